@@ -264,8 +264,9 @@ int gbp_power_normalize_job(const double* sums, const long long* nmodes,
 /* The 3-D FFT fused with the binning (library transform sizes only: power-of
  * two meshes 64..1024 and a plan made without the cuFFT override).  The z and
  * y passes write the partial transform to `spectrum` (the buffer
- * gbp_fft_r2c would fill); the x pass runs inside the binning kernel, so the
- * full spectrum never reaches HBM.  Same outputs and arguments as
+ * gbp_fft_r2c would fill, in a packed layout of their own, without the rows
+ * and columns beyond the last k edge); the x pass runs inside the binning
+ * kernel, so the full spectrum never reaches HBM.  Same outputs and arguments as
  * gbp_fft_r2c followed by gbp_power (src/correlations.py:22-48); the sums
  * agree to float32 round-off (a different, fixed summation order).
  * GBP_ERR_UNSUPPORTED when the plan uses cuFFT. */
@@ -299,7 +300,7 @@ int gbp_particles_power_workspace_size(int64_t n_particles, gbp_fft_plan plan,
                                        gbp_bins bins, int mas, int ells,
                                        size_t* bytes);
 /* Column tile shapes (tx x ty pencils, all of z) of the fused path for an
- * n_mesh^3 mesh, the default first: up to `max` of them into tx[], ty[];
+ * n_mesh^3 mesh, the default of one grid first: up to `max` of them into tx[], ty[];
  * *count = how many there are (no reference counterpart: the tile is the
  * bucket of the particle sort, a tuning choice).  Every shape gives the same
  * results bit for bit; they differ in speed, which the autotuner measures. */

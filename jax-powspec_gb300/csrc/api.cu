@@ -218,13 +218,30 @@ extern "C" int gbp_bins_create(const float* e, int ne, int N, gbp_bins* out) {
     h_is2[k] = (float)(1.0 / (s * s));
     h_eph[k] = make_float2((float)cos(x), (float)sin(x));
   }
+  // items of the x pass + binning: a block of 8 kz columns of one ky row is transformed and binned only
+  // when its smallest |k| (kx = 0, its first kz) is within the last edge
+  std::vector<int> h_items;
+  B->kz_cols = 0;
+  if (own_fft_supported(N)) {
+    for (int y = 0; y < N; ++y) {
+      const long long ky = signed_k(y, N);
+      for (int kb = 0; 8 * kb <= h; ++kb) {
+        if (ky * ky + 64LL * kb * kb > last) break;
+        h_items.push_back(y * XITEM_KB + kb);
+        B->kz_cols = 8 * (kb + 1) > B->kz_cols ? 8 * (kb + 1) : B->kz_cols;
+      }
+    }
+  }
+  B->n_xitems = (int)h_items.size();
+  h_items.push_back(0);
   const size_t o_thr = 0;
   const size_t o_lut = o_thr + align256(h_thr.size() * 4);
   const size_t o_is2 = o_lut + align256(h_lut.size() * 4);
   const size_t o_eph = o_is2 + align256(h_is2.size() * 4);
   const size_t o_nm = o_eph + align256(h_eph.size() * 8);
   const size_t o_ks = o_nm + align256(h_nmodes.size() * 8);
-  const size_t total = o_ks + align256(h_ksum.size() * 8);
+  const size_t o_xi = o_ks + align256(h_ksum.size() * 8);
+  const size_t total = o_xi + align256(h_items.size() * 4);
   cudaGetDevice(&B->device);
   char* blk = nullptr;
   if (cudaMalloc(&blk, total) != cudaSuccess) {
@@ -238,7 +255,8 @@ extern "C" int gbp_bins_create(const float* e, int ne, int N, gbp_bins* out) {
   B->d_eph = reinterpret_cast<float2*>(blk + o_eph);
   B->d_nmodes = reinterpret_cast<long long*>(blk + o_nm);
   B->d_ksum = reinterpret_cast<double*>(blk + o_ks);
-  cudaError_t ce = cudaSuccess;
+  B->d_xitems = reinterpret_cast<int*>(blk + o_xi);
+  cudaError_t ce = cudaMemcpy(B->d_xitems, h_items.data(), h_items.size() * 4, cudaMemcpyHostToDevice);
   if (ce == cudaSuccess) ce = cudaMemcpy(B->d_nmodes, h_nmodes.data(), h_nmodes.size() * 8, cudaMemcpyHostToDevice);
   if (ce == cudaSuccess) ce = cudaMemcpy(B->d_ksum, h_ksum.data(), h_ksum.size() * 8, cudaMemcpyHostToDevice);
   if (ce == cudaSuccess) ce = cudaMemcpy(B->d_thr, h_thr.data(), h_thr.size() * 4, cudaMemcpyHostToDevice);
@@ -282,13 +300,17 @@ extern "C" int gbp_fft_plan_create(int n, int grids, gbp_fft_plan* out, size_t* 
   const char* env = getenv("GBP_FFT_BACKEND");
   const bool force_cufft = env && strcmp(env, "cufft") == 0;
   if (own_fft_supported(n) && !force_cufft) {
-    float2* tw = nullptr;
-    const int st = own_fft_twiddles(n, &tw);
+    float2 *tw = nullptr, *twx = nullptr;
+    int st = own_fft_twiddles(n, &tw);
     if (st) return st;
-    gbp_fft_plan_s* p = new (std::nothrow) gbp_fft_plan_s{true, 0, tw, n, grids, own_fft_pitch(n), 0};
+    // one grid: the packed x transform is half as long (fft.cu)
+    if (grids == 1) st = own_fft_twiddles(n / 2, &twx);
+    gbp_fft_plan_s* p = nullptr;
+    if (!st) p = new (std::nothrow) gbp_fft_plan_s{true, 0, tw, grids == 1 ? twx : tw, n, grids, own_fft_pitch(n), 0};
     if (!p) {
       cudaFree(tw);
-      return GBP_ERR_ALLOC;
+      cudaFree(twx);
+      return st ? st : GBP_ERR_ALLOC;
     }
     *out = p;
     if (ws_bytes) *ws_bytes = 0;
@@ -308,7 +330,7 @@ extern "C" int gbp_fft_plan_create(int n, int grids, gbp_fft_plan* out, size_t* 
     cufftDestroy(h);
     return GBP_ERR_CUFFT;
   }
-  gbp_fft_plan_s* p = new (std::nothrow) gbp_fft_plan_s{false, h, nullptr, n, grids, n / 2 + 1, ws};
+  gbp_fft_plan_s* p = new (std::nothrow) gbp_fft_plan_s{false, h, nullptr, nullptr, n, grids, n / 2 + 1, ws};
   if (!p) {
     cufftDestroy(h);
     return GBP_ERR_ALLOC;
@@ -326,8 +348,12 @@ extern "C" int gbp_fft_plan_pitch(gbp_fft_plan p, int* z_pitch) {
 
 extern "C" int gbp_fft_plan_destroy(gbp_fft_plan p) {
   if (!p) return GBP_ERR_INVALID;
-  if (p->own) cudaFree(p->tw);
-  else cufftDestroy(p->h);
+  if (p->own) {
+    if (p->twx != p->tw) cudaFree(p->twx);
+    cudaFree(p->tw);
+  } else {
+    cufftDestroy(p->h);
+  }
   delete p;
   return GBP_OK;
 }

@@ -19,15 +19,18 @@
 //      shared reductions, no carries).  The scales belong to the 4x4 blocks,
 //      not to the tile, so every tile shape gives the same cells, the same
 //      floats and the same P_l, bit for bit;
-//   2. transforms its pencils along z: the first radix-8 stage reads the
-//      integer cells of two pencils (packed as one complex pencil), converts
-//      them to float and writes the complex buffer that aliases the
-//      accumulators; the remaining stages run in place (fft_pass.cuh),
-//   3. splits each packed spectrum into its two real-input half spectra and
-//      writes the pencils' rows of the z-transformed spectrum (P = N/2 + 8
-//      complex per row, as the library's own transform),
+//   2. transforms its pencils along z in the packed layout (fft.cu): a complex
+//      column is a pencil of both grids, or with one grid two pencils of
+//      adjacent x planes.  The first radix-8 stage reads the integer cells,
+//      converts them to float and writes the complex buffer that aliases the
+//      accumulators; the stages in between run in place (fft_pass.cuh),
+//   3. stores Z(kz) and Z(-kz) from the last stage's registers,
 //   4. adds up the tile's exact integer total at the common scale 2^s_g
 //      (the mean density; stats_kernel folds the tiles).
+//
+// With two grids a tile is taken in units of 4x4 (1024^3: 4x2) pencils whose
+// both grids fit in shared memory together; with one grid the unit is the
+// tile.
 //
 // A block whose densest plane would cost more than SH_MAX bits (a dense
 // clump) sends its whole tile to deposit_fftz_wide_kernel: 64-bit cells, the
@@ -53,20 +56,43 @@ namespace {
 template <int N, int TX_, int TY_>
 struct ColTile {
   static constexpr int TX = TX_, TY = TY_;
-  static constexpr int NPEN = TX * TY;            // pencils per tile; pencil f = lx * TY + ly
-  static constexpr int PAIRS = NPEN / 2;          // complex transforms (pencils 2q, 2q+1)
-  static constexpr int NFFT = PAIRS * N / 16;     // butterfly pairs (two columns) per radix-8 stage
-  static constexpr int NT = NFFT < 256 ? 256 : NFFT;
-  static constexpr int MINB = NT >= 1024 ? 1 : (NT >= 512 ? 2 : 3);   // CTAs per SM the registers are sized for
   static constexpr int SBX = TX / 4, SBY = TY / 4, NSB = SBX * SBY;    // 4x4-pencil scale blocks
-  static constexpr size_t SMEM = (size_t)(NPEN + NSB) * N * sizeof(int);   // cells + per-block plane counts
-  static constexpr size_t SMEM_WIDE = (size_t)NPEN * N * sizeof(long long);
   static_assert(TX % 4 == 0 && TY % 4 == 0, "tiles are whole 4x4 scale blocks");
 };
 
-// Scale block of local pencil column (lx, ly).
-template <class CT>
-__device__ __forceinline__ int scale_block(int lx, int ly) { return (lx >> 2) * CT::SBY + (ly >> 2); }
+// The pencils of a tile that go through shared memory together, as PAIRS
+// packed complex columns: column q = (a, ly) with a = the pencil's x (two
+// grids) or x / 2 (one grid), a = q / UY, ly = q % UY.  Columns 2cp and
+// 2cp + 1 always lie in one scale block.  The unit is the tile where its
+// cells fit UNIT_BYTES, else 4x4 or 4x2 pencils of it.  At 512^3 a unit of
+// 64 KB (512 threads, 64-thread named barriers, two CTAs per SM) beats one
+// of 128 KB in a 1024-thread CTA (0.84 against 0.89 ms for 8x4 tiles of two
+// grids, 4 Mi particles TSC); at 1024^3 4x4 pencils in one CTA beat two
+// visits of the bucket by 4x2 (7.7 against 8.5 ms, 16 Mi PCS).
+template <int N, bool WIDE>
+constexpr size_t UNIT_BYTES = (N == 512 && !WIDE ? 64 : 128) * 1024;
+
+template <int N, int G, class CT, bool WIDE>
+struct Unit {
+  static constexpr size_t PENCIL = (size_t)N * G * (WIDE ? 8 : 4);       // bytes of a pencil's cells
+  static constexpr bool WHOLE = CT::TX * CT::TY * PENCIL <= UNIT_BYTES<N, WIDE>, SQUARE = 16 * PENCIL <= UNIT_BYTES<N, WIDE>;
+  static constexpr int UX = WHOLE ? CT::TX : 4;
+  static constexpr int UY = WHOLE ? CT::TY : (SQUARE ? 4 : 2);
+  static constexpr int NUY = CT::TY / UY, NU = (CT::TX / UX) * NUY;      // units per tile
+  static constexpr int PAIRS = UX * UY * G / 2;
+  static constexpr int SBY = UY >= 4 ? UY / 4 : 1, NSB = UX / 4 * SBY;   // scale blocks it spans
+  static constexpr int NFFT = PAIRS * N / 16;     // butterfly pairs (two columns) per radix-8 stage
+  static constexpr int NT = NFFT < 256 ? 256 : NFFT;
+  static constexpr int MINB = NT >= 1024 ? 1 : (NT >= 512 ? 2 : 3);   // CTAs per SM the registers are sized for
+  static constexpr size_t CELLS = (size_t)2 * PAIRS * N;
+  static constexpr size_t SMEM = CELLS * (WIDE ? 8 : 4) + (WIDE ? 0 : (size_t)CT::NSB * N * 4);  // + plane counts
+  static_assert(CELLS * (WIDE ? 8 : 4) <= UNIT_BYTES<N, WIDE> && NT <= 1024, "a unit fits in shared memory");
+  // First cell of pencil (lx, ly) of a grid.
+  __device__ static __forceinline__ int cell_row(int lx, int ly, int grid) {
+    if constexpr (G == 2) return ((lx * UY + ly) * 2 + grid) * N;
+    else return (((lx >> 1) * UY + ly) * 2 + (lx & 1)) * N;
+  }
+};
 
 // v[b] for a block index known only at run time, by selects (no local memory).
 template <int NSB, class T>
@@ -85,20 +111,26 @@ __device__ __forceinline__ T pick_block(int b, const T (&v)[NSB]) {
 constexpr int SH_MAX = 10;
 constexpr long long WIDE_MARK = (-0x7fffffffffffffffLL - 1);   // tile_mass entry of a tile left to the wide kernel
 
-// Deposit, z transform, split and row stores of one column tile and grid
-// (steps 1-4 above).  WIDE: 64-bit cells.  sh[b]: bits given up by scale
-// block b (its scale 2^(sg - sh[b]), sh[b] <= SH_MAX).  Returns the tile's
-// exact total at the common scale 2^sg (valid in thread 0).
+// Two grids per pass share the entry loads and need no split of the packed
+// spectra: deposit_fft_z 0.052 -> 0.034 ms (128^3, 1 M particles CIC), 0.135
+// -> 0.127 (256^3, 1 M TSC); at 512^3 0.742 -> 0.742 (4 Mi TSC, 4x4 instead
+// of 8x4 tiles), bound by instruction issue (0.59 of the slots) and barriers.
+//
+// Deposit, z transform and row stores of one unit (steps 1-4 above); x0, y0:
+// its first pencil.  WIDE: 64-bit cells.  sh[b]: bits given up by scale block
+// b of the unit (its scale 2^(sg - sh[b]), sh[b] <= SH_MAX).  tm[grid]: the
+// unit's exact totals at the common scale 2^sg (valid in thread 0).
 template <int N, int MAS, int G, class CT, bool WIDE>
-__device__ __forceinline__ long long tile_grid(const DepGeom& g, const float4* __restrict__ entries, unsigned beg,
-                                               unsigned end, int sg, const int (&sh)[CT::NSB], int grid, int x0,
-                                               int y0, const float2* __restrict__ tw, float2* __restrict__ spec,
-                                               unsigned char* smem, long long* s_part) {
+__device__ __forceinline__ void tile_unit(const DepGeom& g, const float4* __restrict__ entries, unsigned beg,
+                                          unsigned end, int sg, const int (&sh)[Unit<N, G, CT, WIDE>::NSB], int x0, int y0,
+                                          int kz_cols, const float2* __restrict__ tw, float2* __restrict__ spec,
+                                          unsigned char* smem, long long (*s_part)[G], long long (&tm)[G]) {
   using Cell = typename std::conditional<WIDE, unsigned long long, int>::type;
-  constexpr int R = MAS, TX = CT::TX, TY = CT::TY, NPEN = CT::NPEN, PAIRS = CT::PAIRS, NT = CT::NT;
-  constexpr int NSB = CT::NSB;
-  constexpr int P = N / 2 + 8, H = N / 2;
-  Cell* acc = reinterpret_cast<Cell*>(smem);                   // [NPEN][N] fixed-point cells
+  using U = Unit<N, G, CT, WIDE>;
+  constexpr int R = MAS, UX = U::UX, UY = U::UY, PAIRS = U::PAIRS, NT = U::NT, NSB = U::NSB;
+  constexpr int P = N / 2 + 8, NX = G == 2 ? N : N / 2;
+  constexpr int SBY = U::SBY;                                  // scale blocks along y
+  Cell* acc = reinterpret_cast<Cell*>(smem);                   // [2 PAIRS][N] fixed-point cells
   float4* cs4 = reinterpret_cast<float4*>(smem);               // [PAIRS/2][N] slots of two columns, alias the cells
   const int tid = threadIdx.x;
   // 2^s and 2^-s of each block: s = sg - sh in [-110, 100], one normal float each
@@ -108,145 +140,161 @@ __device__ __forceinline__ long long tile_grid(const DepGeom& g, const float4* _
     up[b] = ldexpf(1.0f, sg - sh[b]);
     dn[b] = ldexpf(1.0f, sh[b] - sg);
   }
-  const long long gstride = (long long)N * N * P;
 
   {
     uint4* a4 = reinterpret_cast<uint4*>(acc);
-    for (int k = tid; k < (int)(NPEN * N * sizeof(Cell) / 16); k += NT) a4[k] = make_uint4(0u, 0u, 0u, 0u);
+    for (int k = tid; k < (int)(U::CELLS * sizeof(Cell) / 16); k += NT) a4[k] = make_uint4(0u, 0u, 0u, 0u);
   }
   __syncthreads();
   for (unsigned i = beg + tid; i < end; i += NT) {
     const float4 e = entries[i];
-    Axis<R> ax, ay, az;
-    make_axis<MAS, 0, N>(g, e.x, grid, ax);
-    make_axis<MAS, 0, N>(g, e.y, grid, ay);
-    make_axis<MAS, 0, N>(g, e.z, grid, az);
-    int lx[R], ly[R], zz[R];
-    local_nodes<R>(ax, N, x0, TX, lx);
-    local_nodes<R>(ay, N, y0, TY, ly);
-    // z weight times the particle weight at each block's scale (exact: powers of two)
-    float wz[NSB][R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) zz[r] = wrapn(az.first + r, N);
+    for (int grid = 0; grid < G; ++grid) {
+      Axis<R> ax, ay, az;
+      make_axis<MAS, 0, N>(g, e.x, grid, ax);
+      make_axis<MAS, 0, N>(g, e.y, grid, ay);
+      make_axis<MAS, 0, N>(g, e.z, grid, az);
+      int lx[R], ly[R], zz[R];
+      local_nodes<R>(ax, N, x0, UX, lx);
+      local_nodes<R>(ay, N, y0, UY, ly);
+      // z weight times the particle weight at each block's scale (exact: powers of two)
+      float wz[NSB][R];
 #pragma unroll
-    for (int b = 0; b < NSB; ++b) {
-      const float wsc = __fmul_rn(e.w, up[b]);
+      for (int r = 0; r < R; ++r) zz[r] = wrapn(az.first + r, N);
 #pragma unroll
-      for (int r = 0; r < R; ++r) wz[b][r] = __fmul_rn(az.w[r], wsc);
-    }
+      for (int b = 0; b < NSB; ++b) {
+        const float wsc = __fmul_rn(e.w, up[b]);
 #pragma unroll
-    for (int rx = 0; rx < R; ++rx) {
-      if (lx[rx] < 0) continue;
-      // with one block row (TY = 4) the block depends on x only: select the z weights once per x node
-      float wzx[R];
-      if constexpr (CT::SBY == 1) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          float wzb[NSB];
-#pragma unroll
-          for (int k = 0; k < NSB; ++k) wzb[k] = wz[k][r];
-          wzx[r] = pick_block<NSB>(lx[rx] >> 2, wzb);
-        }
+        for (int r = 0; r < R; ++r) wz[b][r] = __fmul_rn(az.w[r], wsc);
       }
 #pragma unroll
-      for (int ry = 0; ry < R; ++ry) {
-        if (ly[ry] < 0) continue;
-        const float wxy = __fmul_rn(ax.w[rx], ay.w[ry]);
-        const int row = (lx[rx] * TY + ly[ry]) * N;
+      for (int rx = 0; rx < R; ++rx) {
+        if (lx[rx] < 0) continue;
+        // with one block row the block depends on x only: select the z weights once per x node
+        float wzx[R];
+        if constexpr (SBY == 1) {
 #pragma unroll
-        for (int rz = 0; rz < R; ++rz) {
-          float wzr;
-          if constexpr (CT::SBY == 1) {
-            wzr = wzx[rz];
-          } else {
+          for (int r = 0; r < R; ++r) {
             float wzb[NSB];
 #pragma unroll
-            for (int k = 0; k < NSB; ++k) wzb[k] = wz[k][rz];
-            wzr = pick_block<NSB>(scale_block<CT>(lx[rx], ly[ry]), wzb);
+            for (int k = 0; k < NSB; ++k) wzb[k] = wz[k][r];
+            wzx[r] = pick_block<NSB>(lx[rx] >> 2, wzb);
           }
-          const int v = __float2int_rn(__fmul_rn(wxy, wzr));
-          if constexpr (WIDE) atomicAdd(&acc[row + zz[rz]], (unsigned long long)(long long)v);
-          else atomicAdd(&acc[row + zz[rz]], v);
+        }
+#pragma unroll
+        for (int ry = 0; ry < R; ++ry) {
+          if (ly[ry] < 0) continue;
+          const float wxy = __fmul_rn(ax.w[rx], ay.w[ry]);
+          const int row = U::cell_row(lx[rx], ly[ry], grid);
+#pragma unroll
+          for (int rz = 0; rz < R; ++rz) {
+            float wzr;
+            if constexpr (SBY == 1) {
+              wzr = wzx[rz];
+            } else {
+              float wzb[NSB];
+#pragma unroll
+              for (int k = 0; k < NSB; ++k) wzb[k] = wz[k][rz];
+              wzr = pick_block<NSB>((lx[rx] >> 2) * SBY + (ly[ry] >> 2), wzb);
+            }
+            const int v = __float2int_rn(__fmul_rn(wxy, wzr));
+            if constexpr (WIDE) atomicAdd(&acc[row + zz[rz]], (unsigned long long)(long long)v);
+            else atomicAdd(&acc[row + zz[rz]], v);
+          }
         }
       }
     }
   }
   __syncthreads();
 
-  // z transform: pencils 2q and 2q+1 are the real and imaginary parts of
-  // column q; a thread transforms columns 2cp and 2cp+1 (pencils 4cp..4cp+3,
-  // one scale block), the same column pair in every stage of the first
-  // (and only) butterfly per thread: cp = tid / (N/8)
-  long long part = 0;
-  auto gin = [&part, &dn, acc](int j, int cp) {
-    const int f = 4 * cp;
-    const float d = pick_block<NSB>(scale_block<CT>(f / TY, f % TY), dn);
+  // z transform: a thread transforms columns 2cp and 2cp+1 (one scale block), the same column pair in
+  // every stage of the first (and only) butterfly per thread: cp = tid / (N/8).  The cells of column q:
+  // the real parts at 2q N, the imaginary parts at (2q + 1) N
+  auto block_of = [](int cp) {
+    const int a = 2 * cp / UY, ly = 2 * cp % UY;
+    return NSB == 1 ? 0 : ((G == 2 ? a : 2 * a) >> 2) * SBY + (ly >> 2);
+  };
+  long long part[G];
+#pragma unroll
+  for (int q = 0; q < G; ++q) part[q] = 0;
+  auto gin = [&part, &dn, &sh, acc, block_of](int j, int cp) {
+    const float d = pick_block<NSB>(block_of(cp), dn);
+    const int f = 1 << pick_block<NSB>(block_of(cp), sh);     // the block's total at the common scale
     float v[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const long long q = (long long)acc[(f + k) * N + j];
-      part += q;
-      v[k] = __fmul_rn(WIDE ? __ll2float_rn(q) : __int2float_rn((int)q), d);   // exact: a power of two
+      const auto q = acc[(4 * cp + k) * N + j];
+      // 32-bit cells: one widening multiply-add each
+      part[G == 2 ? (k & 1) : 0] += (long long)q * f;
+      v[k] = __fmul_rn(WIDE ? __ll2float_rn((long long)q) : __int2float_rn((int)q), d);   // exact: a power of two
     }
     return make_float4(v[0], v[1], v[2], v[3]);
   };
   auto sin_ = [cs4](int j, int cp) { return cs4[cp * N + fft::zsw(j)]; };
   auto sout = [cs4](int j, int cp, float4 v) { cs4[cp * N + fft::zsw(j)] = v; };
+  // columns 2cp and 2cp + 1 are rows y0 + ly and y0 + ly + 1 of plane x0 + a (G = 2) or x0 / 2 + a
+  auto gout = [spec, x0, y0, kz_cols](int k, int cp, float4 v) {
+    const int a = 2 * cp / UY, ly = 2 * cp % UY;
+    float2* o0 = spec + ((long long)((G == 2 ? x0 : x0 / 2) + a) * N + (y0 + ly)) * P;
+    fft::store_packed<N>(o0, o0 + (long long)NX * N * P, P, kz_cols, k, 0, v);
+  };
   // N = 512, 32-bit cells: every stage is radix 8 and the 64 threads of a column pair own its data
   // (the first stage's writes alias the pair's own pencils), so the stages synchronise 64-thread
   // groups only.  64-bit cells span twice the bytes of the complex slots: whole-CTA barriers.
-  constexpr int GS = (!WIDE && N == 512 && NT == PAIRS / 2 * (N / 8)) ? N / 8 : 0;
-  static_assert(CT::NFFT <= NT, "one first-stage butterfly per thread");
-  fft::run_stages2<N, PAIRS / 2, NT, true, true, true, decltype(gin), decltype(sin_), decltype(sout),
-                   decltype(sout), GS>(gin, sin_, sout, sout, tw, tid);
-  {
-    // this thread's cells belong to one scale block: shift its total to the common scale
-    const int cp = tid / (N / 8);
-    if (cp < PAIRS / 2) {
-      int shb[NSB];
+  constexpr int GS = (!WIDE && N == 512 && NT == PAIRS / 2 * (N / 8) && NT / (N / 8) <= fft::MAX_GROUPS) ? N / 8 : 0;
+  static_assert(U::NFFT <= NT, "one first-stage butterfly per thread");
+  fft::run_stages2<N, PAIRS / 2, NT, true, true, false, decltype(gin), decltype(sin_), decltype(sout), decltype(gout),
+                   GS>(gin, sin_, sout, gout, tw, tid);
+  // the unit's exact totals
 #pragma unroll
-      for (int b = 0; b < NSB; ++b) shb[b] = sh[b];
-      part *= (1LL << pick_block<NSB>(scale_block<CT>(4 * cp / TY, 4 * cp % TY), shb));
+  for (int q = 0; q < G; ++q) {
+    for (int o = 16; o > 0; o >>= 1) part[q] += __shfl_xor_sync(0xffffffffu, part[q], o);
+    if ((tid & 31) == 0) s_part[tid >> 5][q] = part[q];
+  }
+  __syncthreads();                                     // also: the next unit reuses the accumulators
+  if (tid == 0) {
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+      tm[q] = 0;
+      for (int k = 0; k < NT / 32; ++k) tm[q] += s_part[k][q];
     }
   }
+}
 
-  // split the packed spectra; write all pencils' rows (row padding -> 0), two k per thread and
-  // 16-byte stores
-  const float2* cs = reinterpret_cast<const float2*>(cs4);
-  float2* out = spec + grid * gstride;
-  constexpr int P2 = P / 2;
-  for (int idx = tid; idx < PAIRS * P2; idx += NT) {
-    const int q = idx / P2, k0 = 2 * (idx - q * P2);
-    const float2* col = cs + (q >> 1) * N * 2 + (q & 1);
-    float2 a[2], b[2];
+// Every unit of a tile; writes the tile's totals.  sh: the shifts of the tile's scale blocks.
+template <int N, int MAS, int G, class CT, bool WIDE>
+__device__ __forceinline__ void tile_units(const DepGeom& g, const float4* __restrict__ entries, unsigned beg,
+                                           unsigned end, int sg, const int (&sh)[CT::NSB], int x0, int y0, int kz_cols,
+                                           const float2* __restrict__ tw, float2* __restrict__ spec,
+                                           unsigned char* smem, long long (*s_part)[G], long long* tile_mass,
+                                           int ntiles, int t) {
+  using U = Unit<N, G, CT, WIDE>;
+  long long total[G];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int k = k0 + h;
-      a[h] = b[h] = make_float2(0.f, 0.f);
-      if (k <= H) {
-        const float2 c = col[fft::zsw(k) * 2];
-        const float2 m = col[fft::zsw((N - k) & (N - 1)) * 2];
-        const float2 cm = make_float2(m.x, -m.y);
-        const float2 sum = fft::cadd(c, cm), dif = fft::cmi(fft::csub(c, cm));
-        a[h] = make_float2(0.5f * sum.x, 0.5f * sum.y);
-        b[h] = make_float2(0.5f * dif.x, 0.5f * dif.y);
-      }
+  for (int q = 0; q < G; ++q) total[q] = 0;
+#pragma unroll 1
+  for (int u = 0; u < U::NU; ++u) {
+    const int ux = u / U::NUY * U::UX, uy = u % U::NUY * U::UY;
+    int shu[U::NSB];
+    if constexpr (U::NU > 1) {
+      static_assert(U::NU == 1 || U::NSB == 1, "a part of a tile lies in one scale block");
+      shu[0] = pick_block<CT::NSB>((ux >> 2) * CT::SBY + (uy >> 2), sh);
+    } else {
+#pragma unroll
+      for (int b = 0; b < U::NSB; ++b) shu[b] = sh[b];
     }
-    const int f0 = 2 * q, f1 = 2 * q + 1;
-    const long long r0 = (long long)(x0 + f0 / TY) * N + (y0 + f0 % TY);
-    const long long r1 = (long long)(x0 + f1 / TY) * N + (y0 + f1 % TY);
-    __stcs(reinterpret_cast<float4*>(out + r0 * P + k0), make_float4(a[0].x, a[0].y, a[1].x, a[1].y));
-    __stcs(reinterpret_cast<float4*>(out + r1 * P + k0), make_float4(b[0].x, b[0].y, b[1].x, b[1].y));
+    long long tm[G];
+    tile_unit<N, MAS, G, CT, WIDE>(g, entries, beg, end, sg, shu, x0 + ux, y0 + uy, kz_cols, tw, spec, smem, s_part,
+                                   tm);
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int q = 0; q < G; ++q) total[q] += tm[q];
+    }
   }
-
-  // the tile's exact total
-  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-  if ((tid & 31) == 0) s_part[tid >> 5] = part;
-  __syncthreads();                                     // also: the next grid reuses the accumulators
-  long long tm = 0;
-  if (tid == 0)
-    for (int k = 0; k < NT / 32; ++k) tm += s_part[k];
-  return tm;
+  if (threadIdx.x == 0) {                              // replaces a wide tile's mark and shifts
+    tile_mass[t] = total[0];
+    tile_mass[(long long)ntiles + t] = G == 2 ? total[G - 1] : 0;
+  }
 }
 
 // Per-block plane counts of a tile (zc [NSB][N], zeroed on entry) and the
@@ -257,7 +305,7 @@ __device__ __forceinline__ long long tile_grid(const DepGeom& g, const float4* _
 template <int N, int MAS, int G, class CT>
 __device__ __forceinline__ bool block_scales(const DepGeom& g, const float4* __restrict__ entries, unsigned beg,
                                              unsigned end, int x0, int y0, int* zc, int* s_max, int (&sh)[CT::NSB]) {
-  constexpr int R = MAS, NT = CT::NT, NSB = CT::NSB, W = R + G - 1;
+  constexpr int R = MAS, NT = Unit<N, G, CT, false>::NT, NSB = CT::NSB, W = R + G - 1;
   const int tid = threadIdx.x;
   // this pass is the tile's first touch of its bucket: a thread issues EB entry loads at once
   constexpr int EB = 4;
@@ -336,15 +384,16 @@ __device__ __forceinline__ bool block_scales(const DepGeom& g, const float4* __r
 }
 
 template <int N, int MAS, int G, class CT>
-__global__ void __launch_bounds__(CT::NT, CT::MINB)
+__global__ void __launch_bounds__(Unit<N, G, CT, false>::NT, Unit<N, G, CT, false>::MINB)
 deposit_fftz_kernel(DepGeom g, const float4* __restrict__ entries, const unsigned* __restrict__ counts,
-                    const unsigned* __restrict__ offsets, const DepCounters* ctr, const float2* __restrict__ tw,
-                    float2* __restrict__ spec, long long* __restrict__ tile_mass) {
+                    const unsigned* __restrict__ offsets, const DepCounters* ctr, int kz_cols,
+                    const float2* __restrict__ tw, float2* __restrict__ spec, long long* __restrict__ tile_mass) {
   pdl_wait();
-  constexpr int NPEN = CT::NPEN, NT = CT::NT, NSB = CT::NSB;
+  using U = Unit<N, G, CT, false>;
+  constexpr int NT = U::NT, NSB = CT::NSB;
   extern __shared__ __align__(16) int acc_smem[];
-  int* zc = acc_smem + NPEN * N;                       // [NSB][N] entries covering each block's planes
-  __shared__ long long s_part[NT / 32];
+  int* zc = acc_smem + U::CELLS;                       // [NSB][N] entries covering each block's planes
+  __shared__ long long s_part[NT / 32][G];
   __shared__ int s_max[NT / 32];
   const int tid = threadIdx.x;
   const int t = blockIdx.x;
@@ -366,11 +415,8 @@ deposit_fftz_kernel(DepGeom g, const float4* __restrict__ entries, const unsigne
     }
     return;
   }
-  for (int grid = 0; grid < G; ++grid) {
-    const long long tm = tile_grid<N, MAS, G, CT, false>(g, entries, beg, end, sg, sh, grid, x0, y0, tw, spec,
-                                                         reinterpret_cast<unsigned char*>(acc_smem), s_part);
-    if (tid == 0) tile_mass[(long long)grid * gridDim.x + t] = tm;   // exact, at the common scale 2^sg
-  }
+  tile_units<N, MAS, G, CT, false>(g, entries, beg, end, sg, sh, x0, y0, kz_cols, tw, spec,
+                                   reinterpret_cast<unsigned char*>(acc_smem), s_part, tile_mass, (int)gridDim.x, t);
 }
 
 // The tiles deposit_fftz_kernel left (tile_mass entry WIDE_MARK, the
@@ -381,14 +427,15 @@ deposit_fftz_kernel(DepGeom g, const float4* __restrict__ entries, const unsigne
 constexpr int WIDE_LIST = 64;                          // marked tiles listed per scan round
 
 template <int N, int MAS, int G, class CT>
-__global__ void __launch_bounds__(CT::NT, CT::MINB)
+__global__ void __launch_bounds__(Unit<N, G, CT, true>::NT, Unit<N, G, CT, true>::MINB)
 deposit_fftz_wide_kernel(DepGeom g, const float4* __restrict__ entries, const unsigned* __restrict__ counts,
-                         const unsigned* __restrict__ offsets, const DepCounters* ctr, const float2* __restrict__ tw,
-                         float2* __restrict__ spec, long long* __restrict__ tile_mass, int ntiles) {
+                         const unsigned* __restrict__ offsets, const DepCounters* ctr, int kz_cols,
+                         const float2* __restrict__ tw, float2* __restrict__ spec, long long* __restrict__ tile_mass,
+                         int ntiles) {
   pdl_wait();
-  constexpr int NT = CT::NT, NSB = CT::NSB;
+  constexpr int NT = Unit<N, G, CT, true>::NT, NSB = CT::NSB;
   extern __shared__ __align__(16) unsigned long long wide_smem[];
-  __shared__ long long s_part[NT / 32];
+  __shared__ long long s_part[NT / 32][G];
   __shared__ int s_list[WIDE_LIST];
   __shared__ int s_n;
   const int sg = fixed_scale_exp(ctr->maxw_bits, 0);
@@ -416,13 +463,8 @@ deposit_fftz_wide_kernel(DepGeom g, const float4* __restrict__ entries, const un
 #pragma unroll
         for (int b = 0; b < NSB; ++b) sh[b] = (int)((packed >> (8 * b)) & 0xff);
         __syncthreads();                               // every thread has read the shifts before they are replaced
-        for (int grid = 0; grid < G; ++grid) {
-          const long long tm = tile_grid<N, MAS, G, CT, true>(g, entries, beg, end, sg, sh, grid, tx * CT::TX,
-                                                              ty * CT::TY, tw, spec,
-                                                              reinterpret_cast<unsigned char*>(wide_smem), s_part);
-          if (threadIdx.x == 0) tile_mass[(long long)grid * ntiles + tt] = tm;   // clears the mark
-        }
-        if (G == 1 && threadIdx.x == 0) tile_mass[(long long)ntiles + tt] = 0;
+        tile_units<N, MAS, G, CT, true>(g, entries, beg, end, sg, sh, tx * CT::TX, ty * CT::TY, kz_cols, tw, spec,
+                                        reinterpret_cast<unsigned char*>(wide_smem), s_part, tile_mass, ntiles, tt);
       }
       __syncthreads();                                 // the marks are replaced before the next scan
     }
@@ -447,48 +489,50 @@ int particles_layout(int64_t n, gbp_fft_plan plan, gbp_bins B, int mas, int ells
 }
 
 template <int N, int MAS, int G, class CT>
-int run_fused(const DepGeom& g, const DepLayout& L, const DepBuffers& b, const float2* tw, float2* spec,
+int run_fused(const DepGeom& g, const DepLayout& L, const DepBuffers& b, int kz_cols, const float2* tw, float2* spec,
               cudaStream_t st) {
+  using U = Unit<N, G, CT, false>;
+  using UW = Unit<N, G, CT, true>;
   int r = bucket_particles<MAS, G, 0>(g, L, b, st);
   if (r) return r;
   auto k = deposit_fftz_kernel<N, MAS, G, CT>;
-  GBP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CT::SMEM));
+  GBP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)U::SMEM));
   {
     GBP_TRACE("deposit_fft_z", st);
-    GBP_CUDA_TRY(launch_pdl(k, dim3(L.ntiles), dim3(CT::NT), CT::SMEM, st, g, b.entries, b.counts, b.offsets, b.ctr,
-                            tw, spec, b.tile_mass));
+    GBP_CUDA_TRY(launch_pdl(k, dim3(L.ntiles), dim3(U::NT), U::SMEM, st, g, b.entries, b.counts, b.offsets, b.ctr,
+                            kz_cols, tw, spec, b.tile_mass));
   }
   // tiles of dense clumps, if any, with 64-bit cells (as many CTAs as fit at once scan the marks: a
   // dense small mesh can send most of its tiles here)
   auto kw = deposit_fftz_wide_kernel<N, MAS, G, CT>;
-  GBP_CUDA_TRY(cudaFuncSetAttribute(kw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CT::SMEM_WIDE));
+  GBP_CUDA_TRY(cudaFuncSetAttribute(kw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)UW::SMEM));
   int dev = 0, sms = 0, per_sm = 0;
   GBP_CUDA_TRY(cudaGetDevice(&dev));
   GBP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  GBP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kw, CT::NT, CT::SMEM_WIDE));
+  GBP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kw, UW::NT, UW::SMEM));
   GBP_TRACE("deposit_fft_z_wide", st);
-  GBP_CUDA_TRY(launch_pdl(kw, dim3(std::max(1, std::min(sms * std::max(per_sm, 1), L.ntiles))), dim3(CT::NT),
-                          CT::SMEM_WIDE, st, g, b.entries, b.counts, b.offsets, b.ctr, tw, spec, b.tile_mass,
-                          L.ntiles));
+  GBP_CUDA_TRY(launch_pdl(kw, dim3(std::max(1, std::min(sms * std::max(per_sm, 1), L.ntiles))), dim3(UW::NT),
+                          UW::SMEM, st, g, b.entries, b.counts, b.offsets, b.ctr, kz_cols, tw, spec,
+                          b.tile_mass, L.ntiles));
   return GBP_OK;
 }
 
 template <int N, class CT>
-int dispatch_mas(int mas, int G, const DepGeom& g, const DepLayout& L, const DepBuffers& b, const float2* tw,
-                 float2* spec, cudaStream_t st) {
+int dispatch_mas(int mas, int G, const DepGeom& g, const DepLayout& L, const DepBuffers& b, int kz_cols,
+                 const float2* tw, float2* spec, cudaStream_t st) {
   if (G == 2) {
     switch (mas) {
-      case GBP_NGP: return run_fused<N, GBP_NGP, 2, CT>(g, L, b, tw, spec, st);
-      case GBP_CIC: return run_fused<N, GBP_CIC, 2, CT>(g, L, b, tw, spec, st);
-      case GBP_TSC: return run_fused<N, GBP_TSC, 2, CT>(g, L, b, tw, spec, st);
-      default: return run_fused<N, GBP_PCS, 2, CT>(g, L, b, tw, spec, st);
+      case GBP_NGP: return run_fused<N, GBP_NGP, 2, CT>(g, L, b, kz_cols, tw, spec, st);
+      case GBP_CIC: return run_fused<N, GBP_CIC, 2, CT>(g, L, b, kz_cols, tw, spec, st);
+      case GBP_TSC: return run_fused<N, GBP_TSC, 2, CT>(g, L, b, kz_cols, tw, spec, st);
+      default: return run_fused<N, GBP_PCS, 2, CT>(g, L, b, kz_cols, tw, spec, st);
     }
   }
   switch (mas) {
-    case GBP_NGP: return run_fused<N, GBP_NGP, 1, CT>(g, L, b, tw, spec, st);
-    case GBP_CIC: return run_fused<N, GBP_CIC, 1, CT>(g, L, b, tw, spec, st);
-    case GBP_TSC: return run_fused<N, GBP_TSC, 1, CT>(g, L, b, tw, spec, st);
-    default: return run_fused<N, GBP_PCS, 1, CT>(g, L, b, tw, spec, st);
+    case GBP_NGP: return run_fused<N, GBP_NGP, 1, CT>(g, L, b, kz_cols, tw, spec, st);
+    case GBP_CIC: return run_fused<N, GBP_CIC, 1, CT>(g, L, b, kz_cols, tw, spec, st);
+    case GBP_TSC: return run_fused<N, GBP_TSC, 1, CT>(g, L, b, kz_cols, tw, spec, st);
+    default: return run_fused<N, GBP_PCS, 1, CT>(g, L, b, kz_cols, tw, spec, st);
   }
 }
 
@@ -515,16 +559,16 @@ int particles_power_n(DepGeom g, int64_t n_launch, gbp_fft_plan plan, gbp_bins B
   GBP_CUDA_TRY(cudaMemsetAsync(b.ctr, 0, zeroed_bytes(L.dep), st));
   r = GBP_ERR_UNSUPPORTED;
   if (tx == 4 && ty == 4) {
-    r = dispatch_mas<N, ColTile<N, 4, 4>>(mas, G, g, L.dep, b, plan->tw, spec, st);
+    r = dispatch_mas<N, ColTile<N, 4, 4>>(mas, G, g, L.dep, b, B->kz_cols, plan->tw, spec, st);
   } else if (tx == 8 && ty == 4) {
-    if constexpr (N <= 512) r = dispatch_mas<N, ColTile<N, 8, 4>>(mas, G, g, L.dep, b, plan->tw, spec, st);
+    if constexpr (N <= 512) r = dispatch_mas<N, ColTile<N, 8, 4>>(mas, G, g, L.dep, b, B->kz_cols, plan->tw, spec, st);
   } else if (tx == 8 && ty == 8) {
-    if constexpr (N == 128 || N == 256) r = dispatch_mas<N, ColTile<N, 8, 8>>(mas, G, g, L.dep, b, plan->tw, spec, st);
+    if constexpr (N == 128 || N == 256) r = dispatch_mas<N, ColTile<N, 8, 8>>(mas, G, g, L.dep, b, B->kz_cols, plan->tw, spec, st);
   }
   if (r) return r;
   r = deposit_stats(b, L.dep, GBP_COMPAT_NONE, G, stats_out, st);
   if (r) return r;
-  r = own_fft_y(N, G, spec, plan->tw, st);
+  r = own_fft_y_packed(N, G, spec, B->kz_cols, B->last_closed, plan->tw, st);
   if (r) return r;
   const double* mass = reinterpret_cast<const double*>(stats_out);   // gbp_deposit_stats starts with mass[2]
   return xbin_power(plan, spec, B, mas, ells, mass, sums_out, nmodes_out, ksum_out, xws, L.xbin, st);

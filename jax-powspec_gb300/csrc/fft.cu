@@ -11,6 +11,22 @@
 //   x pass  in place, same with rows N*P apart (the pipeline fuses it with
 //           the binning instead: xbin.cu)
 //
+// The power spectrum needs no spectrum in that order, and takes the packed
+// transform instead: one complex field c = a + i b of two real ones, whose
+// spectrum Z carries both (A, B) = ((Z(k) + conj Z(-k)) / 2,
+// -i (Z(k) - conj Z(-k)) / 2), is transformed along z, y and x without any
+// split; the binning (xbin.cu) combines Z(k) and Z(-k) where it has both.
+//
+//   two grids   a, b = the two meshes of an interlaced pair; N x planes
+//   one grid    a, b = the x planes 2x', 2x'+1 of the mesh; N/2 x' planes
+//               (the last butterfly of the x transform, F(kx) = A + w^kx B)
+//
+// Layout [2][NX][N][P], NX = N (two grids) or N/2 (one): slab 0 holds Z at
+// kz = 0 .. N/2, slab 1 holds Z at -kz, so both halves of a kz block are
+// aligned and the y pass treats the slabs as two grids.  The split it saves
+// cost the z pass a write and a read of the block in shared memory.
+// Columns and rows beyond the last k edge are not stored.
+//
 // The z rows are padded from N/2+1 to P = N/2+8 complex (64-byte multiples)
 // so every 8-column block of the y and x passes is a whole number of 32-byte
 // sectors; the padding is written as zeros by the z pass.  Same transform as
@@ -98,15 +114,50 @@ fftz_kernel(const float* __restrict__ mesh, float2* __restrict__ out, long long 
   }
 }
 
+// z pass of the packed transform: PAIRS complex columns per CTA, column q =
+// x' N + y of the packed field (G = 2: pencil q of both meshes; G = 1:
+// pencils (2x', y) and (2x'+1, y)).  The last stage stores Z[kz] to slab 0
+// and / or the mirrored entry of slab 1 straight from registers.
+template <int N, int G, int PAIRS>
+__global__ void __launch_bounds__(PAIRS * N / 16)
+fftz_packed_kernel(const float* __restrict__ mesh, float2* __restrict__ out, int kz_cols,
+                   const float2* __restrict__ tw) {
+  pdl_wait();
+  constexpr int NT = PAIRS * N / 16;
+  constexpr int CP = PAIRS / 2;
+  constexpr int NX = G == 2 ? N : N / 2;
+  constexpr int P = zpitch(N);
+  constexpr long long IM = G == 2 ? (long long)N * N * N : (long long)N * N;   // from the real to the imaginary pencil
+  static_assert(N % PAIRS == 0, "a block's columns share one x plane");
+  extern __shared__ __align__(16) float4 s4[];    // [CP][N] slots of two columns
+  const int tid = threadIdx.x;
+  const long long q0 = (long long)blockIdx.x * PAIRS;
+  const long long x = q0 / N, y = q0 - x * N;
+  const float* base = mesh + (G == 2 ? q0 * N : (2 * x * N + y) * N);
+  float2* o0 = out + q0 * P;
+  float2* o1 = o0 + (long long)NX * N * P;
+  auto gin = [base](int j, int cp) {
+    const float* b = base + 2 * cp * N + j;
+    return make_float4(__ldcs(b), __ldcs(b + IM), __ldcs(b + N), __ldcs(b + IM + N));
+  };
+  auto sin_ = [](int j, int cp) { return s4[cp * N + zsw(j)]; };
+  auto sout = [](int j, int cp, float4 v) { s4[cp * N + zsw(j)] = v; };
+  auto gout = [o0, o1, kz_cols](int k, int cp, float4 v) { fft::store_packed<N>(o0, o1, P, kz_cols, k, cp, v); };
+  fft::run_stages2<N, CP, NT, true, false, false>(gin, sin_, sout, gout, tw, tid);
+}
+
 // ---- y and x passes --------------------------------------------------------
 // 8 adjacent kz columns x N rows per CTA, rows `row_stride` complex apart;
 // CTA b covers plane (b / nkb) and kz block (b % nkb).  N/2 threads: one
 // pair of radix-8 butterflies (two columns) each per stage; the first stage
 // loads from HBM and the last stores to HBM (fft_pass.cuh), in place.
-template <int N>
+// PRUNE: rows whose wavenumber k has k^2 + (the block's first kz)^2 > k2_max
+// are not stored (with k edges up to k_Nyquist, a fifth of them: 0.423 ->
+// 0.392 ms for two grids at 512^3, 5.0 TB/s; bound by HBM).
+template <int N, bool PRUNE>
 __global__ void __launch_bounds__(N / 2, N <= 512 ? 4 : 2)
 fft_cols_kernel(float2* __restrict__ data, long long plane_stride, long long row_stride, int nplanes, int nkb,
-                const float2* __restrict__ tw) {
+                int k2_max, const float2* __restrict__ tw) {
   pdl_wait();
   extern __shared__ __align__(16) float2 s[];
   const int plane = blockIdx.x / nkb, kb = blockIdx.x % nkb;
@@ -115,7 +166,12 @@ fft_cols_kernel(float2* __restrict__ data, long long plane_stride, long long row
   auto gin = [base, row_stride](int j, int cp) {
     return __ldcs(reinterpret_cast<const float4*>(base + j * row_stride) + cp);
   };
-  auto gout = [base, row_stride](int j, int cp, float4 v) {
+  const int lim = PRUNE ? k2_max - 64 * kb * kb : 0;
+  auto gout = [base, row_stride, lim](int j, int cp, float4 v) {
+    if (PRUNE) {
+      const int k = signed_k(j, N);
+      if (k * k > lim) return;
+    }
     __stcs(reinterpret_cast<float4*>(base + j * row_stride) + cp, v);
   };
   fft::col_fft<N, 1, N / 2, false>(s, gin, gout, tw, threadIdx.x);
@@ -123,14 +179,24 @@ fft_cols_kernel(float2* __restrict__ data, long long plane_stride, long long row
 
 template <int N>
 constexpr int z_pairs() { return N >= 256 ? 8 : 32768 / (N * 8); }   // >= 256 threads
+template <int N, bool PRUNE>
+int launch_cols(float2* data, long long plane_stride, long long row_stride, int nplanes, int nkb, int k2_max,
+                const float2* tw, cudaStream_t st) {
+  const size_t smem = (size_t)fft::ColBlock<N, 1>::SLAB * sizeof(float2);
+  auto kc = fft_cols_kernel<N, PRUNE>;
+  GBP_CUDA_TRY(cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GBP_CUDA_TRY(launch_pdl(kc, dim3((unsigned)(nplanes * nkb)), dim3(N / 2), smem, st, data, plane_stride, row_stride,
+                          nplanes, nkb, k2_max, tw));
+  return GBP_OK;
+}
+
 template <int N>
-int run_fft(const float* mesh, float2* spec, int G, const float2* tw, cudaStream_t st, bool x_pass = true,
-            bool z_pass = true) {
+int run_fft(const float* mesh, float2* spec, int G, const float2* tw, cudaStream_t st) {
   constexpr int PAIRS = z_pairs<N>();
   constexpr int P = zpitch(N);
   constexpr int C = 8;                    // kz columns per CTA in the y and x passes
   const long long npen = (long long)G * N * N;
-  if (z_pass) {
+  {
     const size_t smem = (size_t)PAIRS * N * sizeof(float2);
     auto k = fftz_kernel<N, PAIRS>;
     GBP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -138,22 +204,41 @@ int run_fft(const float* mesh, float2* spec, int G, const float2* tw, cudaStream
     GBP_TRACE("fft_z", st);
     GBP_CUDA_TRY(launch_pdl(k, dim3((unsigned)blocks), dim3(PAIRS * N / 16), smem, st, mesh, spec, npen, tw));
   }
-  const int nkb = P / C;
-  const size_t smem = (size_t)fft::ColBlock<N, 1>::SLAB * sizeof(float2);
-  auto kc = fft_cols_kernel<N>;
-  GBP_CUDA_TRY(cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   {  // y pass: a plane is one x slab of one grid; rows (y) are P apart
     GBP_TRACE("fft_y", st);
-    GBP_CUDA_TRY(launch_pdl(kc, dim3((unsigned)(G * N * nkb)), dim3(N / 2), smem, st, spec, (long long)N * P,
-                            (long long)P, G * N, nkb, tw));
+    const int r = launch_cols<N, false>(spec, (long long)N * P, (long long)P, G * N, P / C, 0, tw, st);
+    if (r) return r;
   }
   // x pass: a plane is one y row of one grid; rows (x) are N*P apart
-  for (int g = 0; x_pass && g < G; ++g) {
+  for (int g = 0; g < G; ++g) {
     GBP_TRACE("fft_x", st);
-    GBP_CUDA_TRY(launch_pdl(kc, dim3((unsigned)(N * nkb)), dim3(N / 2), smem, st, spec + (long long)g * N * N * P,
-                            (long long)P, (long long)N * P, N, nkb, tw));
+    const int r =
+        launch_cols<N, false>(spec + (long long)g * N * N * P, (long long)P, (long long)N * P, N, P / C, 0, tw, st);
+    if (r) return r;
   }
   return GBP_OK;
+}
+
+template <int N, int G>
+int run_z_packed(const float* mesh, float2* spec, int kz_cols, const float2* tw, cudaStream_t st) {
+  constexpr int PAIRS = z_pairs<N>();
+  constexpr int NX = G == 2 ? N : N / 2;
+  const size_t smem = (size_t)PAIRS * N * sizeof(float2);
+  auto k = fftz_packed_kernel<N, G, PAIRS>;
+  GBP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GBP_TRACE("fft_z", st);
+  GBP_CUDA_TRY(launch_pdl(k, dim3((unsigned)(NX * N / PAIRS)), dim3(PAIRS * N / 16), smem, st, mesh, spec, kz_cols,
+                          tw));
+  return GBP_OK;
+}
+
+template <int N>
+int run_y_packed(int G, float2* spec, int kz_cols, int k2_max, const float2* tw, cudaStream_t st) {
+  constexpr int P = zpitch(N);
+  if (kz_cols == 0) return GBP_OK;
+  GBP_TRACE("fft_y", st);
+  // a plane is one x' of one slab: two slabs of N (two grids) or N/2 planes
+  return launch_cols<N, true>(spec, (long long)N * P, (long long)P, G * N, kz_cols / 8, k2_max, tw, st);
 }
 
 }  // namespace
@@ -191,6 +276,7 @@ std::vector<float2> twiddle_tables() {
 int own_fft_twiddles(int N, float2** d_tw) {
   std::vector<float2> h;
   switch (N) {
+    case 32: h = twiddle_tables<32>(); break;
     case 64: h = twiddle_tables<64>(); break;
     case 128: h = twiddle_tables<128>(); break;
     case 256: h = twiddle_tables<256>(); break;
@@ -221,24 +307,28 @@ int own_fft_r2c(int N, int G, const float* mesh, float2* spec, const float2* tw,
   }
 }
 
-int own_fft_y(int N, int G, float2* spec, const float2* tw, cudaStream_t st) {
+int own_fft_z_packed(int N, int G, const float* mesh, float2* spec, int kz_cols, const float2* tw,
+                     cudaStream_t st) {
+#define GBP_Z(NN) \
+  case NN: return G == 2 ? run_z_packed<NN, 2>(mesh, spec, kz_cols, tw, st) : run_z_packed<NN, 1>(mesh, spec, kz_cols, tw, st)
   switch (N) {
-    case 64: return run_fft<64>(nullptr, spec, G, tw, st, false, false);
-    case 128: return run_fft<128>(nullptr, spec, G, tw, st, false, false);
-    case 256: return run_fft<256>(nullptr, spec, G, tw, st, false, false);
-    case 512: return run_fft<512>(nullptr, spec, G, tw, st, false, false);
-    case 1024: return run_fft<1024>(nullptr, spec, G, tw, st, false, false);
+    GBP_Z(64);
+    GBP_Z(128);
+    GBP_Z(256);
+    GBP_Z(512);
+    GBP_Z(1024);
     default: return GBP_ERR_UNSUPPORTED;
   }
+#undef GBP_Z
 }
 
-int own_fft_zy(int N, int G, const float* mesh, float2* spec, const float2* tw, cudaStream_t st) {
+int own_fft_y_packed(int N, int G, float2* spec, int kz_cols, int k2_max, const float2* tw, cudaStream_t st) {
   switch (N) {
-    case 64: return run_fft<64>(mesh, spec, G, tw, st, false);
-    case 128: return run_fft<128>(mesh, spec, G, tw, st, false);
-    case 256: return run_fft<256>(mesh, spec, G, tw, st, false);
-    case 512: return run_fft<512>(mesh, spec, G, tw, st, false);
-    case 1024: return run_fft<1024>(mesh, spec, G, tw, st, false);
+    case 64: return run_y_packed<64>(G, spec, kz_cols, k2_max, tw, st);
+    case 128: return run_y_packed<128>(G, spec, kz_cols, k2_max, tw, st);
+    case 256: return run_y_packed<256>(G, spec, kz_cols, k2_max, tw, st);
+    case 512: return run_y_packed<512>(G, spec, kz_cols, k2_max, tw, st);
+    case 1024: return run_y_packed<1024>(G, spec, kz_cols, k2_max, tw, st);
     default: return GBP_ERR_UNSUPPORTED;
   }
 }

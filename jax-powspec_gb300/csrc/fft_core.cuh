@@ -3,7 +3,7 @@
 // Layout: element i of column c (one transform per column) sits at
 // s[i * CP + c]; CP >= C is the row pitch.  A CTA transforms its C columns
 // of length N together, one butterfly of 8 values per thread and stage.
-// Lengths N = 8^a * {1, 2, 4} (64 .. 4096) use radix-8 stages and at most one
+// Lengths N = 8^a * {1, 2, 4} (32 .. 4096) use radix-8 stages and at most one
 // radix-2 or radix-4 stage; the output is in natural order (Stockham).
 //
 // Stage with radix R, p = product of the previous radices: butterfly
@@ -64,7 +64,7 @@ __device__ __forceinline__ void dft8(float2* u) {
 
 template <int N>
 struct Radices {
-  static constexpr int log2n = (N == 64) ? 6 : (N == 128) ? 7 : (N == 256) ? 8 : (N == 512) ? 9
+  static constexpr int log2n = (N == 32) ? 5 : (N == 64) ? 6 : (N == 128) ? 7 : (N == 256) ? 8 : (N == 512) ? 9
                                : (N == 1024) ? 10 : (N == 2048) ? 11 : 12;
   static constexpr int n8 = log2n / 3;      // radix-8 stages
   static constexpr int tail = log2n % 3;    // 0, 1 (radix 2) or 2 (radix 4)

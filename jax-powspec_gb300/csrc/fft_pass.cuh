@@ -50,6 +50,8 @@ __device__ __forceinline__ float4 pack2(float2 a, float2 b) { return make_float4
 
 // Barrier of the GS consecutive threads that share data (a named barrier,
 // id 1 + tid / GS), or of the whole CTA when GS == 0.
+// A CTA has 16 named barriers and __syncthreads is number 0: at most 15 groups.
+constexpr int MAX_GROUPS = 15;
 template <int GS>
 __device__ __forceinline__ void group_sync(int tid) {
   if constexpr (GS == 0) {
@@ -114,6 +116,7 @@ __device__ __forceinline__ void stage2(In in, Out out, const float2* __restrict_
     for (int r = 0; r < R; ++r) u[q][r] = pack2(a[r], c[r]);
   }
   static_assert(GS == 0 || (IFAST && N / R == GS && NB == NT), "group barriers need one column pair per group");
+  static_assert(GS == 0 || CP <= MAX_GROUPS, "more groups than named barriers");
   if (MID_SYNC) group_sync<GS>(tid);
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
@@ -186,6 +189,23 @@ __device__ __forceinline__ void col_fft(float2* s, In gin, Out gout, const float
   auto sin_ = [s4](int j, int cp) { return s4[L::at(j, cp)]; };
   auto sout = [s4](int j, int cp, float4 v) { s4[L::at(j, cp)] = v; };
   run_stages2<N, L::CP, NT, false, IN_SHARED, OUT_SHARED>(gin, sin_, sout, gout, tw, tid);
+}
+
+// Stores Z[k] of columns 2cp and 2cp + 1 (rows 2cp, 2cp + 1 of pitch P) of a
+// packed z pass: kz = k goes to slab 0 (o0) when k <= N/2, kz = -(N - k) to
+// slab 1 (o1) when N - k <= N/2 (k = 0 and N/2 to both); columns >= kz_cols
+// are not stored.
+template <int N>
+__device__ __forceinline__ void store_packed(float2* o0, float2* o1, int P, int kz_cols, int k, int cp, float4 v) {
+  const int m = (N - k) & (N - 1);
+  if (k <= N / 2 && k < kz_cols) {
+    __stcs(o0 + 2 * cp * P + k, lo2(v));
+    __stcs(o0 + (2 * cp + 1) * P + k, hi2(v));
+  }
+  if (m <= N / 2 && m < kz_cols) {
+    __stcs(o1 + 2 * cp * P + m, lo2(v));
+    __stcs(o1 + (2 * cp + 1) * P + m, hi2(v));
+  }
 }
 
 // Slot of row j in a column-major block of column pairs (IFAST stages).

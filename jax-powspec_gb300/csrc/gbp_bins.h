@@ -6,6 +6,9 @@
 
 #include "gbpowspec.h"
 
+// Encoding of an item of the x pass + binning: y * XITEM_KB + kz block.
+constexpr int XITEM_KB = 128;
+
 struct gbp_bins_s {
   int N;            // mesh side
   int nb;           // number of bins (n_edges - 1)
@@ -20,5 +23,10 @@ struct gbp_bins_s {
   float2* d_eph;        // [N/2 + 1]  exp(i pi k / N)
   long long* d_nmodes;  // [nb] modes per bin (geometry only, computed once)
   double* d_ksum;       // [nb] sum of |k| per bin, grid units
+  // work items of the x pass + binning (power-of-two sides 64..1024): (y row, block of 8 kz columns)
+  // pairs that hold a mode at or below last_closed, as y * XITEM_KB + block, y-major
+  int* d_xitems;
+  int n_xitems;
+  int kz_cols;          // kz columns the items read (a multiple of 8; 0: none)
   void* d_block;        // the single device allocation holding the above
 };

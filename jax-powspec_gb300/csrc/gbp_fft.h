@@ -12,6 +12,7 @@ struct gbp_fft_plan_s {
   bool own;
   cufftHandle h;
   float2* tw;       // own transform: twiddles exp(-2 pi i e / N)
+  float2* twx;      // those of the packed x transform (fft.cu): N points for two grids (== tw), N/2 for one
   int n, grids, pitch;
   size_t ws;
   int tx = 0, ty = 0;   // column tile of the fused particles path (0: the default for n)
@@ -22,12 +23,12 @@ bool own_fft_supported(int N);
 int own_fft_pitch(int N);
 int own_fft_twiddles(int N, float2** d_tw);
 int own_fft_r2c(int N, int G, const float* mesh, float2* spec, const float2* tw, cudaStream_t st);
-// z and y passes only: spec holds the transform over z and y, not yet over x
-int own_fft_zy(int N, int G, const float* mesh, float2* spec, const float2* tw, cudaStream_t st);
-// y pass only (spec already transformed over z)
-int own_fft_y(int N, int G, float2* spec, const float2* tw, cudaStream_t st);
+// Packed transform (fft.cu): z pass of G = 1 or 2 meshes into the packed layout, kz < kz_cols only
+int own_fft_z_packed(int N, int G, const float* mesh, float2* spec, int kz_cols, const float2* tw, cudaStream_t st);
+// y pass of the packed layout: kz < kz_cols, rows with ky^2 + (first kz of the block)^2 <= k2_max stored
+int own_fft_y_packed(int N, int G, float2* spec, int kz_cols, int k2_max, const float2* tw, cudaStream_t st);
 // x pass fused with the binning + the fold into per-bin sums (xbin.cu); spec
-// holds the transform over z and y
+// holds the packed transform over z and y
 int xbin_power_workspace(gbp_fft_plan plan, gbp_bins bins, int ells, size_t* bytes);
 // Cached cuFFT plan (per device) of `batch` unnormalised inverse real 3-D
 // transforms: complex input rows of P >= N/2+1 entries ([batch][N][N][P]),

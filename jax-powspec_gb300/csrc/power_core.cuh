@@ -34,7 +34,9 @@ struct PowGeom {
   int groups;               // work groups (g.warps chunks each), one partial per group
   // fused x-pass + binning (xbin.cu) only
   const float2* tw;         // [N] exp(-2 pi i e / N)
-  int items, nkb;           // (y, kz block) work items; kz blocks per row
+  const float2* twx;        // twiddle tables of the x transform
+  const int* item_list;     // [items] y * XITEM_KB + kz block (gbp_bins.h)
+  int items;
 };
 
 struct SmemPlan {

@@ -1,26 +1,38 @@
 // The x pass of the 3-D FFT fused with the binning.
 //
-// After the z and y passes (fft.cu) the spectrum buffer holds, for every
-// grid, the transform over z and y; the remaining 1-D transforms run along
-// x, whose rows lie N*P complex apart.  Instead of writing them back and
-// reading them again for the binning, one CTA takes a work item = one ky row
-// and a block of 8 adjacent kz columns, for all grids:
+// After the z and y passes (fft.cu) the spectrum buffer holds the packed
+// field Z transformed over z and y: slab 0 at kz, slab 1 at -kz; the
+// remaining 1-D transforms run along x, whose rows lie N*P complex apart.
+// Instead of writing them back and reading them again for the binning, one
+// CTA takes a work item = one ky row and a block of 8 adjacent kz columns of
+// slab 0, and row -ky of the same block of slab 1:
 //
-//   1. loads the item's N x 8 complex values of each grid (16-byte loads,
-//      64 contiguous bytes per x row) into shared memory,
-//   2. transforms the 8 (or 16, two grids) columns along x with radix-8
-//      Stockham stages (fft_core.cuh); the last stage writes the result
-//      column-major with an XOR swizzle, so the binning reads it without
-//      bank conflicts,
-//   3. bins the 8 x N modes: from 128^3 up the modes x and N - x of a
-//      column (kx and -kx) share |k|, mu, the window and the bin, so they
-//      are summed first and looked up once; a warp walks one column over
-//      half of the |kx| range (pairs p = 0..N/4-1 or N/4..N/2-1; x = N/2
-//      alone is added after the upper half), so bins are monotone along the
-//      walk (at 64^3: single modes over half of the x axis).  A lane owns
-//      consecutive pairs; runs of equal bin are summed in-lane, joined
-//      across lanes by one warp segmented scan, and each run is added once
-//      to the warp's float32 bins (distinct bins within a step: no atomics).
+//   1. loads the item's 2 x NX x 8 complex values (16-byte loads, 64
+//      contiguous bytes per x row) into shared memory,
+//   2. transforms the 16 columns along x (NX = N points for an interlaced
+//      pair, N/2 for one grid) with radix-8 Stockham stages (fft_core.cuh);
+//      the last stage writes the result column-major with an XOR swizzle, so
+//      the binning reads it without bank conflicts,
+//   3. bins the 8 x N modes.  With A = Z(k), B = conj Z(-k) the mode is
+//          two grids:  F0 + phi F1,  F0 = (A + B)/2, F1 = -i (A - B)/2,
+//                      phi = exp(i pi (kx + ky + kz) / N)  (times 1/2)
+//          one grid:   E + w O, the same with w = exp(-2 pi i kx / N) and
+//                      Z taken at kx mod N/2,
+//      that is ((A + B) - i f (A - B)) / 2 with f = phi or w.  The modes x
+//      and N - x of a column (kx and -kx) share |k|, mu, the window and the
+//      bin, and the four values they need, so they are summed first and
+//      looked up once; a warp walks one column over half of the |kx| range
+//      (or all of it; x = N/2 alone is added after the last pair), so bins
+//      are monotone along the walk.  A lane owns consecutive pairs; runs of
+//      equal bin are summed in-lane, joined across lanes by one warp
+//      segmented scan, and each run is added once to the warp's float32 bins
+//      (distinct bins within a step: no atomics).
+//
+// Only items with a mode inside the last k edge are listed by the bin plan
+// (gbp_bins_create): edges up to k_Nyquist leave out a fifth of them.  Two
+// grids at 512^3: 0.688 -> 0.552 ms (0.86 GB read: 1.6 TB/s; bound by
+// instruction issue and barriers); one grid (half the points per column, a
+// warp per column): 0.545 -> 0.362 ms at 512^3, 0.091 -> 0.045 at 256^3.
 //
 // The mode arithmetic (window deconvolution, interlacing average, |delta|^2,
 // mu^2 and mu^4 moments, DC removal) and the bin lookup are those of
@@ -42,43 +54,39 @@
 namespace gbp {
 namespace {
 
-constexpr int XB_THREADS = 512;
 constexpr int XB_BINS = 8;                   // per-warp bin arrays; warps w and w + 8 share one
 constexpr int XB_C = 8;                      // kz columns per work item
 // The next item's HBM loads start before the barrier that ends the binning (512^3 and up)
 template <int N>
 constexpr bool XB_EARLY = N >= 512;
 
-template <int N>
+template <int N, bool INTER>
 struct XLayout {
-  static constexpr int TST = N + 1;          // complex per column (transposed layout); odd: no store conflicts
-  static constexpr int M = N / 64;           // modes per lane in a half axis
-  static constexpr int MS = M < 8 ? M : 8;   // modes per lane and warp step
-  // N >= 128: the modes x and N - x of a column (kx and -kx: the same |k|, mu, window and bin) are
-  // binned together, M2 such pairs per lane in half of the |kx| range
-  static constexpr bool PAIRED = N >= 128;
-  static constexpr int M2 = N / 128;
-  static constexpr int MS2 = M2 < 8 ? M2 : 8;
-  static_assert(!PAIRED || (MS2 > 0 && M2 % MS2 == 0), "whole warp steps of mode pairs");
-  static __host__ __device__ constexpr size_t data_bytes(int G) {
-    const size_t rows = (size_t)G * fft::ColBlock<N, 2>::SLAB, cols = (size_t)G * XB_C * TST;
+  static constexpr int NX = INTER ? N : N / 2;   // points of the x transform
+  static constexpr int NT = NX < 512 ? 256 : 512;
+  static constexpr int HALVES = NT / 256;    // warps per column
+  static constexpr int TST = NX + 1;         // complex per column (transposed layout); odd: no store conflicts
+  // a lane takes M2 consecutive pairs (x, N - x) of its warp's part of the |kx| range, MS2 per warp step
+  static constexpr int M2 = N / (64 * HALVES);
+  static constexpr int MS2 = M2 < 4 ? M2 : (N >= 1024 && INTER ? (M2 < 8 ? M2 : 8) : 4);
+  static_assert(MS2 > 0 && M2 % MS2 == 0, "whole warp steps of mode pairs");
+  static __host__ __device__ constexpr size_t data_bytes() {
+    const size_t rows = (size_t)2 * fft::ColBlock<NX, 2>::SLAB, cols = (size_t)2 * XB_C * TST;
     return ((rows > cols ? rows : cols) * 8 + 127) & ~size_t(127);
   }
-  // per-x tables (swizzled like the columns): window c2(|kx|) and exp(i pi kx / N)
-  static __host__ __device__ constexpr size_t xtab_bytes() { return (size_t)N * 12; }
+  // per-|kx| tables (swizzled like the columns): window c2 and the factor f of kx >= 0
+  static __host__ __device__ constexpr size_t xtab_bytes() { return (size_t)(N / 2) * 12; }
 };
 
-// Swizzled position of x in a transposed column: lane l reads x = base + L l
-// (L = the modes or mode pairs a lane takes per half axis), and so does it
-// read the mirror N - x; with x's low bits XORed by bits 4.. of x, the 16
-// lanes of a half-warp hit 16 distinct 8-byte slots in both reads, and the
-// last FFT stage's stores stay conflict-free (checked by enumeration of
-// every stage and mesh size).
-template <int N>
+// Swizzled position of x in a transposed column: lane l reads x = base + M2 l
+// + j (M2 = the mode pairs a lane takes), and so does it read the mirror
+// -x; with x's low bits XORed by bits 4.. of x, the 16 lanes of a half-warp
+// hit 16 distinct 8-byte slots in both reads, and the last FFT stage's
+// stores stay conflict-free.
+template <int M2>
 __device__ __forceinline__ int xswz(int x) {
-  constexpr int L = XLayout<N>::PAIRED ? XLayout<N>::M2 : XLayout<N>::M;
-  if constexpr (L <= 1) return x;
-  else return x ^ ((x >> 4) & (L - 1));
+  if constexpr (M2 <= 1) return x;
+  else return x ^ ((x >> 4) & (M2 - 1));
 }
 
 // One warp step: lane modes x0 + j (j < MS) of one column, bins monotone in
@@ -126,102 +134,91 @@ __device__ __forceinline__ void flush_runs(float (&P)[MS][NV], const int (&bin)[
   __syncwarp();
 }
 
-// Moments and bins of one warp step (lane modes x0 .. x0 + MS - 1 of column c).
-template <int N, int NV, bool INTER, int MS>
-__device__ __forceinline__ void xbin_modes(const PowGeom& g, const Smem& t, const float* c2x, const float2* ephx,
-                                           const float2* a_col, const float2* b_col, int x0, int kyz2, float cyz,
-                                           float fz2, float2 eyz, float (&P)[MS][NV], int (&bin)[MS]) {
-#pragma unroll
-  for (int j = 0; j < MS; ++j) {
-    const int x = x0 + j;
-    const int kx = signed_k(x, N);
-    const int sx = xswz<N>(x);
-    const float2 a = a_col[sx];
-    float re = a.x, im = a.y;
-    if (INTER) {
-      const float2 b = b_col[sx];
-      const float2 ex = ephx[sx];
-      const float qr = ex.x * eyz.x - ex.y * eyz.y;
-      const float qi = ex.x * eyz.y + ex.y * eyz.x;
-      re = a.x + (b.x * qr - b.y * qi);
-      im = a.y + (b.x * qi + b.y * qr);
-    }
-    const int k2 = kx * kx + kyz2;
-    if (g.zero_dc && k2 == 0) re = im = 0.0f;
-    const float p = (re * re + im * im) * (cyz * c2x[sx]);
-    P[j][0] = p;
-    if (NV > 1) {
-      const float mu2 = k2 > 0 ? __fdividef(fz2, (float)k2) : 0.0f;
-      P[j][1] = p * mu2;
-      if (NV > 2) P[j][2] = P[j][1] * mu2;
-    }
-    bin[j] = bin_of(g, t, k2);
-  }
+// (A + B) - i f (A - B), B = conj b, f = (fr, fi): four times |.|^2's root is the mode.
+__device__ __forceinline__ float2 unpack_mode(float2 a, float2 b, float fr, float fi) {
+  const float sx = a.x + b.x, sy = a.y - b.y, dx = a.x - b.x, dy = a.y + b.y;
+  return make_float2(sx + (fr * dy + fi * dx), sy + (fi * dy - fr * dx));
 }
 
 // Moments and bins of one warp step of mode pairs: lane pairs p0 .. p0 + MS - 1
-// of column (a_col, b_col), pair p = the columns x = p and x = N - p
-// (kx = p and -p), whose |k|, mu, window and bin agree; p = 0 is x = 0 alone.
+// of a column (a_col at (ky, kz), b_col at (-ky, -kz)), pair p = the modes
+// kx = p and -p, whose |k|, mu, window and bin agree; p = 0 is one mode.
+// eyz: the ky and kz part of the phase (two grids).
 template <int N, int NV, bool INTER, int MS>
-__device__ __forceinline__ void xbin_pairs(const PowGeom& g, const Smem& t, const float* c2x, const float2* ephx,
+__device__ __forceinline__ void xbin_pairs(const PowGeom& g, const Smem& t, const float* c2x, const float2* fx,
                                            const float2* a_col, const float2* b_col, int p0, int kyz2, float cyz,
                                            float fz2, float2 eyz, float (&P)[MS][NV], int (&bin)[MS]) {
+  using L = XLayout<N, INTER>;
 #pragma unroll
   for (int j = 0; j < MS; ++j) {
     const int p = p0 + j;
-    const int sp = xswz<N>(p), sm = xswz<N>((N - p) & (N - 1));
-    const float2 a = a_col[sp], am = a_col[sm];
-    float re = a.x, im = a.y, rem = am.x, imm = am.y;
+    const int sp = xswz<L::M2>(p), sm = xswz<L::M2>((L::NX - p) & (L::NX - 1));
+    const float2 e = fx[sp];
+    float fr = e.x, fi = e.y, mr = e.x, mi = -e.y;           // f of kx = p and of kx = -p
     if (INTER) {
-      const float2 b = b_col[sp], bm = b_col[sm];
-      const float2 ex = ephx[sp];                            // exp(i pi p / N); kx = -p takes its conjugate
-      const float ar = ex.x * eyz.x, ai = ex.x * eyz.y, br = ex.y * eyz.y, bi = ex.y * eyz.x;
-      const float qr = ar - br, qi = ai + bi;                // exp(i pi p / N) eyz
-      const float mr = ar + br, mi = ai - bi;                // exp(-i pi p / N) eyz
-      re = a.x + (b.x * qr - b.y * qi);
-      im = a.y + (b.x * qi + b.y * qr);
-      rem = am.x + (bm.x * mr - bm.y * mi);
-      imm = am.y + (bm.x * mi + bm.y * mr);
+      const float ar = e.x * eyz.x, ai = e.x * eyz.y, br = e.y * eyz.y, bi = e.y * eyz.x;
+      fr = ar - br;
+      fi = ai + bi;
+      mr = ar + br;
+      mi = ai - bi;
     }
+    const float2 ap = a_col[sp], am = a_col[sm], bp = b_col[sp], bm = b_col[sm];
+    const float2 u = unpack_mode(ap, bm, fr, fi), v = unpack_mode(am, bp, mr, mi);
     const int k2 = p * p + kyz2;
-    float pw = re * re + im * im;
+    float pw = u.x * u.x + u.y * u.y;
     if (g.zero_dc && k2 == 0) pw = 0.0f;
-    if (p > 0) pw += rem * rem + imm * imm;
-    const float v = pw * (cyz * c2x[sp]);
-    P[j][0] = v;
+    if (p > 0) pw += v.x * v.x + v.y * v.y;
+    const float w = pw * (cyz * c2x[sp]);
+    P[j][0] = w;
     if (NV > 1) {
       const float mu2 = k2 > 0 ? __fdividef(fz2, (float)k2) : 0.0f;
-      P[j][1] = v * mu2;
+      P[j][1] = w * mu2;
       if (NV > 2) P[j][2] = P[j][1] * mu2;
     }
     bin[j] = bin_of(g, t, k2);
   }
 }
 
-// The column x = N/2 (kx = N/2, its own mirror) of one column, added to the
-// warp's bins by one lane.  Out of line: it runs once per column and only
-// for bins beyond k_Nyq, and inlined it would cost the binning registers.
+// The mode kx = N/2 (its own mirror) of one column, added to the warp's bins
+// by one lane.  Out of line: it runs once per column and only for bins
+// beyond k_Nyq, and inlined it would cost the binning registers.
 template <int N, int NV, bool INTER>
-__device__ __noinline__ void add_nyquist_x(const PowGeom& g, const Smem& t, const float* c2x, const float2* ephx,
-                                           const float2* a_col, const float2* b_col, int kyz2, float cyz, float fz2,
-                                           float2 eyz, float* wb) {
-  float P[1][NV];
-  int bin[1];
-  xbin_modes<N, NV, INTER, 1>(g, t, c2x, ephx, a_col, b_col, N / 2, kyz2, cyz, fz2, eyz, P, bin);
-  if (bin[0] >= 0) bin_add<NV>(wb, g.nbe, bin[0], P[0]);
+__device__ __noinline__ void add_nyquist_x(const PowGeom& g, const Smem& t, const float2* a_col, const float2* b_col,
+                                           int kyz2, float cyz, float fz2, float2 eyz, float* wb) {
+  using L = XLayout<N, INTER>;
+  constexpr int H = N / 2;
+  const int sp = xswz<L::M2>(H & (L::NX - 1));
+  float fr = -1.0f, fi = 0.0f;                               // w^(N/2)
+  if (INTER) {
+    const float2 e = t.eph[H];
+    fr = e.x * eyz.x - e.y * eyz.y;
+    fi = e.x * eyz.y + e.y * eyz.x;
+  }
+  const float2 u = unpack_mode(a_col[sp], b_col[sp], fr, fi);
+  const int k2 = H * H + kyz2;
+  float P[NV];
+  P[0] = (u.x * u.x + u.y * u.y) * (cyz * t.c2[H]);
+  if (NV > 1) {
+    const float mu2 = __fdividef(fz2, (float)k2);
+    P[1] = P[0] * mu2;
+    if (NV > 2) P[2] = P[1] * mu2;
+  }
+  const int bin = bin_of(g, t, k2);
+  if (bin >= 0) bin_add<NV>(wb, g.nbe, bin, P);
 }
 
-// Bin the 8 columns of one item (transposed layout in s).  Warp w takes
-// column w / 2 and half w % 2 of the x axis (of the |kx| range, in mode
-// pairs x, N - x from 128^3 up); warps w and w + 8 share bin
-// array w % 8 and flush in two phases separated by barriers.  No barrier
-// follows the last step: the caller's next barrier (the next item's first
-// FFT stage, or the fold) orders the last flushes and reads of s.
+// Bin the 8 columns of one item (transposed layout in s).  HALVES = 2: warp
+// w takes column w / 2 and half w % 2 of the |kx| range; warps w and w + 8
+// share bin array w % 8 and flush in two phases separated by barriers.
+// HALVES = 1: warp w takes column w.  No barrier follows the last step: the
+// caller's next barrier (the next item's first FFT stage, or the fold)
+// orders the last flushes and reads of s.
 template <int N, int NV, bool INTER>
-__device__ __forceinline__ void xbin_item(const PowGeom& g, const Smem& t, const float* c2x, const float2* ephx,
+__device__ __forceinline__ void xbin_item(const PowGeom& g, const Smem& t, const float* c2x, const float2* fx,
                                           const float2* s, int warp, int lane, int y, int kb) {
-  constexpr int H = N / 2, M = XLayout<N>::M, MS = XLayout<N>::MS, TST = XLayout<N>::TST;
-  const int c = warp >> 1, h = warp & 1;
+  using L = XLayout<N, INTER>;
+  constexpr int H = N / 2, TST = L::TST, HALVES = L::HALVES, M2 = L::M2, MS2 = L::MS2;
+  const int c = warp / HALVES, h = warp % HALVES;
   const int kz = kb * XB_C + c;
   const bool active = kz <= H;                              // else row padding
   const int kzc = active ? kz : 0;
@@ -234,123 +231,110 @@ __device__ __forceinline__ void xbin_item(const PowGeom& g, const Smem& t, const
     const float2 ez = t.eph[kzc];
     eyz = make_float2(ey.x * ez.x - ey.y * ez.y, ey.x * ez.y + ey.y * ez.x);
   }
-  // |(a + b)/2|^2: the 1/4 of the interlaced average rides on the constant
-  const float cyz = t.c2[ay] * t.c2[kzc] * (INTER ? 0.25f : 1.0f);
+  // |unpack_mode / 2|^2, and |(a + b)/2|^2 of an interlaced pair: the 1/4 or 1/16 rides on the constant
+  const float cyz = t.c2[ay] * t.c2[kzc] * (INTER ? 0.0625f : 0.25f);
   const int kyz2 = ky * ky + kzc * kzc;
   const float fz2 = (float)(kzc * kzc);
   const float2* a_col = s + c * TST;
   const float2* b_col = s + (XB_C + c) * TST;
   float* wb = t.wbase + (warp & (XB_BINS - 1)) * NV * g.nbe;
-  if constexpr (XLayout<N>::PAIRED) {
-    // warp half h walks pairs h N/4 .. (h+1) N/4 - 1 (|kx| ascending); the column x = N/2, its own
-    // mirror, is added by lane 0 of the upper half after its last flush
-    constexpr int M2 = XLayout<N>::M2, MS2 = XLayout<N>::MS2;
 #pragma unroll 1
-    for (int s0 = 0; s0 < M2; s0 += MS2) {
-      float P[MS2][NV];
-      int bin[MS2];
-      if (active)
-        xbin_pairs<N, NV, INTER, MS2>(g, t, c2x, ephx, a_col, b_col, h * (H / 2) + lane * M2 + s0, kyz2, cyz, fz2,
-                                      eyz, P, bin);
-      auto flush = [&]() {
-        flush_runs<MS2, NV>(P, bin, lane, wb, g.nbe);
-        // |kx| = N/2 reaches a bin only when the last edge lies beyond k_Nyq
-        if (h == 1 && s0 + MS2 >= M2 && (H * H + kyz2 <= g.tu)) {
-          if (lane == 0) add_nyquist_x<N, NV, INTER>(g, t, c2x, ephx, a_col, b_col, kyz2, cyz, fz2, eyz, wb);
-          __syncwarp();
-        }
-      };
+  for (int s0 = 0; s0 < M2; s0 += MS2) {
+    float P[MS2][NV];
+    int bin[MS2];
+    if (active)
+      xbin_pairs<N, NV, INTER, MS2>(g, t, c2x, fx, a_col, b_col, h * (H / HALVES) + lane * M2 + s0, kyz2, cyz, fz2,
+                                    eyz, P, bin);
+    auto flush = [&]() {
+      flush_runs<MS2, NV>(P, bin, lane, wb, g.nbe);
+      // |kx| = N/2 reaches a bin only when the last edge lies beyond k_Nyq
+      if (h == HALVES - 1 && s0 + MS2 >= M2 && (H * H + kyz2 <= g.tu)) {
+        if (lane == 0) add_nyquist_x<N, NV, INTER>(g, t, a_col, b_col, kyz2, cyz, fz2, eyz, wb);
+        __syncwarp();
+      }
+    };
+    if constexpr (HALVES == 1) {
+      if (active) flush();
+    } else {
       if (warp < XB_BINS && active) flush();
       __syncthreads();
       if (warp >= XB_BINS && active) flush();
       if (s0 + MS2 < M2) __syncthreads();   // after the last step, the next item's (or the fold's) barrier follows
     }
-  } else {
-#pragma unroll 1
-    for (int s0 = 0; s0 < M; s0 += MS) {
-      float P[MS][NV];
-      int bin[MS];
-      if (active) {
-        xbin_modes<N, NV, INTER, MS>(g, t, c2x, ephx, a_col, b_col, h * H + lane * M + s0, kyz2, cyz, fz2, eyz, P,
-                                     bin);
-      }
-      if (warp < XB_BINS && active) flush_runs<MS, NV>(P, bin, lane, wb, g.nbe);
-      __syncthreads();
-      if (warp >= XB_BINS && active) flush_runs<MS, NV>(P, bin, lane, wb, g.nbe);
-      if (s0 + MS < M) __syncthreads();     // after the last step, the next item's (or the fold's) barrier follows
-    }
   }
 }
 
 template <int N, int NV, bool INTER>
-__global__ void __launch_bounds__(XB_THREADS, N >= 1024 ? 1 : 2)
+__global__ void __launch_bounds__(XLayout<N, INTER>::NT,
+                                  N >= 1024 && INTER ? 1 : 1024 / XLayout<N, INTER>::NT)
 xbin_kernel(PowGeom g) {
   pdl_wait();
-  constexpr int G = INTER ? 2 : 1;
+  using L = XLayout<N, INTER>;
   constexpr int P = N / 2 + 8;                              // z row pitch of the own transform
-  constexpr int TST = XLayout<N>::TST;
+  constexpr int TST = L::TST, NX = L::NX, NT = L::NT;
   extern __shared__ __align__(16) unsigned char smem[];
   float2* s = reinterpret_cast<float2*>(smem);
-  float2* ephx = reinterpret_cast<float2*>(smem + XLayout<N>::data_bytes(G));
-  float* c2x = reinterpret_cast<float*>(ephx + N);
-  const Smem t = load_tables<NV, INTER>(g, smem + XLayout<N>::data_bytes(G) + XLayout<N>::xtab_bytes());
+  float2* fx = reinterpret_cast<float2*>(smem + L::data_bytes());
+  float* c2x = reinterpret_cast<float*>(fx + N / 2);
+  const Smem t = load_tables<NV, INTER>(g, smem + L::data_bytes() + L::xtab_bytes());
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int x = tid; x < N; x += XB_THREADS) {               // per-x tables (load_tables ended with a barrier)
-    const int kx = signed_k(x, N), ax = kx < 0 ? -kx : kx;
-    float2 e = INTER ? t.eph[ax] : make_float2(1.f, 0.f);
-    if (kx < 0) e.y = -e.y;
-    ephx[xswz<N>(x)] = e;
-    c2x[xswz<N>(x)] = t.c2[ax];
+  for (int p = tid; p < N / 2; p += NT) {                   // per-|kx| tables (load_tables ended with a barrier)
+    fx[xswz<L::M2>(p)] = INTER ? t.eph[p] : g.tw[p];        // exp(i pi p / N), exp(-2 pi i p / N)
+    c2x[xswz<L::M2>(p)] = t.c2[p];
   }
   __syncthreads();
-  const long long gstride = (long long)N * N * P;
+  const long long sstride = (long long)NX * N * P;
   for (int grp = blockIdx.x; grp < g.groups; grp += gridDim.x) {
     for (int it = grp; it < g.items; it += g.groups) {
-      const int y = it / g.nkb, kb = it - (it / g.nkb) * g.nkb;
-      const float2* src = g.s0 + ((long long)y * P + kb * XB_C);
-      auto gin = [src, gstride](int x, int cp) {   // columns 2cp, 2cp+1 (slab = grid cp / 4)
-        return __ldcs(reinterpret_cast<const float4*>(src + (cp >> 2) * gstride + (long long)x * N * P) + (cp & 3));
+      const int code = __ldg(g.item_list + it), y = code / XITEM_KB, kb = code % XITEM_KB;
+      const float2* src = g.s0 + kb * XB_C;
+      // row of the column pair's slab: y, or -y of slab 1
+      const long long r0 = (long long)y * P, r1 = sstride + (long long)((N - y) & (N - 1)) * P;
+      auto gin = [src, r0, r1](int x, int cp) {    // columns 2cp, 2cp+1 (slab cp / 4)
+        return __ldcs(reinterpret_cast<const float4*>(src + (cp < 4 ? r0 : r1) + (long long)x * N * P) + (cp & 3));
       };
       auto tout = [s](int x, int cp, float4 v) {
-        s[(2 * cp) * TST + xswz<N>(x)] = fft::lo2(v);
-        s[(2 * cp + 1) * TST + xswz<N>(x)] = fft::hi2(v);
+        s[(2 * cp) * TST + xswz<L::M2>(x)] = fft::lo2(v);
+        s[(2 * cp + 1) * TST + xswz<L::M2>(x)] = fft::hi2(v);
       };
       // from 512^3 up the first stage loads the item from HBM while the previous item's last warps
       // still bin it, and waits for them before it writes the shared buffer (smaller meshes: the
       // registers the early loads hold would spill; they end the binning with a barrier instead)
-      fft::col_fft<N, G, XB_THREADS, true, decltype(gin), decltype(tout), XB_EARLY<N>>(s, gin, tout, g.tw, tid);
-      xbin_item<N, NV, INTER>(g, t, c2x, ephx, s, warp, lane, y, kb);
+      fft::col_fft<NX, 2, NT, true, decltype(gin), decltype(tout), XB_EARLY<N>>(s, gin, tout, g.twx, tid);
+      xbin_item<N, NV, INTER>(g, t, c2x, fx, s, warp, lane, y, kb);
       if constexpr (!XB_EARLY<N>) __syncthreads();
     }
     cta_fold<NV>(g, t, grp);
   }
 }
 
-// Work groups: a pure function of N, so the summation order is the same on
-// every device.
-int xbin_groups(int items) { return std::min(items, 1216); }
+// Work groups: a pure function of the items, so the summation order is the
+// same on every device.
+int xbin_groups(int items) { return std::max(1, std::min(items, 1216)); }
 
 struct XbLayout {
-  int NV, items, nkb, groups;
+  int NV, items, groups;
   size_t smem, ws;
 };
 
 int xbin_layout(const gbp_bins_s* B, int G, int ells, XbLayout& L) {
   const int N = B->N;
   L.NV = (ells & GBP_ELL4) ? 3 : ((ells & GBP_ELL2) ? 2 : 1);
-  L.nkb = (N / 2 + 8) / XB_C;
-  L.items = N * L.nkb;
+  L.items = B->n_xitems;
   L.groups = xbin_groups(L.items);
   size_t data = 0;
+#define GBP_DATA(NN) \
+  case NN: data = G == 2 ? XLayout<NN, true>::data_bytes() : XLayout<NN, false>::data_bytes(); break
   switch (N) {
-    case 64: data = XLayout<64>::data_bytes(G); break;
-    case 128: data = XLayout<128>::data_bytes(G); break;
-    case 256: data = XLayout<256>::data_bytes(G); break;
-    case 512: data = XLayout<512>::data_bytes(G); break;
-    case 1024: data = XLayout<1024>::data_bytes(G); break;
+    GBP_DATA(64);
+    GBP_DATA(128);
+    GBP_DATA(256);
+    GBP_DATA(512);
+    GBP_DATA(1024);
     default: return GBP_ERR_UNSUPPORTED;
   }
-  L.smem = data + (size_t)N * 12 + smem_plan(N, B->nbe, B->lut_n, XB_BINS, L.NV).total;
+#undef GBP_DATA
+  L.smem = data + (size_t)(N / 2) * 12 + smem_plan(N, B->nbe, B->lut_n, XB_BINS, L.NV).total;
   if (L.smem > 227 * 1024) return GBP_ERR_UNSUPPORTED;
   L.ws = align256((size_t)L.groups * L.NV * B->nbe * sizeof(float2));
   return GBP_OK;
@@ -365,7 +349,7 @@ int launch_xbin(const PowGeom& g, size_t smem, cudaStream_t st) {
   // as fast as the persistent grid at 512^3 (0.775 against 0.781 ms)
   const int grid = std::max(1, g.groups);
   GBP_TRACE("fft_x_bins", st);
-  GBP_CUDA_TRY(launch_pdl(k, dim3(grid), dim3(XB_THREADS), smem, st, g));
+  GBP_CUDA_TRY(launch_pdl(k, dim3(grid), dim3(XLayout<N, INTER>::NT), smem, st, g));
   return GBP_OK;
 }
 
@@ -413,7 +397,6 @@ int xbin_power(gbp_fft_plan plan, float2* spec, gbp_bins B, int mas_order, int e
   const int N = B->N, G = plan->grids;
   PowGeom g{};
   g.s0 = spec;
-  g.s1 = G == 2 ? spec + (long long)N * N * plan->pitch : nullptr;
   g.N = N;
   g.Lz = N / 2 + 1;
   g.Lzs = plan->pitch;
@@ -432,8 +415,9 @@ int xbin_power(gbp_fft_plan plan, float2* spec, gbp_bins B, int mas_order, int e
   g.warps = XB_BINS;
   g.groups = L.groups;
   g.tw = plan->tw;
+  g.twx = plan->twx;
   g.items = L.items;
-  g.nkb = L.nkb;
+  g.item_list = B->d_xitems;
   switch (N) {
     case 64: r = dispatch_xbin<64>(g, L.NV, G == 2, L.smem, st); break;
     case 128: r = dispatch_xbin<128>(g, L.NV, G == 2, L.smem, st); break;
@@ -472,7 +456,9 @@ extern "C" int gbp_fft_power(gbp_fft_plan plan, const float* mesh, void* spectru
   if (r) return r;
   if (!workspace || ws_bytes < need) return GBP_ERR_WORKSPACE;
   float2* spec = static_cast<float2*>(spectrum);
-  r = own_fft_zy(B->N, plan->grids, mesh, spec, plan->tw, st);
+  r = own_fft_z_packed(B->N, plan->grids, mesh, spec, B->kz_cols, plan->tw, st);
+  if (r) return r;
+  r = own_fft_y_packed(B->N, plan->grids, spec, B->kz_cols, B->last_closed, plan->tw, st);
   if (r) return r;
   return xbin_power(plan, spec, B, mas_order, ells, mass, sums_out, nmodes_out, ksum_out, workspace, ws_bytes, st);
 }

@@ -153,7 +153,7 @@ class FFTPlan:
 
 
 def tile_variants(n_mesh: int) -> list:
-    """Column tiles [(tx, ty), ...] of the fused path for an n_mesh^3 mesh, the default first ([] when the
+    """Column tiles [(tx, ty), ...] of the fused path for an n_mesh^3 mesh, the default (of one grid) first ([] when the
     mesh size has no fused path)."""
     tx, ty, cnt = (C.c_int * 8)(), (C.c_int * 8)(), C.c_int(0)
     st = _lib.load().gbp_column_tile_variants(int(n_mesh), tx, ty, 8, C.byref(cnt))
