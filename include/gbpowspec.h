@@ -96,9 +96,8 @@ typedef struct gbp_deposit_stats {
 } gbp_deposit_stats;
 
 /* flags bit: a tile's bucket outgrew the fixed capacity the one-pass
- * bucketing gives it (a strongly clustered catalogue), so the buckets were
- * rebuilt by a scan and a second scatter; the results are the same, the
- * call took longer. */
+ * bucketing gives it (a strongly clustered catalogue), and its surplus went
+ * through per-tile lists; the results are the same. */
 #define GBP_STATS_REFILLED 1
 
 int gbp_deposit_workspace_size(int64_t n_particles, int n_mesh, int mas,
@@ -291,9 +290,9 @@ int gbp_fft_power(gbp_fft_plan plan, const float* mesh, void* spectrum,
  * binning and the normalisation use) followed by gbp_fft_power; `spectrum`
  * is scratch of the plan's spectrum size.  The particles are bucketed by
  * column tile in one pass into buckets of fixed capacity (twice the mean
- * fill of a uniform catalogue of n_particles, plus 64); a catalogue that
- * overflows one (a dense clump) is re-bucketed by a scan and a second pass
- * in the same call, same results, GBP_STATS_REFILLED in stats_out->flags.
+ * fill of a uniform catalogue of n_particles, plus 64); what overflows one
+ * (a dense clump) goes to lists that the tile collects in the same call, same
+ * results, GBP_STATS_REFILLED in stats_out->flags.
  * Replaces src/mas.py:88-153 + src/correlations.py:7-56 for the production
  * path. */
 int gbp_particles_power_workspace_size(int64_t n_particles, gbp_fft_plan plan,

@@ -33,8 +33,9 @@
 // tile.
 //
 // A block whose densest plane would cost more than SH_MAX bits (a dense
-// clump) sends its whole tile to deposit_fftz_wide_kernel: 64-bit cells, the
-// clumped blocks at the common scale, the others at their own.
+// clump) makes its whole tile wide: 64-bit cells (4x2 or 4x4 pencils at a
+// time in the same shared memory), the clumped blocks at the common scale,
+// the others at their own.
 //
 // Then the y pass (fft.cu) and the x pass fused with the binning (xbin.cu)
 // finish the transform and the P_l sums.  HBM traffic per grid: the
@@ -64,29 +65,32 @@ struct ColTile {
 // packed complex columns: column q = (a, ly) with a = the pencil's x (two
 // grids) or x / 2 (one grid), a = q / UY, ly = q % UY.  Columns 2cp and
 // 2cp + 1 always lie in one scale block.  The unit is the tile where its
-// cells fit UNIT_BYTES, else 4x4 or 4x2 pencils of it.  At 512^3 a unit of
-// 64 KB (512 threads, 64-thread named barriers, two CTAs per SM) beats one
-// of 128 KB in a 1024-thread CTA (0.84 against 0.89 ms for 8x4 tiles of two
-// grids, 4 Mi particles TSC); at 1024^3 4x4 pencils in one CTA beat two
-// visits of the bucket by 4x2 (7.7 against 8.5 ms, 16 Mi PCS).
-template <int N, bool WIDE>
-constexpr size_t UNIT_BYTES = (N == 512 && !WIDE ? 64 : 128) * 1024;
+// cells fit UNIT_BYTES, else 4x4 pencils of it; with 64-bit cells half of
+// that or less.  At 512^3 a unit of 64 KB (512 threads, 64-thread named
+// barriers, two CTAs per SM) beats one of 128 KB in a 1024-thread CTA (0.84
+// against 0.89 ms for 8x4 tiles of two grids, 4 Mi particles TSC); at 1024^3
+// 4x4 pencils in one CTA beat two visits of the bucket by 4x2 (7.7 against
+// 8.5 ms, 16 Mi PCS).
+template <int N>
+constexpr size_t UNIT_BYTES = (N == 512 ? 64 : 128) * 1024;
 
 template <int N, int G, class CT, bool WIDE>
 struct Unit {
-  static constexpr size_t PENCIL = (size_t)N * G * (WIDE ? 8 : 4);       // bytes of a pencil's cells
-  static constexpr bool WHOLE = CT::TX * CT::TY * PENCIL <= UNIT_BYTES<N, WIDE>, SQUARE = 16 * PENCIL <= UNIT_BYTES<N, WIDE>;
-  static constexpr int UX = WHOLE ? CT::TX : 4;
-  static constexpr int UY = WHOLE ? CT::TY : (SQUARE ? 4 : 2);
+  static constexpr size_t PENCIL = (size_t)N * G * sizeof(int);          // bytes of a pencil's 32-bit cells
+  static constexpr bool WHOLE = CT::TX * CT::TY * PENCIL <= UNIT_BYTES<N>;
+  static constexpr int NARROW_X = WHOLE ? CT::TX : 4, NARROW_Y = WHOLE ? CT::TY : 4;
+  static constexpr int UX = WIDE ? 4 : NARROW_X;
+  static constexpr int UY = WIDE ? (NARROW_X * NARROW_Y == 16 ? 2 : 4) : NARROW_Y;
   static constexpr int NUY = CT::TY / UY, NU = (CT::TX / UX) * NUY;      // units per tile
   static constexpr int PAIRS = UX * UY * G / 2;
   static constexpr int SBY = UY >= 4 ? UY / 4 : 1, NSB = UX / 4 * SBY;   // scale blocks it spans
-  static constexpr int NFFT = PAIRS * N / 16;     // butterfly pairs (two columns) per radix-8 stage
+  // threads of the CTA: a butterfly pair (two columns) of the 32-bit unit's radix-8 stages each
+  static constexpr int NFFT = NARROW_X * NARROW_Y * G * N / 32;
   static constexpr int NT = NFFT < 256 ? 256 : NFFT;
   static constexpr int MINB = NT >= 1024 ? 1 : (NT >= 512 ? 2 : 3);   // CTAs per SM the registers are sized for
   static constexpr size_t CELLS = (size_t)2 * PAIRS * N;
-  static constexpr size_t SMEM = CELLS * (WIDE ? 8 : 4) + (WIDE ? 0 : (size_t)CT::NSB * N * 4);  // + plane counts
-  static_assert(CELLS * (WIDE ? 8 : 4) <= UNIT_BYTES<N, WIDE> && NT <= 1024, "a unit fits in shared memory");
+  static constexpr size_t SMEM = CELLS * sizeof(int) + (size_t)CT::NSB * N * sizeof(int);   // + plane counts
+  static_assert(UX * UY * (WIDE ? 2 : 1) <= NARROW_X * NARROW_Y && NT <= 1024, "64-bit cells fit the same bytes");
   // First cell of pencil (lx, ly) of a grid.
   __device__ static __forceinline__ int cell_row(int lx, int ly, int grid) {
     if constexpr (G == 2) return ((lx * UY + ly) * 2 + grid) * N;
@@ -106,10 +110,9 @@ __device__ __forceinline__ T pick_block(int b, const T (&v)[NSB]) {
 // Bits of resolution a block may give up to its 32-bit cells.  A block whose
 // densest z plane is covered by more than 2^(SH_MAX + WBIT) entries (a dense
 // clump: a halo, a point mass) is deposited with 64-bit cells at the common
-// scale instead, by deposit_fftz_wide_kernel: with the coarse quantum the
-// rounding of many identical contributions adds up instead of averaging out.
+// scale instead: with the coarse quantum the rounding of many identical
+// contributions adds up instead of averaging out.
 constexpr int SH_MAX = 10;
-constexpr long long WIDE_MARK = (-0x7fffffffffffffffLL - 1);   // tile_mass entry of a tile left to the wide kernel
 
 // Two grids per pass share the entry loads and need no split of the packed
 // spectra: deposit_fft_z 0.052 -> 0.034 ms (128^3, 1 M particles CIC), 0.135
@@ -121,9 +124,8 @@ constexpr long long WIDE_MARK = (-0x7fffffffffffffffLL - 1);   // tile_mass entr
 // b of the unit (its scale 2^(sg - sh[b]), sh[b] <= SH_MAX).  tm[grid]: the
 // unit's exact totals at the common scale 2^sg (valid in thread 0).
 template <int N, int MAS, int G, class CT, bool WIDE>
-__device__ __forceinline__ void tile_unit(const DepGeom& g, const float4* __restrict__ entries, unsigned beg,
-                                          unsigned end, int sg, const int (&sh)[Unit<N, G, CT, WIDE>::NSB], int x0, int y0,
-                                          int kz_cols, const float2* __restrict__ tw, float2* __restrict__ spec,
+__device__ __forceinline__ void tile_unit(const DepGeom& g, const TileEntries& te, int sg, const int (&sh)[Unit<N, G, CT, WIDE>::NSB],
+                                          int x0, int y0, int kz_cols, const float2* __restrict__ tw, float2* __restrict__ spec,
                                           unsigned char* smem, long long (*s_part)[G], long long (&tm)[G]) {
   using Cell = typename std::conditional<WIDE, unsigned long long, int>::type;
   using U = Unit<N, G, CT, WIDE>;
@@ -146,8 +148,12 @@ __device__ __forceinline__ void tile_unit(const DepGeom& g, const float4* __rest
     for (int k = tid; k < (int)(U::CELLS * sizeof(Cell) / 16); k += NT) a4[k] = make_uint4(0u, 0u, 0u, 0u);
   }
   __syncthreads();
-  for (unsigned i = beg + tid; i < end; i += NT) {
-    const float4 e = entries[i];
+#pragma unroll 1
+  for (int q = 0; q < 2; ++q) {
+  const float4* ep = q ? te.p[1] : te.p[0];
+  const unsigned en = q ? te.n[1] : te.n[0];
+  for (unsigned i = tid; i < en; i += NT) {
+    const float4 e = ep[i];
 #pragma unroll
     for (int grid = 0; grid < G; ++grid) {
       Axis<R> ax, ay, az;
@@ -205,6 +211,7 @@ __device__ __forceinline__ void tile_unit(const DepGeom& g, const float4* __rest
       }
     }
   }
+  }
   __syncthreads();
 
   // z transform: a thread transforms columns 2cp and 2cp+1 (one scale block), the same column pair in
@@ -242,7 +249,7 @@ __device__ __forceinline__ void tile_unit(const DepGeom& g, const float4* __rest
   // (the first stage's writes alias the pair's own pencils), so the stages synchronise 64-thread
   // groups only.  64-bit cells span twice the bytes of the complex slots: whole-CTA barriers.
   constexpr int GS = (!WIDE && N == 512 && NT == PAIRS / 2 * (N / 8) && NT / (N / 8) <= fft::MAX_GROUPS) ? N / 8 : 0;
-  static_assert(U::NFFT <= NT, "one first-stage butterfly per thread");
+  static_assert(PAIRS * N / 16 <= NT, "one first-stage butterfly per thread");
   fft::run_stages2<N, PAIRS / 2, NT, true, true, false, decltype(gin), decltype(sin_), decltype(sout), decltype(gout),
                    GS>(gin, sin_, sout, gout, tw, tid);
   // the unit's exact totals
@@ -263,11 +270,10 @@ __device__ __forceinline__ void tile_unit(const DepGeom& g, const float4* __rest
 
 // Every unit of a tile; writes the tile's totals.  sh: the shifts of the tile's scale blocks.
 template <int N, int MAS, int G, class CT, bool WIDE>
-__device__ __forceinline__ void tile_units(const DepGeom& g, const float4* __restrict__ entries, unsigned beg,
-                                           unsigned end, int sg, const int (&sh)[CT::NSB], int x0, int y0, int kz_cols,
-                                           const float2* __restrict__ tw, float2* __restrict__ spec,
-                                           unsigned char* smem, long long (*s_part)[G], long long* tile_mass,
-                                           int ntiles, int t) {
+__device__ __forceinline__ void tile_units(const DepGeom& g, const TileEntries& te, int sg, const int (&sh)[CT::NSB],
+                                           int x0, int y0, int kz_cols, const float2* __restrict__ tw,
+                                           float2* __restrict__ spec, unsigned char* smem, long long (*s_part)[G],
+                                           long long* tile_mass, int ntiles, int t) {
   using U = Unit<N, G, CT, WIDE>;
   long long total[G];
 #pragma unroll
@@ -284,17 +290,31 @@ __device__ __forceinline__ void tile_units(const DepGeom& g, const float4* __res
       for (int b = 0; b < U::NSB; ++b) shu[b] = sh[b];
     }
     long long tm[G];
-    tile_unit<N, MAS, G, CT, WIDE>(g, entries, beg, end, sg, shu, x0 + ux, y0 + uy, kz_cols, tw, spec, smem, s_part,
+    tile_unit<N, MAS, G, CT, WIDE>(g, te, sg, shu, x0 + ux, y0 + uy, kz_cols, tw, spec, smem, s_part,
                                    tm);
     if (threadIdx.x == 0) {
 #pragma unroll
       for (int q = 0; q < G; ++q) total[q] += tm[q];
     }
   }
-  if (threadIdx.x == 0) {                              // replaces a wide tile's mark and shifts
+  if (threadIdx.x == 0) {
     tile_mass[t] = total[0];
     tile_mass[(long long)ntiles + t] = G == 2 ? total[G - 1] : 0;
   }
+}
+
+// The same with 64-bit cells, out of line: tiles of dense clumps are rare,
+// and inlined their code would cost the others registers.  packed: 8 bits of
+// shift per scale block.
+template <int N, int MAS, int G, class CT>
+__device__ __noinline__ void tile_units_wide(const DepGeom& g, TileEntries te, int sg, unsigned packed, int x0, int y0,
+                                             int kz_cols, const float2* __restrict__ tw, float2* __restrict__ spec,
+                                             unsigned char* smem, long long (*s_part)[G], long long* tile_mass,
+                                             int ntiles, int t) {
+  int sh[CT::NSB];
+#pragma unroll
+  for (int b = 0; b < CT::NSB; ++b) sh[b] = (int)((packed >> (8 * b)) & 0xffu);
+  tile_units<N, MAS, G, CT, true>(g, te, sg, sh, x0, y0, kz_cols, tw, spec, smem, s_part, tile_mass, ntiles, t);
 }
 
 // Per-block plane counts of a tile (zc [NSB][N], zeroed on entry) and the
@@ -303,22 +323,26 @@ __device__ __forceinline__ void tile_units(const DepGeom& g, const float4* __res
 // plane z when its nodes (any grid) reach b's 4 x-columns, its 4 y-columns
 // and z.
 template <int N, int MAS, int G, class CT>
-__device__ __forceinline__ bool block_scales(const DepGeom& g, const float4* __restrict__ entries, unsigned beg,
-                                             unsigned end, int x0, int y0, int* zc, int* s_max, int (&sh)[CT::NSB]) {
+__device__ __forceinline__ bool block_scales(const DepGeom& g, const TileEntries& te, int x0, int y0, int* zc,
+                                             int* s_max, int (&sh)[CT::NSB]) {
   constexpr int R = MAS, NT = Unit<N, G, CT, false>::NT, NSB = CT::NSB, W = R + G - 1;
   const int tid = threadIdx.x;
   // this pass is the tile's first touch of its bucket: a thread issues EB entry loads at once
   constexpr int EB = 4;
-  for (unsigned i0 = beg + tid; i0 < end; i0 += EB * NT) {
+#pragma unroll 1
+  for (int q = 0; q < 2; ++q) {
+  const float4* ep = q ? te.p[1] : te.p[0];
+  const unsigned en = q ? te.n[1] : te.n[0];
+  for (unsigned i0 = tid; i0 < en; i0 += EB * NT) {
     float4 ev[EB];
 #pragma unroll
     for (int k = 0; k < EB; ++k) {
       const unsigned i = i0 + k * NT;
-      ev[k] = i < end ? entries[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      ev[k] = i < en ? ep[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
     for (int k = 0; k < EB; ++k) {
-      if (i0 + k * NT >= end) break;
+      if (i0 + k * NT >= en) break;
       const float4 e = ev[k];
       // the union of the grids' nodes along each axis: first .. last (the second grid's first node
       // is the first grid's or the next one), as the bucketing counts them.  Every entry of the
@@ -361,6 +385,7 @@ __device__ __forceinline__ bool block_scales(const DepGeom& g, const float4* __r
             for (int zn = first[2]; zn <= last[2]; ++zn) atomicAdd(&zc[(bx * CT::SBY + by) * N + wrapn(zn, N)], 1);
     }
   }
+  }
   __syncthreads();
   // a node weight of TSC (<= 0.75^3) or PCS (<= (2/3)^3) is below 1/2: one more bit
   constexpr int WBIT = (MAS == GBP_TSC || MAS == GBP_PCS) ? 1 : 0;
@@ -385,8 +410,8 @@ __device__ __forceinline__ bool block_scales(const DepGeom& g, const float4* __r
 
 template <int N, int MAS, int G, class CT>
 __global__ void __launch_bounds__(Unit<N, G, CT, false>::NT, Unit<N, G, CT, false>::MINB)
-deposit_fftz_kernel(DepGeom g, const float4* __restrict__ entries, const unsigned* __restrict__ counts,
-                    const unsigned* __restrict__ offsets, const DepCounters* ctr, int kz_cols,
+deposit_fftz_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ entries, const unsigned* __restrict__ counts,
+                    const unsigned* __restrict__ offsets, const __grid_constant__ Spill sp, DepCounters* ctr, int kz_cols,
                     const float2* __restrict__ tw, float2* __restrict__ spec, long long* __restrict__ tile_mass) {
   pdl_wait();
   using U = Unit<N, G, CT, false>;
@@ -399,75 +424,22 @@ deposit_fftz_kernel(DepGeom g, const float4* __restrict__ entries, const unsigne
   const int t = blockIdx.x;
   const int ty = t % g.nt[1], tx = t / g.nt[1];
   const int x0 = tx * CT::TX, y0 = ty * CT::TY;
-  unsigned beg, end;
-  tile_range(g, t, counts, offsets, ctr, beg, end);
+  const TileEntries te = tile_entries(g, t, entries, counts, offsets, sp, ctr);
   const int sg = fixed_scale_exp(ctr->maxw_bits, 0);
   for (int k = tid; k < NSB * N; k += NT) zc[k] = 0;
   __syncthreads();
   int sh[NSB];
-  if (block_scales<N, MAS, G, CT>(g, entries, beg, end, x0, y0, zc, s_max, sh)) {
-    // a dense clump: the wide kernel takes this tile (the clumped blocks at the common scale)
-    if (tid == 0) {
-      long long packed = 0;
-      for (int b = 0; b < NSB; ++b) packed |= (long long)(sh[b] > SH_MAX ? 0 : sh[b]) << (8 * b);
-      tile_mass[t] = WIDE_MARK;
-      tile_mass[(long long)gridDim.x + t] = packed;    // the second grid's slot is free until the wide kernel
-    }
-    return;
-  }
-  tile_units<N, MAS, G, CT, false>(g, entries, beg, end, sg, sh, x0, y0, kz_cols, tw, spec,
-                                   reinterpret_cast<unsigned char*>(acc_smem), s_part, tile_mass, (int)gridDim.x, t);
-}
-
-// The tiles deposit_fftz_kernel left (tile_mass entry WIDE_MARK, the
-// blocks' shifts packed in the second slot): 64-bit cells.  Persistent:
-// CTA b owns a contiguous range of tiles, finds its marked ones with one
-// parallel scan (such tiles are rare; with none, that scan is all a CTA
-// does) and processes them in turn.
-constexpr int WIDE_LIST = 64;                          // marked tiles listed per scan round
-
-template <int N, int MAS, int G, class CT>
-__global__ void __launch_bounds__(Unit<N, G, CT, true>::NT, Unit<N, G, CT, true>::MINB)
-deposit_fftz_wide_kernel(DepGeom g, const float4* __restrict__ entries, const unsigned* __restrict__ counts,
-                         const unsigned* __restrict__ offsets, const DepCounters* ctr, int kz_cols,
-                         const float2* __restrict__ tw, float2* __restrict__ spec, long long* __restrict__ tile_mass,
-                         int ntiles) {
-  pdl_wait();
-  constexpr int NT = Unit<N, G, CT, true>::NT, NSB = CT::NSB;
-  extern __shared__ __align__(16) unsigned long long wide_smem[];
-  __shared__ long long s_part[NT / 32][G];
-  __shared__ int s_list[WIDE_LIST];
-  __shared__ int s_n;
-  const int sg = fixed_scale_exp(ctr->maxw_bits, 0);
-  const int per = (ntiles + gridDim.x - 1) / gridDim.x;
-  const int t0 = blockIdx.x * per, t1 = min(ntiles, t0 + per);
-  for (int base = t0; base < t1; base += NT) {
-    for (;;) {                                         // list the marked tiles of [base, base + NT), 64 at a time
-      if (threadIdx.x == 0) s_n = 0;
-      __syncthreads();
-      const int t = base + (int)threadIdx.x;
-      if (t < t1 && tile_mass[t] == WIDE_MARK) {
-        const int k = atomicAdd(&s_n, 1);
-        if (k < WIDE_LIST) s_list[k] = t;
-      }
-      __syncthreads();
-      const int n = min(s_n, WIDE_LIST);
-      if (n == 0) break;                               // uniform over the CTA
-      for (int k = 0; k < n; ++k) {
-        const int tt = s_list[k];
-        const int ty = tt % g.nt[1], tx = tt / g.nt[1];
-        unsigned beg, end;
-        tile_range(g, tt, counts, offsets, ctr, beg, end);
-        const long long packed = tile_mass[(long long)ntiles + tt];
-        int sh[NSB];
+  const bool heavy = block_scales<N, MAS, G, CT>(g, te, x0, y0, zc, s_max, sh);
+  unsigned char* cells = reinterpret_cast<unsigned char*>(acc_smem);
+  if (heavy) {                                         // uniform over the CTA
+    unsigned packed = 0;
 #pragma unroll
-        for (int b = 0; b < NSB; ++b) sh[b] = (int)((packed >> (8 * b)) & 0xff);
-        __syncthreads();                               // every thread has read the shifts before they are replaced
-        tile_units<N, MAS, G, CT, true>(g, entries, beg, end, sg, sh, tx * CT::TX, ty * CT::TY, kz_cols, tw, spec,
-                                        reinterpret_cast<unsigned char*>(wide_smem), s_part, tile_mass, ntiles, tt);
-      }
-      __syncthreads();                                 // the marks are replaced before the next scan
-    }
+    for (int b = 0; b < NSB; ++b) packed |= (unsigned)(sh[b] > SH_MAX ? 0 : sh[b]) << (8 * b);
+    tile_units_wide<N, MAS, G, CT>(g, te, sg, packed, x0, y0, kz_cols, tw, spec, cells, s_part, tile_mass,
+                                   (int)gridDim.x, t);
+  } else {
+    tile_units<N, MAS, G, CT, false>(g, te, sg, sh, x0, y0, kz_cols, tw, spec, cells, s_part, tile_mass,
+                                     (int)gridDim.x, t);
   }
 }
 
@@ -492,28 +464,15 @@ template <int N, int MAS, int G, class CT>
 int run_fused(const DepGeom& g, const DepLayout& L, const DepBuffers& b, int kz_cols, const float2* tw, float2* spec,
               cudaStream_t st) {
   using U = Unit<N, G, CT, false>;
-  using UW = Unit<N, G, CT, true>;
   int r = bucket_particles<MAS, G, 0>(g, L, b, st);
   if (r) return r;
   auto k = deposit_fftz_kernel<N, MAS, G, CT>;
   GBP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)U::SMEM));
   {
     GBP_TRACE("deposit_fft_z", st);
-    GBP_CUDA_TRY(launch_pdl(k, dim3(L.ntiles), dim3(U::NT), U::SMEM, st, g, b.entries, b.counts, b.offsets, b.ctr,
-                            kz_cols, tw, spec, b.tile_mass));
+    GBP_CUDA_TRY(launch_pdl(k, dim3(L.ntiles), dim3(U::NT), U::SMEM, st, g, b.entries, b.counts, b.offsets, b.spill,
+                            b.ctr, kz_cols, tw, spec, b.tile_mass));
   }
-  // tiles of dense clumps, if any, with 64-bit cells (as many CTAs as fit at once scan the marks: a
-  // dense small mesh can send most of its tiles here)
-  auto kw = deposit_fftz_wide_kernel<N, MAS, G, CT>;
-  GBP_CUDA_TRY(cudaFuncSetAttribute(kw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)UW::SMEM));
-  int dev = 0, sms = 0, per_sm = 0;
-  GBP_CUDA_TRY(cudaGetDevice(&dev));
-  GBP_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  GBP_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kw, UW::NT, UW::SMEM));
-  GBP_TRACE("deposit_fft_z_wide", st);
-  GBP_CUDA_TRY(launch_pdl(kw, dim3(std::max(1, std::min(sms * std::max(per_sm, 1), L.ntiles))), dim3(UW::NT),
-                          UW::SMEM, st, g, b.entries, b.counts, b.offsets, b.ctr, kz_cols, tw, spec,
-                          b.tile_mass, L.ntiles));
   return GBP_OK;
 }
 

@@ -18,10 +18,10 @@
 //                      the mesh exactly once.
 //   5. stats_kernel    folds the per-block partial sums in a fixed order.
 //
-// With enough particles per tile, passes 1-3 are one: fill_kernel gives
-// each tile a bucket of fixed capacity and writes every entry at the slot
-// its count atomic returns; scan and scatter (from those counts) run only if
-// a bucket overflowed (deposit_core.cuh, deposit_layout).
+// Passes 1-3 are one unless a large mesh holds few particles: fill_kernel
+// gives each tile a bucket of fixed capacity and writes every entry at the
+// slot its count atomic returns, or on the tile's spill lists when the bucket
+// is full (deposit_core.cuh, deposit_layout).
 //
 // Integer accumulation makes each cell's sum independent of particle order
 // and scheduling, so the mesh is bitwise reproducible; no float atomics are
@@ -43,8 +43,9 @@ namespace {
 // sums are exact whatever the order of the adds.
 template <int MAS, int G, int CM>
 __global__ void __launch_bounds__(DEP_THREADS)
-deposit_kernel(DepGeom g, const float4* __restrict__ entries, const unsigned* __restrict__ counts,
-               const unsigned* __restrict__ offsets, const DepCounters* ctr, const float* __restrict__ mesh_in,
+deposit_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ entries, const unsigned* __restrict__ counts,
+               const unsigned* __restrict__ offsets, const __grid_constant__ Spill sp, DepCounters* ctr,
+               const float* __restrict__ mesh_in,
                float* __restrict__ mesh_out, long long* __restrict__ tile_mass) {
   pdl_wait();
   constexpr int R = Scheme<MAS, CM>::R;
@@ -57,8 +58,7 @@ deposit_kernel(DepGeom g, const float4* __restrict__ entries, const unsigned* __
   const int x0 = tx * g.td[0], y0 = ty * g.td[1], z0 = tz * g.td[2];
   const int ex = min(g.td[0], g.N - x0), ey = min(g.td[1], g.N - y0), ez = min(g.td[2], g.N - z0);
 
-  unsigned beg, end;
-  tile_range(g, t, counts, offsets, ctr, beg, end);
+  const TileEntries te = tile_entries(g, t, entries, counts, offsets, sp, ctr);
   const int s = fixed_scale_exp(ctr->maxw_bits, CM);
   const float sc = ldexpf(1.0f, s);
   const float inv_sc = ldexpf(1.0f, -s);
@@ -72,8 +72,12 @@ deposit_kernel(DepGeom g, const float4* __restrict__ entries, const unsigned* __
       for (int k = threadIdx.x; k < 2 * TILE3 / 4; k += DEP_THREADS) a4[k] = make_uint4(0u, 0u, 0u, 0u);
     }
     __syncthreads();
-    for (unsigned i = beg + threadIdx.x; i < end; i += DEP_THREADS) {
-      const float4 e = entries[i];
+#pragma unroll 1
+    for (int q = 0; q < 2; ++q) {
+    const float4* ep = q ? te.p[1] : te.p[0];
+    const unsigned en = q ? te.n[1] : te.n[0];
+    for (unsigned i = threadIdx.x; i < en; i += DEP_THREADS) {
+      const float4 e = ep[i];
       Axis<R> ax, ay, az;
       make_axis<MAS, CM>(g, e.x, grid, ax);
       make_axis<MAS, CM>(g, e.y, grid, ay);
@@ -113,6 +117,7 @@ deposit_kernel(DepGeom g, const float4* __restrict__ entries, const unsigned* __
           }
         }
       }
+    }
     }
     __syncthreads();
 
@@ -162,8 +167,7 @@ deposit_kernel(DepGeom g, const float4* __restrict__ entries, const unsigned* __
   }
 }
 
-// Buckets of a fixed capacity filled in one pass (count, scan and scatter
-// only when one overflows), as on the fused path.
+// Buckets of a fixed capacity filled in one pass, as on the fused path.
 constexpr bool kMeshFill = true;
 
 template <int MAS, int G, int CM>
@@ -177,7 +181,7 @@ int run_scheme(const DepGeom& g, const DepLayout& L, const DepBuffers& b, const 
                                     (int)smem));
   GBP_TRACE("deposit_tiles", st);
   GBP_CUDA_TRY(launch_pdl(deposit_kernel<MAS, G, CM>, dim3(L.ntiles), dim3(DEP_THREADS), smem, st, g, b.entries,
-                          b.counts, b.offsets, b.ctr, mesh_in, mesh_out, b.tile_mass));
+                          b.counts, b.offsets, b.spill, b.ctr, mesh_in, mesh_out, b.tile_mass));
   return GBP_OK;
 }
 

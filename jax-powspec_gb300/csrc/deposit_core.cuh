@@ -245,8 +245,20 @@ __device__ __forceinline__ ff warp_ff_sum(ff v) {
 
 struct DepCounters {           // zeroed by one memset per call
   unsigned int maxw_bits;
-  unsigned int overflow;       // fill path: some tile has more entries than its bucket holds
-  unsigned int pad_[2];
+  unsigned int n_spill;        // fill path: entries beyond their bucket's capacity
+  unsigned int n_extra;        // spilled entries listed by their tiles so far (tile_entries)
+  unsigned int pad_;
+};
+
+// Fill path: the entries beyond a bucket's capacity.  Entry s is particle
+// node[s].x of tile tile[s]; heads holds HEADS lists per tile of them
+// (node index + 1, 0 ends a list), linked through node[s].y.
+constexpr unsigned HEADS = CSTRIDE;
+struct Spill {
+  unsigned* heads;      // [ntiles * HEADS], zeroed
+  uint2* node;          // [n * maxrep]
+  unsigned* tile;       // [n * maxrep]
+  float4* extra;        // [n * maxrep] (u, w) of the tiles that gathered theirs
 };
 
 // Block reductions of the weight statistics in a fixed order (deterministic
@@ -320,15 +332,25 @@ count_kernel(DepGeom gp, unsigned* __restrict__ counts, DepCounters* ctr, float4
 // Passes 1 and 3 at once (fill path: buckets of a fixed capacity g.tcap, tile
 // t's at entry t * tcap).  The count of tile t that a particle's atomic
 // returns is also its slot in t's bucket, so the entry is written right away;
-// a slot beyond the capacity is not written and raises ctr->overflow, after
-// which the scan and scatter passes (they run only then) rebuild all buckets
-// packed, from these counts: every attempt was counted.  The statistics are
-// those of count_kernel, over the same particle blocks.  Registers for 5
-// CTAs per SM: its returning atomics want warps in flight (0.151 -> 0.142 ms
-// for 4 Mi particles at 512^3 against 4 CTAs per SM).
+// a slot beyond the capacity puts the particle on one of the tile's spill
+// lists instead, which the tile's CTA collects (tile_entries), so a clump
+// costs its own tile and no second pass over the catalogue (a scan and a
+// scatter that rebuilt all buckets cost 0.15 of the 0.57 ms of a clustered
+// 4 Mi particle 512^3 CIC deposit, now 0.43, and two idle launches when
+// nothing overflowed).  The statistics are those of count_kernel, over the
+// same particle blocks.
+// Registers for 5 CTAs per SM: its returning atomics want warps in flight
+// (0.151 -> 0.142 ms for 4 Mi particles at 512^3 against 4 CTAs per SM).
+__device__ __forceinline__ void spill_entry(const Spill& sp, DepCounters* ctr, int t, int k) {
+  const unsigned i = blockIdx.x * (CNT_THREADS * CNT_ITEMS) + k * CNT_THREADS + threadIdx.x;   // as load_batch
+  const unsigned s = atomicAdd(&ctr->n_spill, 1u);
+  sp.tile[s] = (unsigned)t;
+  sp.node[s] = make_uint2(i, atomicExch(&sp.heads[(size_t)t * HEADS + (s & (HEADS - 1))], s + 1u));
+}
+
 template <int MAS, int G, int CM>
 __global__ void __launch_bounds__(CNT_THREADS, 5)
-fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entries, DepCounters* ctr,
+fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entries, Spill sp, DepCounters* ctr,
             float4* block_stats, uint2* block_counts) {
   pdl_wait();
   DepGeom g = gp;
@@ -337,7 +359,6 @@ fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entr
   float maxw = 0.0f;
   ff sw{0.f, 0.f}, sw2{0.f, 0.f};
   unsigned kept = 0, bad = 0;
-  bool over = false;
   Batch bt;
   load_batch(g, bt, blockIdx.x);
 #pragma unroll
@@ -370,7 +391,7 @@ fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entr
       for (int q = 0; q < 8; ++q)
         if (tt[q] >= 0) {
           if (slot[q] < tcap) entries[(unsigned)tt[q] * tcap + slot[q]] = e;
-          else over = true;
+          else spill_entry(sp, ctr, tt[q], k);
         }
     } else {
       for (int a = 0; a < nx; ++a)
@@ -379,76 +400,85 @@ fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entr
             const int t = (pick3(a, x0, x1, x2) * g.nt[1] + pick3(b, y0, y1, y2)) * g.nt[2] + pick3(c, z0, z1, z2);
             const unsigned slot = atomicAdd(&counts[t * CSTRIDE], 1u);
             if (slot < tcap) entries[(unsigned)t * tcap + slot] = e;
-            else over = true;
+            else spill_entry(sp, ctr, t, k);
           }
     }
     maxw = fmaxf(maxw, fabsf(w));
     sw = ff_add_f(sw, w);
     sw2 = ff_add_f(sw2, __fmul_rn(w, w));
   }
-  if (over) atomicOr(&ctr->overflow, 1u);
   flush_block_stats(maxw, sw, sw2, kept, bad, ctr, block_stats, block_counts);
 }
 
-// Pass 2 of the fill path, run only when a bucket overflowed (one CTA:
-// otherwise it returns at once): exclusive scan of the tile counts.
-constexpr int FSCAN_THREADS = 1024;
-__global__ void __launch_bounds__(FSCAN_THREADS)
-gated_scan_kernel(const unsigned* __restrict__ counts, unsigned* __restrict__ offsets, int ntiles,
-                  const DepCounters* ctr) {
-  pdl_wait();
-  if (ctr->overflow == 0u) return;
-  __shared__ unsigned s_warp[FSCAN_THREADS / 32];
-  const int per = (ntiles + FSCAN_THREADS - 1) / FSCAN_THREADS;
-  const int a = min(ntiles, (int)threadIdx.x * per), b = min(ntiles, a + per);
-  unsigned sum = 0;
-  for (int i = a; i < b; ++i) sum += counts[(long long)i * CSTRIDE];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  unsigned inc = sum;                                  // inclusive scan within the warp
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned v = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += v;
+// The entries of one tile in two parts: n[0] in its bucket, n[1] beyond its
+// capacity (fill path).  Loops over a tile's entries take the parts in turn:
+// the rare second one costs the first nothing per entry.
+struct TileEntries {
+  const float4* p[2];
+  unsigned n[2];
+};
+
+// Collects a tile's n spilled particles into a slice of `extra` of its own
+// (every thread of the block calls).  One warp walks the tile's HEADS lists;
+// a tile that holds more than 64 entries per list and a sixteenth of all
+// spilled ones (a point mass) has the block look through them all instead.
+__device__ __noinline__ const float4* gather_spilled(const DepGeom& gp, const Spill& sp, DepCounters* ctr, int t,
+                                                     unsigned n) {
+  __shared__ unsigned s_base, s_n;
+  if (threadIdx.x == 0) {
+    s_base = atomicAdd(&ctr->n_extra, n);
+    s_n = 0;
   }
-  if (lane == 31) s_warp[wid] = inc;
   __syncthreads();
-  if (wid == 0) {
-    unsigned v = s_warp[lane], w = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned u = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += u;
+  float4* out = sp.extra + s_base;
+  DepGeom g = gp;
+  resolve_job(g);
+  auto put = [&](unsigned i) {
+    const unsigned q = atomicAdd(&s_n, 1u);
+    float u[3];
+    grid_coords(g, g.x[i], g.y[i], g.z[i], u);
+    if (q < n) out[q] = make_float4(u[0], u[1], u[2], g.w ? g.w[i] : 1.0f);
+  };
+  const unsigned all = ctr->n_spill;
+  if (n > 64 * HEADS && n > all / 16) {
+    for (unsigned k = threadIdx.x; k < all; k += blockDim.x)
+      if (sp.tile[k] == (unsigned)t) put(sp.node[k].x);
+  } else if (threadIdx.x < HEADS) {
+    unsigned v = sp.heads[(size_t)t * HEADS + threadIdx.x];
+    for (unsigned k = 0; v != 0u && k < n; ++k) {
+      const uint2 nd = sp.node[v - 1u];
+      put(nd.x);
+      v = nd.y;
     }
-    s_warp[lane] = w - v;                              // exclusive prefix of the warp totals
   }
   __syncthreads();
-  unsigned run = s_warp[wid] + inc - sum;
-  for (int i = a; i < b; ++i) {
-    offsets[i] = run;
-    run += counts[(long long)i * CSTRIDE];
-  }
+  return out;
 }
 
-// First entry and end of tile t's bucket: fixed-capacity buckets unless the
-// fill path overflowed (then, as on the count path, packed at the scanned
-// offsets); the counts are the same on both paths.
-__device__ __forceinline__ void tile_range(const DepGeom& g, int t, const unsigned* counts, const unsigned* offsets,
-                                           const DepCounters* ctr, unsigned& beg, unsigned& end) {
+// Every thread of the block calls; ends with the list complete.
+__device__ __forceinline__ TileEntries tile_entries(const DepGeom& g, int t, const float4* entries,
+                                                    const unsigned* counts, const unsigned* offsets, const Spill& sp,
+                                                    DepCounters* ctr) {
+  TileEntries te;
   const unsigned c = counts[(long long)t * CSTRIDE];
-  beg = (g.tcap && ctr->overflow == 0u) ? (unsigned)t * g.tcap : offsets[t];
-  end = beg + c;
+  te.n[0] = g.tcap ? min(c, g.tcap) : c;
+  te.n[1] = c - te.n[0];
+  te.p[0] = entries + (g.tcap ? (size_t)t * g.tcap : (size_t)offsets[t]);
+  te.p[1] = te.n[1] ? gather_spilled(g, sp, ctr, t, te.n[1]) : te.p[0];
+  return te;
 }
 
 // Pass 3: append (u_x, u_y, u_z, w) to every touched tile's bucket.
 template <int MAS, int G, int CM>
 __global__ void __launch_bounds__(CNT_THREADS, 4)
 scatter_kernel(DepGeom gp, const unsigned* __restrict__ offsets, unsigned* __restrict__ fills,
-               float4* __restrict__ entries, const DepCounters* gate) {
+               float4* __restrict__ entries) {
   pdl_wait();
-  if (gate && gate->overflow == 0u) return;            // fill path: the buckets are complete
   DepGeom g = gp;
   resolve_job(g);
-  for (long long blk = blockIdx.x; blk * (CNT_THREADS * CNT_ITEMS) < g.n; blk += gridDim.x) {
+  {
     Batch bt;
-    load_batch(g, bt, blk);
+    load_batch(g, bt, blockIdx.x);
 #pragma unroll
     for (int k = 0; k < CNT_ITEMS; ++k) {
       if (!bt.in[k]) continue;
@@ -601,7 +631,7 @@ stats_kernel(const DepCounters* ctr, const float4* block_stats, const uint2* blo
     out->n_kept = tk;
     out->n_nonfinite = tbad;
     out->scale_exp = s;
-    out->flags = ctr->overflow ? GBP_STATS_REFILLED : 0;
+    out->flags = ctr->n_spill ? GBP_STATS_REFILLED : 0;
   }
 }
 
@@ -609,16 +639,14 @@ struct DepLayout {
   int td[3], ts[3], nt[3], ntiles, maxrep, nblocks;
   unsigned tcap;        // fill path: entries per bucket (0: count path)
   size_t nentries;      // entries the bucket buffer holds
+  size_t nspill;        // fill path: entries that may lie beyond their buckets
   size_t scan_bytes;
   size_t total;
 };
 
-// Blocks of the fill path's fallback scatter (a grid-stride loop; when no
-// bucket overflowed they return at once).
-constexpr int FILL_SCATTER_BLOCKS = 1216;
-
 // Bytes at the start of the workspace that one memset clears per call: the
-// counters, the tiles' entry counts and their fill counters (adjacent).
+// counters, the tiles' entry counts and their fill counters or spill list
+// heads (adjacent).
 inline size_t zeroed_bytes(const DepLayout& L) {
   return align256(sizeof(DepCounters)) + 2 * align256((size_t)L.ntiles * CSTRIDE * sizeof(unsigned));
 }
@@ -653,9 +681,9 @@ int max_tiles_axis(int N, int tdim, int width) {
 // to the bucket of each tile its stencil (all grids) touches.  fill: buckets
 // of a fixed capacity, twice the mean fill m of a uniform catalogue of n
 // particles plus 64 (a span of `width` nodes reaches the next tile along an
-// axis with probability (width - 1) / td), so that one pass fills them
-// unless the catalogue is strongly clustered; the count path when m < 32
-// (few particles per tile: small buffers matter more than the pass).  Wider
+// axis with probability (width - 1) / td), so that spills are rare unless the
+// catalogue is strongly clustered; the count path when m < 32 and the buckets
+// would still take more than 256 MB (a large mesh with few particles).  Wider
 // buckets cost the one pass time: the same entries written over a larger
 // range (3 m + 64 instead of 2 m + 64: 0.169 against 0.147 ms for 4 Mi
 // particles at 512^3).
@@ -683,23 +711,26 @@ int deposit_layout(int64_t n, int N, int mas, int interlace, int compat, const i
   L.nblocks = (int)((n + (long long)CNT_THREADS * CNT_ITEMS - 1) / ((long long)CNT_THREADS * CNT_ITEMS));
   L.tcap = 0;
   L.nentries = (size_t)n * L.maxrep + 1;
+  L.nspill = 0;
   if (fill && n > 0) {
     double rep = 1.0;
     for (int a = 0; a < 3; ++a)
       if (L.td[a] < N) rep *= 1.0 + (double)(width - 1) / (double)L.td[a];
     const double mean = (double)n * rep / (double)L.ntiles;
     const double cap = 4.0 * std::ceil((2.0 * mean + 64.0) / 4.0);
-    if (mean >= 32.0 && cap * (double)L.ntiles < 4294967295.0) {
+    if ((mean >= 32.0 || cap * (double)L.ntiles <= 16777216.0) && cap * (double)L.ntiles < 4294967295.0) {
       L.tcap = (unsigned)cap;
-      L.nentries = std::max(L.nentries, (size_t)L.tcap * (size_t)L.ntiles + 1);
+      L.nspill = L.nentries;
+      L.nentries = (size_t)L.tcap * (size_t)L.ntiles + 1;
     }
   }
   L.scan_bytes = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, L.scan_bytes, strided_counts(nullptr), (unsigned*)nullptr, L.ntiles);
+  if (!L.tcap) cub::DeviceScan::ExclusiveSum(nullptr, L.scan_bytes, strided_counts(nullptr), (unsigned*)nullptr, L.ntiles);
   const size_t nbl = (size_t)(L.nblocks > 0 ? L.nblocks : 1);
   L.total = zeroed_bytes(L) + align256((size_t)L.ntiles * 4) + align256(nbl * sizeof(float4)) +
             align256(nbl * sizeof(uint2)) + align256((size_t)L.ntiles * 2 * sizeof(long long)) +
-            align256(L.nentries * sizeof(float4)) + align256(L.scan_bytes);
+            align256(L.nentries * sizeof(float4)) + align256(L.scan_bytes) + align256(L.nspill * sizeof(uint2)) +
+            align256(L.nspill * sizeof(unsigned)) + align256(L.nspill * sizeof(float4));
   return GBP_OK;
 }
 
@@ -707,13 +738,14 @@ int deposit_layout(int64_t n, int N, int mas, int interlace, int compat, const i
 struct DepBuffers {
   DepCounters* ctr;
   unsigned* counts;      // [ntiles * CSTRIDE] entries per tile (count pass)
-  unsigned* fills;       // [ntiles * CSTRIDE] entries written so far (scatter pass)
+  unsigned* fills;       // [ntiles * CSTRIDE] entries written so far (count path's scatter)
   unsigned* offsets;     // [ntiles] first entry of each tile (exclusive scan of the counts)
   float4* block_stats;
   uint2* block_counts;
   long long* tile_mass;
   float4* entries;
   void* scan_tmp;
+  Spill spill;           // fill path (its heads share the bytes of fills)
 };
 
 inline DepBuffers carve_deposit(void* workspace, const DepLayout& L) {
@@ -729,6 +761,10 @@ inline DepBuffers carve_deposit(void* workspace, const DepLayout& L) {
   b.tile_mass = cv.take<long long>((size_t)L.ntiles * 2);
   b.entries = cv.take<float4>(L.nentries);
   b.scan_tmp = cv.take<char>(L.scan_bytes);
+  b.spill.heads = b.fills;
+  b.spill.node = cv.take<uint2>(L.nspill);
+  b.spill.tile = cv.take<unsigned>(L.nspill);
+  b.spill.extra = cv.take<float4>(L.nspill);
   return b;
 }
 
@@ -737,22 +773,10 @@ inline DepBuffers carve_deposit(void* workspace, const DepLayout& L) {
 template <int MAS, int G, int CM>
 int bucket_particles(const DepGeom& g, const DepLayout& L, const DepBuffers& b, cudaStream_t st) {
   if (L.tcap) {
-    // fill path: one pass; the scan and the scatter return at once unless a bucket overflowed
     if (L.nblocks > 0) {
       GBP_TRACE("deposit_fill", st);
       GBP_CUDA_TRY(launch_pdl(fill_kernel<MAS, G, CM>, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts,
-                              b.entries, b.ctr, b.block_stats, b.block_counts));
-    }
-    {
-      GBP_TRACE("deposit_scan", st);
-      GBP_CUDA_TRY(launch_pdl(gated_scan_kernel, dim3(1), dim3(FSCAN_THREADS), 0, st, b.counts, b.offsets,
-                              L.ntiles, b.ctr));
-    }
-    if (L.nblocks > 0) {
-      GBP_TRACE("deposit_scatter", st);
-      GBP_CUDA_TRY(launch_pdl(scatter_kernel<MAS, G, CM>, dim3(std::min(L.nblocks, FILL_SCATTER_BLOCKS)),
-                              dim3(CNT_THREADS), 0, st, g, b.offsets, b.fills, b.entries,
-                              static_cast<const DepCounters*>(b.ctr)));
+                              b.entries, b.spill, b.ctr, b.block_stats, b.block_counts));
     }
     return GBP_OK;
   }
@@ -770,7 +794,7 @@ int bucket_particles(const DepGeom& g, const DepLayout& L, const DepBuffers& b, 
   if (L.nblocks > 0) {
     GBP_TRACE("deposit_scatter", st);
     GBP_CUDA_TRY(launch_pdl(scatter_kernel<MAS, G, CM>, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.offsets,
-                            b.fills, b.entries, static_cast<const DepCounters*>(nullptr)));
+                            b.fills, b.entries));
   }
   return GBP_OK;
 }
