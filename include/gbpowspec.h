@@ -411,6 +411,31 @@ int gbp_deposit_backward(const float* x, const float* y, const float* z,
                          float* grad_x, float* grad_y, float* grad_z,
                          float* grad_w, gbp_stream_t stream);
 
+/* The same adjoint on the packed spectrum that gbp_fft_power or
+ * gbp_particles_power leaves in its `spectrum` buffer (library transform
+ * sizes; read only): dLoss/d(mesh cell) into grad_mesh, and scal [2]
+ * (device, double) = the explicit dependences of P_l on a weight w_i,
+ * dLoss/dM through L^3/M^2 and -2 L^3/M^2 dLoss/dP_0 (times w_i; 0 unless
+ * subtract_shot).  pk: the forward result; a NaN gradient or one into an
+ * empty bin counts as 0.  gbp_deposit_backward_total: gbp_deposit_backward
+ * with those two added to grad_w. */
+int gbp_power_backward_packed_workspace_size(gbp_fft_plan plan, gbp_bins bins,
+                                             size_t* bytes);
+int gbp_power_backward_packed(const void* packed, gbp_fft_plan plan,
+                              gbp_bins bins, int mas_order,
+                              const double* grad_pk, const double* pk,
+                              const long long* nmodes, const double* mass,
+                              double box_size, int subtract_shot,
+                              float* grad_mesh, double* scal, void* workspace,
+                              size_t workspace_bytes, gbp_stream_t stream);
+int gbp_deposit_backward_total(const float* x, const float* y, const float* z,
+                               const float* w, int64_t n_particles, float xmin,
+                               float ymin, float zmin, float inv_cell,
+                               int n_mesh, int mas, int interlace,
+                               const float* grad_mesh, const double* scal,
+                               float* grad_x, float* grad_y, float* grad_z,
+                               float* grad_w, gbp_stream_t stream);
+
 /* ---- Lanes: resident per-mock pipelines for batching and serving --------
  * No reference counterpart (the reference computes one mock per call).
  * A lane owns every buffer one mock needs and, with GBP_LANE_GRAPH, a CUDA

@@ -177,6 +177,70 @@ fft_cols_kernel(float2* __restrict__ data, long long plane_stride, long long row
   fft::col_fft<N, 1, N / 2, false>(s, gin, gout, tw, threadIdx.x);
 }
 
+// Inverse of the packed transform along y, in place: rows whose ky^2 + (the
+// block's first kz)^2 > k2_max hold nothing and are taken as zeros; every row
+// of every x plane is stored.  (An inverse transform is a forward one with
+// real and imaginary parts swapped before and after.)
+template <int N>
+__global__ void __launch_bounds__(N / 2, N <= 512 ? 4 : 2)
+fft_cols_inv_kernel(float2* __restrict__ data, int nplanes, int nkb, int k2_max, const float2* __restrict__ tw) {
+  pdl_wait();
+  constexpr int P = zpitch(N);
+  extern __shared__ __align__(16) float2 s[];
+  const int plane = blockIdx.x / nkb, kb = blockIdx.x % nkb;
+  if (plane >= nplanes) return;
+  float2* base = data + (long long)plane * N * P + kb * 8;
+  const int lim = k2_max - 64 * kb * kb;
+  auto gin = [base, lim](int j, int cp) {
+    const int k = signed_k(j, N);
+    if (k * k > lim) return make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 v = __ldcs(reinterpret_cast<const float4*>(base + (long long)j * P) + cp);
+    return make_float4(v.y, v.x, v.w, v.z);
+  };
+  auto gout = [base](int j, int cp, float4 v) {
+    __stcs(reinterpret_cast<float4*>(base + (long long)j * P) + cp, make_float4(v.y, v.x, v.w, v.z));
+  };
+  fft::col_fft<N, 1, N / 2, false>(s, gin, gout, tw, threadIdx.x);
+}
+
+// Inverse z pass of the packed transform: real fields out (the layout of
+// fftz_packed_kernel's input), kz >= kz_cols taken as zero.
+template <int N, int G, int PAIRS>
+__global__ void __launch_bounds__(PAIRS * N / 16)
+fftz_unpack_kernel(const float2* __restrict__ spec, float* __restrict__ mesh, int kz_cols,
+                   const float2* __restrict__ tw) {
+  pdl_wait();
+  constexpr int NT = PAIRS * N / 16;
+  constexpr int CP = PAIRS / 2;
+  constexpr int NX = G == 2 ? N : N / 2;
+  constexpr int P = zpitch(N);
+  constexpr long long IM = G == 2 ? (long long)N * N * N : (long long)N * N;
+  extern __shared__ __align__(16) float4 s4[];    // [CP][N] slots of two columns
+  const int tid = threadIdx.x;
+  const long long q0 = (long long)blockIdx.x * PAIRS;
+  const long long x = q0 / N, y = q0 - x * N;
+  float* base = mesh + (G == 2 ? q0 * N : (2 * x * N + y) * N);
+  const float2* i0 = spec + q0 * P;
+  const float2* i1 = i0 + (long long)NX * N * P;
+  auto gin = [i0, i1, kz_cols](int j, int cp) {
+    const int k = j <= N / 2 ? j : N - j;
+    if (k >= kz_cols) return make_float4(0.f, 0.f, 0.f, 0.f);
+    const float2* b = (j <= N / 2 ? i0 : i1) + (2 * cp) * P + k;
+    const float2 u = __ldcs(b), v = __ldcs(b + P);
+    return make_float4(u.y, u.x, v.y, v.x);
+  };
+  auto sin_ = [](int j, int cp) { return s4[cp * N + zsw(j)]; };
+  auto sout = [](int j, int cp, float4 v) { s4[cp * N + zsw(j)] = v; };
+  auto gout = [base](int j, int cp, float4 v) {
+    float* b = base + 2 * cp * N + j;
+    __stcs(b, v.y);
+    __stcs(b + IM, v.x);
+    __stcs(b + N, v.w);
+    __stcs(b + IM + N, v.z);
+  };
+  fft::run_stages2<N, CP, NT, true, false, false>(gin, sin_, sout, gout, tw, tid);
+}
+
 template <int N>
 constexpr int z_pairs() { return N >= 256 ? 8 : 32768 / (N * 8); }   // >= 256 threads
 template <int N, bool PRUNE>
@@ -239,6 +303,31 @@ int run_y_packed(int G, float2* spec, int kz_cols, int k2_max, const float2* tw,
   GBP_TRACE("fft_y", st);
   // a plane is one x' of one slab: two slabs of N (two grids) or N/2 planes
   return launch_cols<N, true>(spec, (long long)N * P, (long long)P, G * N, kz_cols / 8, k2_max, tw, st);
+}
+
+template <int N>
+int run_y_inverse(int G, float2* spec, int kz_cols, int k2_max, const float2* tw, cudaStream_t st) {
+  if (kz_cols == 0) return GBP_OK;
+  const size_t smem = (size_t)fft::ColBlock<N, 1>::SLAB * sizeof(float2);
+  auto k = fft_cols_inv_kernel<N>;
+  GBP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GBP_TRACE("fft_y_inverse", st);
+  GBP_CUDA_TRY(launch_pdl(k, dim3((unsigned)(G * N * (kz_cols / 8))), dim3(N / 2), smem, st, spec, G * N, kz_cols / 8,
+                          k2_max, tw));
+  return GBP_OK;
+}
+
+template <int N, int G>
+int run_z_unpack(const float2* spec, float* mesh, int kz_cols, const float2* tw, cudaStream_t st) {
+  constexpr int PAIRS = z_pairs<N>();
+  constexpr int NX = G == 2 ? N : N / 2;
+  const size_t smem = (size_t)PAIRS * N * sizeof(float2);
+  auto k = fftz_unpack_kernel<N, G, PAIRS>;
+  GBP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  GBP_TRACE("fft_z_inverse", st);
+  GBP_CUDA_TRY(launch_pdl(k, dim3((unsigned)(NX * N / PAIRS)), dim3(PAIRS * N / 16), smem, st, spec, mesh, kz_cols,
+                          tw));
+  return GBP_OK;
 }
 
 }  // namespace
@@ -331,6 +420,31 @@ int own_fft_y_packed(int N, int G, float2* spec, int kz_cols, int k2_max, const 
     case 1024: return run_y_packed<1024>(G, spec, kz_cols, k2_max, tw, st);
     default: return GBP_ERR_UNSUPPORTED;
   }
+}
+
+int own_fft_y_inverse(int N, int G, float2* spec, int kz_cols, int k2_max, const float2* tw, cudaStream_t st) {
+  switch (N) {
+    case 64: return run_y_inverse<64>(G, spec, kz_cols, k2_max, tw, st);
+    case 128: return run_y_inverse<128>(G, spec, kz_cols, k2_max, tw, st);
+    case 256: return run_y_inverse<256>(G, spec, kz_cols, k2_max, tw, st);
+    case 512: return run_y_inverse<512>(G, spec, kz_cols, k2_max, tw, st);
+    case 1024: return run_y_inverse<1024>(G, spec, kz_cols, k2_max, tw, st);
+    default: return GBP_ERR_UNSUPPORTED;
+  }
+}
+
+int own_fft_z_unpack(int N, int G, const float2* spec, float* mesh, int kz_cols, const float2* tw, cudaStream_t st) {
+#define GBP_Z(NN) \
+  case NN: return G == 2 ? run_z_unpack<NN, 2>(spec, mesh, kz_cols, tw, st) : run_z_unpack<NN, 1>(spec, mesh, kz_cols, tw, st)
+  switch (N) {
+    GBP_Z(64);
+    GBP_Z(128);
+    GBP_Z(256);
+    GBP_Z(512);
+    GBP_Z(1024);
+    default: return GBP_ERR_UNSUPPORTED;
+  }
+#undef GBP_Z
 }
 
 }  // namespace gbp

@@ -44,50 +44,12 @@
 // instead of writing and reading them three more times.
 #include <algorithm>
 
-#include "fft_core.cuh"
-#include "fft_pass.cuh"
-#include "gbp_bins.h"
-#include "gbp_fft.h"
-#include "gbp_internal.cuh"
-#include "power_core.cuh"
+#include "xpass.cuh"
 
 namespace gbp {
 namespace {
 
 constexpr int XB_BINS = 8;                   // per-warp bin arrays; warps w and w + 8 share one
-constexpr int XB_C = 8;                      // kz columns per work item
-// The next item's HBM loads start before the barrier that ends the binning (512^3 and up)
-template <int N>
-constexpr bool XB_EARLY = N >= 512;
-
-template <int N, bool INTER>
-struct XLayout {
-  static constexpr int NX = INTER ? N : N / 2;   // points of the x transform
-  static constexpr int NT = NX < 512 ? 256 : 512;
-  static constexpr int HALVES = NT / 256;    // warps per column
-  static constexpr int TST = NX + 1;         // complex per column (transposed layout); odd: no store conflicts
-  // a lane takes M2 consecutive pairs (x, N - x) of its warp's part of the |kx| range, MS2 per warp step
-  static constexpr int M2 = N / (64 * HALVES);
-  static constexpr int MS2 = M2 < 4 ? M2 : (N >= 1024 && INTER ? (M2 < 8 ? M2 : 8) : 4);
-  static_assert(MS2 > 0 && M2 % MS2 == 0, "whole warp steps of mode pairs");
-  static __host__ __device__ constexpr size_t data_bytes() {
-    const size_t rows = (size_t)2 * fft::ColBlock<NX, 2>::SLAB, cols = (size_t)2 * XB_C * TST;
-    return ((rows > cols ? rows : cols) * 8 + 127) & ~size_t(127);
-  }
-  // per-|kx| tables (swizzled like the columns): window c2 and the factor f of kx >= 0
-  static __host__ __device__ constexpr size_t xtab_bytes() { return (size_t)(N / 2) * 12; }
-};
-
-// Swizzled position of x in a transposed column: lane l reads x = base + M2 l
-// + j (M2 = the mode pairs a lane takes), and so does it read the mirror
-// -x; with x's low bits XORed by bits 4.. of x, the 16 lanes of a half-warp
-// hit 16 distinct 8-byte slots in both reads, and the last FFT stage's
-// stores stay conflict-free.
-template <int M2>
-__device__ __forceinline__ int xswz(int x) {
-  if constexpr (M2 <= 1) return x;
-  else return x ^ ((x >> 4) & (M2 - 1));
-}
 
 // One warp step: lane modes x0 + j (j < MS) of one column, bins monotone in
 // lane order; sums runs and adds each once to the warp's bins.
@@ -132,12 +94,6 @@ __device__ __forceinline__ void flush_runs(float (&P)[MS][NV], const int (&bin)[
   }
   if (!next_cont && bin[MS - 1] >= 0) bin_add<NV>(wb, nbe, bin[MS - 1], T);
   __syncwarp();
-}
-
-// (A + B) - i f (A - B), B = conj b, f = (fr, fi): four times |.|^2's root is the mode.
-__device__ __forceinline__ float2 unpack_mode(float2 a, float2 b, float fr, float fi) {
-  const float sx = a.x + b.x, sy = a.y - b.y, dx = a.x - b.x, dy = a.y + b.y;
-  return make_float2(sx + (fr * dy + fi * dx), sy + (fi * dy - fr * dx));
 }
 
 // Moments and bins of one warp step of mode pairs: lane pairs p0 .. p0 + MS - 1
@@ -270,8 +226,7 @@ __global__ void __launch_bounds__(XLayout<N, INTER>::NT,
 xbin_kernel(PowGeom g) {
   pdl_wait();
   using L = XLayout<N, INTER>;
-  constexpr int P = N / 2 + 8;                              // z row pitch of the own transform
-  constexpr int TST = L::TST, NX = L::NX, NT = L::NT;
+  constexpr int NT = L::NT;
   extern __shared__ __align__(16) unsigned char smem[];
   float2* s = reinterpret_cast<float2*>(smem);
   float2* fx = reinterpret_cast<float2*>(smem + L::data_bytes());
@@ -283,24 +238,13 @@ xbin_kernel(PowGeom g) {
     c2x[xswz<L::M2>(p)] = t.c2[p];
   }
   __syncthreads();
-  const long long sstride = (long long)NX * N * P;
   for (int grp = blockIdx.x; grp < g.groups; grp += gridDim.x) {
     for (int it = grp; it < g.items; it += g.groups) {
       const int code = __ldg(g.item_list + it), y = code / XITEM_KB, kb = code % XITEM_KB;
-      const float2* src = g.s0 + kb * XB_C;
-      // row of the column pair's slab: y, or -y of slab 1
-      const long long r0 = (long long)y * P, r1 = sstride + (long long)((N - y) & (N - 1)) * P;
-      auto gin = [src, r0, r1](int x, int cp) {    // columns 2cp, 2cp+1 (slab cp / 4)
-        return __ldcs(reinterpret_cast<const float4*>(src + (cp < 4 ? r0 : r1) + (long long)x * N * P) + (cp & 3));
-      };
-      auto tout = [s](int x, int cp, float4 v) {
-        s[(2 * cp) * TST + xswz<L::M2>(x)] = fft::lo2(v);
-        s[(2 * cp + 1) * TST + xswz<L::M2>(x)] = fft::hi2(v);
-      };
       // from 512^3 up the first stage loads the item from HBM while the previous item's last warps
       // still bin it, and waits for them before it writes the shared buffer (smaller meshes: the
       // registers the early loads hold would spill; they end the binning with a barrier instead)
-      fft::col_fft<NX, 2, NT, true, decltype(gin), decltype(tout), XB_EARLY<N>>(s, gin, tout, g.twx, tid);
+      x_forward<N, INTER, XB_EARLY<N>>(s, g.s0, y, kb, g.twx, tid);
       xbin_item<N, NV, INTER>(g, t, c2x, fx, s, warp, lane, y, kb);
       if constexpr (!XB_EARLY<N>) __syncthreads();
     }

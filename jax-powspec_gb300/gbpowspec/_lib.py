@@ -137,6 +137,10 @@ SIGNATURES = [
     ("gbp_power_backward", _i, [_vp, _vp, _vp, _i, _vp, _vp, _vp, _d, _vp, _vp, _sz, _vp]),
     ("gbp_deposit_backward", _i, [_vp, _vp, _vp, _vp, _i64, _f, _f, _f, _f, _i, _i, _i, _vp, _vp, _vp, _vp, _vp,
                                   _vp]),
+    ("gbp_power_backward_packed_workspace_size", _i, [_vp, _vp, C.POINTER(_sz)]),
+    ("gbp_power_backward_packed", _i, [_vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _d, _i, _vp, _vp, _vp, _sz, _vp]),
+    ("gbp_deposit_backward_total", _i, [_vp, _vp, _vp, _vp, _i64, _f, _f, _f, _f, _i, _i, _i, _vp, _vp, _vp, _vp,
+                                        _vp, _vp, _vp]),
     ("gbp_trace_enable", _i, [_i]),
     ("gbp_trace_collect", _i, [_vp, _i, C.POINTER(_i)]),
 ]

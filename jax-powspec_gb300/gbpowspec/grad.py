@@ -10,14 +10,15 @@ noise), as a torch.autograd.Function whose backward pass runs on the GPU:
     loss = ((pk[:, 0] - target) ** 2).sum()
     loss.backward()                                                      # x.grad, y.grad, z.grad, w.grad
 
-Forward: deposit (gbp_deposit) -> R2C (gbp_fft_r2c, spectra kept) -> binning
-(gbp_power) -> normalisation.  Backward: gbp_power_backward forms the adjoint
-spectrum from dLoss/dP and transforms it back to gradient meshes (C2R);
-gbp_deposit_backward gathers them at the particles with the B-spline
-derivatives; the explicit dependence of L^3/M^2 and of the shot noise on the
-weights (M = sum w, Q = sum w^2) is added here:
+Forward: deposit (gbp_deposit) -> packed transform + binning (gbp_fft_power, the
+packed spectrum kept) -> normalisation.  Backward: gbp_power_backward_packed
+forms the adjoint spectrum from dLoss/dP and transforms it back to gradient
+meshes; gbp_deposit_backward_total gathers them at the particles with the
+B-spline derivatives and adds the explicit dependence of L^3/M^2 and of the
+shot noise on the weights (M = sum w, Q = sum w^2):
     dP_l/dM = -2 P_l / M,   dP_0/dQ = -L^3 / M^2.
-Empty bins (NaN) carry no gradient.
+Meshes that need cuFFT go through gbp_fft_r2c, gbp_power and
+gbp_power_backward.  Empty bins (NaN) carry no gradient.
 """
 from __future__ import annotations
 
@@ -49,10 +50,14 @@ class _PowerFn(torch.autograd.Function):
                                       mas=cfg.mas_order, interlace=cfg.interlace)
         plan = _native.fft_plan(N, G, dev)
         spec = torch.empty(plan.spectrum_floats, dtype=torch.float32, device=dev)
-        plan.execute(mesh, spec)
         bins = _native.bins_for(cfg.kedges_grid(), N, dev)
         mask = _lib.ELL0 | _lib.ELL2 | _lib.ELL4
-        sums = _native.power(spec, G, bins, mas_order=cfg.mas_order, ells=mask, z_pitch=plan.pitch, mass=stats)
+        ctx.packed = _native.fft_power_workspace_size(plan, bins, mask) is not None
+        if ctx.packed:
+            sums = _native.fft_power(plan, mesh, spec, bins, mas_order=cfg.mas_order, ells=mask, mass=stats)
+        else:
+            plan.execute(mesh, spec)
+            sums = _native.power(spec, G, bins, mas_order=cfg.mas_order, ells=mask, z_pitch=plan.pitch, mass=stats)
         pk, _ = _native.normalize(sums, n_mesh=N, box_size=cfg.box_size, mass=stats, stats=stats,
                                   subtract_shot=cfg.shot_noise)
         ctx.cfg, ctx.plan, ctx.bins = cfg, plan, bins
@@ -68,37 +73,46 @@ class _PowerFn(torch.autograd.Function):
         dev = xs.device
         N, G = cfg.n_mesh, cfg.grids
         ws = ws if ctx.has_w else None
-        g = torch.nan_to_num(grad_pk.detach().to(torch.float64), nan=0.0).contiguous()
-        empty = ~torch.isfinite(pk)
-        g = torch.where(empty, torch.zeros_like(g), g)
         lib = _lib.load()
-        need = C.c_size_t(0)
-        check(lib.gbp_power_backward_workspace_size(plan.handle, C.byref(need)), "gbp_power_backward_workspace_size")
-        wsb = _native.workspace(need.value, dev)
         gmesh = torch.empty((G, N, N, N), dtype=torch.float32, device=dev)
         stream = _native._stream_of(dev)
-        check(lib.gbp_power_backward(_p(spec), plan.handle, bins.handle, cfg.mas_order, _p(g), _p(nmodes),
-                                     _p(stats), float(cfg.box_size), _p(gmesh), _p(wsb), wsb.numel(), stream),
-              "gbp_power_backward")
+        need = C.c_size_t(0)
         n = xs.numel()
         gx, gy, gz = (torch.empty(n, dtype=torch.float32, device=dev) for _ in range(3))
-        gw = torch.empty(n, dtype=torch.float32, device=dev)
+        want_w = ctx.has_w and ctx.needs_input_grad[3]
+        gw = torch.empty(n, dtype=torch.float32, device=dev) if want_w else None
         inv = float(np.float32(N / cfg.box_size))
         o = [float(np.float32(v)) for v in cfg.origin]
-        check(lib.gbp_deposit_backward(_p(xs), _p(ys), _p(zs), _p(ws), n, o[0], o[1], o[2], inv, N, cfg.mas_order,
-                                       int(cfg.interlace), _p(gmesh), _p(gx), _p(gy), _p(gz), _p(gw), stream),
-              "gbp_deposit_backward")
-        grad_w = None
-        if ctx.has_w and ctx.needs_input_grad[3]:
-            st = _native.read_stats(stats)
-            M = float(st.mass[0])
-            pk0 = torch.nan_to_num(pk, nan=0.0)
-            c_mass = float((g * (-2.0 * pk0 / M)).sum())               # dP_l/dM = -2 P_l / M
-            grad_w = gw.to(torch.float64) + c_mass
-            if cfg.shot_noise:
-                grad_w = grad_w - 2.0 * ws.to(torch.float64) * (cfg.box_size ** 3 / M ** 2) * float(g[:, 0].sum())
-            grad_w = grad_w.to(ws.dtype)
-        return gx, gy, gz, grad_w, None
+        if ctx.packed:
+            g = grad_pk.detach().to(torch.float64).contiguous()
+            check(lib.gbp_power_backward_packed_workspace_size(plan.handle, bins.handle, C.byref(need)),
+                  "gbp_power_backward_packed_workspace_size")
+            wsb = _native.workspace(need.value, dev)
+            scal = torch.empty(2, dtype=torch.float64, device=dev)
+            check(lib.gbp_power_backward_packed(_p(spec), plan.handle, bins.handle, cfg.mas_order, _p(g), _p(pk),
+                                                _p(nmodes), _p(stats), float(cfg.box_size), int(cfg.shot_noise),
+                                                _p(gmesh), _p(scal), _p(wsb), wsb.numel(), stream),
+                  "gbp_power_backward_packed")
+        else:
+            g = torch.nan_to_num(grad_pk.detach().to(torch.float64), nan=0.0).contiguous()
+            g = torch.where(torch.isfinite(pk), g, torch.zeros_like(g))
+            check(lib.gbp_power_backward_workspace_size(plan.handle, C.byref(need)),
+                  "gbp_power_backward_workspace_size")
+            wsb = _native.workspace(need.value, dev)
+            check(lib.gbp_power_backward(_p(spec), plan.handle, bins.handle, cfg.mas_order, _p(g), _p(nmodes),
+                                         _p(stats), float(cfg.box_size), _p(gmesh), _p(wsb), wsb.numel(), stream),
+                  "gbp_power_backward")
+            scal = None
+            if want_w:
+                M = stats[:8].view(torch.float64)                          # gbp_deposit_stats starts with mass[2]
+                pk0 = torch.nan_to_num(pk, nan=0.0)
+                shot = -2.0 * cfg.box_size ** 3 * int(cfg.shot_noise)
+                scal = torch.cat([(g * (-2.0 * pk0 / M)).sum().reshape(1),  # dP_l/dM = -2 P_l / M
+                                  shot / M ** 2 * g[:, 0].sum()])
+        check(lib.gbp_deposit_backward_total(_p(xs), _p(ys), _p(zs), _p(ws), n, o[0], o[1], o[2], inv, N,
+                                             cfg.mas_order, int(cfg.interlace), _p(gmesh), _p(scal), _p(gx), _p(gy),
+                                             _p(gz), _p(gw), stream), "gbp_deposit_backward_total")
+        return gx, gy, gz, gw, None
 
 
 def power_multipoles_diff(x, y, z, w=None, *, box_size: float, n_mesh: int, mas: str = "tsc", interlace: bool = True,
