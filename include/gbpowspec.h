@@ -370,6 +370,17 @@ int gbp_xi(gbp_fft_plan plan, const float* delta, void* spectrum, float* field,
            double* sums_out, long long* counts_out, void* workspace,
            size_t workspace_bytes, gbp_stream_t stream);
 
+/* gbp_xi without the field, for the library's transform sizes
+ * (GBP_ERR_UNSUPPORTED otherwise): only the separations within the last edge
+ * are formed; same sums and counts to float32 round-off.  `spectrum` is
+ * scratch of the plan's spectrum size. */
+int gbp_xi_shells_workspace_size(gbp_fft_plan plan, gbp_bins bins,
+                                 size_t* bytes);
+int gbp_xi_shells(gbp_fft_plan plan, const float* delta, void* spectrum,
+                  gbp_bins bins, int mas_order, int nan_mu_at_origin,
+                  double* sums_out, long long* counts_out, void* workspace,
+                  size_t workspace_bytes, gbp_stream_t stream);
+
 /* Bispectrum of a density contrast mesh (src/correlations.py:334-462
  * bispec): shells |k| in [k_i - kF, k_i + kF) around k_1, k_2 and every
  * k_3(theta), each a run of elementary bins of `bins` (edges in kF units:

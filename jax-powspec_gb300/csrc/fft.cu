@@ -151,10 +151,11 @@ fftz_packed_kernel(const float* __restrict__ mesh, float2* __restrict__ out, int
 // CTA b covers plane (b / nkb) and kz block (b % nkb).  N/2 threads: one
 // pair of radix-8 butterflies (two columns) each per stage; the first stage
 // loads from HBM and the last stores to HBM (fft_pass.cuh), in place.
-// PRUNE: rows whose wavenumber k has k^2 + (the block's first kz)^2 > k2_max
-// are not stored (with k edges up to k_Nyquist, a fifth of them: 0.423 ->
-// 0.392 ms for two grids at 512^3, 5.0 TB/s; bound by HBM).
-template <int N, bool PRUNE>
+// PRUNE = 1: rows whose wavenumber k has k^2 + (the block's first kz)^2 >
+// k2_max are not stored (with k edges up to k_Nyquist, a fifth of them: 0.423 ->
+// 0.392 ms for two grids at 512^3, 5.0 TB/s; bound by HBM).  PRUNE = 2: the
+// same with the plane's number in place of kz (real-space rows, xi.cu).
+template <int N, int PRUNE>
 __global__ void __launch_bounds__(N / 2, N <= 512 ? 4 : 2)
 fft_cols_kernel(float2* __restrict__ data, long long plane_stride, long long row_stride, int nplanes, int nkb,
                 int k2_max, const float2* __restrict__ tw) {
@@ -166,7 +167,7 @@ fft_cols_kernel(float2* __restrict__ data, long long plane_stride, long long row
   auto gin = [base, row_stride](int j, int cp) {
     return __ldcs(reinterpret_cast<const float4*>(base + j * row_stride) + cp);
   };
-  const int lim = PRUNE ? k2_max - 64 * kb * kb : 0;
+  const int lim = PRUNE == 1 ? k2_max - 64 * kb * kb : k2_max - plane * plane;
   auto gout = [base, row_stride, lim](int j, int cp, float4 v) {
     if (PRUNE) {
       const int k = signed_k(j, N);
@@ -243,7 +244,7 @@ fftz_unpack_kernel(const float2* __restrict__ spec, float* __restrict__ mesh, in
 
 template <int N>
 constexpr int z_pairs() { return N >= 256 ? 8 : 32768 / (N * 8); }   // >= 256 threads
-template <int N, bool PRUNE>
+template <int N, int PRUNE>
 int launch_cols(float2* data, long long plane_stride, long long row_stride, int nplanes, int nkb, int k2_max,
                 const float2* tw, cudaStream_t st) {
   const size_t smem = (size_t)fft::ColBlock<N, 1>::SLAB * sizeof(float2);
@@ -270,14 +271,14 @@ int run_fft(const float* mesh, float2* spec, int G, const float2* tw, cudaStream
   }
   {  // y pass: a plane is one x slab of one grid; rows (y) are P apart
     GBP_TRACE("fft_y", st);
-    const int r = launch_cols<N, false>(spec, (long long)N * P, (long long)P, G * N, P / C, 0, tw, st);
+    const int r = launch_cols<N, 0>(spec, (long long)N * P, (long long)P, G * N, P / C, 0, tw, st);
     if (r) return r;
   }
   // x pass: a plane is one y row of one grid; rows (x) are N*P apart
   for (int g = 0; g < G; ++g) {
     GBP_TRACE("fft_x", st);
     const int r =
-        launch_cols<N, false>(spec + (long long)g * N * N * P, (long long)P, (long long)N * P, N, P / C, 0, tw, st);
+        launch_cols<N, 0>(spec + (long long)g * N * N * P, (long long)P, (long long)N * P, N, P / C, 0, tw, st);
     if (r) return r;
   }
   return GBP_OK;
@@ -302,7 +303,15 @@ int run_y_packed(int G, float2* spec, int kz_cols, int k2_max, const float2* tw,
   if (kz_cols == 0) return GBP_OK;
   GBP_TRACE("fft_y", st);
   // a plane is one x' of one slab: two slabs of N (two grids) or N/2 planes
-  return launch_cols<N, true>(spec, (long long)N * P, (long long)P, G * N, kz_cols / 8, k2_max, tw, st);
+  return launch_cols<N, 1>(spec, (long long)N * P, (long long)P, G * N, kz_cols / 8, k2_max, tw, st);
+}
+
+template <int N>
+int run_y_shells(float2* spec, int nplanes, int r2_max, const float2* tw, cudaStream_t st) {
+  constexpr int P = zpitch(N);
+  if (nplanes == 0) return GBP_OK;
+  GBP_TRACE("fft_y", st);
+  return launch_cols<N, 2>(spec, (long long)N * P, (long long)P, nplanes, P / 8, r2_max, tw, st);
 }
 
 template <int N>
@@ -445,6 +454,17 @@ int own_fft_z_unpack(int N, int G, const float2* spec, float* mesh, int kz_cols,
     default: return GBP_ERR_UNSUPPORTED;
   }
 #undef GBP_Z
+}
+
+int own_fft_y_shells(int N, float2* spec, int nplanes, int r2_max, const float2* tw, cudaStream_t st) {
+  switch (N) {
+    case 64: return run_y_shells<64>(spec, nplanes, r2_max, tw, st);
+    case 128: return run_y_shells<128>(spec, nplanes, r2_max, tw, st);
+    case 256: return run_y_shells<256>(spec, nplanes, r2_max, tw, st);
+    case 512: return run_y_shells<512>(spec, nplanes, r2_max, tw, st);
+    case 1024: return run_y_shells<1024>(spec, nplanes, r2_max, tw, st);
+    default: return GBP_ERR_UNSUPPORTED;
+  }
 }
 
 }  // namespace gbp

@@ -31,6 +31,8 @@ int own_fft_y_packed(int N, int G, float2* spec, int kz_cols, int k2_max, const 
 // block)^2 <= k2_max, in place; inverse z pass into the real fields (unnormalised, as the forward passes)
 int own_fft_y_inverse(int N, int G, float2* spec, int kz_cols, int k2_max, const float2* tw, cudaStream_t st);
 int own_fft_z_unpack(int N, int G, const float2* spec, float* mesh, int kz_cols, const float2* tw, cudaStream_t st);
+// Forward y pass of x planes 0 .. nplanes - 1 of [x][N][P]; rows y with x^2 + y^2 <= r2_max stored
+int own_fft_y_shells(int N, float2* spec, int nplanes, int r2_max, const float2* tw, cudaStream_t st);
 // x pass fused with the binning + the fold into per-bin sums (xbin.cu); spec
 // holds the packed transform over z and y
 int xbin_power_workspace(gbp_fft_plan plan, gbp_bins bins, int ells, size_t* bytes);

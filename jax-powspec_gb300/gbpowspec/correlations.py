@@ -155,7 +155,7 @@ def reference_sedges(s_edges, box_size, n_mesh: int):
 
 
 def _xi(d: torch.Tensor, box: np.float32, s_edges, nan_mu_at_origin: bool):
-    """(r3D, xi3D, Nmodes3D) of a density contrast mesh through gbp_xi."""
+    """(r3D, xi3D, Nmodes3D) of a density contrast mesh through gbp_xi_shells (library transform sizes) or gbp_xi."""
     import ctypes as C
     N = int(d.shape[0])
     dev = d.device
@@ -164,16 +164,23 @@ def _xi(d: torch.Tensor, box: np.float32, s_edges, nan_mu_at_origin: bool):
     plan = _native.fft_plan(N, 1, dev)
     lib = _lib.load()
     need = C.c_size_t(0)
-    _lib.check(lib.gbp_xi_workspace_size(plan.handle, bins.handle, C.byref(need)), "gbp_xi_workspace_size")
     spec = torch.empty(plan.spectrum_floats, dtype=torch.float32, device=dev)
-    field = torch.empty((N, N, N), dtype=torch.float32, device=dev)
-    ws = _native.workspace(need.value, dev)
     nb = bins.n_bins
     sums = torch.empty((nb, 3), dtype=torch.float64, device=dev)
     counts = torch.empty(nb, dtype=torch.int64, device=dev)
     p = lambda t: C.c_void_p(t.data_ptr())
-    _lib.check(lib.gbp_xi(plan.handle, p(d), p(spec), p(field), bins.handle, 2, int(nan_mu_at_origin), p(sums),
-                          p(counts), p(ws), ws.numel(), _native._stream_of(dev)), "gbp_xi")
+    st = lib.gbp_xi_shells_workspace_size(plan.handle, bins.handle, C.byref(need))
+    if st != _lib.GBP_ERR_UNSUPPORTED:
+        _lib.check(st, "gbp_xi_shells_workspace_size")
+        ws = _native.workspace(need.value, dev)
+        _lib.check(lib.gbp_xi_shells(plan.handle, p(d), p(spec), bins.handle, 2, int(nan_mu_at_origin), p(sums),
+                                     p(counts), p(ws), ws.numel(), _native._stream_of(dev)), "gbp_xi_shells")
+    else:
+        _lib.check(lib.gbp_xi_workspace_size(plan.handle, bins.handle, C.byref(need)), "gbp_xi_workspace_size")
+        field = torch.empty((N, N, N), dtype=torch.float32, device=dev)
+        ws = _native.workspace(need.value, dev)
+        _lib.check(lib.gbp_xi(plan.handle, p(d), p(spec), p(field), bins.handle, 2, int(nan_mu_at_origin), p(sums),
+                              p(counts), p(ws), ws.numel(), _native._stream_of(dev)), "gbp_xi")
     n3 = float(N) ** 3
     nm = counts.to(torch.float64)
     nm = torch.where(nm == 0, torch.full_like(nm, float("inf")), nm)               # :180
