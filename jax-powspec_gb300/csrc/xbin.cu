@@ -51,51 +51,6 @@ namespace {
 
 constexpr int XB_BINS = 8;                   // per-warp bin arrays; warps w and w + 8 share one
 
-// One warp step: lane modes x0 + j (j < MS) of one column, bins monotone in
-// lane order; sums runs and adds each once to the warp's bins.
-template <int MS, int NV>
-__device__ __forceinline__ void flush_runs(float (&P)[MS][NV], const int (&bin)[MS], int lane, float* wb, int nbe) {
-  bool start[MS];
-  start[0] = true;
-#pragma unroll
-  for (int j = 1; j < MS; ++j) {
-    start[j] = bin[j] != bin[j - 1];
-    if (!start[j]) {
-#pragma unroll
-      for (int q = 0; q < NV; ++q) P[j][q] += P[j - 1][q];
-    }
-  }
-  bool multi = false;
-#pragma unroll
-  for (int j = 1; j < MS; ++j) multi = multi || start[j];
-  const int prev_last = __shfl_up_sync(0xffffffffu, bin[MS - 1], 1);
-  const bool cont = lane > 0 && bin[0] == prev_last;       // the lane's first run continues the previous lane's last
-  const unsigned heads = __ballot_sync(0xffffffffu, multi || !cont);
-  float T[NV];
-#pragma unroll
-  for (int q = 0; q < NV; ++q) T[q] = P[MS - 1][q];
-  seg_scan<NV>(T, heads, lane);
-  float Tprev[NV];
-#pragma unroll
-  for (int q = 0; q < NV; ++q) Tprev[q] = __shfl_up_sync(0xffffffffu, T[q], 1);
-  const bool next_cont = __shfl_down_sync(0xffffffffu, cont, 1) && lane < 31;
-  // runs that end inside the lane: the first of them absorbs the carry from earlier lanes
-  bool carry = cont && multi;
-#pragma unroll
-  for (int j = 0; j < MS - 1; ++j) {
-    if (start[j + 1]) {
-      if (carry) {
-#pragma unroll
-        for (int q = 0; q < NV; ++q) P[j][q] += Tprev[q];
-        carry = false;
-      }
-      if (bin[j] >= 0) bin_add<NV>(wb, nbe, bin[j], P[j]);
-    }
-  }
-  if (!next_cont && bin[MS - 1] >= 0) bin_add<NV>(wb, nbe, bin[MS - 1], T);
-  __syncwarp();
-}
-
 // Moments and bins of one warp step of mode pairs: lane pairs p0 .. p0 + MS - 1
 // of a column (a_col at (ky, kz), b_col at (-ky, -kz)), pair p = the modes
 // kx = p and -p, whose |k|, mu, window and bin agree; p = 0 is one mode.

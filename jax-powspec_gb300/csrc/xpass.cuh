@@ -21,10 +21,13 @@ constexpr int XB_C = 8;                      // kz columns per work item
 template <int N>
 constexpr bool XB_EARLY = N >= 512;
 
-template <int N, bool INTER>
+// Threads of a CTA that transforms one item (INTER: N points along x, else N/2).
+constexpr int x_threads(int N, bool inter) { return (inter ? N : N / 2) < 512 ? 256 : 512; }
+
+template <int N, bool INTER, int NT_ = x_threads(N, INTER)>
 struct XLayout {
   static constexpr int NX = INTER ? N : N / 2;   // points of the x transform
-  static constexpr int NT = NX < 512 ? 256 : 512;
+  static constexpr int NT = NT_;
   static constexpr int HALVES = NT / 256;    // warps per column
   static constexpr int TST = NX + 1;         // complex per column (transposed layout); odd: no store conflicts
   // a lane takes M2 consecutive pairs (x, N - x) of its warp's part of the |kx| range, MS2 per warp step
@@ -56,19 +59,66 @@ __device__ __forceinline__ float2 unpack_mode(float2 a, float2 b, float fr, floa
   return make_float2(sx + (fr * dy + fi * dx), sy + (fi * dy - fr * dx));
 }
 
+// One warp step: lane modes x0 + j (j < MS) of one column, bins monotone in
+// lane order; sums runs and adds each once to the warp's bins.
+template <int MS, int NV>
+__device__ __forceinline__ void flush_runs(float (&P)[MS][NV], const int (&bin)[MS], int lane, float* wb, int nbe) {
+  bool start[MS];
+  start[0] = true;
+#pragma unroll
+  for (int j = 1; j < MS; ++j) {
+    start[j] = bin[j] != bin[j - 1];
+    if (!start[j]) {
+#pragma unroll
+      for (int q = 0; q < NV; ++q) P[j][q] += P[j - 1][q];
+    }
+  }
+  bool multi = false;
+#pragma unroll
+  for (int j = 1; j < MS; ++j) multi = multi || start[j];
+  const int prev_last = __shfl_up_sync(0xffffffffu, bin[MS - 1], 1);
+  const bool cont = lane > 0 && bin[0] == prev_last;       // the lane's first run continues the previous lane's last
+  const unsigned heads = __ballot_sync(0xffffffffu, multi || !cont);
+  float T[NV];
+#pragma unroll
+  for (int q = 0; q < NV; ++q) T[q] = P[MS - 1][q];
+  seg_scan<NV>(T, heads, lane);
+  float Tprev[NV];
+#pragma unroll
+  for (int q = 0; q < NV; ++q) Tprev[q] = __shfl_up_sync(0xffffffffu, T[q], 1);
+  const bool next_cont = __shfl_down_sync(0xffffffffu, cont, 1) && lane < 31;
+  // runs that end inside the lane: the first of them absorbs the carry from earlier lanes
+  bool carry = cont && multi;
+#pragma unroll
+  for (int j = 0; j < MS - 1; ++j) {
+    if (start[j + 1]) {
+      if (carry) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) P[j][q] += Tprev[q];
+        carry = false;
+      }
+      if (bin[j] >= 0) bin_add<NV>(wb, nbe, bin[j], P[j]);
+    }
+  }
+  if (!next_cont && bin[MS - 1] >= 0) bin_add<NV>(wb, nbe, bin[MS - 1], T);
+  __syncwarp();
+}
+
 // Loads item (y, kb) of the packed spectrum `spec` (transformed over z and y)
 // and transforms its 16 columns along x into s (transposed, swizzled); ends
-// with a barrier.  IN_SHARED: see fft::col_fft.
-template <int N, bool INTER, bool IN_SHARED>
+// with a barrier.  IN_SHARED: see fft::col_fft.  planes: how many row planes
+// of [N][P] apart consecutive x' lie (the slabs NX * planes of them).
+template <int N, bool INTER, bool IN_SHARED, int NT = x_threads(N, INTER)>
 __device__ __forceinline__ void x_forward(float2* s, const float2* __restrict__ spec, int y, int kb,
-                                          const float2* __restrict__ twx, int tid) {
-  using L = XLayout<N, INTER>;
+                                          const float2* __restrict__ twx, int tid, int planes = 1) {
+  using L = XLayout<N, INTER, NT>;
   constexpr int P = N / 2 + 8, TST = L::TST;
   const float2* src = spec + kb * XB_C;
   // row of the column pair's slab: y, or -y of slab 1
-  const long long r0 = (long long)y * P, r1 = (long long)L::NX * N * P + (long long)((N - y) & (N - 1)) * P;
-  auto gin = [src, r0, r1](int x, int cp) {    // columns 2cp, 2cp+1 (slab cp / 4)
-    return __ldcs(reinterpret_cast<const float4*>(src + (cp < 4 ? r0 : r1) + (long long)x * N * P) + (cp & 3));
+  const long long r0 = (long long)y * P, r1 = (long long)L::NX * planes * N * P + (long long)((N - y) & (N - 1)) * P;
+  auto gin = [src, r0, r1, planes](int x, int cp) {    // columns 2cp, 2cp+1 (slab cp / 4)
+    return __ldcs(reinterpret_cast<const float4*>(src + (cp < 4 ? r0 : r1) + (long long)x * planes * N * P) +
+                  (cp & 3));
   };
   auto tout = [s](int x, int cp, float4 v) {
     s[(2 * cp) * TST + xswz<L::M2>(x)] = fft::lo2(v);
