@@ -58,6 +58,27 @@ deposit_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ ent
   const int x0 = tx * g.td[0], y0 = ty * g.td[1], z0 = tz * g.td[2];
   const int ex = min(g.td[0], g.N - x0), ey = min(g.td[1], g.N - y0), ez = min(g.td[2], g.N - z0);
 
+  // The drop-ins add to a mesh, one grid: its cells are read, and the accumulators cleared, ahead of the
+  // chain count -> bucket entries, which they do not depend on (512^3, 4 Mi particles: 0.335 -> 0.282 ms,
+  // 1.07 GB, 3.8 TB/s).  With two grids the registers cost more than the latency (0.137 -> 0.157 at 360^3).
+  constexpr bool EARLY = CM != 0;
+  constexpr int CELLS4 = TILE3 / 4 / DEP_THREADS;      // float4s of the tile per thread
+  float4 base[EARLY ? CELLS4 : 1];
+  if (EARLY) {
+    const long long n = g.N;
+    if (g.vec_ok && ez == TILE && (g.N & 3) == 0 && mesh_in) {
+#pragma unroll
+      for (int q = 0; q < CELLS4; ++q) {
+        const int k = threadIdx.x + q * DEP_THREADS;
+        const int lz = (k % (TILE / 4)) * 4, ly = (k / (TILE / 4)) % TILE, lx = k / (TILE * TILE / 4);
+        if (lx < ex && ly < ey)
+          base[EARLY ? q : 0] =
+              __ldcs(reinterpret_cast<const float4*>(mesh_in + ((x0 + lx) * n + (y0 + ly)) * n + (z0 + lz)));
+      }
+    }
+    uint4* a4 = reinterpret_cast<uint4*>(acc32);
+    for (int k = threadIdx.x; k < 2 * TILE3 / 4; k += DEP_THREADS) a4[k] = make_uint4(0u, 0u, 0u, 0u);
+  }
   const TileEntries te = tile_entries(g, t, entries, counts, offsets, sp, ctr);
   const int s = fixed_scale_exp(ctr->maxw_bits, CM);
   const float sc = ldexpf(1.0f, s);
@@ -67,7 +88,7 @@ deposit_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ ent
   const bool vec4 = g.vec_ok && (ez == TILE) && ((g.N & 3) == 0);
 
   for (int grid = 0; grid < G; ++grid) {
-    {
+    if (!EARLY) {
       uint4* a4 = reinterpret_cast<uint4*>(acc32);
       for (int k = threadIdx.x; k < 2 * TILE3 / 4; k += DEP_THREADS) a4[k] = make_uint4(0u, 0u, 0u, 0u);
     }
@@ -124,9 +145,9 @@ deposit_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ ent
     // Write this grid's tile once; sum it exactly for the mean density.
     long long part = 0;
     if (vec4) {
-      for (int k = threadIdx.x; k < TILE3 / 4; k += DEP_THREADS) {
+      auto cell4 = [&](int k, const float4& early) {
         const int lz = (k % (TILE / 4)) * 4, ly = (k / (TILE / 4)) % TILE, lx = k / (TILE * TILE / 4);
-        if (lx >= ex || ly >= ey) continue;
+        if (lx >= ex || ly >= ey) return;
         const int c0 = (lx * TILE + ly) * TILE + lz;
         const uint4 l4 = *reinterpret_cast<const uint4*>(lo + c0);
         const uint4 h4 = *reinterpret_cast<const uint4*>(hi + c0);
@@ -139,10 +160,16 @@ deposit_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ ent
                                fixed_to_float(q3, inv_sc));
         const long long gi = grid * M + ((x0 + lx) * N + (y0 + ly)) * N + (z0 + lz);
         if (mesh_in) {
-          const float4 b = *reinterpret_cast<const float4*>(mesh_in + gi);
+          const float4 b = EARLY ? early : *reinterpret_cast<const float4*>(mesh_in + gi);
           v = make_float4(__fadd_rn(b.x, v.x), __fadd_rn(b.y, v.y), __fadd_rn(b.z, v.z), __fadd_rn(b.w, v.w));
         }
         *reinterpret_cast<float4*>(mesh_out + gi) = v;
+      };
+      if constexpr (EARLY) {
+#pragma unroll
+        for (int q = 0; q < CELLS4; ++q) cell4(threadIdx.x + q * DEP_THREADS, base[q]);
+      } else {
+        for (int k = threadIdx.x; k < TILE3 / 4; k += DEP_THREADS) cell4(k, base[0]);
       }
     } else {
       for (int k = threadIdx.x; k < TILE3; k += DEP_THREADS) {
