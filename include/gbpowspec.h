@@ -289,10 +289,11 @@ int gbp_fft_power(gbp_fft_plan plan, const float* mesh, void* spectrum,
  * Outputs as gbp_deposit (stats_out, required: it carries the mass the
  * binning and the normalisation use) followed by gbp_fft_power; `spectrum`
  * is scratch of the plan's spectrum size.  The particles are bucketed by
- * column tile in one pass into buckets of fixed capacity (twice the mean
- * fill of a uniform catalogue of n_particles, plus 64); what overflows one
- * (a dense clump) goes to lists that the tile collects in the same call, same
- * results, GBP_STATS_REFILLED in stats_out->flags.
+ * column tile in one pass, each written once, into buckets of fixed capacity
+ * (twice the mean fill of a uniform catalogue of n_particles and a little);
+ * what overflows one (a dense clump) goes to lists that the tile collects in
+ * the same call, same results.  GBP_STATS_REFILLED in stats_out->flags: some
+ * tile holds more than twice the mean plus 64 entries.
  * Replaces src/mas.py:88-153 + src/correlations.py:7-56 for the production
  * path. */
 int gbp_particles_power_workspace_size(int64_t n_particles, gbp_fft_plan plan,

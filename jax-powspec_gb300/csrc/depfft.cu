@@ -3,7 +3,7 @@
 //
 // The column tile (TX x TY pencils over all of z) is a plan option:
 // gbp_fft_plan_set_tiles picks one of column_tile_variants(N); zero means
-// the default (8x4 at 256^3, and at 512^3 with one grid; 4x4 otherwise).  Every shape gives
+// the default (8x4 at 256^3 and 512^3 with one grid, else 4x4).  Every shape gives
 // the same P_l bit for bit (fixed-point scales per 4x4 block, see
 // depfft_impl.cuh); they differ in speed only.
 #include <cstdint>
@@ -60,9 +60,10 @@ int plan_tiles(gbp_fft_plan plan, int& tx, int& ty) {
   if (!plan || tile_variants(plan->n, v) == 0) return GBP_ERR_UNSUPPORTED;
   tx = plan->tx ? plan->tx : v[0][0];
   ty = plan->ty ? plan->ty : v[0][1];
-  // two grids at 512^3: a unit is 4x4 pencils, and an 8x4 bucket would be read twice (4 Mi particles TSC
-  // 1.91 against 1.96 ms per mock, CIC 1.65 against 1.70; 9 M PCS 3.25 against 3.07)
-  if (!plan->tx && plan->n == 512 && plan->grids == 2) tx = ty = 4;
+  // two grids: both grids' cells of 4x4 pencils go through shared memory at once, and a particle is written
+  // to its bucket once whatever the tile (512^3, 4 Mi particles TSC 1.81 against 1.87 ms per mock with 8x4,
+  // 9 M PCS 2.64 against 2.93, 0.5 M TSC 1.57 against 1.54; 256^3, 1 M TSC 0.282 against 0.286)
+  if (!plan->tx && (plan->n == 512 || plan->n == 256) && plan->grids == 2) tx = ty = 4;
   return GBP_OK;
 }
 

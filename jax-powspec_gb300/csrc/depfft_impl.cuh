@@ -5,8 +5,9 @@
 //
 // The mesh is never written.  Particles are bucketed (deposit_core.cuh) by
 // column tile: TX x TY pencils spanning the whole z axis (the tile shape is
-// a plan option: 4x4, 8x4 or 8x8, see column_tile_variants), so a stencil is
-// replicated across x and y tile faces only.  One CTA per column tile:
+// a plan option: 4x4, 8x4 or 8x8, see column_tile_variants), each in the tile
+// of its first node, by which faces its stencil crosses.  One CTA per column
+// tile reads its own bucket and the crossing parts of three neighbours':
 //
 //   1. accumulates its bucket in shared memory as 32-bit fixed point.  Each
 //      4x4-pencil block of the tile has a scale of its own, 2^s with
@@ -89,7 +90,8 @@ struct Unit {
   static constexpr int NT = NFFT < 256 ? 256 : NFFT;
   static constexpr int MINB = NT >= 1024 ? 1 : (NT >= 512 ? 2 : 3);   // CTAs per SM the registers are sized for
   static constexpr size_t CELLS = (size_t)2 * PAIRS * N;
-  static constexpr size_t SMEM = CELLS * sizeof(int) + (size_t)CT::NSB * N * sizeof(int);   // + plane counts
+  static constexpr int LIST = 4 * NT;              // entries whose places are kept between the two passes
+  static constexpr size_t SMEM = (CELLS + (size_t)CT::NSB * N + LIST) * sizeof(int);   // cells, plane counts, list
   static_assert(UX * UY * (WIDE ? 2 : 1) <= NARROW_X * NARROW_Y && NT <= 1024, "64-bit cells fit the same bytes");
   // First cell of pencil (lx, ly) of a grid.
   __device__ static __forceinline__ int cell_row(int lx, int ly, int grid) {
@@ -124,9 +126,10 @@ constexpr int SH_MAX = 10;
 // b of the unit (its scale 2^(sg - sh[b]), sh[b] <= SH_MAX).  tm[grid]: the
 // unit's exact totals at the common scale 2^sg (valid in thread 0).
 template <int N, int MAS, int G, class CT, bool WIDE>
-__device__ __forceinline__ void tile_unit(const DepGeom& g, const TileEntries& te, int sg, const int (&sh)[Unit<N, G, CT, WIDE>::NSB],
+__device__ __forceinline__ void tile_unit(const DepGeom& g, const ColEntries& te, int sg, const int (&sh)[Unit<N, G, CT, WIDE>::NSB],
                                           int x0, int y0, int kz_cols, const float2* __restrict__ tw, float2* __restrict__ spec,
-                                          unsigned char* smem, long long (*s_part)[G], long long (&tm)[G]) {
+                                          unsigned char* smem, const unsigned* list, long long (*s_part)[G],
+                                          long long (&tm)[G]) {
   using Cell = typename std::conditional<WIDE, unsigned long long, int>::type;
   using U = Unit<N, G, CT, WIDE>;
   constexpr int R = MAS, UX = U::UX, UY = U::UY, PAIRS = U::PAIRS, NT = U::NT, NSB = U::NSB;
@@ -150,10 +153,9 @@ __device__ __forceinline__ void tile_unit(const DepGeom& g, const TileEntries& t
   __syncthreads();
 #pragma unroll 1
   for (int q = 0; q < 2; ++q) {
-  const float4* ep = q ? te.p[1] : te.p[0];
   const unsigned en = q ? te.n[1] : te.n[0];
   for (unsigned i = tid; i < en; i += NT) {
-    const float4 e = ep[i];
+    const float4 e = q ? te.extra[i] : __ldg(te.entries + (i < U::LIST ? list[i] : column_index(te, i)));
 #pragma unroll
     for (int grid = 0; grid < G; ++grid) {
       Axis<R> ax, ay, az;
@@ -270,10 +272,10 @@ __device__ __forceinline__ void tile_unit(const DepGeom& g, const TileEntries& t
 
 // Every unit of a tile; writes the tile's totals.  sh: the shifts of the tile's scale blocks.
 template <int N, int MAS, int G, class CT, bool WIDE>
-__device__ __forceinline__ void tile_units(const DepGeom& g, const TileEntries& te, int sg, const int (&sh)[CT::NSB],
+__device__ __forceinline__ void tile_units(const DepGeom& g, const ColEntries& te, int sg, const int (&sh)[CT::NSB],
                                            int x0, int y0, int kz_cols, const float2* __restrict__ tw,
-                                           float2* __restrict__ spec, unsigned char* smem, long long (*s_part)[G],
-                                           long long* tile_mass, int ntiles, int t) {
+                                           float2* __restrict__ spec, unsigned char* smem, const unsigned* list,
+                                           long long (*s_part)[G], long long* tile_mass, int ntiles, int t) {
   using U = Unit<N, G, CT, WIDE>;
   long long total[G];
 #pragma unroll
@@ -290,8 +292,8 @@ __device__ __forceinline__ void tile_units(const DepGeom& g, const TileEntries& 
       for (int b = 0; b < U::NSB; ++b) shu[b] = sh[b];
     }
     long long tm[G];
-    tile_unit<N, MAS, G, CT, WIDE>(g, te, sg, shu, x0 + ux, y0 + uy, kz_cols, tw, spec, smem, s_part,
-                                   tm);
+    tile_unit<N, MAS, G, CT, WIDE>(g, te, sg, shu, x0 + ux, y0 + uy, kz_cols, tw, spec, smem, list,
+                                   s_part, tm);
     if (threadIdx.x == 0) {
 #pragma unroll
       for (int q = 0; q < G; ++q) total[q] += tm[q];
@@ -307,14 +309,15 @@ __device__ __forceinline__ void tile_units(const DepGeom& g, const TileEntries& 
 // and inlined their code would cost the others registers.  packed: 8 bits of
 // shift per scale block.
 template <int N, int MAS, int G, class CT>
-__device__ __noinline__ void tile_units_wide(const DepGeom& g, TileEntries te, int sg, unsigned packed, int x0, int y0,
+__device__ __noinline__ void tile_units_wide(const DepGeom& g, ColEntries te, int sg, unsigned packed, int x0, int y0,
                                              int kz_cols, const float2* __restrict__ tw, float2* __restrict__ spec,
-                                             unsigned char* smem, long long (*s_part)[G], long long* tile_mass,
-                                             int ntiles, int t) {
+                                             unsigned char* smem, const unsigned* list, long long (*s_part)[G],
+                                             long long* tile_mass, int ntiles, int t) {
   int sh[CT::NSB];
 #pragma unroll
   for (int b = 0; b < CT::NSB; ++b) sh[b] = (int)((packed >> (8 * b)) & 0xffu);
-  tile_units<N, MAS, G, CT, true>(g, te, sg, sh, x0, y0, kz_cols, tw, spec, smem, s_part, tile_mass, ntiles, t);
+  tile_units<N, MAS, G, CT, true>(g, te, sg, sh, x0, y0, kz_cols, tw, spec, smem, list, s_part, tile_mass, ntiles,
+                                  t);
 }
 
 // Per-block plane counts of a tile (zc [NSB][N], zeroed on entry) and the
@@ -323,22 +326,31 @@ __device__ __noinline__ void tile_units_wide(const DepGeom& g, TileEntries te, i
 // plane z when its nodes (any grid) reach b's 4 x-columns, its 4 y-columns
 // and z.
 template <int N, int MAS, int G, class CT>
-__device__ __forceinline__ bool block_scales(const DepGeom& g, const TileEntries& te, int x0, int y0, int* zc,
-                                             int* s_max, int (&sh)[CT::NSB]) {
+__device__ __forceinline__ bool block_scales(const DepGeom& g, const ColEntries& te, int x0, int y0, int* zc,
+                                             unsigned* list, int* s_max, int (&sh)[CT::NSB]) {
   constexpr int R = MAS, NT = Unit<N, G, CT, false>::NT, NSB = CT::NSB, W = R + G - 1;
+  constexpr unsigned LIST = Unit<N, G, CT, false>::LIST;
   const int tid = threadIdx.x;
   // this pass is the tile's first touch of its bucket: a thread issues EB entry loads at once
   constexpr int EB = 4;
 #pragma unroll 1
   for (int q = 0; q < 2; ++q) {
-  const float4* ep = q ? te.p[1] : te.p[0];
   const unsigned en = q ? te.n[1] : te.n[0];
   for (unsigned i0 = tid; i0 < en; i0 += EB * NT) {
     float4 ev[EB];
 #pragma unroll
     for (int k = 0; k < EB; ++k) {
       const unsigned i = i0 + k * NT;
-      ev[k] = i < en ? ep[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      ev[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i < en) {
+        if (q) {
+          ev[k] = te.extra[i];
+        } else {
+          const unsigned at = column_index(te, i);
+          if (i < LIST) list[i] = at;                  // read by this thread only, in the deposit
+          ev[k] = __ldg(te.entries + at);
+        }
+      }
     }
 #pragma unroll
     for (int k = 0; k < EB; ++k) {
@@ -411,34 +423,37 @@ __device__ __forceinline__ bool block_scales(const DepGeom& g, const TileEntries
 template <int N, int MAS, int G, class CT>
 __global__ void __launch_bounds__(Unit<N, G, CT, false>::NT, Unit<N, G, CT, false>::MINB)
 deposit_fftz_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ entries, const unsigned* __restrict__ counts,
-                    const unsigned* __restrict__ offsets, const __grid_constant__ Spill sp, DepCounters* ctr, int kz_cols,
+                    const __grid_constant__ Spill sp, DepCounters* ctr, int kz_cols,
                     const float2* __restrict__ tw, float2* __restrict__ spec, long long* __restrict__ tile_mass) {
   pdl_wait();
   using U = Unit<N, G, CT, false>;
   constexpr int NT = U::NT, NSB = CT::NSB;
   extern __shared__ __align__(16) int acc_smem[];
   int* zc = acc_smem + U::CELLS;                       // [NSB][N] entries covering each block's planes
+  unsigned* list = reinterpret_cast<unsigned*>(zc + NSB * N);
   __shared__ long long s_part[NT / 32][G];
   __shared__ int s_max[NT / 32];
+  __shared__ ColRuns s_runs;
   const int tid = threadIdx.x;
   const int t = blockIdx.x;
   const int ty = t % g.nt[1], tx = t / g.nt[1];
   const int x0 = tx * CT::TX, y0 = ty * CT::TY;
-  const TileEntries te = tile_entries(g, t, entries, counts, offsets, sp, ctr);
+  const ColEntries te = column_entries(g, tx, ty, entries, counts, sp, ctr, s_runs);
+  if (tid == 0 && te.n[0] + te.n[1] > g.flag_cap) atomicOr(&ctr->outgrown, 1u);
   const int sg = fixed_scale_exp(ctr->maxw_bits, 0);
   for (int k = tid; k < NSB * N; k += NT) zc[k] = 0;
   __syncthreads();
   int sh[NSB];
-  const bool heavy = block_scales<N, MAS, G, CT>(g, te, x0, y0, zc, s_max, sh);
+  const bool heavy = block_scales<N, MAS, G, CT>(g, te, x0, y0, zc, list, s_max, sh);
   unsigned char* cells = reinterpret_cast<unsigned char*>(acc_smem);
   if (heavy) {                                         // uniform over the CTA
     unsigned packed = 0;
 #pragma unroll
     for (int b = 0; b < NSB; ++b) packed |= (unsigned)(sh[b] > SH_MAX ? 0 : sh[b]) << (8 * b);
-    tile_units_wide<N, MAS, G, CT>(g, te, sg, packed, x0, y0, kz_cols, tw, spec, cells, s_part, tile_mass,
-                                   (int)gridDim.x, t);
+    tile_units_wide<N, MAS, G, CT>(g, te, sg, packed, x0, y0, kz_cols, tw, spec, cells, list, s_part,
+                                   tile_mass, (int)gridDim.x, t);
   } else {
-    tile_units<N, MAS, G, CT, false>(g, te, sg, sh, x0, y0, kz_cols, tw, spec, cells, s_part, tile_mass,
+    tile_units<N, MAS, G, CT, false>(g, te, sg, sh, x0, y0, kz_cols, tw, spec, cells, list, s_part, tile_mass,
                                      (int)gridDim.x, t);
   }
 }
@@ -451,8 +466,7 @@ struct PartLayout {
 int particles_layout(int64_t n, gbp_fft_plan plan, gbp_bins B, int mas, int ells, int tx, int ty, PartLayout& L) {
   if (!plan || !B || plan->n != B->N) return GBP_ERR_INVALID;
   if (!plan->own || (plan->grids != 1 && plan->grids != 2)) return GBP_ERR_UNSUPPORTED;
-  const int tile[3] = {tx, ty, B->N};
-  int st = deposit_layout(n, B->N, mas, plan->grids == 2, GBP_COMPAT_NONE, tile, L.dep, true);
+  int st = column_layout(n, B->N, mas, plan->grids == 2, tx, ty, L.dep);
   if (st) return st;
   st = xbin_power_workspace(plan, B, ells, &L.xbin);
   if (st) return st;
@@ -464,13 +478,13 @@ template <int N, int MAS, int G, class CT>
 int run_fused(const DepGeom& g, const DepLayout& L, const DepBuffers& b, int kz_cols, const float2* tw, float2* spec,
               cudaStream_t st) {
   using U = Unit<N, G, CT, false>;
-  int r = bucket_particles<MAS, G, 0>(g, L, b, st);
+  int r = bucket_columns<MAS, G>(g, L, b, st);
   if (r) return r;
   auto k = deposit_fftz_kernel<N, MAS, G, CT>;
   GBP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)U::SMEM));
   {
     GBP_TRACE("deposit_fft_z", st);
-    GBP_CUDA_TRY(launch_pdl(k, dim3(L.ntiles), dim3(U::NT), U::SMEM, st, g, b.entries, b.counts, b.offsets, b.spill,
+    GBP_CUDA_TRY(launch_pdl(k, dim3(L.ntiles), dim3(U::NT), U::SMEM, st, g, b.entries, b.counts, b.spill,
                             b.ctr, kz_cols, tw, spec, b.tile_mass));
   }
   return GBP_OK;
@@ -513,6 +527,8 @@ int particles_power_n(DepGeom g, int64_t n_launch, gbp_fft_plan plan, gbp_bins B
   for (int a = 0; a < 3; ++a) { g.td[a] = L.dep.td[a]; g.ts[a] = L.dep.ts[a]; g.nt[a] = L.dep.nt[a]; }
   g.vec_ok = 0;
   g.tcap = L.dep.tcap;
+  g.flag_cap = L.dep.flag_cap;
+  for (int c = 0; c < 4; ++c) { g.ccap[c] = L.dep.ccap[c]; g.coff[c] = L.dep.coff[c]; }
   const int G = plan->grids;
   float2* spec = static_cast<float2*>(spectrum);
   GBP_CUDA_TRY(cudaMemsetAsync(b.ctr, 0, zeroed_bytes(L.dep), st));

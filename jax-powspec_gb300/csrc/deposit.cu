@@ -80,6 +80,7 @@ deposit_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ ent
     for (int k = threadIdx.x; k < 2 * TILE3 / 4; k += DEP_THREADS) a4[k] = make_uint4(0u, 0u, 0u, 0u);
   }
   const TileEntries te = tile_entries(g, t, entries, counts, offsets, sp, ctr);
+  if (threadIdx.x == 0 && te.n[0] + te.n[1] > g.flag_cap) atomicOr(&ctr->outgrown, 1u);
   const int s = fixed_scale_exp(ctr->maxw_bits, CM);
   const float sc = ldexpf(1.0f, s);
   const float inv_sc = ldexpf(1.0f, -s);
@@ -219,6 +220,7 @@ int deposit_launch(DepGeom g, const DepLayout& L, int64_t n, int mas, int G, int
   const DepBuffers b = carve_deposit(workspace, L);
   for (int a = 0; a < 3; ++a) { g.td[a] = L.td[a]; g.ts[a] = L.ts[a]; g.nt[a] = L.nt[a]; }
   g.tcap = L.tcap;
+  g.flag_cap = L.flag_cap;
   g.vec_ok = ((reinterpret_cast<uintptr_t>(mesh_out) | reinterpret_cast<uintptr_t>(mesh_in)) & 15u) == 0;
   GBP_CUDA_TRY(cudaMemsetAsync(b.ctr, 0, zeroed_bytes(L), stream));
   int st;

@@ -43,17 +43,26 @@ struct DepGeom {
   const gbp_job* job;  // non-null: particles, n and box geometry are read from here
   long long cap;       // job mode: the capacity the launches were sized for
   unsigned tcap;       // > 0: buckets of a fixed capacity, tile t's at entry t * tcap (fill path)
+  unsigned flag_cap;   // entries of a tile beyond which GBP_STATS_REFILLED is reported
+  unsigned ccap[4];    // column tiles: capacity of each class's part of a bucket
+  unsigned coff[4];    // and where in the bucket it starts
 };
 
 // Job mode: the particle pointers, count and box geometry come from a
 // gbp_job in device memory (one broadcast load per thread), so the launch
-// parameters do not depend on the mock.
-__device__ __forceinline__ void resolve_job(DepGeom& g) {
-  if (!g.job) return;
-  const gbp_job j = *g.job;
-  g.x = j.x; g.y = j.y; g.z = j.z; g.w = j.w;
-  g.n = j.n < 0 ? 0 : (j.n > g.cap ? g.cap : j.n);   // the buckets hold `cap` particles at most
-  g.ox = j.xmin; g.oy = j.ymin; g.oz = j.zmin; g.inv_cell = j.inv_cell;
+// parameters do not depend on the mock.  A compile-time choice: with the job's
+// and the parameters' fields merged at run time the compiler (nvcc 13.0) kept
+// the parameters' x beside the job's y, z and n.
+template <bool JOB>
+__device__ __forceinline__ DepGeom catalogue_of(const DepGeom& gp) {
+  DepGeom g = gp;
+  if constexpr (JOB) {
+    const gbp_job j = *gp.job;
+    g.x = j.x; g.y = j.y; g.z = j.z; g.w = j.w;
+    g.n = j.n < 0 ? 0 : (j.n > gp.cap ? gp.cap : j.n);   // the buckets hold `cap` particles at most
+    g.ox = j.xmin; g.oy = j.ymin; g.oz = j.zmin; g.inv_cell = j.inv_cell;
+  }
+  return g;
 }
 
 // Node index reduced into [0, N).  Stencil nodes lie within a few cells of
@@ -246,20 +255,29 @@ __device__ __forceinline__ ff warp_ff_sum(ff v) {
 struct DepCounters {           // zeroed by one memset per call
   unsigned int maxw_bits;
   unsigned int n_spill;        // fill path: entries beyond their bucket's capacity
-  unsigned int n_extra;        // spilled entries listed by their tiles so far (tile_entries)
-  unsigned int pad_;
+  unsigned int n_extra;        // spilled entries gathered by their tiles so far
+  unsigned int outgrown;       // some tile has more entries than DepGeom::flag_cap
 };
 
-// Fill path: the entries beyond a bucket's capacity.  Entry s is particle
-// node[s].x of tile tile[s]; heads holds HEADS lists per tile of them
-// (node index + 1, 0 ends a list), linked through node[s].y.
+// Fill path: the entries beyond a bucket's capacity.  heads holds HEADS lists
+// per tile of them (node + 1, 0 ends a list), linked through next.
 constexpr unsigned HEADS = CSTRIDE;
 struct Spill {
   unsigned* heads;      // [ntiles * HEADS], zeroed
-  uint2* node;          // [n * maxrep]
-  unsigned* tile;       // [n * maxrep]
-  float4* extra;        // [n * maxrep] (u, w) of the tiles that gathered theirs
+  unsigned* next;       // [nspill]
+  unsigned* tile;       // [nspill] (column tiles: 4 * tile + class)
+  float4* entry;        // [nspill] (u, w)
+  float4* extra;        // [nextra] copies gathered by the tiles, contiguous per tile
 };
+
+// Puts an entry on list `head`; `lists` (a power of two) of them start at it.
+__device__ __forceinline__ void spill_entry(const Spill& sp, DepCounters* ctr, unsigned tile, size_t head,
+                                            unsigned lists, const float4& e) {
+  const unsigned s = atomicAdd(&ctr->n_spill, 1u);
+  sp.tile[s] = tile;
+  sp.entry[s] = e;
+  sp.next[s] = atomicExch(&sp.heads[head + (s & (lists - 1))], s + 1u);
+}
 
 // Block reductions of the weight statistics in a fixed order (deterministic
 // partials per particle block), and the global max |w|.
@@ -293,13 +311,12 @@ __device__ __forceinline__ void flush_block_stats(float maxw, ff sw, ff sw2, uns
 }
 
 // Pass 1: tile occupancy counts + weight statistics.
-template <int MAS, int G, int CM>
+template <int MAS, int G, int CM, bool JOB>
 __global__ void __launch_bounds__(CNT_THREADS)
 count_kernel(DepGeom gp, unsigned* __restrict__ counts, DepCounters* ctr, float4* block_stats,
              uint2* block_counts) {
   pdl_wait();
-  DepGeom g = gp;
-  resolve_job(g);
+  const DepGeom g = catalogue_of<JOB>(gp);
   float maxw = 0.0f;
   ff sw{0.f, 0.f}, sw2{0.f, 0.f};
   unsigned kept = 0, bad = 0;
@@ -341,20 +358,12 @@ count_kernel(DepGeom gp, unsigned* __restrict__ counts, DepCounters* ctr, float4
 // same particle blocks.
 // Registers for 5 CTAs per SM: its returning atomics want warps in flight
 // (0.151 -> 0.142 ms for 4 Mi particles at 512^3 against 4 CTAs per SM).
-__device__ __forceinline__ void spill_entry(const Spill& sp, DepCounters* ctr, int t, int k) {
-  const unsigned i = blockIdx.x * (CNT_THREADS * CNT_ITEMS) + k * CNT_THREADS + threadIdx.x;   // as load_batch
-  const unsigned s = atomicAdd(&ctr->n_spill, 1u);
-  sp.tile[s] = (unsigned)t;
-  sp.node[s] = make_uint2(i, atomicExch(&sp.heads[(size_t)t * HEADS + (s & (HEADS - 1))], s + 1u));
-}
-
-template <int MAS, int G, int CM>
+template <int MAS, int G, int CM, bool JOB>
 __global__ void __launch_bounds__(CNT_THREADS, 5)
 fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entries, Spill sp, DepCounters* ctr,
             float4* block_stats, uint2* block_counts) {
   pdl_wait();
-  DepGeom g = gp;
-  resolve_job(g);
+  const DepGeom g = catalogue_of<JOB>(gp);
   const unsigned tcap = g.tcap;
   float maxw = 0.0f;
   ff sw{0.f, 0.f}, sw2{0.f, 0.f};
@@ -391,7 +400,7 @@ fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entr
       for (int q = 0; q < 8; ++q)
         if (tt[q] >= 0) {
           if (slot[q] < tcap) entries[(unsigned)tt[q] * tcap + slot[q]] = e;
-          else spill_entry(sp, ctr, tt[q], k);
+          else spill_entry(sp, ctr, (unsigned)tt[q], (size_t)tt[q] * HEADS, HEADS, e);
         }
     } else {
       for (int a = 0; a < nx; ++a)
@@ -400,7 +409,7 @@ fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entr
             const int t = (pick3(a, x0, x1, x2) * g.nt[1] + pick3(b, y0, y1, y2)) * g.nt[2] + pick3(c, z0, z1, z2);
             const unsigned slot = atomicAdd(&counts[t * CSTRIDE], 1u);
             if (slot < tcap) entries[(unsigned)t * tcap + slot] = e;
-            else spill_entry(sp, ctr, t, k);
+            else spill_entry(sp, ctr, (unsigned)t, (size_t)t * HEADS, HEADS, e);
           }
     }
     maxw = fmaxf(maxw, fabsf(w));
@@ -408,6 +417,191 @@ fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entr
     sw2 = ff_add_f(sw2, __fmul_rn(w, w));
   }
   flush_block_stats(maxw, sw, sw2, kept, bad, ctr, block_stats, block_counts);
+}
+
+// Column tiles (TX x TY pencils over all of z; power-of-two meshes, TX, TY >=
+// 4): a particle is written once, to the tile of its first node in x and y,
+// into the part of the bucket of its class: 2 * (its nodes reach the next
+// tile in x) + (in y).  A tile's entries are then nine runs (column_entries):
+// its own four parts, the left neighbour's two that cross in x, the lower
+// neighbour's two that cross in y, the diagonal one's that crosses in both.
+// One atomic and one 16-byte store per particle instead of one per tile it
+// touches (3.1 for TSC with two grids and 4x4 tiles): the returning atomics
+// set this pass's time, 15 us per million (512^3, 4 Mi particles TSC, two
+// grids: 0.190 -> 0.063 ms; 256^3, 1 M: 0.047 -> 0.022; 1024^3, 16 Mi PCS:
+// 1.28 -> 0.32), for 2 % more in the kernel that finds the runs.
+constexpr int CLS = CSTRIDE / 4;              // words between a tile's four class counters (a sector each)
+constexpr int CLS_HEADS = HEADS / 4;          // spill lists per tile and class
+
+// v[c] by selects (no local memory).
+__device__ __forceinline__ unsigned pick4(unsigned c, const unsigned (&v)[4]) {
+  return (c & 2u) ? ((c & 1u) ? v[3] : v[2]) : ((c & 1u) ? v[1] : v[0]);
+}
+
+template <int MAS, int G>
+__device__ __forceinline__ int column_axis(const DepGeom& g, int ax, float u, int& cross) {
+  Axis<MAS> a;
+  make_axis<MAS, 0>(g, u, 0, a);
+  int last = a.first + MAS - 1;
+  if constexpr (G == 2) {
+    Axis<MAS> b;
+    make_axis<MAS, 0>(g, u, 1, b);
+    last = b.first + MAS - 1;                 // b.first is a.first or a.first + 1
+  }
+  const int f = a.first & (g.N - 1);
+  cross = (f & (g.td[ax] - 1)) + (last - a.first) >= g.td[ax] ? 1 : 0;
+  return f >> g.ts[ax];
+}
+
+template <int MAS, int G, bool JOB>
+__global__ void __launch_bounds__(CNT_THREADS, 5)
+fill_columns_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entries, Spill sp,
+                    DepCounters* ctr, float4* block_stats, uint2* block_counts) {
+  pdl_wait();
+  const DepGeom g = catalogue_of<JOB>(gp);
+  float maxw = 0.0f;
+  ff sw{0.f, 0.f}, sw2{0.f, 0.f};
+  unsigned kept = 0, bad = 0;
+  Batch bt;
+  load_batch(g, bt, blockIdx.x);
+  float4 e[CNT_ITEMS];
+  int tc[CNT_ITEMS];                          // 4 * tile + class, -1: dropped
+  unsigned slot[CNT_ITEMS];
+#pragma unroll
+  for (int k = 0; k < CNT_ITEMS; ++k) {       // every particle's claim in flight before the first store
+    tc[k] = -1;
+    if (!bt.in[k]) continue;
+    float u[3];
+    const float w = bt.w[k];
+    if (!grid_coords(g, bt.x[k], bt.y[k], bt.z[k], u)) { ++bad; continue; }
+    int cx, cy;
+    const int tx = column_axis<MAS, G>(g, 0, u[0], cx), ty = column_axis<MAS, G>(g, 1, u[1], cy);
+    ++kept;
+    e[k] = make_float4(u[0], u[1], u[2], w);
+    const int t = tx * g.nt[1] + ty, c = 2 * cx + cy;
+    tc[k] = 4 * t + c;
+    slot[k] = atomicAdd(&counts[(size_t)t * CSTRIDE + c * CLS], 1u);
+    maxw = fmaxf(maxw, fabsf(w));
+    sw = ff_add_f(sw, w);
+    sw2 = ff_add_f(sw2, __fmul_rn(w, w));
+  }
+#pragma unroll
+  for (int k = 0; k < CNT_ITEMS; ++k) {
+    if (tc[k] < 0) continue;
+    const unsigned t = (unsigned)tc[k] >> 2, c = (unsigned)tc[k] & 3u;
+    if (slot[k] < pick4(c, g.ccap)) {
+      entries[(size_t)t * g.tcap + pick4(c, g.coff) + slot[k]] = e[k];
+    } else {
+      spill_entry(sp, ctr, (unsigned)tc[k], (size_t)t * HEADS + c * CLS_HEADS, CLS_HEADS, e[k]);
+    }
+  }
+  flush_block_stats(maxw, sw, sw2, kept, bad, ctr, block_stats, block_counts);
+}
+
+// The nine runs of a column tile's entries: entry i of the buckets lies at
+// i + delta[r], r the last run with pre[r] <= i (runs 9.. never are).
+struct ColRuns {
+  unsigned pre[16], delta[16];
+  unsigned spilled[9], code[9];               // entries beyond the bucket, 4 * tile + class
+  unsigned total, n_spilled, base, fill;
+};
+
+struct ColEntries {
+  const float4* entries;
+  const ColRuns* runs;
+  const float4* extra;
+  unsigned n[2];                              // in buckets, spilled
+};
+
+// Where entry i of the buckets lies.
+__device__ __forceinline__ unsigned column_index(const ColEntries& te, unsigned i) {
+  const ColRuns& r = *te.runs;
+  int q = i >= r.pre[8] ? 8 : 0;
+  if (i >= r.pre[q + 4]) q += 4;
+  if (i >= r.pre[q + 2]) q += 2;
+  if (i >= r.pre[q + 1]) q += 1;
+  return i + r.delta[q];
+}
+
+// Collects a column tile's spilled entries into a slice of sp.extra of its own
+// (every thread of the block calls): run by run, eight lanes walk the lists of
+// the run's class; a run that holds more than 64 entries per list and a
+// sixteenth of all spilled ones (a point mass) has the block look through
+// them all instead.
+__device__ __noinline__ const float4* gather_columns(const Spill& sp, DepCounters* ctr, ColRuns& r) {
+  if (threadIdx.x == 0) {
+    r.base = atomicAdd(&ctr->n_extra, r.n_spilled);
+    r.fill = 0;
+  }
+  __syncthreads();
+  float4* out = sp.extra + r.base;
+  auto put = [&](unsigned s) {
+    const unsigned q = atomicAdd(&r.fill, 1u);
+    if (q < r.n_spilled) out[q] = sp.entry[s];
+  };
+  const unsigned all = ctr->n_spill;
+  for (int k = 0; k < 9; ++k) {
+    const unsigned n = r.spilled[k], code = r.code[k];
+    if (n > 64 * CLS_HEADS && n > all / 16) {
+      for (unsigned j = threadIdx.x; j < all; j += blockDim.x)
+        if (sp.tile[j] == code) put(j);
+    } else if (n && threadIdx.x < CLS_HEADS) {
+      unsigned v = sp.heads[(size_t)(code >> 2) * HEADS + (code & 3u) * CLS_HEADS + threadIdx.x];
+      for (unsigned j = 0; v != 0u && j < n; ++j) {
+        put(v - 1u);
+        v = sp.next[v - 1u];
+      }
+    }
+  }
+  __syncthreads();
+  return out;
+}
+
+// Every thread of the block calls; ends with a barrier.
+__device__ __forceinline__ ColEntries column_entries(const DepGeom& g, int tx, int ty, const float4* entries,
+                                                     const unsigned* counts, const Spill& sp, DepCounters* ctr,
+                                                     ColRuns& r) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    unsigned m = 0, code = 0, c = 0;
+    if (lane < 9) {
+      // own 0..3 | left, crossing in x: 2, 3 | lower, crossing in y: 1, 3 | diagonal: 3
+      const int dx = (lane == 4 || lane == 5 || lane == 8) ? 1 : 0, dy = lane >= 6 ? 1 : 0;
+      const int cls = lane < 4 ? lane : (lane == 4 ? 2 : (lane == 6 ? 1 : 3));
+      const int ntx = g.nt[0], nty = g.nt[1];
+      const int t = ((tx + ntx - dx) & (ntx - 1)) * nty + ((ty + nty - dy) & (nty - 1));
+      code = 4u * t + cls;
+      c = counts[(size_t)t * CSTRIDE + cls * CLS];
+      m = min(c, g.ccap[cls]);
+    }
+    unsigned inc = m;
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+      const unsigned v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    const unsigned all = __reduce_add_sync(0xffffffffu, c - m);
+    if (lane < 16) {
+      const unsigned first = lane < 9 ? (code >> 2) * g.tcap + g.coff[code & 3u] : 0u;
+      r.pre[lane] = lane < 9 ? inc - m : 0xffffffffu;
+      r.delta[lane] = first - (inc - m);
+      if (lane < 9) {
+        r.spilled[lane] = c - m;
+        r.code[lane] = code;
+      }
+      if (lane == 8) r.total = inc;
+      if (lane == 0) r.n_spilled = all;
+    }
+  }
+  __syncthreads();
+  ColEntries te;
+  te.entries = entries;
+  te.runs = &r;
+  te.n[0] = r.total;
+  te.n[1] = r.n_spilled;
+  te.extra = nullptr;
+  if (te.n[1]) te.extra = gather_columns(sp, ctr, r);
+  return te;
 }
 
 // The entries of one tile in two parts: n[0] in its bucket, n[1] beyond its
@@ -418,12 +612,11 @@ struct TileEntries {
   unsigned n[2];
 };
 
-// Collects a tile's n spilled particles into a slice of `extra` of its own
+// Collects a tile's n spilled entries into a slice of `extra` of its own
 // (every thread of the block calls).  One warp walks the tile's HEADS lists;
 // a tile that holds more than 64 entries per list and a sixteenth of all
 // spilled ones (a point mass) has the block look through them all instead.
-__device__ __noinline__ const float4* gather_spilled(const DepGeom& gp, const Spill& sp, DepCounters* ctr, int t,
-                                                     unsigned n) {
+__device__ __noinline__ const float4* gather_spilled(const Spill& sp, DepCounters* ctr, int t, unsigned n) {
   __shared__ unsigned s_base, s_n;
   if (threadIdx.x == 0) {
     s_base = atomicAdd(&ctr->n_extra, n);
@@ -431,24 +624,19 @@ __device__ __noinline__ const float4* gather_spilled(const DepGeom& gp, const Sp
   }
   __syncthreads();
   float4* out = sp.extra + s_base;
-  DepGeom g = gp;
-  resolve_job(g);
-  auto put = [&](unsigned i) {
+  auto put = [&](unsigned s) {
     const unsigned q = atomicAdd(&s_n, 1u);
-    float u[3];
-    grid_coords(g, g.x[i], g.y[i], g.z[i], u);
-    if (q < n) out[q] = make_float4(u[0], u[1], u[2], g.w ? g.w[i] : 1.0f);
+    if (q < n) out[q] = sp.entry[s];
   };
   const unsigned all = ctr->n_spill;
   if (n > 64 * HEADS && n > all / 16) {
     for (unsigned k = threadIdx.x; k < all; k += blockDim.x)
-      if (sp.tile[k] == (unsigned)t) put(sp.node[k].x);
+      if (sp.tile[k] == (unsigned)t) put(k);
   } else if (threadIdx.x < HEADS) {
     unsigned v = sp.heads[(size_t)t * HEADS + threadIdx.x];
     for (unsigned k = 0; v != 0u && k < n; ++k) {
-      const uint2 nd = sp.node[v - 1u];
-      put(nd.x);
-      v = nd.y;
+      put(v - 1u);
+      v = sp.next[v - 1u];
     }
   }
   __syncthreads();
@@ -464,18 +652,17 @@ __device__ __forceinline__ TileEntries tile_entries(const DepGeom& g, int t, con
   te.n[0] = g.tcap ? min(c, g.tcap) : c;
   te.n[1] = c - te.n[0];
   te.p[0] = entries + (g.tcap ? (size_t)t * g.tcap : (size_t)offsets[t]);
-  te.p[1] = te.n[1] ? gather_spilled(g, sp, ctr, t, te.n[1]) : te.p[0];
+  te.p[1] = te.n[1] ? gather_spilled(sp, ctr, t, te.n[1]) : te.p[0];
   return te;
 }
 
 // Pass 3: append (u_x, u_y, u_z, w) to every touched tile's bucket.
-template <int MAS, int G, int CM>
+template <int MAS, int G, int CM, bool JOB>
 __global__ void __launch_bounds__(CNT_THREADS, 4)
 scatter_kernel(DepGeom gp, const unsigned* __restrict__ offsets, unsigned* __restrict__ fills,
                float4* __restrict__ entries) {
   pdl_wait();
-  DepGeom g = gp;
-  resolve_job(g);
+  const DepGeom g = catalogue_of<JOB>(gp);
   {
     Batch bt;
     load_batch(g, bt, blockIdx.x);
@@ -631,15 +818,18 @@ stats_kernel(const DepCounters* ctr, const float4* block_stats, const uint2* blo
     out->n_kept = tk;
     out->n_nonfinite = tbad;
     out->scale_exp = s;
-    out->flags = ctr->n_spill ? GBP_STATS_REFILLED : 0;
+    out->flags = ctr->outgrown ? GBP_STATS_REFILLED : 0;
   }
 }
 
 struct DepLayout {
   int td[3], ts[3], nt[3], ntiles, maxrep, nblocks;
   unsigned tcap;        // fill path: entries per bucket (0: count path)
+  unsigned flag_cap;    // DepGeom::flag_cap
+  unsigned ccap[4], coff[4];   // column tiles: each class's part of the bucket
   size_t nentries;      // entries the bucket buffer holds
   size_t nspill;        // fill path: entries that may lie beyond their buckets
+  size_t nextra;        // and copies of them that the tiles may gather
   size_t scan_bytes;
   size_t total;
 };
@@ -659,6 +849,19 @@ struct StrideLoad {
 inline thrust::transform_iterator<StrideLoad, thrust::counting_iterator<int>> strided_counts(const unsigned* p) {
   return thrust::make_transform_iterator(thrust::counting_iterator<int>(0), StrideLoad{p});
 }
+
+void finish_layout(DepLayout& L);
+
+// Mean entries per tile of a uniform catalogue of n particles (a span of
+// `width` nodes reaches the next tile along an axis with probability
+// (width - 1) / td), and the capacity of a bucket for it.
+double mean_fill(int64_t n, int N, int width, const DepLayout& L) {
+  double rep = 1.0;
+  for (int a = 0; a < 3; ++a)
+    if (L.td[a] < N) rep *= 1.0 + (double)(width - 1) / (double)L.td[a];
+  return (double)n * rep / (double)L.ntiles;
+}
+double bucket_capacity(double mean) { return 4.0 * std::ceil((2.0 * mean + 64.0) / 4.0); }
 
 // Largest number of distinct tiles a run of `width` consecutive nodes can
 // touch along one periodic axis (exact, by enumeration).
@@ -711,27 +914,71 @@ int deposit_layout(int64_t n, int N, int mas, int interlace, int compat, const i
   L.nblocks = (int)((n + (long long)CNT_THREADS * CNT_ITEMS - 1) / ((long long)CNT_THREADS * CNT_ITEMS));
   L.tcap = 0;
   L.nentries = (size_t)n * L.maxrep + 1;
-  L.nspill = 0;
+  L.nspill = L.nextra = 0;
+  L.flag_cap = 0xffffffffu;
   if (fill && n > 0) {
-    double rep = 1.0;
-    for (int a = 0; a < 3; ++a)
-      if (L.td[a] < N) rep *= 1.0 + (double)(width - 1) / (double)L.td[a];
-    const double mean = (double)n * rep / (double)L.ntiles;
-    const double cap = 4.0 * std::ceil((2.0 * mean + 64.0) / 4.0);
+    const double mean = mean_fill(n, N, width, L), cap = bucket_capacity(mean);
+    if (mean >= 32.0) L.flag_cap = (unsigned)std::min(cap, 4294967295.0);
     if ((mean >= 32.0 || cap * (double)L.ntiles <= 16777216.0) && cap * (double)L.ntiles < 4294967295.0) {
       L.tcap = (unsigned)cap;
-      L.nspill = L.nentries;
+      L.nspill = L.nextra = L.nentries;
       L.nentries = (size_t)L.tcap * (size_t)L.ntiles + 1;
     }
   }
+  finish_layout(L);
+  return GBP_OK;
+}
+
+// Column tiles of tx x ty pencils (both powers of two >= 4 that divide N/2),
+// always one pass: class c's part of a bucket holds twice its mean fill of a
+// uniform catalogue plus 48 (what overflows it costs a list;
+// GBP_STATS_REFILLED is reported at the capacity a bucket of all the tile's
+// entries would have).  Nodes first .. last of all grids span MAS - 1 cells,
+// or half a cell more on average with two grids, so they reach the next tile
+// along an axis with probability span / tx.
+int column_layout(int64_t n, int N, int mas, int interlace, int tx, int ty, DepLayout& L) {
+  if (n < 0) return GBP_ERR_INVALID;
+  if (mas < GBP_NGP || mas > GBP_PCS) return GBP_ERR_INVALID;
+  const int td[3] = {tx, ty, N};
+  L.maxrep = 4;
+  for (int a = 0; a < 3; ++a) {
+    L.td[a] = td[a];
+    L.ts[a] = __builtin_ctz(td[a]);
+    L.nt[a] = N / td[a];
+  }
+  L.ntiles = L.nt[0] * L.nt[1];
+  if ((double)n * L.maxrep >= 4294967295.0) return GBP_ERR_UNSUPPORTED;
+  L.nblocks = (int)((n + (long long)CNT_THREADS * CNT_ITEMS - 1) / ((long long)CNT_THREADS * CNT_ITEMS));
+  const double all = mean_fill(n, N, mas + (interlace ? 1 : 0), L);
+  L.flag_cap = all >= 32.0 ? (unsigned)std::min(bucket_capacity(all), 4294967295.0) : 0xffffffffu;
+  const double span = mas - 1 + (interlace ? 0.5 : 0.0), mean = (double)n / (double)L.ntiles;
+  double off = 0.0;
+  for (int c = 0; c < 4; ++c) {
+    const double px = span / tx, py = span / ty;
+    const double m = mean * ((c & 2) ? px : 1.0 - px) * ((c & 1) ? py : 1.0 - py);
+    const double cap = 4.0 * std::ceil((2.0 * m + 48.0) / 4.0);
+    L.coff[c] = (unsigned)off;
+    L.ccap[c] = (unsigned)cap;
+    off += cap;
+  }
+  if (off * (double)L.ntiles >= 4294967295.0) return GBP_ERR_UNSUPPORTED;
+  L.tcap = (unsigned)off;
+  L.nentries = (size_t)L.tcap * (size_t)L.ntiles + 1;
+  L.nspill = (size_t)n + 1;
+  L.nextra = (size_t)n * L.maxrep + 1;
+  finish_layout(L);
+  return GBP_OK;
+}
+
+// The rest of a layout, from its tiles, blocks and buckets.
+void finish_layout(DepLayout& L) {
   L.scan_bytes = 0;
   if (!L.tcap) cub::DeviceScan::ExclusiveSum(nullptr, L.scan_bytes, strided_counts(nullptr), (unsigned*)nullptr, L.ntiles);
   const size_t nbl = (size_t)(L.nblocks > 0 ? L.nblocks : 1);
   L.total = zeroed_bytes(L) + align256((size_t)L.ntiles * 4) + align256(nbl * sizeof(float4)) +
             align256(nbl * sizeof(uint2)) + align256((size_t)L.ntiles * 2 * sizeof(long long)) +
-            align256(L.nentries * sizeof(float4)) + align256(L.scan_bytes) + align256(L.nspill * sizeof(uint2)) +
-            align256(L.nspill * sizeof(unsigned)) + align256(L.nspill * sizeof(float4));
-  return GBP_OK;
+            align256(L.nentries * sizeof(float4)) + align256(L.scan_bytes) + 2 * align256(L.nspill * sizeof(unsigned)) +
+            align256(L.nspill * sizeof(float4)) + align256(L.nextra * sizeof(float4));
 }
 
 // Workspace slices shared by both deposit paths.
@@ -762,9 +1009,10 @@ inline DepBuffers carve_deposit(void* workspace, const DepLayout& L) {
   b.entries = cv.take<float4>(L.nentries);
   b.scan_tmp = cv.take<char>(L.scan_bytes);
   b.spill.heads = b.fills;
-  b.spill.node = cv.take<uint2>(L.nspill);
+  b.spill.next = cv.take<unsigned>(L.nspill);
   b.spill.tile = cv.take<unsigned>(L.nspill);
-  b.spill.extra = cv.take<float4>(L.nspill);
+  b.spill.entry = cv.take<float4>(L.nspill);
+  b.spill.extra = cv.take<float4>(L.nextra);
   return b;
 }
 
@@ -772,17 +1020,18 @@ inline DepBuffers carve_deposit(void* workspace, const DepLayout& L) {
 // workspace must be zero on entry).
 template <int MAS, int G, int CM>
 int bucket_particles(const DepGeom& g, const DepLayout& L, const DepBuffers& b, cudaStream_t st) {
+  const bool job = g.job != nullptr;                 // B-spline deposits only
   if (L.tcap) {
     if (L.nblocks > 0) {
       GBP_TRACE("deposit_fill", st);
-      GBP_CUDA_TRY(launch_pdl(fill_kernel<MAS, G, CM>, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts,
+      GBP_CUDA_TRY(launch_pdl(job ? fill_kernel<MAS, G, CM, CM == 0> : fill_kernel<MAS, G, CM, false>, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts,
                               b.entries, b.spill, b.ctr, b.block_stats, b.block_counts));
     }
     return GBP_OK;
   }
   if (L.nblocks > 0) {
     GBP_TRACE("deposit_count", st);
-    GBP_CUDA_TRY(launch_pdl(count_kernel<MAS, G, CM>, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts, b.ctr,
+    GBP_CUDA_TRY(launch_pdl(job ? count_kernel<MAS, G, CM, CM == 0> : count_kernel<MAS, G, CM, false>, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts, b.ctr,
                             b.block_stats, b.block_counts));
   }
   {
@@ -793,9 +1042,20 @@ int bucket_particles(const DepGeom& g, const DepLayout& L, const DepBuffers& b, 
   }
   if (L.nblocks > 0) {
     GBP_TRACE("deposit_scatter", st);
-    GBP_CUDA_TRY(launch_pdl(scatter_kernel<MAS, G, CM>, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.offsets,
+    GBP_CUDA_TRY(launch_pdl(job ? scatter_kernel<MAS, G, CM, CM == 0> : scatter_kernel<MAS, G, CM, false>, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.offsets,
                             b.fills, b.entries));
   }
+  return GBP_OK;
+}
+
+// The same for column tiles.
+template <int MAS, int G>
+int bucket_columns(const DepGeom& g, const DepLayout& L, const DepBuffers& b, cudaStream_t st) {
+  if (L.nblocks == 0) return GBP_OK;
+  GBP_TRACE("deposit_fill", st);
+  auto k = g.job ? fill_columns_kernel<MAS, G, true> : fill_columns_kernel<MAS, G, false>;
+  GBP_CUDA_TRY(launch_pdl(k, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts,
+                          b.entries, b.spill, b.ctr, b.block_stats, b.block_counts));
   return GBP_OK;
 }
 

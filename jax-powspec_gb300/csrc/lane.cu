@@ -115,6 +115,20 @@ int lane_sizes(int N, int mas, int interlace, int ells, gbp_bins bins, long long
   int st = gbp_fft_plan_pitch(plan, &s.pitch);
   if (st) return st;
   s.particles = gbp_particles_power_workspace_size(cap, plan, bins, mas, ells, &s.pow) == GBP_OK;
+  if (s.particles) {            // the largest over the tile shapes: a lane's size does not depend on its tile
+    int tx[8], ty[8], nv = 0, tx0 = 0, ty0 = 0;
+    st = gbp_fft_plan_tiles(plan, &tx0, &ty0);
+    if (!st) st = gbp_column_tile_variants(N, tx, ty, 8, &nv);
+    for (int i = 0; !st && i < nv && i < 8; ++i) {
+      size_t b = 0;
+      st = gbp_fft_plan_set_tiles(plan, tx[i], ty[i]);
+      if (!st) st = gbp_particles_power_workspace_size(cap, plan, bins, mas, ells, &b);
+      s.pow = b > s.pow ? b : s.pow;
+    }
+    if (st) return st;
+    st = gbp_fft_plan_set_tiles(plan, tx0, ty0);
+    if (st) return st;
+  }
   if (s.particles) {            // one fused call: no mesh, one workspace
     s.mesh = 0;
     s.dep = 0;
