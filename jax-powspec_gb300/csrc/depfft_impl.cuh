@@ -27,7 +27,7 @@
 //      accumulators; the stages in between run in place (fft_pass.cuh),
 //   3. stores Z(kz) and Z(-kz) from the last stage's registers,
 //   4. adds up the tile's exact integer total at the common scale 2^s_g
-//      (the mean density; stats_kernel folds the tiles).
+//      (the mean density).
 //
 // With two grids a tile is taken in units of 4x4 (1024^3: 4x2) pencils whose
 // both grids fit in shared memory together; with one grid the unit is the
@@ -275,7 +275,7 @@ template <int N, int MAS, int G, class CT, bool WIDE>
 __device__ __forceinline__ void tile_units(const DepGeom& g, const ColEntries& te, int sg, const int (&sh)[CT::NSB],
                                            int x0, int y0, int kz_cols, const float2* __restrict__ tw,
                                            float2* __restrict__ spec, unsigned char* smem, const unsigned* list,
-                                           long long (*s_part)[G], long long* tile_mass, int ntiles, int t) {
+                                           long long (*s_part)[G], long long* tile_mass) {
   using U = Unit<N, G, CT, WIDE>;
   long long total[G];
 #pragma unroll
@@ -300,8 +300,8 @@ __device__ __forceinline__ void tile_units(const DepGeom& g, const ColEntries& t
     }
   }
   if (threadIdx.x == 0) {
-    tile_mass[t] = total[0];
-    tile_mass[(long long)ntiles + t] = G == 2 ? total[G - 1] : 0;
+#pragma unroll
+    for (int q = 0; q < G; ++q) tile_mass[(size_t)q * gridDim.x + blockIdx.x] = total[q];
   }
 }
 
@@ -312,12 +312,11 @@ template <int N, int MAS, int G, class CT>
 __device__ __noinline__ void tile_units_wide(const DepGeom& g, ColEntries te, int sg, unsigned packed, int x0, int y0,
                                              int kz_cols, const float2* __restrict__ tw, float2* __restrict__ spec,
                                              unsigned char* smem, const unsigned* list, long long (*s_part)[G],
-                                             long long* tile_mass, int ntiles, int t) {
+                                             long long* tile_mass) {
   int sh[CT::NSB];
 #pragma unroll
   for (int b = 0; b < CT::NSB; ++b) sh[b] = (int)((packed >> (8 * b)) & 0xffu);
-  tile_units<N, MAS, G, CT, true>(g, te, sg, sh, x0, y0, kz_cols, tw, spec, smem, list, s_part, tile_mass, ntiles,
-                                  t);
+  tile_units<N, MAS, G, CT, true>(g, te, sg, sh, x0, y0, kz_cols, tw, spec, smem, list, s_part, tile_mass);
 }
 
 // Per-block plane counts of a tile (zc [NSB][N], zeroed on entry) and the
@@ -450,11 +449,9 @@ deposit_fftz_kernel(const __grid_constant__ DepGeom g, const float4* __restrict_
     unsigned packed = 0;
 #pragma unroll
     for (int b = 0; b < NSB; ++b) packed |= (unsigned)(sh[b] > SH_MAX ? 0 : sh[b]) << (8 * b);
-    tile_units_wide<N, MAS, G, CT>(g, te, sg, packed, x0, y0, kz_cols, tw, spec, cells, list, s_part,
-                                   tile_mass, (int)gridDim.x, t);
+    tile_units_wide<N, MAS, G, CT>(g, te, sg, packed, x0, y0, kz_cols, tw, spec, cells, list, s_part, tile_mass);
   } else {
-    tile_units<N, MAS, G, CT, false>(g, te, sg, sh, x0, y0, kz_cols, tw, spec, cells, list, s_part, tile_mass,
-                                     (int)gridDim.x, t);
+    tile_units<N, MAS, G, CT, false>(g, te, sg, sh, x0, y0, kz_cols, tw, spec, cells, list, s_part, tile_mass);
   }
 }
 
@@ -541,12 +538,18 @@ int particles_power_n(DepGeom g, int64_t n_launch, gbp_fft_plan plan, gbp_bins B
     if constexpr (N == 128 || N == 256) r = dispatch_mas<N, ColTile<N, 8, 8>>(mas, G, g, L.dep, b, B->kz_cols, plan->tw, spec, st);
   }
   if (r) return r;
-  r = deposit_stats(b, L.dep, GBP_COMPAT_NONE, G, stats_out, st);
-  if (r) return r;
+  // up to 256^3 the statistics are a block of the last fold (as fast as a kernel of its own less the launch,
+  // 3 us at 256^3, 2 % of a 128^3 batch); beyond, that block would outlast the fold (1024^3: 78 against 29 + 20 us)
+  StatsFold stats = stats_fold(b, L.dep, GBP_COMPAT_NONE, G, stats_out);
+  if (N > 256) {
+    r = deposit_stats(b, L.dep, GBP_COMPAT_NONE, G, stats_out, st);
+    if (r) return r;
+    stats.out = nullptr;
+  }
   r = own_fft_y_packed(N, G, spec, B->kz_cols, B->last_closed, plan->tw, st);
   if (r) return r;
   const double* mass = reinterpret_cast<const double*>(stats_out);   // gbp_deposit_stats starts with mass[2]
-  return xbin_power(plan, spec, B, mas, ells, mass, sums_out, nmodes_out, ksum_out, xws, L.xbin, st);
+  return xbin_power(plan, spec, B, mas, ells, mass, sums_out, nmodes_out, ksum_out, xws, L.xbin, st, stats);
 }
 
 }  // namespace

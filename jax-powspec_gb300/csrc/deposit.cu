@@ -16,7 +16,8 @@
 //                      each add is a native 32-bit atomic on the low word plus
 //                      a carry into the high word), then writes its cells of
 //                      the mesh exactly once.
-//   5. stats_kernel    folds the per-block partial sums in a fixed order.
+//   5. stats_kernel    folds the per-block partial sums in a fixed order (the
+//                      exact integer totals need none).
 //
 // Passes 1-3 are one unless a large mesh holds few particles: fill_kernel
 // gives each tile a bucket of fixed capacity and writes every entry at the

@@ -11,6 +11,7 @@
 #include <thrust/iterator/counting_iterator.h>
 #include <thrust/iterator/transform_iterator.h>
 
+#include "deposit_stats.cuh"
 #include "gbp_internal.cuh"
 
 namespace gbp {
@@ -244,21 +245,6 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-__device__ __forceinline__ ff warp_ff_sum(ff v) {
-  for (int o = 16; o > 0; o >>= 1) {
-    ff t{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
-    v = ff_add(v, t);
-  }
-  return v;
-}
-
-struct DepCounters {           // zeroed by one memset per call
-  unsigned int maxw_bits;
-  unsigned int n_spill;        // fill path: entries beyond their bucket's capacity
-  unsigned int n_extra;        // spilled entries gathered by their tiles so far
-  unsigned int outgrown;       // some tile has more entries than DepGeom::flag_cap
-};
-
 // Fill path: the entries beyond a bucket's capacity.  heads holds HEADS lists
 // per tile of them (node + 1, 0 ends a list), linked through next.
 constexpr unsigned HEADS = CSTRIDE;
@@ -282,7 +268,7 @@ __device__ __forceinline__ void spill_entry(const Spill& sp, DepCounters* ctr, u
 // Block reductions of the weight statistics in a fixed order (deterministic
 // partials per particle block), and the global max |w|.
 __device__ __forceinline__ void flush_block_stats(float maxw, ff sw, ff sw2, unsigned kept, unsigned bad,
-                                                  DepCounters* ctr, float4* block_stats, uint2* block_counts) {
+                                                  DepCounters* ctr, float4* block_stats) {
   __shared__ float s_max[CNT_THREADS / 32];
   __shared__ ff s_sw[CNT_THREADS / 32], s_sw2[CNT_THREADS / 32];
   __shared__ unsigned s_kept, s_bad;
@@ -305,7 +291,8 @@ __device__ __forceinline__ void flush_block_stats(float maxw, ff sw, ff sw2, uns
       b = ff_add(b, s_sw2[k]);
     }
     block_stats[blockIdx.x] = make_float4(a.hi, a.lo, b.hi, b.lo);
-    block_counts[blockIdx.x] = make_uint2(s_kept, s_bad);
+    if (s_kept) atomicAdd(&ctr->kept, (unsigned long long)s_kept);
+    if (s_bad) atomicAdd(&ctr->bad, (unsigned long long)s_bad);
     if (m > 0.f) atomicMax(&ctr->maxw_bits, __float_as_uint(m));
   }
 }
@@ -313,8 +300,7 @@ __device__ __forceinline__ void flush_block_stats(float maxw, ff sw, ff sw2, uns
 // Pass 1: tile occupancy counts + weight statistics.
 template <int MAS, int G, int CM, bool JOB>
 __global__ void __launch_bounds__(CNT_THREADS)
-count_kernel(DepGeom gp, unsigned* __restrict__ counts, DepCounters* ctr, float4* block_stats,
-             uint2* block_counts) {
+count_kernel(DepGeom gp, unsigned* __restrict__ counts, DepCounters* ctr, float4* block_stats) {
   pdl_wait();
   const DepGeom g = catalogue_of<JOB>(gp);
   float maxw = 0.0f;
@@ -343,7 +329,7 @@ count_kernel(DepGeom gp, unsigned* __restrict__ counts, DepCounters* ctr, float4
     sw = ff_add_f(sw, w);
     sw2 = ff_add_f(sw2, __fmul_rn(w, w));
   }
-  flush_block_stats(maxw, sw, sw2, kept, bad, ctr, block_stats, block_counts);
+  flush_block_stats(maxw, sw, sw2, kept, bad, ctr, block_stats);
 }
 
 // Passes 1 and 3 at once (fill path: buckets of a fixed capacity g.tcap, tile
@@ -361,7 +347,7 @@ count_kernel(DepGeom gp, unsigned* __restrict__ counts, DepCounters* ctr, float4
 template <int MAS, int G, int CM, bool JOB>
 __global__ void __launch_bounds__(CNT_THREADS, 5)
 fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entries, Spill sp, DepCounters* ctr,
-            float4* block_stats, uint2* block_counts) {
+            float4* block_stats) {
   pdl_wait();
   const DepGeom g = catalogue_of<JOB>(gp);
   const unsigned tcap = g.tcap;
@@ -416,7 +402,7 @@ fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entr
     sw = ff_add_f(sw, w);
     sw2 = ff_add_f(sw2, __fmul_rn(w, w));
   }
-  flush_block_stats(maxw, sw, sw2, kept, bad, ctr, block_stats, block_counts);
+  flush_block_stats(maxw, sw, sw2, kept, bad, ctr, block_stats);
 }
 
 // Column tiles (TX x TY pencils over all of z; power-of-two meshes, TX, TY >=
@@ -456,7 +442,7 @@ __device__ __forceinline__ int column_axis(const DepGeom& g, int ax, float u, in
 template <int MAS, int G, bool JOB>
 __global__ void __launch_bounds__(CNT_THREADS, 5)
 fill_columns_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entries, Spill sp,
-                    DepCounters* ctr, float4* block_stats, uint2* block_counts) {
+                    DepCounters* ctr, float4* block_stats) {
   pdl_wait();
   const DepGeom g = catalogue_of<JOB>(gp);
   float maxw = 0.0f;
@@ -495,7 +481,7 @@ fill_columns_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restric
       spill_entry(sp, ctr, (unsigned)tc[k], (size_t)t * HEADS + c * CLS_HEADS, CLS_HEADS, e[k]);
     }
   }
-  flush_block_stats(maxw, sw, sw2, kept, bad, ctr, block_stats, block_counts);
+  flush_block_stats(maxw, sw, sw2, kept, bad, ctr, block_stats);
 }
 
 // The nine runs of a column tile's entries: entry i of the buckets lies at
@@ -710,20 +696,6 @@ scatter_kernel(DepGeom gp, const unsigned* __restrict__ offsets, unsigned* __res
   }
 }
 
-// Fixed-point exponent s: one contribution w * W (|W| <= 1, or <= 8 for the
-// reference CIC, whose fractions can leave [0,1) off the box) is an integer
-// below 2^30 in magnitude, so it fits one 32-bit atomic on the low word; the
-// 64-bit cell sums hold n * 2^30 without overflow for any n < 2^32.
-// Float32 and integer operations only (GB300's FP64 rate is tiny).
-__device__ __forceinline__ int fixed_scale_exp(unsigned maxw_bits, int compat) {
-  const float maxw = __uint_as_float(maxw_bits);
-  if (!(maxw > 0.0f) || !(maxw < 3.0e38f)) return 0;
-  int ew;
-  frexpf(maxw, &ew);                            // maxw < 2^ew
-  const int s = 30 - ew - (compat ? 3 : 0);
-  return s < -100 ? -100 : (s > 100 ? 100 : s);
-}
-
 // int64 fixed-point value -> float32 (two exact 32-bit halves, one rounding in the FMA).
 __device__ __forceinline__ float fixed_to_float(long long q, float inv_sc) {
   const int hi = (int)(q >> 32);
@@ -742,84 +714,12 @@ __device__ __forceinline__ void local_nodes(const Axis<R>& a, int N, int t0, int
   }
 }
 
-// Pass 5: fold the per-block statistics and the per-tile mass totals into
-// gbp_deposit_stats.  Float partials are folded in a fixed order; integer
-// totals are exact in any order.
-constexpr int STATS_THREADS = 1024;
-__global__ void __launch_bounds__(STATS_THREADS)
-stats_kernel(const DepCounters* ctr, const float4* block_stats, const uint2* block_counts, int nblocks,
-             const long long* tile_mass, int ntiles, int compat, int G, gbp_deposit_stats* out) {
+// Pass 5 of the mesh deposit: gbp_deposit_stats from the counters and the
+// per-block partials (the fused path folds them in power_reduce_kernel).
+__global__ void __launch_bounds__(STATS_LANES)
+stats_kernel(StatsFold f) {
   pdl_wait();
-  __shared__ ff s_a[32], s_b[32];
-  __shared__ long long s_m[2][32], s_c[2][32];
-  ff a{0.f, 0.f}, b{0.f, 0.f};
-  long long kept = 0, bad = 0, m0 = 0, m1 = 0;
-  // a thread adds blocks k = tid, tid + blockDim, ... in that order; the loads of SU of them are issued
-  // before the adds
-  constexpr int SU = 4;
-  const int nt = blockDim.x;
-  for (int k0 = threadIdx.x; k0 < nblocks; k0 += SU * nt) {
-    float4 v[SU];
-    uint2 c[SU];
-#pragma unroll
-    for (int u = 0; u < SU; ++u) {
-      const int k = k0 + u * nt;
-      v[u] = k < nblocks ? block_stats[k] : make_float4(0.f, 0.f, 0.f, 0.f);
-      c[u] = k < nblocks ? block_counts[k] : make_uint2(0u, 0u);
-    }
-#pragma unroll
-    for (int u = 0; u < SU; ++u) {
-      if (k0 + u * nt >= nblocks) break;
-      a = ff_add(a, ff{v[u].x, v[u].y});
-      b = ff_add(b, ff{v[u].z, v[u].w});
-      kept += c[u].x;
-      bad += c[u].y;
-    }
-  }
-  for (int k0 = threadIdx.x; k0 < ntiles; k0 += SU * nt) {       // integers: any order
-#pragma unroll
-    for (int u = 0; u < SU; ++u) {
-      const int k = k0 + u * nt;
-      if (k < ntiles) {
-        m0 += tile_mass[k];
-        if (G == 2) m1 += tile_mass[ntiles + k];
-      }
-    }
-  }
-  a = warp_ff_sum(a);
-  b = warp_ff_sum(b);
-  for (int o = 16; o > 0; o >>= 1) {
-    kept += __shfl_xor_sync(0xffffffffu, kept, o);
-    bad += __shfl_xor_sync(0xffffffffu, bad, o);
-    m0 += __shfl_xor_sync(0xffffffffu, m0, o);
-    m1 += __shfl_xor_sync(0xffffffffu, m1, o);
-  }
-  const int wid = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    s_a[wid] = a; s_b[wid] = b;
-    s_c[0][wid] = kept; s_c[1][wid] = bad;
-    s_m[0][wid] = m0; s_m[1][wid] = m1;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ff ta{0.f, 0.f}, tb{0.f, 0.f};
-    long long tk = 0, tbad = 0, tm[2] = {0, 0};
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
-      ta = ff_add(ta, s_a[k]);
-      tb = ff_add(tb, s_b[k]);
-      tk += s_c[0][k]; tbad += s_c[1][k];
-      tm[0] += s_m[0][k]; tm[1] += s_m[1][k];
-    }
-    const int s = fixed_scale_exp(ctr->maxw_bits, compat);
-    const double inv = ldexp(1.0, -s);
-    for (int grid = 0; grid < 2; ++grid) out->mass[grid] = grid < G ? (double)tm[grid] * inv : 0.0;
-    out->sum_w = (double)ta.hi + (double)ta.lo;
-    out->sum_w2 = (double)tb.hi + (double)tb.lo;
-    out->n_kept = tk;
-    out->n_nonfinite = tbad;
-    out->scale_exp = s;
-    out->flags = ctr->outgrown ? GBP_STATS_REFILLED : 0;
-  }
+  fold_stats<STATS_LANES>(f);
 }
 
 struct DepLayout {
@@ -975,8 +875,7 @@ void finish_layout(DepLayout& L) {
   L.scan_bytes = 0;
   if (!L.tcap) cub::DeviceScan::ExclusiveSum(nullptr, L.scan_bytes, strided_counts(nullptr), (unsigned*)nullptr, L.ntiles);
   const size_t nbl = (size_t)(L.nblocks > 0 ? L.nblocks : 1);
-  L.total = zeroed_bytes(L) + align256((size_t)L.ntiles * 4) + align256(nbl * sizeof(float4)) +
-            align256(nbl * sizeof(uint2)) + align256((size_t)L.ntiles * 2 * sizeof(long long)) +
+  L.total = zeroed_bytes(L) + align256((size_t)L.ntiles * 2 * sizeof(long long)) + align256((size_t)L.ntiles * 4) + align256(nbl * sizeof(float4)) +
             align256(L.nentries * sizeof(float4)) + align256(L.scan_bytes) + 2 * align256(L.nspill * sizeof(unsigned)) +
             align256(L.nspill * sizeof(float4)) + align256(L.nextra * sizeof(float4));
 }
@@ -988,8 +887,7 @@ struct DepBuffers {
   unsigned* fills;       // [ntiles * CSTRIDE] entries written so far (count path's scatter)
   unsigned* offsets;     // [ntiles] first entry of each tile (exclusive scan of the counts)
   float4* block_stats;
-  uint2* block_counts;
-  long long* tile_mass;
+  long long* tile_mass;  // [2][ntiles]
   float4* entries;
   void* scan_tmp;
   Spill spill;           // fill path (its heads share the bytes of fills)
@@ -1004,7 +902,6 @@ inline DepBuffers carve_deposit(void* workspace, const DepLayout& L) {
   b.fills = cv.take<unsigned>((size_t)L.ntiles * CSTRIDE);
   b.offsets = cv.take<unsigned>(L.ntiles);
   b.block_stats = cv.take<float4>(nbl);
-  b.block_counts = cv.take<uint2>(nbl);
   b.tile_mass = cv.take<long long>((size_t)L.ntiles * 2);
   b.entries = cv.take<float4>(L.nentries);
   b.scan_tmp = cv.take<char>(L.scan_bytes);
@@ -1025,14 +922,14 @@ int bucket_particles(const DepGeom& g, const DepLayout& L, const DepBuffers& b, 
     if (L.nblocks > 0) {
       GBP_TRACE("deposit_fill", st);
       GBP_CUDA_TRY(launch_pdl(job ? fill_kernel<MAS, G, CM, CM == 0> : fill_kernel<MAS, G, CM, false>, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts,
-                              b.entries, b.spill, b.ctr, b.block_stats, b.block_counts));
+                              b.entries, b.spill, b.ctr, b.block_stats));
     }
     return GBP_OK;
   }
   if (L.nblocks > 0) {
     GBP_TRACE("deposit_count", st);
     GBP_CUDA_TRY(launch_pdl(job ? count_kernel<MAS, G, CM, CM == 0> : count_kernel<MAS, G, CM, false>, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts, b.ctr,
-                            b.block_stats, b.block_counts));
+                            b.block_stats));
   }
   {
     GBP_TRACE("deposit_scan", st);
@@ -1055,16 +952,18 @@ int bucket_columns(const DepGeom& g, const DepLayout& L, const DepBuffers& b, cu
   GBP_TRACE("deposit_fill", st);
   auto k = g.job ? fill_columns_kernel<MAS, G, true> : fill_columns_kernel<MAS, G, false>;
   GBP_CUDA_TRY(launch_pdl(k, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts,
-                          b.entries, b.spill, b.ctr, b.block_stats, b.block_counts));
+                          b.entries, b.spill, b.ctr, b.block_stats));
   return GBP_OK;
+}
+
+inline StatsFold stats_fold(const DepBuffers& b, const DepLayout& L, int compat, int G, gbp_deposit_stats* out) {
+  return StatsFold{b.ctr, b.block_stats, L.nblocks, compat, G, b.tile_mass, L.ntiles, out};
 }
 
 inline int deposit_stats(const DepBuffers& b, const DepLayout& L, int compat, int G, gbp_deposit_stats* out,
                          cudaStream_t st) {
   GBP_TRACE("deposit_stats", st);
-  GBP_CUDA_TRY(launch_pdl(stats_kernel, dim3(1), dim3(STATS_THREADS), 0, st, static_cast<const DepCounters*>(b.ctr),
-                          static_cast<const float4*>(b.block_stats), static_cast<const uint2*>(b.block_counts),
-                          L.nblocks, static_cast<const long long*>(b.tile_mass), L.ntiles, compat, G, out));
+  GBP_CUDA_TRY(launch_pdl(stats_kernel, dim3(1), dim3(STATS_LANES), 0, st, stats_fold(b, L, compat, G, out)));
   return GBP_OK;
 }
 

@@ -19,6 +19,7 @@ struct gbp_fft_plan_s {
 };
 
 namespace gbp {
+struct StatsFold;   // deposit_stats.cuh
 bool own_fft_supported(int N);
 int own_fft_pitch(int N);
 int own_fft_twiddles(int N, float2** d_tw);
@@ -46,7 +47,8 @@ int c2r_plan(int N, int P, int batch, cufftHandle* h, size_t* ws);
 // and the transform enqueued under a lock, so concurrent callers cannot mix
 // them up.  `in` is overwritten (cuFFT's multi-dimensional C2R).
 int c2r_exec(int N, int P, int batch, const float2* in, float* out, void* work, cudaStream_t st);
+// (stats: the deposit statistics to fold in the same launch, out = nullptr for none)
 int xbin_power(gbp_fft_plan plan, float2* spec, gbp_bins bins, int mas_order, int ells, const double* mass,
                double* sums_out, long long* nmodes_out, double* ksum_out, void* ws, size_t ws_bytes,
-               cudaStream_t st);
+               cudaStream_t st, const StatsFold& stats);
 }  // namespace gbp

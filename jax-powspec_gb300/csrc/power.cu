@@ -357,7 +357,7 @@ int launch_power(const void* spectrum, int G, int Lzs, gbp_bins B, int mas_order
   GBP_CUDA_TRY(launch_pdl(power_reduce_kernel, dim3(B->nb), dim3(FOLD_THREADS), 0, stream,
                           static_cast<const float2*>(part_ff), L.C, L.NV, B->nb, B->nbe,
                           static_cast<const long long*>(B->d_nmodes), static_cast<const double*>(B->d_ksum), sums_out,
-                          nmodes_out, (ells & GBP_KSUM) ? ksum_out : nullptr));
+                          nmodes_out, (ells & GBP_KSUM) ? ksum_out : nullptr, StatsFold{}));
   return GBP_OK;
 }
 

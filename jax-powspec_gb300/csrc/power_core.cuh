@@ -5,6 +5,7 @@
 
 #include <math.h>
 
+#include "deposit_stats.cuh"
 #include "gbp_bins.h"
 #include "gbp_internal.cuh"
 
@@ -245,13 +246,18 @@ __device__ __forceinline__ void fold_bin(const float2* __restrict__ part_ff, int
 
 // One block per bin (FOLD_THREADS threads): fold the CTA partials into double
 // moment totals and form the Legendre sums; copy the plan's geometry per bin.
+// stats.out: one more block folds the deposit's statistics, which only the
+// normalisation after it reads.
 __global__ void __launch_bounds__(FOLD_THREADS)
 power_reduce_kernel(const float2* __restrict__ part_ff, int C, int NV, int nb, int nbe,
                     const long long* __restrict__ plan_nmodes, const double* __restrict__ plan_ksum,
-                    double* sums_out, long long* nmodes_out, double* ksum_out) {
+                    double* sums_out, long long* nmodes_out, double* ksum_out, StatsFold stats) {
   pdl_wait();
   const int b = blockIdx.x;
-  if (b >= nb) return;                         // uniform over the block
+  if (b >= nb) {                               // uniform over the block
+    if (stats.out) fold_stats<FOLD_THREADS>(stats);
+    return;
+  }
   double m[3] = {0.0, 0.0, 0.0};
   if (b < nbe) fold_bin<3>(part_ff, C, NV, nbe, b, m);
   if (threadIdx.x == 0) {

@@ -281,7 +281,7 @@ int xbin_power_workspace(gbp_fft_plan plan, gbp_bins B, int ells, size_t* bytes)
 
 int xbin_power(gbp_fft_plan plan, float2* spec, gbp_bins B, int mas_order, int ells, const double* mass,
                double* sums_out, long long* nmodes_out, double* ksum_out, void* workspace, size_t ws_bytes,
-               cudaStream_t st) {
+               cudaStream_t st, const StatsFold& stats) {
   if (!plan || !spec || !B || !sums_out || !nmodes_out) return GBP_ERR_INVALID;
   if (plan->n != B->N) return GBP_ERR_INVALID;
   if (!plan->own || (plan->grids != 1 && plan->grids != 2)) return GBP_ERR_UNSUPPORTED;
@@ -327,10 +327,10 @@ int xbin_power(gbp_fft_plan plan, float2* spec, gbp_bins B, int mas_order, int e
   }
   if (r) return r;
   GBP_TRACE("power_reduce", st);
-  GBP_CUDA_TRY(launch_pdl(power_reduce_kernel, dim3(B->nb), dim3(FOLD_THREADS), 0, st,
+  GBP_CUDA_TRY(launch_pdl(power_reduce_kernel, dim3(B->nb + (stats.out ? 1 : 0)), dim3(FOLD_THREADS), 0, st,
                           static_cast<const float2*>(g.part_ff), L.groups, L.NV, B->nb, B->nbe,
                           static_cast<const long long*>(B->d_nmodes), static_cast<const double*>(B->d_ksum), sums_out,
-                          nmodes_out, (ells & GBP_KSUM) ? ksum_out : nullptr));
+                          nmodes_out, (ells & GBP_KSUM) ? ksum_out : nullptr, stats));
   return GBP_OK;
 }
 
@@ -359,5 +359,5 @@ extern "C" int gbp_fft_power(gbp_fft_plan plan, const float* mesh, void* spectru
   if (r) return r;
   r = own_fft_y_packed(B->N, plan->grids, spec, B->kz_cols, B->last_closed, plan->tw, st);
   if (r) return r;
-  return xbin_power(plan, spec, B, mas_order, ells, mass, sums_out, nmodes_out, ksum_out, workspace, ws_bytes, st);
+  return xbin_power(plan, spec, B, mas_order, ells, mass, sums_out, nmodes_out, ksum_out, workspace, ws_bytes, st, StatsFold{});
 }
