@@ -292,7 +292,7 @@ bispec_y_kernel(PowGeom g, const int* __restrict__ shell_bins, int k2_max, int n
   auto gin = [base, lim](int j, int cp) {
     const int k = signed_k(j, N);
     if (k * k > lim) return make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 v = __ldcs(reinterpret_cast<const float4*>(base + (long long)j * P) + cp);
+    const float4 v = __ldcg(reinterpret_cast<const float4*>(base + (long long)j * P) + cp);
     return make_float4(v.y, v.x, v.w, v.z);
   };
   auto gout = [base](int j, int cp, float4 v) {
@@ -321,7 +321,7 @@ bispec_z_kernel(PowGeom g, const int* __restrict__ shell_bins, int k2_max, int k
   const float2* i2 = i0 + 2 * sstride;
   auto load = [lim, pstride](const float2* row, int k, int cp) {   // row y0 + cp of planes 2x', 2x'+1
     if (64 * (k >> 3) * (k >> 3) > lim) return make_float4(0.f, 0.f, 0.f, 0.f);
-    const float2 u = __ldcs(row + cp * P + k), v = __ldcs(row + pstride + cp * P + k);
+    const float2 u = __ldcg(row + cp * P + k), v = __ldcg(row + pstride + cp * P + k);
     return make_float4(u.x, u.y, v.x, v.y);
   };
   auto agin = [&](int j, int cp) {

@@ -78,7 +78,7 @@ fftz_kernel(const float* __restrict__ mesh, float2* __restrict__ out, long long 
   auto gin = [base, npen](int j, int cp) {      // pencils 4cp .. 4cp+3 at z = j
     float v[4];
 #pragma unroll
-    for (int f = 0; f < 4; ++f) v[f] = 4 * cp + f < npen ? __ldcs(base + (4 * cp + f) * N + j) : 0.0f;
+    for (int f = 0; f < 4; ++f) v[f] = 4 * cp + f < npen ? __ldcg(base + (4 * cp + f) * N + j) : 0.0f;
     return make_float4(v[0], v[1], v[2], v[3]);
   };
   auto sin_ = [](int j, int cp) { return s4[cp * N + zsw(j)]; };
@@ -138,7 +138,7 @@ fftz_packed_kernel(const float* __restrict__ mesh, float2* __restrict__ out, int
   float2* o1 = o0 + (long long)NX * N * P;
   auto gin = [base](int j, int cp) {
     const float* b = base + 2 * cp * N + j;
-    return make_float4(__ldcs(b), __ldcs(b + IM), __ldcs(b + N), __ldcs(b + IM + N));
+    return make_float4(__ldcg(b), __ldcg(b + IM), __ldcg(b + N), __ldcg(b + IM + N));
   };
   auto sin_ = [](int j, int cp) { return s4[cp * N + zsw(j)]; };
   auto sout = [](int j, int cp, float4 v) { s4[cp * N + zsw(j)] = v; };
@@ -150,7 +150,11 @@ fftz_packed_kernel(const float* __restrict__ mesh, float2* __restrict__ out, int
 // 8 adjacent kz columns x N rows per CTA, rows `row_stride` complex apart;
 // CTA b covers plane (b / nkb) and kz block (b % nkb).  N/2 threads: one
 // pair of radix-8 butterflies (two columns) each per stage; the first stage
-// loads from HBM and the last stores to HBM (fft_pass.cuh), in place.
+// loads from HBM and the last stores to HBM (fft_pass.cuh), in place.  A row's
+// 64 bytes are half of a 128-byte line: ordinary L2 policy (.cg) lets the CTA
+// of the other half find it there, which evict-first (.cs) did not; the planes
+// go last to first, as the previous pass wrote the last ones last.  Two grids
+// at 512^3: 0.402 -> 0.327 ms, one 0.201 -> 0.168; 256^3: 0.053 -> 0.046.
 // PRUNE = 1: rows whose wavenumber k has k^2 + (the block's first kz)^2 >
 // k2_max are not stored (with k edges up to k_Nyquist, a fifth of them: 0.423 ->
 // 0.392 ms for two grids at 512^3, 5.0 TB/s; bound by HBM).  PRUNE = 2: the
@@ -161,11 +165,11 @@ fft_cols_kernel(float2* __restrict__ data, long long plane_stride, long long row
                 int k2_max, const float2* __restrict__ tw) {
   pdl_wait();
   extern __shared__ __align__(16) float2 s[];
-  const int plane = blockIdx.x / nkb, kb = blockIdx.x % nkb;
-  if (plane >= nplanes) return;
+  const int plane = nplanes - 1 - blockIdx.x / nkb, kb = blockIdx.x % nkb;
+  if (plane < 0) return;
   float2* base = data + plane * plane_stride + kb * 8;
   auto gin = [base, row_stride](int j, int cp) {
-    return __ldcs(reinterpret_cast<const float4*>(base + j * row_stride) + cp);
+    return __ldcg(reinterpret_cast<const float4*>(base + j * row_stride) + cp);
   };
   const int lim = PRUNE == 1 ? k2_max - 64 * kb * kb : k2_max - plane * plane;
   auto gout = [base, row_stride, lim](int j, int cp, float4 v) {
@@ -173,7 +177,7 @@ fft_cols_kernel(float2* __restrict__ data, long long plane_stride, long long row
       const int k = signed_k(j, N);
       if (k * k > lim) return;
     }
-    __stcs(reinterpret_cast<float4*>(base + j * row_stride) + cp, v);
+    __stcg(reinterpret_cast<float4*>(base + j * row_stride) + cp, v);
   };
   fft::col_fft<N, 1, N / 2, false>(s, gin, gout, tw, threadIdx.x);
 }
@@ -188,18 +192,18 @@ fft_cols_inv_kernel(float2* __restrict__ data, int nplanes, int nkb, int k2_max,
   pdl_wait();
   constexpr int P = zpitch(N);
   extern __shared__ __align__(16) float2 s[];
-  const int plane = blockIdx.x / nkb, kb = blockIdx.x % nkb;
-  if (plane >= nplanes) return;
+  const int plane = nplanes - 1 - blockIdx.x / nkb, kb = blockIdx.x % nkb;
+  if (plane < 0) return;
   float2* base = data + (long long)plane * N * P + kb * 8;
   const int lim = k2_max - 64 * kb * kb;
   auto gin = [base, lim](int j, int cp) {
     const int k = signed_k(j, N);
     if (k * k > lim) return make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 v = __ldcs(reinterpret_cast<const float4*>(base + (long long)j * P) + cp);
+    const float4 v = __ldcg(reinterpret_cast<const float4*>(base + (long long)j * P) + cp);
     return make_float4(v.y, v.x, v.w, v.z);
   };
   auto gout = [base](int j, int cp, float4 v) {
-    __stcs(reinterpret_cast<float4*>(base + (long long)j * P) + cp, make_float4(v.y, v.x, v.w, v.z));
+    __stcg(reinterpret_cast<float4*>(base + (long long)j * P) + cp, make_float4(v.y, v.x, v.w, v.z));
   };
   fft::col_fft<N, 1, N / 2, false>(s, gin, gout, tw, threadIdx.x);
 }
@@ -227,7 +231,7 @@ fftz_unpack_kernel(const float2* __restrict__ spec, float* __restrict__ mesh, in
     const int k = j <= N / 2 ? j : N - j;
     if (k >= kz_cols) return make_float4(0.f, 0.f, 0.f, 0.f);
     const float2* b = (j <= N / 2 ? i0 : i1) + (2 * cp) * P + k;
-    const float2 u = __ldcs(b), v = __ldcs(b + P);
+    const float2 u = __ldcg(b), v = __ldcg(b + P);
     return make_float4(u.y, u.x, v.y, v.x);
   };
   auto sin_ = [](int j, int cp) { return s4[cp * N + zsw(j)]; };

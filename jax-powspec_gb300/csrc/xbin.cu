@@ -30,7 +30,8 @@
 //
 // Only items with a mode inside the last k edge are listed by the bin plan
 // (gbp_bins_create): edges up to k_Nyquist leave out a fifth of them.  Two
-// grids at 512^3: 0.688 -> 0.552 ms (0.86 GB read: 1.6 TB/s; bound by
+// grids at 512^3: 0.688 -> 0.552 ms, 0.526 with loads that keep their lines in
+// L2 for the neighbouring kz block (0.86 GB read: 1.6 TB/s; bound by
 // instruction issue and barriers); one grid (half the points per column, a
 // warp per column): 0.545 -> 0.362 ms at 512^3, 0.091 -> 0.045 at 256^3.
 //

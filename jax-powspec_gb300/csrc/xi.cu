@@ -189,7 +189,7 @@ xi_z_kernel(PowGeom g, const float2* __restrict__ h, int chunks, int nan_origin)
       auto row_y = [ym, rows](int m) { return m <= ym ? m : N - rows + m; };
       auto at = [&](int f, int kz) {                                       // h of pencil f of the item
         const int m = m0 + f;
-        return m < rows ? __ldcs(h + ((long long)x * N + row_y(m)) * P + kz) : make_float2(0.f, 0.f);
+        return m < rows ? __ldcg(h + ((long long)x * N + row_y(m)) * P + kz) : make_float2(0.f, 0.f);
       };
       auto gin = [&](int j, int cp) {                                      // columns 2cp, 2cp+1: pencils 4cp .. 4cp+3
         const int kz = j <= H ? j : N - j;

@@ -117,7 +117,7 @@ __device__ __forceinline__ void x_forward(float2* s, const float2* __restrict__ 
   // row of the column pair's slab: y, or -y of slab 1
   const long long r0 = (long long)y * P, r1 = (long long)L::NX * planes * N * P + (long long)((N - y) & (N - 1)) * P;
   auto gin = [src, r0, r1, planes](int x, int cp) {    // columns 2cp, 2cp+1 (slab cp / 4)
-    return __ldcs(reinterpret_cast<const float4*>(src + (cp < 4 ? r0 : r1) + (long long)x * planes * N * P) +
+    return __ldcg(reinterpret_cast<const float4*>(src + (cp < 4 ? r0 : r1) + (long long)x * planes * N * P) +
                   (cp & 3));
   };
   auto tout = [s](int x, int cp, float4 v) {
