@@ -52,7 +52,7 @@
 //   f. bispec_xbin_kernel: x passes of an item of the contrast and of both
 //      products, and the four sums, binned as in xbin.cu.
 //
-// 256^3, k1 = 0.1, k2 = 0.2, 20 angles, L = 2500: 0.857 -> 0.45 ms of kernels (x 0.050, y 0.051, z 0.107,
+// 256^3, k1 = 0.1, k2 = 0.2, 20 angles, L = 2500: 0.857 -> 0.43 ms of kernels (x 0.050, y 0.051, z 0.107,
 // x + bins 0.116).
 //
 // Shell membership is the reference's float32 rule, k = sqrtf(k^2) >=
@@ -418,8 +418,8 @@ bispec_xbin_kernel(PowGeom g, const float2* __restrict__ pair, int k2_max, int p
       const int ky = signed_k(y, N), ay = ky < 0 ? -ky : ky;
       if (ky * ky + 64 * kb * kb > k2_max) continue;                     // uniform over the block
       x_forward<N, false, false, NT>(sd, g.s0, y, kb, g.twx, tid);
-      x_forward<N, false, false, NT>(sd + FIELD, pair, y, kb, g.twx, tid, 2);
-      x_forward<N, false, false, NT>(sd + 2 * FIELD, pair + (long long)N * P, y, kb, g.twx, tid, 2);
+      x_forward<N, false, false, NT, 1>(sd + FIELD, pair, y, kb, g.twx, tid, 2);
+      x_forward<N, false, false, NT, 1>(sd + 2 * FIELD, pair + (long long)N * P, y, kb, g.twx, tid, 2);
       const int c = warp / HALVES, h = warp % HALVES, kz = kb * XB_C + c;
       const bool active = kz <= H;
       const int kzc = active ? kz : 0;
@@ -527,7 +527,7 @@ int run_bispec_packed(gbp_fft_plan plan, PowGeom g, const BpLayout& L, const int
       GBP_CUDA_TRY(launch_pdl(k, dim3(N * N / PAIRS), dim3(PAIRS * N / 16), smem, st, g, shell_bins, L.k2_max,
                               L.kz_cols, data));
     }
-    const int r = own_fft_y_packed(N, 2, data, L.kz_cols, L.k2_max, plan->tw, st);
+    const int r = own_fft_y_rows(N, 2 * N, data, L.kz_cols, L.k2_max, plan->tw, st);
     if (r) return r;
   }
   auto k = bispec_xbin_kernel<N>;

@@ -244,8 +244,8 @@ __device__ __forceinline__ void tile_unit(const DepGeom& g, const ColEntries& te
   // columns 2cp and 2cp + 1 are rows y0 + ly and y0 + ly + 1 of plane x0 + a (G = 2) or x0 / 2 + a
   auto gout = [spec, x0, y0, kz_cols](int k, int cp, float4 v) {
     const int a = 2 * cp / UY, ly = 2 * cp % UY;
-    float2* o0 = spec + ((long long)((G == 2 ? x0 : x0 / 2) + a) * N + (y0 + ly)) * P;
-    fft::store_packed<N>(o0, o0 + (long long)NX * N * P, P, kz_cols, k, 0, v);
+    float2* o0 = spec + fft::PackedRows<N>::at((G == 2 ? x0 : x0 / 2) + a, y0 + ly);
+    fft::store_packed<N>(o0, o0 + (long long)NX * N * P, fft::PackedRows<N>::ROW, kz_cols, k, v);
   };
   // N = 512, 32-bit cells: every stage is radix 8 and the 64 threads of a column pair own its data
   // (the first stage's writes alias the pair's own pencils), so the stages synchronise 64-thread

@@ -24,7 +24,10 @@
 // Layout [2][NX][N][P], NX = N (two grids) or N/2 (one): slab 0 holds Z at
 // kz = 0 .. N/2, slab 1 holds Z at -kz, so both halves of a kz block are
 // aligned and the y pass treats the slabs as two grids.  The split it saves
-// cost the z pass a write and a read of the block in shared memory.
+// cost the z pass a write and a read of the block in shared memory.  The x
+// planes are interleaved four by four in blocks of 8 kz (fft::PackedRows): a
+// block of one plane is half a 128-byte line, and the x pass, which reads one
+// block of every plane for its row, finds four planes' blocks side by side.
 // Columns and rows beyond the last k edge are not stored.
 //
 // The z rows are padded from N/2+1 to P = N/2+8 complex (64-byte multiples)
@@ -47,6 +50,7 @@ namespace {
 using fft::cadd;
 using fft::cmi;
 using fft::csub;
+using fft::PACK_W;
 
 __host__ __device__ constexpr int zpitch(int N) { return N / 2 + 8; }
 
@@ -114,10 +118,11 @@ fftz_kernel(const float* __restrict__ mesh, float2* __restrict__ out, long long 
   }
 }
 
-// z pass of the packed transform: PAIRS complex columns per CTA, column q =
-// x' N + y of the packed field (G = 2: pencil q of both meshes; G = 1:
-// pencils (2x', y) and (2x'+1, y)).  The last stage stores Z[kz] to slab 0
-// and / or the mirrored entry of slab 1 straight from registers.
+// z pass of the packed transform: PAIRS complex columns per CTA, column (x', y)
+// of the packed field (G = 2: pencil (x', y) of both meshes; G = 1: pencils
+// (2x', y) and (2x'+1, y)).  The CTA takes PACK_W planes x PAIRS / PACK_W rows,
+// so it fills whole lines of the interleaved planes.  The last stage stores
+// Z[kz] to slab 0 and / or the mirrored entry of slab 1 straight from registers.
 template <int N, int G, int PAIRS>
 __global__ void __launch_bounds__(PAIRS * N / 16)
 fftz_packed_kernel(const float* __restrict__ mesh, float2* __restrict__ out, int kz_cols,
@@ -128,46 +133,62 @@ fftz_packed_kernel(const float* __restrict__ mesh, float2* __restrict__ out, int
   constexpr int NX = G == 2 ? N : N / 2;
   constexpr int P = zpitch(N);
   constexpr long long IM = G == 2 ? (long long)N * N * N : (long long)N * N;   // from the real to the imaginary pencil
-  static_assert(N % PAIRS == 0, "a block's columns share one x plane");
+  static_assert(PAIRS % PACK_W == 0 && N % (PAIRS / PACK_W) == 0, "whole blocks of rows");
   extern __shared__ __align__(16) float4 s4[];    // [CP][N] slots of two columns
   const int tid = threadIdx.x;
-  const long long q0 = (long long)blockIdx.x * PAIRS;
-  const long long x = q0 / N, y = q0 - x * N;
-  const float* base = mesh + (G == 2 ? q0 * N : (2 * x * N + y) * N);
-  float2* o0 = out + q0 * P;
+  using R = fft::PackedRows<N>;
+  constexpr int ROWS = PAIRS / PACK_W;
+  const int x = blockIdx.x / (N / ROWS) * PACK_W, y = blockIdx.x % (N / ROWS) * ROWS;
+  constexpr long long XM = G == 2 ? (long long)N * N : 2LL * N * N;            // mesh: from one packed plane to the next
+  const float* base = mesh + x * XM + (long long)y * N;
+  float2* o0 = out + R::at(x, y);
   float2* o1 = o0 + (long long)NX * N * P;
   auto gin = [base](int j, int cp) {
-    const float* b = base + 2 * cp * N + j;
-    return make_float4(__ldcg(b), __ldcg(b + IM), __ldcg(b + N), __ldcg(b + IM + N));
+    const float* b = base + 2 * cp % PACK_W * XM + 2 * cp / PACK_W * N + j;    // planes 2cp % PACK_W and the next
+    return make_float4(__ldcg(b), __ldcg(b + IM), __ldcg(b + XM), __ldcg(b + IM + XM));
   };
   auto sin_ = [](int j, int cp) { return s4[cp * N + zsw(j)]; };
   auto sout = [](int j, int cp, float4 v) { s4[cp * N + zsw(j)] = v; };
-  auto gout = [o0, o1, kz_cols](int k, int cp, float4 v) { fft::store_packed<N>(o0, o1, P, kz_cols, k, cp, v); };
+  auto gout = [o0, o1, kz_cols](int k, int cp, float4 v) {
+    const int c = 2 * cp / PACK_W * R::ROW + 2 * cp % PACK_W * 8;
+    fft::store_packed<N>(o0 + c, o1 + c, 8, kz_cols, k, v);
+  };
   fft::run_stages2<N, CP, NT, true, false, false>(gin, sin_, sout, gout, tw, tid);
 }
+
+// Interleaved planes a CTA of the packed y passes takes together (below: measured)
+template <int N>
+constexpr int Y_PLANES = N <= 512 ? 2 : 1;
 
 // ---- y and x passes --------------------------------------------------------
 // 8 adjacent kz columns x N rows per CTA, rows `row_stride` complex apart;
 // CTA b covers plane (b / nkb) and kz block (b % nkb).  N/2 threads: one
 // pair of radix-8 butterflies (two columns) each per stage; the first stage
-// loads from HBM and the last stores to HBM (fft_pass.cuh), in place.  A row's
-// 64 bytes are half of a 128-byte line: ordinary L2 policy (.cg) lets the CTA
-// of the other half find it there, which evict-first (.cs) did not; the planes
-// go last to first, as the previous pass wrote the last ones last.  Two grids
-// at 512^3: 0.402 -> 0.327 ms, one 0.201 -> 0.168; 256^3: 0.053 -> 0.046.
+// loads from HBM and the last stores to HBM (fft_pass.cuh), in place.  Loads
+// and stores use the ordinary L2 policy (.cg), so the CTA that takes the other
+// half of a line finds it there, which evict-first (.cs) did not, and the
+// planes go last to first, as the previous pass wrote the last ones last.
+// Rows with interleaved planes (W > 1): a CTA takes SL planes of one block.
+// Two grids at 512^3: 0.402 -> 0.327 (policy) -> 0.310 ms (two planes; one by
+// one 0.338), 6.2 TB/s; one grid 0.201 -> 0.158; 256^3 0.053 -> 0.041, with as
+// many CTAs as fill the SM.  At 1024^3 two planes fill the SM with one CTA
+// (3.66 ms) and one by one takes 3.33 ms; rows of one plane took 3.07, which
+// the x pass pays for (xbin.cu).  Bound by HBM.
 // PRUNE = 1: rows whose wavenumber k has k^2 + (the block's first kz)^2 >
-// k2_max are not stored (with k edges up to k_Nyquist, a fifth of them: 0.423 ->
-// 0.392 ms for two grids at 512^3, 5.0 TB/s; bound by HBM).  PRUNE = 2: the
-// same with the plane's number in place of kz (real-space rows, xi.cu).
-template <int N, int PRUNE>
-__global__ void __launch_bounds__(N / 2, N <= 512 ? 4 : 2)
+// k2_max are not stored (with k edges up to k_Nyquist, a fifth of them).
+// PRUNE = 2: the same with the plane's number in place of kz (real-space rows,
+// xi.cu).
+template <int N, int PRUNE, int W, int SL = W == 1 ? 1 : Y_PLANES<N>>
+__global__ void __launch_bounds__(N / 2 * SL, N >= 256 ? 2048 / (N * SL) : 4)
 fft_cols_kernel(float2* __restrict__ data, long long plane_stride, long long row_stride, int nplanes, int nkb,
                 int k2_max, const float2* __restrict__ tw) {
   pdl_wait();
   extern __shared__ __align__(16) float2 s[];
-  const int plane = nplanes - 1 - blockIdx.x / nkb, kb = blockIdx.x % nkb;
+  constexpr int WS = W / SL;
+  const int grp = blockIdx.x / (WS * nkb), sub = blockIdx.x - grp * WS * nkb;
+  const int plane = nplanes - (grp * WS + sub % WS + 1) * SL, kb = sub / WS;
   if (plane < 0) return;
-  float2* base = data + plane * plane_stride + kb * 8;
+  float2* base = data + (W > 1 ? fft::PackedRows<N, W>::plane(plane) : plane * plane_stride) + kb * 8 * W;
   auto gin = [base, row_stride](int j, int cp) {
     return __ldcg(reinterpret_cast<const float4*>(base + j * row_stride) + cp);
   };
@@ -179,33 +200,35 @@ fft_cols_kernel(float2* __restrict__ data, long long plane_stride, long long row
     }
     __stcg(reinterpret_cast<float4*>(base + j * row_stride) + cp, v);
   };
-  fft::col_fft<N, 1, N / 2, false>(s, gin, gout, tw, threadIdx.x);
+  fft::col_fft<N, SL, N / 2 * SL, false>(s, gin, gout, tw, threadIdx.x);
 }
 
 // Inverse of the packed transform along y, in place: rows whose ky^2 + (the
 // block's first kz)^2 > k2_max hold nothing and are taken as zeros; every row
 // of every x plane is stored.  (An inverse transform is a forward one with
 // real and imaginary parts swapped before and after.)
-template <int N>
-__global__ void __launch_bounds__(N / 2, N <= 512 ? 4 : 2)
+template <int N, int SL = Y_PLANES<N>>
+__global__ void __launch_bounds__(N / 2 * SL, N >= 256 ? 2048 / (N * SL) : 4)
 fft_cols_inv_kernel(float2* __restrict__ data, int nplanes, int nkb, int k2_max, const float2* __restrict__ tw) {
   pdl_wait();
-  constexpr int P = zpitch(N);
   extern __shared__ __align__(16) float2 s[];
-  const int plane = nplanes - 1 - blockIdx.x / nkb, kb = blockIdx.x % nkb;
+  using R = fft::PackedRows<N>;
+  constexpr int WS = PACK_W / SL;
+  const int grp = blockIdx.x / (WS * nkb), sub = blockIdx.x - grp * WS * nkb;
+  const int plane = nplanes - (grp * WS + sub % WS + 1) * SL, kb = sub / WS;
   if (plane < 0) return;
-  float2* base = data + (long long)plane * N * P + kb * 8;
+  float2* base = data + R::plane(plane) + kb * R::BLOCK;
   const int lim = k2_max - 64 * kb * kb;
   auto gin = [base, lim](int j, int cp) {
     const int k = signed_k(j, N);
     if (k * k > lim) return make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 v = __ldcg(reinterpret_cast<const float4*>(base + (long long)j * P) + cp);
+    const float4 v = __ldcg(reinterpret_cast<const float4*>(base + (long long)j * R::ROW) + cp);
     return make_float4(v.y, v.x, v.w, v.z);
   };
   auto gout = [base](int j, int cp, float4 v) {
-    __stcg(reinterpret_cast<float4*>(base + (long long)j * P) + cp, make_float4(v.y, v.x, v.w, v.z));
+    __stcg(reinterpret_cast<float4*>(base + (long long)j * R::ROW) + cp, make_float4(v.y, v.x, v.w, v.z));
   };
-  fft::col_fft<N, 1, N / 2, false>(s, gin, gout, tw, threadIdx.x);
+  fft::col_fft<N, SL, N / 2 * SL, false>(s, gin, gout, tw, threadIdx.x);
 }
 
 // Inverse z pass of the packed transform: real fields out (the layout of
@@ -222,39 +245,42 @@ fftz_unpack_kernel(const float2* __restrict__ spec, float* __restrict__ mesh, in
   constexpr long long IM = G == 2 ? (long long)N * N * N : (long long)N * N;
   extern __shared__ __align__(16) float4 s4[];    // [CP][N] slots of two columns
   const int tid = threadIdx.x;
-  const long long q0 = (long long)blockIdx.x * PAIRS;
-  const long long x = q0 / N, y = q0 - x * N;
-  float* base = mesh + (G == 2 ? q0 * N : (2 * x * N + y) * N);
-  const float2* i0 = spec + q0 * P;
+  using R = fft::PackedRows<N>;
+  constexpr int ROWS = PAIRS / PACK_W;
+  const int x = blockIdx.x / (N / ROWS) * PACK_W, y = blockIdx.x % (N / ROWS) * ROWS;
+  constexpr long long XM = G == 2 ? (long long)N * N : 2LL * N * N;
+  float* base = mesh + x * XM + (long long)y * N;
+  const float2* i0 = spec + R::at(x, y);
   const float2* i1 = i0 + (long long)NX * N * P;
   auto gin = [i0, i1, kz_cols](int j, int cp) {
     const int k = j <= N / 2 ? j : N - j;
     if (k >= kz_cols) return make_float4(0.f, 0.f, 0.f, 0.f);
-    const float2* b = (j <= N / 2 ? i0 : i1) + (2 * cp) * P + k;
-    const float2 u = __ldcg(b), v = __ldcg(b + P);
+    const float2* b = (j <= N / 2 ? i0 : i1) + 2 * cp / PACK_W * R::ROW + 2 * cp % PACK_W * 8 + R::kz(k);
+    const float2 u = __ldcg(b), v = __ldcg(b + 8);
     return make_float4(u.y, u.x, v.y, v.x);
   };
   auto sin_ = [](int j, int cp) { return s4[cp * N + zsw(j)]; };
   auto sout = [](int j, int cp, float4 v) { s4[cp * N + zsw(j)] = v; };
   auto gout = [base](int j, int cp, float4 v) {
-    float* b = base + 2 * cp * N + j;
+    float* b = base + 2 * cp % PACK_W * XM + 2 * cp / PACK_W * N + j;
     __stcs(b, v.y);
     __stcs(b + IM, v.x);
-    __stcs(b + N, v.w);
-    __stcs(b + IM + N, v.z);
+    __stcs(b + XM, v.w);
+    __stcs(b + IM + XM, v.z);
   };
   fft::run_stages2<N, CP, NT, true, false, false>(gin, sin_, sout, gout, tw, tid);
 }
 
 template <int N>
 constexpr int z_pairs() { return N >= 256 ? 8 : 32768 / (N * 8); }   // >= 256 threads
-template <int N, int PRUNE>
+template <int N, int PRUNE, int W>
 int launch_cols(float2* data, long long plane_stride, long long row_stride, int nplanes, int nkb, int k2_max,
                 const float2* tw, cudaStream_t st) {
-  const size_t smem = (size_t)fft::ColBlock<N, 1>::SLAB * sizeof(float2);
-  auto kc = fft_cols_kernel<N, PRUNE>;
+  constexpr int SL = W == 1 ? 1 : Y_PLANES<N>;
+  const size_t smem = (size_t)SL * fft::ColBlock<N, SL>::SLAB * sizeof(float2);
+  auto kc = fft_cols_kernel<N, PRUNE, W, SL>;
   GBP_CUDA_TRY(cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  GBP_CUDA_TRY(launch_pdl(kc, dim3((unsigned)(nplanes * nkb)), dim3(N / 2), smem, st, data, plane_stride, row_stride,
+  GBP_CUDA_TRY(launch_pdl(kc, dim3((unsigned)(nplanes / SL * nkb)), dim3(N / 2 * SL), smem, st, data, plane_stride, row_stride,
                           nplanes, nkb, k2_max, tw));
   return GBP_OK;
 }
@@ -275,14 +301,14 @@ int run_fft(const float* mesh, float2* spec, int G, const float2* tw, cudaStream
   }
   {  // y pass: a plane is one x slab of one grid; rows (y) are P apart
     GBP_TRACE("fft_y", st);
-    const int r = launch_cols<N, 0>(spec, (long long)N * P, (long long)P, G * N, P / C, 0, tw, st);
+    const int r = launch_cols<N, 0, 1>(spec, (long long)N * P, (long long)P, G * N, P / C, 0, tw, st);
     if (r) return r;
   }
   // x pass: a plane is one y row of one grid; rows (x) are N*P apart
   for (int g = 0; g < G; ++g) {
     GBP_TRACE("fft_x", st);
     const int r =
-        launch_cols<N, 0>(spec + (long long)g * N * N * P, (long long)P, (long long)N * P, N, P / C, 0, tw, st);
+        launch_cols<N, 0, 1>(spec + (long long)g * N * N * P, (long long)P, (long long)N * P, N, P / C, 0, tw, st);
     if (r) return r;
   }
   return GBP_OK;
@@ -302,12 +328,14 @@ int run_z_packed(const float* mesh, float2* spec, int kz_cols, const float2* tw,
 }
 
 template <int N>
-int run_y_packed(int G, float2* spec, int kz_cols, int k2_max, const float2* tw, cudaStream_t st) {
+int run_y_packed(int G, bool rows, float2* spec, int kz_cols, int k2_max, const float2* tw, cudaStream_t st) {
   constexpr int P = zpitch(N);
   if (kz_cols == 0) return GBP_OK;
   GBP_TRACE("fft_y", st);
   // a plane is one x' of one slab: two slabs of N (two grids) or N/2 planes
-  return launch_cols<N, 1>(spec, (long long)N * P, (long long)P, G * N, kz_cols / 8, k2_max, tw, st);
+  if (rows) return launch_cols<N, 1, 1>(spec, (long long)N * P, (long long)P, G * N, kz_cols / 8, k2_max, tw, st);
+  using R = fft::PackedRows<N>;
+  return launch_cols<N, 1, PACK_W>(spec, 0, (long long)R::ROW, G * N, kz_cols / 8, k2_max, tw, st);
 }
 
 template <int N>
@@ -315,17 +343,18 @@ int run_y_shells(float2* spec, int nplanes, int r2_max, const float2* tw, cudaSt
   constexpr int P = zpitch(N);
   if (nplanes == 0) return GBP_OK;
   GBP_TRACE("fft_y", st);
-  return launch_cols<N, 2>(spec, (long long)N * P, (long long)P, nplanes, P / 8, r2_max, tw, st);
+  return launch_cols<N, 2, 1>(spec, (long long)N * P, (long long)P, nplanes, P / 8, r2_max, tw, st);
 }
 
 template <int N>
 int run_y_inverse(int G, float2* spec, int kz_cols, int k2_max, const float2* tw, cudaStream_t st) {
   if (kz_cols == 0) return GBP_OK;
-  const size_t smem = (size_t)fft::ColBlock<N, 1>::SLAB * sizeof(float2);
-  auto k = fft_cols_inv_kernel<N>;
+  constexpr int SL = Y_PLANES<N>;
+  const size_t smem = (size_t)SL * fft::ColBlock<N, SL>::SLAB * sizeof(float2);
+  auto k = fft_cols_inv_kernel<N, SL>;
   GBP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   GBP_TRACE("fft_y_inverse", st);
-  GBP_CUDA_TRY(launch_pdl(k, dim3((unsigned)(G * N * (kz_cols / 8))), dim3(N / 2), smem, st, spec, G * N, kz_cols / 8,
+  GBP_CUDA_TRY(launch_pdl(k, dim3((unsigned)(G * N / SL * (kz_cols / 8))), dim3(N / 2 * SL), smem, st, spec, G * N, kz_cols / 8,
                           k2_max, tw));
   return GBP_OK;
 }
@@ -426,11 +455,22 @@ int own_fft_z_packed(int N, int G, const float* mesh, float2* spec, int kz_cols,
 
 int own_fft_y_packed(int N, int G, float2* spec, int kz_cols, int k2_max, const float2* tw, cudaStream_t st) {
   switch (N) {
-    case 64: return run_y_packed<64>(G, spec, kz_cols, k2_max, tw, st);
-    case 128: return run_y_packed<128>(G, spec, kz_cols, k2_max, tw, st);
-    case 256: return run_y_packed<256>(G, spec, kz_cols, k2_max, tw, st);
-    case 512: return run_y_packed<512>(G, spec, kz_cols, k2_max, tw, st);
-    case 1024: return run_y_packed<1024>(G, spec, kz_cols, k2_max, tw, st);
+    case 64: return run_y_packed<64>(G, false, spec, kz_cols, k2_max, tw, st);
+    case 128: return run_y_packed<128>(G, false, spec, kz_cols, k2_max, tw, st);
+    case 256: return run_y_packed<256>(G, false, spec, kz_cols, k2_max, tw, st);
+    case 512: return run_y_packed<512>(G, false, spec, kz_cols, k2_max, tw, st);
+    case 1024: return run_y_packed<1024>(G, false, spec, kz_cols, k2_max, tw, st);
+    default: return GBP_ERR_UNSUPPORTED;
+  }
+}
+
+int own_fft_y_rows(int N, int nplanes, float2* spec, int kz_cols, int k2_max, const float2* tw, cudaStream_t st) {
+  switch (N) {
+    case 64: return run_y_packed<64>(nplanes / N, true, spec, kz_cols, k2_max, tw, st);
+    case 128: return run_y_packed<128>(nplanes / N, true, spec, kz_cols, k2_max, tw, st);
+    case 256: return run_y_packed<256>(nplanes / N, true, spec, kz_cols, k2_max, tw, st);
+    case 512: return run_y_packed<512>(nplanes / N, true, spec, kz_cols, k2_max, tw, st);
+    case 1024: return run_y_packed<1024>(nplanes / N, true, spec, kz_cols, k2_max, tw, st);
     default: return GBP_ERR_UNSUPPORTED;
   }
 }

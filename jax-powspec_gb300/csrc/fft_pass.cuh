@@ -3,7 +3,10 @@
 //
 //   * each thread transforms the same butterfly of two adjacent columns at
 //     once: every shared or global access moves 16 bytes (two complex
-//     values), and the two butterflies share one set of twiddle factors;
+//     values), the two butterflies share one set of twiddle factors, and
+//     their additions are single f32x2 instructions (values that cross shared
+//     memory between stages are kept as two real and two imaginary parts, so
+//     they need no rearranging): 1-4 % of each pass;
 //   * the twiddles come from per-stage tables, w_r(k) = exp(-2 pi i r k /
 //     (R p)) for r < 8 stored contiguously per k (four 16-byte loads);
 //   * the first stage reads its inputs from wherever they are (HBM, or
@@ -68,9 +71,10 @@ __device__ __forceinline__ void group_sync(int tid) {
 // column pair b / (N/R) (consecutive lanes, consecutive rows); otherwise
 // column pair b % CP, butterfly b / CP.  GS > 0 (IFAST, N/R == GS threads per
 // column pair, one butterfly each): the barriers cover only the threads of
-// one column pair, whose data no other thread touches.
-template <int N, int R, int CP, int NT, bool MID_SYNC, bool END_SYNC, bool IFAST, class In, class Out,
-          int GS = 0>
+// one column pair, whose data no other thread touches.  PLANAR_IN / PLANAR_OUT: a
+// float4 holds (re, re, im, im) of the two columns, else (re, im, re, im).
+template <int N, int R, int CP, int NT, bool MID_SYNC, bool END_SYNC, bool IFAST, bool PLANAR_IN, bool PLANAR_OUT,
+          class In, class Out, int GS = 0>
 __device__ __forceinline__ void stage2(In in, Out out, const float2* __restrict__ tw, int p, int tid) {
   constexpr int NB = CP * (N / R);
   constexpr int PER = (NB + NT - 1) / NT;
@@ -82,11 +86,12 @@ __device__ __forceinline__ void stage2(In in, Out out, const float2* __restrict_
     const int cp = IFAST ? b / (N / R) : b % CP, i = IFAST ? b % (N / R) : b / CP;
 #pragma unroll
     for (int r = 0; r < R; ++r) u[q][r] = in(i + r * (N / R), cp);
-    float2 a[R], c[R];
+    Pair a[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      a[r] = lo2(u[q][r]);
-      c[r] = hi2(u[q][r]);
+      const float4 v = u[q][r];
+      a[r] = PLANAR_IN ? Pair{make_float2(v.x, v.y), make_float2(v.z, v.w)}
+                       : Pair{make_float2(v.x, v.z), make_float2(v.y, v.w)};
     }
     if (p > 1) {
       const int k = i & (p - 1);
@@ -94,26 +99,17 @@ __device__ __forceinline__ void stage2(In in, Out out, const float2* __restrict_
 #pragma unroll
       for (int rr = 0; rr < R / 2; ++rr) {
         const float4 w = __ldg(t4 + rr);
-        if (rr > 0) {
-          a[2 * rr] = cmul(a[2 * rr], lo2(w));
-          c[2 * rr] = cmul(c[2 * rr], lo2(w));
-        }
+        if (rr > 0) a[2 * rr] = cmul(a[2 * rr], lo2(w));
         a[2 * rr + 1] = cmul(a[2 * rr + 1], hi2(w));
-        c[2 * rr + 1] = cmul(c[2 * rr + 1], hi2(w));
       }
     }
-    if constexpr (R == 8) {
-      dft8(a);
-      dft8(c);
-    } else if constexpr (R == 4) {
-      dft4(a);
-      dft4(c);
-    } else {
-      dft2(a[0], a[1]);
-      dft2(c[0], c[1]);
-    }
+    if constexpr (R == 8) dft8(a);
+    else if constexpr (R == 4) dft4(a);
+    else dft2(a[0], a[1]);
 #pragma unroll
-    for (int r = 0; r < R; ++r) u[q][r] = pack2(a[r], c[r]);
+    for (int r = 0; r < R; ++r)
+      u[q][r] = PLANAR_OUT ? make_float4(a[r].re.x, a[r].re.y, a[r].im.x, a[r].im.y)
+                           : make_float4(a[r].re.x, a[r].im.x, a[r].re.y, a[r].im.y);
   }
   static_assert(GS == 0 || (IFAST && N / R == GS && NB == NT), "group barriers need one column pair per group");
   static_assert(GS == 0 || CP <= MAX_GROUPS, "more groups than named barriers");
@@ -145,25 +141,25 @@ __device__ __forceinline__ void run_stages2(GIn gin, SIn sin_, SOut sout, GOut g
   using RD = Radices<N>;
   static_assert(RD::stages >= 2, "at least two stages");
   static_assert(GS == 0 || RD::tail == 0, "group barriers need radix-8 stages only");
-  stage2<N, 8, CP, NT, IN_SHARED, true, IFAST, GIn, SOut, GS>(gin, sout, tw, 1, tid);
+  stage2<N, 8, CP, NT, IN_SHARED, true, IFAST, false, true, GIn, SOut, GS>(gin, sout, tw, 1, tid);
   int p = 8;
   if constexpr (RD::tail == 0) {
 #pragma unroll
     for (int st = 1; st < RD::n8 - 1; ++st) {
-      stage2<N, 8, CP, NT, true, true, IFAST, SIn, SOut, GS>(sin_, sout, tw, p, tid);
+      stage2<N, 8, CP, NT, true, true, IFAST, true, true, SIn, SOut, GS>(sin_, sout, tw, p, tid);
       p *= 8;
     }
     // the last stage's outputs may be read by any thread: a CTA barrier ends it
-    stage2<N, 8, CP, NT, OUT_SHARED, false, IFAST, SIn, GOut, GS>(sin_, gout, tw, p, tid);
+    stage2<N, 8, CP, NT, OUT_SHARED, false, IFAST, true, false, SIn, GOut, GS>(sin_, gout, tw, p, tid);
     if (OUT_SHARED) __syncthreads();
   } else {
 #pragma unroll
     for (int st = 1; st < RD::n8; ++st) {
-      stage2<N, 8, CP, NT, true, true, IFAST>(sin_, sout, tw, p, tid);
+      stage2<N, 8, CP, NT, true, true, IFAST, true, true>(sin_, sout, tw, p, tid);
       p *= 8;
     }
-    if constexpr (RD::tail == 1) stage2<N, 2, CP, NT, OUT_SHARED, OUT_SHARED, IFAST>(sin_, gout, tw, p, tid);
-    else stage2<N, 4, CP, NT, OUT_SHARED, OUT_SHARED, IFAST>(sin_, gout, tw, p, tid);
+    if constexpr (RD::tail == 1) stage2<N, 2, CP, NT, OUT_SHARED, OUT_SHARED, IFAST, true, false>(sin_, gout, tw, p, tid);
+    else stage2<N, 4, CP, NT, OUT_SHARED, OUT_SHARED, IFAST, true, false>(sin_, gout, tw, p, tid);
   }
 }
 
@@ -191,20 +187,36 @@ __device__ __forceinline__ void col_fft(float2* s, In gin, Out gout, const float
   run_stages2<N, L::CP, NT, false, IN_SHARED, OUT_SHARED>(gin, sin_, sout, gout, tw, tid);
 }
 
-// Stores Z[k] of columns 2cp and 2cp + 1 (rows 2cp, 2cp + 1 of pitch P) of a
-// packed z pass: kz = k goes to slab 0 (o0) when k <= N/2, kz = -(N - k) to
-// slab 1 (o1) when N - k <= N/2 (k = 0 and N/2 to both); columns >= kz_cols
-// are not stored.
+// Rows of a packed spectrum (slabs of x planes, rows y, N/2 + 8 complex kz):
+// W planes are interleaved in blocks of 8 kz (64 bytes), so the x pass, which
+// reads one block of every plane, finds W of them side by side.  Its time at
+// 512^3, two grids: W = 1 0.527 ms, 2 0.458, 4 0.438, all planes 0.435.  N and
+// N / 2 planes of a slab are multiples of 4.
+constexpr int PACK_W = 4;
+template <int N, int W = PACK_W>
+struct PackedRows {
+  static constexpr int P = N / 2 + 8, ROW = W * P, BLOCK = 8 * W;      // from a row, a kz block, to the next
+  __device__ static __forceinline__ long long plane(int x) {
+    return (long long)(x / W) * W * N * P + (x % W) * 8;
+  }
+  __device__ static __forceinline__ long long at(int x, int y) { return plane(x) + (long long)y * ROW; }
+  __device__ static __forceinline__ int kz(int k) { return (k >> 3) * BLOCK + (k & 7); }
+};
+
+// Stores Z[k] of two columns of a packed z pass, whose entries lie `step`
+// apart: kz = k goes to slab 0 (o0) when k <= N/2, kz = -(N - k) to slab 1
+// (o1) as entry N - k when N - k <= N/2; only kz < kz_cols are kept.
 template <int N>
-__device__ __forceinline__ void store_packed(float2* o0, float2* o1, int P, int kz_cols, int k, int cp, float4 v) {
+__device__ __forceinline__ void store_packed(float2* o0, float2* o1, int step, int kz_cols, int k, float4 v) {
+  using R = PackedRows<N>;
   const int m = (N - k) & (N - 1);
   if (k <= N / 2 && k < kz_cols) {
-    __stcs(o0 + 2 * cp * P + k, lo2(v));
-    __stcs(o0 + (2 * cp + 1) * P + k, hi2(v));
+    __stcs(o0 + R::kz(k), lo2(v));
+    __stcs(o0 + step + R::kz(k), hi2(v));
   }
   if (m <= N / 2 && m < kz_cols) {
-    __stcs(o1 + 2 * cp * P + m, lo2(v));
-    __stcs(o1 + (2 * cp + 1) * P + m, hi2(v));
+    __stcs(o1 + R::kz(m), lo2(v));
+    __stcs(o1 + step + R::kz(m), hi2(v));
   }
 }
 

@@ -28,6 +28,8 @@ int own_fft_r2c(int N, int G, const float* mesh, float2* spec, const float2* tw,
 int own_fft_z_packed(int N, int G, const float* mesh, float2* spec, int kz_cols, const float2* tw, cudaStream_t st);
 // y pass of the packed layout: kz < kz_cols, rows with ky^2 + (first kz of the block)^2 <= k2_max stored
 int own_fft_y_packed(int N, int G, float2* spec, int kz_cols, int k2_max, const float2* tw, cudaStream_t st);
+// the same for nplanes (a multiple of N) x planes of plain rows [x][N][P]
+int own_fft_y_rows(int N, int nplanes, float2* spec, int kz_cols, int k2_max, const float2* tw, cudaStream_t st);
 // Inverse y pass of a packed spectrum that holds only kz < kz_cols and rows with ky^2 + (first kz of the
 // block)^2 <= k2_max, in place; inverse z pass into the real fields (unnormalised, as the forward passes)
 int own_fft_y_inverse(int N, int G, float2* spec, int kz_cols, int k2_max, const float2* tw, cudaStream_t st);

@@ -263,10 +263,11 @@ grad_x_kernel(PowGeom g, const float4* __restrict__ coef, float2* __restrict__ o
       const float2 u = s[(2 * cp) * TST + xswz<M2>(x)], v = s[(2 * cp + 1) * TST + xswz<M2>(x)];
       return make_float4(u.y, u.x, v.y, v.x);
     };
-    float2* dst = out + kb * XB_C;
-    const long long r0 = (long long)y * P, r1 = (long long)NX * N * P + (long long)((N - y) & (N - 1)) * P;
+    using R = fft::PackedRows<N>;
+    float2* dst = out + kb * R::BLOCK;
+    const long long r0 = (long long)y * R::ROW, r1 = R::plane(NX) + (long long)((N - y) & (N - 1)) * R::ROW;
     auto gout = [dst, r0, r1](int x, int cp, float4 v) {
-      __stcs(reinterpret_cast<float4*>(dst + (cp < 4 ? r0 : r1) + (long long)x * N * P) + (cp & 3),
+      __stcs(reinterpret_cast<float4*>(dst + (cp < 4 ? r0 : r1) + R::plane(x)) + (cp & 3),
              make_float4(v.y, v.x, v.w, v.z));
     };
     fft::col_fft<NX, 2, NT, false, decltype(gin), decltype(gout), true>(s, gin, gout, g.twx, tid);

@@ -31,9 +31,12 @@
 // Only items with a mode inside the last k edge are listed by the bin plan
 // (gbp_bins_create): edges up to k_Nyquist leave out a fifth of them.  Two
 // grids at 512^3: 0.688 -> 0.552 ms, 0.526 with loads that keep their lines in
-// L2 for the neighbouring kz block (0.86 GB read: 1.6 TB/s; bound by
-// instruction issue and barriers); one grid (half the points per column, a
-// warp per column): 0.545 -> 0.362 ms at 512^3, 0.091 -> 0.045 at 256^3.
+// L2, 0.438 with interleaved planes (0.86 GB read: 2.0 TB/s; 1024^3 5.16 ->
+// 4.34 ms, 256^3 0.074 -> 0.063); one grid (half the points per column, a warp
+// per column): 0.545 -> 0.362, 0.330, 0.285 ms at 512^3.  Bound by barriers,
+// shared-memory wavefronts (half the pipe) and issue (0.4 of the slots).  Items
+// of 4 columns (half the threads per barrier) took 0.543 ms, for their 32-byte
+// rows, before the interleaving.
 //
 // The mode arithmetic (window deconvolution, interlacing average, |delta|^2,
 // mu^2 and mu^4 moments, DC removal) and the bin lookup are those of

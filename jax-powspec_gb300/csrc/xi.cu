@@ -20,7 +20,7 @@
 // it back along x in the same kernel, storing the x planes within the last
 // edge; the y pass stores the rows within it; the z pass bins its pencils in
 // shared memory, z and -z together, with weight 2 for 0 < x < N/2.
-// 256^3, r < 0.2 L: 0.404 -> 0.161 ms of kernels (z 0.035, y 0.026, x 0.064,
+// 256^3, r < 0.2 L: 0.404 -> 0.157 ms of kernels (z 0.035, y 0.026, x 0.064,
 // y of 52 planes 0.012, z + bins 0.017; the field path's C2R alone took 0.098
 // and its binning 0.144).
 //

@@ -106,19 +106,20 @@ __device__ __forceinline__ void flush_runs(float (&P)[MS][NV], const int (&bin)[
 
 // Loads item (y, kb) of the packed spectrum `spec` (transformed over z and y)
 // and transforms its 16 columns along x into s (transposed, swizzled); ends
-// with a barrier.  IN_SHARED: see fft::col_fft.  planes: how many row planes
-// of [N][P] apart consecutive x' lie (the slabs NX * planes of them).
-template <int N, bool INTER, bool IN_SHARED, int NT = x_threads(N, INTER)>
+// with a barrier.  IN_SHARED: see fft::col_fft.  W: interleaved planes
+// (fft::PackedRows); W = 1: plain rows, consecutive x' `planes` planes of
+// [N][P] apart (the slabs NX * planes of them).
+template <int N, bool INTER, bool IN_SHARED, int NT = x_threads(N, INTER), int W = fft::PACK_W>
 __device__ __forceinline__ void x_forward(float2* s, const float2* __restrict__ spec, int y, int kb,
                                           const float2* __restrict__ twx, int tid, int planes = 1) {
   using L = XLayout<N, INTER, NT>;
-  constexpr int P = N / 2 + 8, TST = L::TST;
-  const float2* src = spec + kb * XB_C;
+  using R = fft::PackedRows<N, W>;
+  constexpr int TST = L::TST;
+  const float2* src = spec + kb * R::BLOCK;
   // row of the column pair's slab: y, or -y of slab 1
-  const long long r0 = (long long)y * P, r1 = (long long)L::NX * planes * N * P + (long long)((N - y) & (N - 1)) * P;
+  const long long r0 = (long long)y * R::ROW, r1 = R::plane(L::NX * planes) + (long long)((N - y) & (N - 1)) * R::ROW;
   auto gin = [src, r0, r1, planes](int x, int cp) {    // columns 2cp, 2cp+1 (slab cp / 4)
-    return __ldcg(reinterpret_cast<const float4*>(src + (cp < 4 ? r0 : r1) + (long long)x * planes * N * P) +
-                  (cp & 3));
+    return __ldcg(reinterpret_cast<const float4*>(src + (cp < 4 ? r0 : r1) + R::plane(x * planes)) + (cp & 3));
   };
   auto tout = [s](int x, int cp, float4 v) {
     s[(2 * cp) * TST + xswz<L::M2>(x)] = fft::lo2(v);
