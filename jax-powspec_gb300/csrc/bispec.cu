@@ -52,7 +52,7 @@
 //   f. bispec_xbin_kernel: x passes of an item of the contrast and of both
 //      products, and the four sums, binned as in xbin.cu.
 //
-// 256^3, k1 = 0.1, k2 = 0.2, 20 angles, L = 2500: 0.857 -> 0.43 ms of kernels (x 0.050, y 0.051, z 0.107,
+// 256^3, k1 = 0.1, k2 = 0.2, 20 angles, L = 2500: 0.857 -> 0.43 ms of kernels (x 0.050, y 0.051, z 0.101,
 // x + bins 0.116).
 //
 // Shell membership is the reference's float32 rule, k = sqrtf(k^2) >=
@@ -301,6 +301,14 @@ bispec_y_kernel(PowGeom g, const int* __restrict__ shell_bins, int k2_max, int n
   fft::col_fft<N, 1, N / 2, false>(sy, gin, gout, g.tw, threadIdx.x);
 }
 
+// Column stages whose barriers cover the threads of a column pair, or a warp (bispec_z at 256^3: 0.106 -> 0.101 ms).
+template <int N, int CP, int NT, bool IN_SHARED, bool OUT_SHARED, class GIn, class SIn, class SOut, class GOut>
+__device__ __forceinline__ void bz_stages(GIn gin, SIn sin_, SOut sout, GOut gout, const float2* __restrict__ tw,
+                                          int tid) {
+  fft::run_stages2<N, CP, NT, true, IN_SHARED, OUT_SHARED, GIn, SIn, SOut, GOut, fft::GROUP<N>>(gin, sin_, sout, gout,
+                                                                                            tw, tid);
+}
+
 // PAIRS pencils per CTA (two x planes, PAIRS / 2 rows): a and b back along z,
 // products, forward along z into the pencils' own rows of slabs 0 and 1 (read
 // before they are written): plane 2x' for delta_1 delta_2, 2x'+1 for I_1 I_2.
@@ -333,8 +341,8 @@ bispec_z_kernel(PowGeom g, const int* __restrict__ shell_bins, int k2_max, int k
   auto asout = [sz_ = sz](int j, int cp, float4 v) { sz_[cp * N + fft::zsw(j)] = v; };
   auto bsin = [sb](int j, int cp) { return sb[cp * N + fft::zsw(j)]; };
   auto bsout = [sb](int j, int cp, float4 v) { sb[cp * N + fft::zsw(j)] = v; };
-  fft::run_stages2<N, CP, NT, true, false, true>(agin, asin, asout, asout, g.tw, tid);
-  fft::run_stages2<N, CP, NT, true, false, true>(bgin, bsin, bsout, bsout, g.tw, tid);
+  bz_stages<N, CP, NT, false, true>(agin, asin, asout, asout, g.tw, tid);
+  bz_stages<N, CP, NT, false, true>(bgin, bsin, bsout, bsout, g.tw, tid);
   // one column of each product per row (the swapped parts of a multiply to the same)
   auto cgin = [&](int j, int cp) {
     const float4 a = asin(j, cp), b = bsin(j, cp);
@@ -351,7 +359,7 @@ bispec_z_kernel(PowGeom g, const int* __restrict__ shell_bins, int k2_max, int k
       __stcs(i1 + pstride + cp * P + m, fft::hi2(v));
     }
   };
-  fft::run_stages2<N, CP, NT, true, true, false>(cgin, asin, asout, cgout, g.tw, tid);
+  bz_stages<N, CP, NT, true, false>(cgin, asin, asout, cgout, g.tw, tid);
 }
 
 template <int N>

@@ -247,10 +247,10 @@ __device__ __forceinline__ void tile_unit(const DepGeom& g, const ColEntries& te
     float2* o0 = spec + fft::PackedRows<N>::at((G == 2 ? x0 : x0 / 2) + a, y0 + ly);
     fft::store_packed<N>(o0, o0 + (long long)NX * N * P, fft::PackedRows<N>::ROW, kz_cols, k, v);
   };
-  // N = 512, 32-bit cells: every stage is radix 8 and the 64 threads of a column pair own its data
-  // (the first stage's writes alias the pair's own pencils), so the stages synchronise 64-thread
-  // groups only.  64-bit cells span twice the bytes of the complex slots: whole-CTA barriers.
-  constexpr int GS = (!WIDE && N == 512 && NT == PAIRS / 2 * (N / 8) && NT / (N / 8) <= fft::MAX_GROUPS) ? N / 8 : 0;
+  // 32-bit cells: the N / 8 threads of a column pair own its data (the first stage's writes alias the
+  // pair's own pencils), so the stages synchronise groups of them only, a warp's or a named barrier
+  // each.  64-bit cells span twice the bytes of the complex slots: whole-CTA barriers.
+  constexpr int GS = WIDE ? 0 : fft::Z_GROUP<N>;
   static_assert(PAIRS * N / 16 <= NT, "one first-stage butterfly per thread");
   fft::run_stages2<N, PAIRS / 2, NT, true, true, false, decltype(gin), decltype(sin_), decltype(sout), decltype(gout),
                    GS>(gin, sin_, sout, gout, tw, tid);

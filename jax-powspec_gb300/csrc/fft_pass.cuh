@@ -55,10 +55,22 @@ __device__ __forceinline__ float4 pack2(float2 a, float2 b) { return make_float4
 // id 1 + tid / GS), or of the whole CTA when GS == 0.
 // A CTA has 16 named barriers and __syncthreads is number 0: at most 15 groups.
 constexpr int MAX_GROUPS = 15;
+
+// Threads of a group that owns whole column pairs (N / 8 threads each, at least a warp), and the rule of the z
+// passes: from 512 up, where a pair's threads are two warps or more, groups (deposit and z pass at 1024^3, one CTA of
+// 1024 threads per SM: 7.95 -> 7.78 ms); below, a CTA barrier keeps a block's loads and stores together (256^3, two
+// meshes: z 0.053 ms, inverse 0.051; with a warp per pair 0.056 and 0.055).
+template <int N>
+constexpr int GROUP = N / 8 < 32 ? 32 : N / 8;
+template <int N>
+constexpr int Z_GROUP = N >= 512 ? GROUP<N> : 0;
+
 template <int GS>
 __device__ __forceinline__ void group_sync(int tid) {
   if constexpr (GS == 0) {
     __syncthreads();
+  } else if constexpr (GS == 32) {
+    __syncwarp();
   } else {
     static_assert(GS % 32 == 0, "named barriers count whole warps");
     asm volatile("bar.sync %0, %1;" ::"r"(1 + tid / GS), "n"(GS) : "memory");
@@ -69,19 +81,27 @@ __device__ __forceinline__ void group_sync(int tid) {
 // MID_SYNC separates the reads from the writes (in-place shared stages);
 // END_SYNC publishes the writes.  IFAST: thread b owns butterfly b % (N/R) of
 // column pair b / (N/R) (consecutive lanes, consecutive rows); otherwise
-// column pair b % CP, butterfly b / CP.  GS > 0 (IFAST, N/R == GS threads per
-// column pair, one butterfly each): the barriers cover only the threads of
-// one column pair, whose data no other thread touches.  PLANAR_IN / PLANAR_OUT: a
+// column pair b % CP, butterfly b / CP.  GS > 0 (IFAST, N / 8 threads per
+// column pair): a group of GS threads owns GS * 8 / N column pairs, whose data
+// no other thread touches, and the barriers cover the group only.
+// PLANAR_IN / PLANAR_OUT: a
 // float4 holds (re, re, im, im) of the two columns, else (re, im, re, im).
 template <int N, int R, int CP, int NT, bool MID_SYNC, bool END_SYNC, bool IFAST, bool PLANAR_IN, bool PLANAR_OUT,
           class In, class Out, int GS = 0>
 __device__ __forceinline__ void stage2(In in, Out out, const float2* __restrict__ tw, int p, int tid) {
   constexpr int NB = CP * (N / R);
-  constexpr int PER = (NB + NT - 1) / NT;
+  constexpr int PER = GS > 0 ? 8 / R : (NB + NT - 1) / NT;
+  static_assert(GS == 0 || (IFAST && GS == GROUP<N> && CP * (N / 8) % GS == 0 && CP * (N / 8) <= NT),
+                "whole groups, one first-stage butterfly per thread");
+  static_assert(GS <= 32 || NT / GS <= MAX_GROUPS, "more groups than named barriers");
+  // number of butterfly q of the thread, column pair by column pair
+  constexpr int STEP = GS > 0 ? GS : NT;
+  const int b0 = GS > 0 && PER > 1 ? tid + tid / STEP * STEP * (PER - 1) : tid;
+  auto number = [b0](int q) { return b0 + q * STEP; };
   float4 u[PER][R];
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
-    const int b = tid + q * NT;
+    const int b = number(q);
     if (PER * NT != NB && b >= NB) continue;
     const int cp = IFAST ? b / (N / R) : b % CP, i = IFAST ? b % (N / R) : b / CP;
 #pragma unroll
@@ -111,12 +131,10 @@ __device__ __forceinline__ void stage2(In in, Out out, const float2* __restrict_
       u[q][r] = PLANAR_OUT ? make_float4(a[r].re.x, a[r].re.y, a[r].im.x, a[r].im.y)
                            : make_float4(a[r].re.x, a[r].im.x, a[r].re.y, a[r].im.y);
   }
-  static_assert(GS == 0 || (IFAST && N / R == GS && NB == NT), "group barriers need one column pair per group");
-  static_assert(GS == 0 || CP <= MAX_GROUPS, "more groups than named barriers");
   if (MID_SYNC) group_sync<GS>(tid);
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
-    const int b = tid + q * NT;
+    const int b = number(q);
     if (PER * NT != NB && b >= NB) continue;
     const int cp = IFAST ? b / (N / R) : b % CP, i = IFAST ? b % (N / R) : b / CP;
     const int k = i & (p - 1);
@@ -135,12 +153,11 @@ __device__ __forceinline__ void stage2(In in, Out out, const float2* __restrict_
 // reads (each then reads everything before it writes; OUT_SHARED also ends
 // with a barrier).
 template <int N, int CP, int NT, bool IFAST, bool IN_SHARED, bool OUT_SHARED, class GIn, class SIn, class SOut,
-          class GOut, int GS = 0>
+          class GOut, int GS = IFAST ? Z_GROUP<N> : 0>
 __device__ __forceinline__ void run_stages2(GIn gin, SIn sin_, SOut sout, GOut gout, const float2* __restrict__ tw,
                                             int tid) {
   using RD = Radices<N>;
   static_assert(RD::stages >= 2, "at least two stages");
-  static_assert(GS == 0 || RD::tail == 0, "group barriers need radix-8 stages only");
   stage2<N, 8, CP, NT, IN_SHARED, true, IFAST, false, true, GIn, SOut, GS>(gin, sout, tw, 1, tid);
   int p = 8;
   if constexpr (RD::tail == 0) {
@@ -155,11 +172,12 @@ __device__ __forceinline__ void run_stages2(GIn gin, SIn sin_, SOut sout, GOut g
   } else {
 #pragma unroll
     for (int st = 1; st < RD::n8; ++st) {
-      stage2<N, 8, CP, NT, true, true, IFAST, true, true>(sin_, sout, tw, p, tid);
+      stage2<N, 8, CP, NT, true, true, IFAST, true, true, SIn, SOut, GS>(sin_, sout, tw, p, tid);
       p *= 8;
     }
-    if constexpr (RD::tail == 1) stage2<N, 2, CP, NT, OUT_SHARED, OUT_SHARED, IFAST, true, false>(sin_, gout, tw, p, tid);
-    else stage2<N, 4, CP, NT, OUT_SHARED, OUT_SHARED, IFAST, true, false>(sin_, gout, tw, p, tid);
+    constexpr int R = RD::tail == 1 ? 2 : 4;
+    stage2<N, R, CP, NT, OUT_SHARED, false, IFAST, true, false, SIn, GOut, GS>(sin_, gout, tw, p, tid);
+    if (OUT_SHARED) __syncthreads();
   }
 }
 
