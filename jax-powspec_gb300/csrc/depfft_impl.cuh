@@ -109,6 +109,15 @@ __device__ __forceinline__ T pick_block(int b, const T (&v)[NSB]) {
   return r;
 }
 
+// Sum over the warp, in every lane: three 26-bit parts (12 signed bits in the
+// last), each summed in 32 bits without overflow.
+__device__ __forceinline__ long long warp_sum(long long v) {
+  const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)v & 0x3ffffffu);
+  const unsigned mid = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 26) & 0x3ffffffu);
+  const int hi = __reduce_add_sync(0xffffffffu, (int)(v >> 52));
+  return (long long)lo + ((long long)mid << 26) + (long long)((unsigned long long)(long long)hi << 52);
+}
+
 // Bits of resolution a block may give up to its 32-bit cells.  A block whose
 // densest z plane is covered by more than 2^(SH_MAX + WBIT) entries (a dense
 // clump: a halo, a point mass) is deposited with 64-bit cells at the common
@@ -118,8 +127,10 @@ constexpr int SH_MAX = 10;
 
 // Two grids per pass share the entry loads and need no split of the packed
 // spectra: deposit_fft_z 0.052 -> 0.034 ms (128^3, 1 M particles CIC), 0.135
-// -> 0.127 (256^3, 1 M TSC); at 512^3 0.742 -> 0.742 (4 Mi TSC, 4x4 instead
-// of 8x4 tiles), bound by instruction issue (0.59 of the slots) and barriers.
+// -> 0.127 (256^3, 1 M TSC); at 512^3 0.752 (4 Mi TSC, 4x4 instead of
+// 8x4 tiles: 0.742 before, with twice the bucket fill), at 1024^3 6.87 -> 7.78
+// (16 Mi PCS; the fill 1.28 -> 0.32).  Bound by the shared-memory pipe (0.71 of
+// its wavefronts at 512^3), instruction issue (0.56 of the slots) and barriers.
 //
 // Deposit, z transform and row stores of one unit (steps 1-4 above); x0, y0:
 // its first pencil.  WIDE: 64-bit cells.  sh[b]: bits given up by scale block
@@ -129,7 +140,7 @@ template <int N, int MAS, int G, class CT, bool WIDE>
 __device__ __forceinline__ void tile_unit(const DepGeom& g, const ColEntries& te, int sg, const int (&sh)[Unit<N, G, CT, WIDE>::NSB],
                                           int x0, int y0, int kz_cols, const float2* __restrict__ tw, float2* __restrict__ spec,
                                           unsigned char* smem, const unsigned* list, long long (*s_part)[G],
-                                          long long (&tm)[G]) {
+                                          long long (&tm)[G], bool clear) {
   using Cell = typename std::conditional<WIDE, unsigned long long, int>::type;
   using U = Unit<N, G, CT, WIDE>;
   constexpr int R = MAS, UX = U::UX, UY = U::UY, PAIRS = U::PAIRS, NT = U::NT, NSB = U::NSB;
@@ -146,11 +157,11 @@ __device__ __forceinline__ void tile_unit(const DepGeom& g, const ColEntries& te
     dn[b] = ldexpf(1.0f, sh[b] - sg);
   }
 
-  {
+  if (clear) {
     uint4* a4 = reinterpret_cast<uint4*>(acc);
     for (int k = tid; k < (int)(U::CELLS * sizeof(Cell) / 16); k += NT) a4[k] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
   }
-  __syncthreads();
 #pragma unroll 1
   for (int q = 0; q < 2; ++q) {
   const unsigned en = q ? te.n[1] : te.n[0];
@@ -257,16 +268,13 @@ __device__ __forceinline__ void tile_unit(const DepGeom& g, const ColEntries& te
   // the unit's exact totals
 #pragma unroll
   for (int q = 0; q < G; ++q) {
-    for (int o = 16; o > 0; o >>= 1) part[q] += __shfl_xor_sync(0xffffffffu, part[q], o);
+    part[q] = warp_sum(part[q]);
     if ((tid & 31) == 0) s_part[tid >> 5][q] = part[q];
   }
   __syncthreads();                                     // also: the next unit reuses the accumulators
-  if (tid == 0) {
+  if (tid < 32) {                                      // one warp: the block ends with this
 #pragma unroll
-    for (int q = 0; q < G; ++q) {
-      tm[q] = 0;
-      for (int k = 0; k < NT / 32; ++k) tm[q] += s_part[k][q];
-    }
+    for (int q = 0; q < G; ++q) tm[q] = warp_sum(tid < NT / 32 ? s_part[tid][q] : 0ll);
   }
 }
 
@@ -293,7 +301,7 @@ __device__ __forceinline__ void tile_units(const DepGeom& g, const ColEntries& t
     }
     long long tm[G];
     tile_unit<N, MAS, G, CT, WIDE>(g, te, sg, shu, x0 + ux, y0 + uy, kz_cols, tw, spec, smem, list,
-                                   s_part, tm);
+                                   s_part, tm, U::NU > 1 && u > 0);
     if (threadIdx.x == 0) {
 #pragma unroll
       for (int q = 0; q < G; ++q) total[q] += tm[q];
@@ -408,9 +416,8 @@ __device__ __forceinline__ bool block_scales(const DepGeom& g, const ColEntries&
     cmax = __reduce_max_sync(0xffffffffu, cmax);
     if ((tid & 31) == 0) s_max[tid >> 5] = cmax;
     __syncthreads();
-    cmax = 0;
-    for (int k = 0; k < NT / 32; ++k) cmax = max(cmax, s_max[k]);
-    __syncthreads();                                   // s_max is reused by the next block
+    cmax = __reduce_max_sync(0xffffffffu, (tid & 31) < NT / 32 ? s_max[tid & 31] : 0);
+    if (b + 1 < NSB) __syncthreads();                  // s_max is reused by the next block
     const unsigned cnt = (unsigned)cmax;
     const int lg = cnt > 1u ? 32 - __clz(cnt - 1u) : 0;  // ceil(log2(entries per plane))
     sh[b] = lg > WBIT ? lg - WBIT : 0;                 // block scale 2^(sg - sh), never finer than 2^sg
@@ -437,6 +444,8 @@ deposit_fftz_kernel(const __grid_constant__ DepGeom g, const float4* __restrict_
   const int t = blockIdx.x;
   const int ty = t % g.nt[1], tx = t / g.nt[1];
   const int x0 = tx * CT::TX, y0 = ty * CT::TY;
+  static_assert(U::CELLS * sizeof(int) >= Unit<N, G, CT, true>::CELLS * 8, "the 64-bit cells lie in what is cleared");
+  for (int k = tid; k < (int)(U::CELLS / 4); k += NT) reinterpret_cast<uint4*>(acc_smem)[k] = make_uint4(0u, 0u, 0u, 0u);
   const ColEntries te = column_entries(g, tx, ty, entries, counts, sp, ctr, s_runs);
   if (tid == 0 && te.n[0] + te.n[1] > g.flag_cap) atomicOr(&ctr->outgrown, 1u);
   const int sg = fixed_scale_exp(ctr->maxw_bits, 0);
