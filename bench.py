@@ -169,26 +169,29 @@ def _cfg_json():
             "parallelism": "replicas"}
 
 
-def kernel_bytes(n: int, N: int, G: int) -> dict:
-    """Algorithmic bytes per launch of each traced kernel (what the algorithm must move)."""
+def kernel_bytes(n: int, N: int, G: int, k_last: float) -> dict:
+    """Algorithmic bytes per launch of each traced kernel (what the algorithm must move); k_last = the last k edge
+    in units of kF.  The fused path stores columns kz within it, and after the y pass rows (ky, kz) within it."""
+    import numpy as np
     M = N ** 3
     Mh = N * N * (N // 2 + 1)
+    kz = np.arange(N // 2 + 1)
+    ky = np.minimum(np.arange(N), N - np.arange(N))
+    cols = N * N * int((kz <= k_last).sum())
+    rows = N * int((ky[:, None] ** 2 + kz[None, :] ** 2 <= k_last ** 2).sum())
     return {
-        # one-pass bucketing: read x, y, z (the bucket writes are implementation traffic); its scan and
-        # scatter return at once unless a bucket overflowed, so they get no byte count
-        "deposit_fill": 12 * n,
-        "deposit_count": 12 * n,                  # count path (small catalogues): read x, y, z
+        "deposit_fill": 12 * n,                   # read x, y, z (the bucket writes are implementation traffic)
+        "deposit_count": 12 * n,                  # count path (large meshes with few particles): read x, y, z
         # deposit fused with the z pass: every particle read once, the z-transformed half spectra written
-        # once (the bucket entries it actually reads, 16 B per particle and touched tile, are
-        # implementation traffic, as is the spectrum rows' padding)
-        "deposit_fft_z": 12 * n + G * 8 * Mh,
+        # once (the 16 B bucket entries it actually reads are implementation traffic, as is the padding)
+        "deposit_fft_z": 12 * n + G * 8 * cols,
         "deposit_tiles": 4 * G * M,               # write every cell of the G meshes once
         "fft_z": G * (4 * M + 8 * Mh),            # read the meshes, write half-spectra
-        "fft_y": G * 16 * Mh,                     # read + write all grids' spectra
+        "fft_y": G * 8 * (cols + rows),           # read the z-transformed spectra, write the rows that are binned
         "fft_x": 16 * Mh,                         # read + write one grid's spectrum
         "cufft_r2c": G * (4 * M + 8 * Mh),
         "power_bins": G * 8 * Mh,                 # read the spectra once
-        "fft_x_bins": G * 8 * Mh,                 # read the z,y-transformed spectra once (x pass + binning)
+        "fft_x_bins": G * 8 * rows,               # read the z,y-transformed spectra once (x pass + binning)
     }
 
 
@@ -207,7 +210,7 @@ def trace_breakdown(ps, xd, yd, zd, reps: int, n: int) -> dict:
         d[0] += 1
         d[1] += ms
     N, G = ps.cfg.n_mesh, ps.cfg.grids
-    alg = kernel_bytes(n, N, G)
+    alg = kernel_bytes(n, N, G, float(ps.cfg.kedges_grid()[-1]))
     out = {}
     for name, (cnt, tot) in per.items():
         mean = tot / cnt
@@ -639,8 +642,7 @@ def main():
                 "h2d_alone_gbs": arena.nbytes / t_h2d / 1e9, "clocks": clk_e2e,
                 "path": "BatchRunner.run_from_host (pinned H2D of every mock, chunk by chunk on a copy stream "
                         "overlapping the lanes) + P_l D2H"},
-        # per mock: the traced stages (the scan stage is two cub kernels) + lane_begin + lane_end; per batch
-        # call: one descriptor kernel per lane
+        # per mock: the traced stages + lane_begin + lane_end; per batch call: one descriptor kernel per lane
         "gpu_launches": int(round(per_mock_launches + 1 + 2)) * args.steps * B + lanes * args.steps,
         "clocks": clk,
         **extra,
