@@ -57,7 +57,7 @@ def _upload(a: np.ndarray, dev: torch.device) -> torch.Tensor:
     """A small host table on the device, through a pinned copy that torch's host allocator keeps until the transfer,
     enqueued on the current stream, is done (pageable memory may be read by the GPU after the call returns where it
     can reach host pages).  Waiting for the transfer, as a blocking copy does, left the GPU idle for 0.1-0.3 ms a call
-    (256^3: xi_vec 0.33 -> 0.24 ms, bispec 1.11 -> 0.81).  Under stream capture the blocking copy refuses, as a
+    (256^3: xi_vec 0.33 -> 0.24 ms, bispec 1.11 -> 0.81; the pinned copies cost 20-30 us each of that back).  Under stream capture the blocking copy refuses, as a
     graph would keep the table's address."""
     t = torch.from_numpy(a)
     if torch.cuda.is_current_stream_capturing():
@@ -196,7 +196,7 @@ def _xi(d: torch.Tensor, box: np.float32, s_edges, nan_mu_at_origin: bool):
     n3 = float(N) ** 3
     nm = counts.to(torch.float64)
     nm.masked_fill_(nm == 0, float("inf"))                                         # :180
-    xi = sums / nm[:, None] / (n3 * n3) * _upload(np.array([1.0, 5.0, 9.0]), dev)
+    xi = sums / nm[:, None] / (n3 * n3) * torch.arange(1.0, 10.0, 4.0, dtype=torch.float64, device=dev)  # 2 l + 1
     r3d = ((_F32(0.5) * (kedges[1:] + kedges[:-1])) * (box * _F32(1.0) / _F32(N))).astype(np.float32)  # :185
     return _upload(r3d, dev), xi.to(torch.float32), nm.to(torch.float32)
 
