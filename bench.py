@@ -654,19 +654,18 @@ def main():
 
 
 # DRAM bytes (read + write) per launch from one ncu capture of the same kernels
-# (--set full, --clock-control none) on 512^3 with 1,048,576 particles,
-# keyed by (kernel, mesh, particles).  The y pass and the x pass + binning
-# move only spectra, so their traffic does not depend on the particle count.
-# The deposit/z kernel writes the z-transformed spectra (1.048 GB, particle
-# independent) and reads its bucket entries (0.037 GB at 1,048,576
-# particles, in proportion to the particles): 1.047 + 4 x 0.037 GB for the
+# (--clock-control none) on 512^3 with 1,048,576 particles, keyed by (kernel,
+# mesh, particles).  The y pass and the x pass + binning move only spectra, so
+# their traffic does not depend on the particle count.  The deposit/z kernel
+# writes the z-transformed spectra (particle independent) and reads its bucket
+# entries, in proportion to the particles: 1.015 + 4 x 0.026 GB for the
 # 4,194,304-particle workload.
-# The one-pass bucketing's entries are still in L2 when it ends (their DRAM
-# writes fall in the deposit/z kernel's window), so it gets no figure.
+# The bucketing's entries are still in L2 when it ends (their DRAM writes fall
+# in the deposit/z kernel's window), so it gets no figure.
 PROFILED_TRAFFIC = {
-    ("deposit_fft_z", 512, 4_194_304): 1_046_520_000 + 4 * 37_453_000,
-    ("fft_y", 512, 4_194_304): 1_107_458_000 + 1_053_273_000,
-    ("fft_x_bins", 512, 4_194_304): 1_107_381_000 + 5_776_000,
+    ("deposit_fft_z", 512, 4_194_304): 1_015_250_000 + 4 * 25_819_000,
+    ("fft_y", 512, 4_194_304): 1_073_804_000 + 789_685_000,
+    ("fft_x_bins", 512, 4_194_304): 852_411_000 + 30_465_000,
 }
 
 
