@@ -88,9 +88,9 @@ struct Unit {
   // threads of the CTA: a butterfly pair (two columns) of the 32-bit unit's radix-8 stages each
   static constexpr int NFFT = NARROW_X * NARROW_Y * G * N / 32;
   static constexpr int NT = NFFT < 256 ? 256 : NFFT;
-  // the kernel waits at the barriers between its phases, and a fourth (64 registers a thread) and a fifth block (48) of
-  // 256 threads hide them: 256^3 TSC weighted 253 -> 243 -> 238 us a call, 24 mocks of 128^3 1543 -> 1443 -> 1402
-  static constexpr int MINB = NT >= 1024 ? 1 : (NT >= 512 ? 2 : 5);   // CTAs per SM the registers are sized for
+  // 64 registers a thread for every size: the kernel waits at the barriers between its phases, and a fourth
+  // block of 256 threads hides them (256^3 TSC weighted 253 -> 244 us a call, 24 mocks of 128^3 1543 -> 1446)
+  static constexpr int MINB = NT >= 1024 ? 1 : (NT >= 512 ? 2 : 4);   // CTAs per SM the registers are sized for
   static constexpr size_t CELLS = (size_t)2 * PAIRS * N;
   static constexpr int LIST = 4 * NT;              // entries whose places are kept between the two passes
   static constexpr size_t SMEM = (CELLS + (size_t)CT::NSB * N + LIST) * sizeof(int);   // cells, plane counts, list
