@@ -96,7 +96,11 @@ struct Axis {
 // reference's node convention: node i sits at xmin + i*H).  `half` shifts
 // the particle by +half a cell (the second, interlaced grid).  NC > 0: the
 // mesh side as a power-of-two constant (the cell index wraps with a mask,
-// the same value as pmod for every int).
+// the same value as pmod for every int).  Every operation is an intrinsic: as
+// plain expressions the compiler chose per kernel instance which products to
+// fuse, and two tile shapes of one build could then differ in the last bits
+// of their cells (nvcc 13.0 with registers for five CTAs per SM in the
+// deposit/z kernel: 64^3 PCS).
 template <int MAS, int NC = 0>
 __device__ __forceinline__ void axis_bspline(float u, int N, int half, Axis<MAS>& a) {
   static_assert(NC == 0 || (NC & (NC - 1)) == 0, "NC is a power of two");
@@ -120,18 +124,23 @@ __device__ __forceinline__ void axis_bspline(float u, int N, int half, Axis<MAS>
     const int up = d >= 0.5f ? 1 : 0;           // nearest node is i+up
     const float s = up ? __fsub_rn(d, 1.0f) : d;  // offset from it, [-0.5, 0.5)
     a.first = i + up - 1;
-    const float l = 0.5f - s, r = 0.5f + s;
-    a.w[0] = 0.5f * l * l;
-    a.w[1] = 0.75f - s * s;
-    a.w[2] = 0.5f * r * r;
+    const float l = __fsub_rn(0.5f, s), r = __fadd_rn(0.5f, s);
+    a.w[0] = __fmul_rn(__fmul_rn(0.5f, l), l);
+    a.w[1] = __fmaf_rn(-s, s, 0.75f);
+    a.w[2] = __fmul_rn(__fmul_rn(0.5f, r), r);
   } else {                                      // PCS (cubic B-spline)
-    const float t = d, m = 1.0f - d;
+    const float t = d, m = __fsub_rn(1.0f, d);
     const float c6 = 1.0f / 6.0f;
     a.first = i - 1;
-    a.w[0] = m * m * m * c6;
-    a.w[1] = (4.0f - 6.0f * t * t + 3.0f * t * t * t) * c6;
-    a.w[2] = (4.0f - 6.0f * m * m + 3.0f * m * m * m) * c6;
-    a.w[3] = t * t * t * c6;
+    auto cube = [c6](float v) { return __fmul_rn(__fmul_rn(__fmul_rn(v, v), v), c6); };
+    auto inner = [c6](float v) {                // (4 - 6 v^2 + 3 v^3) / 6
+      const float q = __fmaf_rn(__fmul_rn(-6.0f, v), v, 4.0f);
+      return __fmul_rn(__fmaf_rn(__fmul_rn(__fmul_rn(3.0f, v), v), v, q), c6);
+    };
+    a.w[0] = cube(m);
+    a.w[1] = inner(t);
+    a.w[2] = inner(m);
+    a.w[3] = cube(t);
   }
 }
 
