@@ -170,7 +170,6 @@ extern "C" int gbp_bins_create(const float* e, int ne, int N, gbp_bins* out) {
   B->nb = ne - 1;
   B->nbe = reach > 0 ? reach : 1;
   B->last_closed = last;
-  B->last_bin = thr[ne - 2];
   const long long K = kmax2_of(N);
   int sh = 0;
   while (((K >> sh) + 1) > LUT_MAX) ++sh;

@@ -493,8 +493,7 @@ int bp_layout(const gbp_fft_plan_s* plan, const gbp_bins_s* B, BpLayout& L) {
     case 1024: st = bp_layout_n<1024>(B, L); break;
   }
   if (st) return st;
-  // the last elementary bin is never a shell's: nothing from its lower edge on is needed
-  L.k2_max = std::min(B->last_closed, B->last_bin - 1);
+  L.k2_max = B->last_closed;      // shells may take in the last elementary bin
   L.kz_cols = 0;
   for (int kb = 0; 8 * kb <= N / 2 && 64LL * kb * kb <= L.k2_max; ++kb) L.kz_cols = 8 * (kb + 1);
   L.items = N * (P / 8);

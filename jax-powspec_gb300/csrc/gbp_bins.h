@@ -16,7 +16,6 @@ struct gbp_bins_s {
   int lut_shift;    // lut[k2 >> lut_shift] = #thresholds <= (k2 >> shift) << shift
   int lut_n;
   int32_t last_closed;
-  int32_t last_bin;     // smallest k^2 at or above the lower edge of the last bin
   int device;
   int* d_thr;           // [nbe + 1]
   int* d_lut;           // [lut_n]

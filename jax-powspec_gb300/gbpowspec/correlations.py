@@ -236,11 +236,10 @@ def bispec_shells(box_size, k1, k2, theta):
 
 
 def _elementary_bins(k_min: np.ndarray, k_max: np.ndarray):
-    """Sorted distinct shell limits (+ one edge above them all, so that the closed last bin of the
-    histogram rule is never a shell's) and each shell's [first, one-past-last) elementary bin."""
+    """Sorted distinct shell limits (+ the next float32 as one edge above them all, so that the closed last bin of
+    the histogram rule is never a shell's) and each shell's [first, one-past-last) elementary bin."""
     e = np.unique(np.concatenate([k_min, k_max]).astype(np.float32))
-    top = _F32(e[-1] + max(_F32(1.0), abs(e[-1])))
-    edges = np.append(e, top).astype(np.float32)
+    edges = np.append(e, np.nextafter(e[-1], _F32(np.inf))).astype(np.float32)
     lo = np.searchsorted(edges, k_min, side="left")
     hi = np.searchsorted(edges, k_max, side="left")
     return edges, np.stack([lo, hi], axis=1).astype(np.int32)
