@@ -127,6 +127,75 @@ __device__ __forceinline__ long long warp_sum(long long v) {
 // contributions adds up instead of averaging out.
 constexpr int SH_MAX = 10;
 
+template <int N, int G, class CT, bool WIDE>
+using UnitCell = typename std::conditional<WIDE, unsigned long long, int>::type;
+
+// Adds entry e (all grids) to the cells of the unit at (x0, y0); up: 2^s of
+// its scale blocks.
+template <int N, int MAS, int G, class CT, bool WIDE>
+__device__ __forceinline__ void add_entry(const DepGeom& g, const float4& e,
+                                          const float (&up)[Unit<N, G, CT, WIDE>::NSB], int x0, int y0,
+                                          UnitCell<N, G, CT, WIDE>* acc) {
+  using U = Unit<N, G, CT, WIDE>;
+  constexpr int R = MAS, UX = U::UX, UY = U::UY, NSB = U::NSB, SBY = U::SBY;
+#pragma unroll
+  for (int grid = 0; grid < G; ++grid) {
+    Axis<R> ax, ay, az;
+    make_axis<MAS, 0, N>(g, e.x, grid, ax);
+    make_axis<MAS, 0, N>(g, e.y, grid, ay);
+    make_axis<MAS, 0, N>(g, e.z, grid, az);
+    int lx[R], ly[R], zz[R];
+    local_nodes<R>(ax, N, x0, UX, lx);
+    local_nodes<R>(ay, N, y0, UY, ly);
+    // z weight times the particle weight at each block's scale (exact: powers of two)
+    float wz[NSB][R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) zz[r] = wrapn(az.first + r, N);
+#pragma unroll
+    for (int b = 0; b < NSB; ++b) {
+      const float wsc = __fmul_rn(e.w, up[b]);
+#pragma unroll
+      for (int r = 0; r < R; ++r) wz[b][r] = __fmul_rn(az.w[r], wsc);
+    }
+#pragma unroll
+    for (int rx = 0; rx < R; ++rx) {
+      if (lx[rx] < 0) continue;
+      // with one block row the block depends on x only: select the z weights once per x node
+      float wzx[R];
+      if constexpr (SBY == 1) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          float wzb[NSB];
+#pragma unroll
+          for (int k = 0; k < NSB; ++k) wzb[k] = wz[k][r];
+          wzx[r] = pick_block<NSB>(lx[rx] >> 2, wzb);
+        }
+      }
+#pragma unroll
+      for (int ry = 0; ry < R; ++ry) {
+        if (ly[ry] < 0) continue;
+        const float wxy = __fmul_rn(ax.w[rx], ay.w[ry]);
+        const int row = U::cell_row(lx[rx], ly[ry], grid);
+#pragma unroll
+        for (int rz = 0; rz < R; ++rz) {
+          float wzr;
+          if constexpr (SBY == 1) {
+            wzr = wzx[rz];
+          } else {
+            float wzb[NSB];
+#pragma unroll
+            for (int k = 0; k < NSB; ++k) wzb[k] = wz[k][rz];
+            wzr = pick_block<NSB>((lx[rx] >> 2) * SBY + (ly[ry] >> 2), wzb);
+          }
+          const int v = __float2int_rn(__fmul_rn(wxy, wzr));
+          if constexpr (WIDE) atomicAdd(&acc[row + zz[rz]], (unsigned long long)(long long)v);
+          else atomicAdd(&acc[row + zz[rz]], v);
+        }
+      }
+    }
+  }
+}
+
 // Two grids per pass share the entry loads and need no split of the packed
 // spectra: deposit_fft_z 0.052 -> 0.034 ms (128^3, 1 M particles CIC), 0.135
 // -> 0.127 (256^3, 1 M TSC); at 512^3 0.752 (4 Mi TSC, 4x4 instead of
@@ -137,15 +206,16 @@ constexpr int SH_MAX = 10;
 // Deposit, z transform and row stores of one unit (steps 1-4 above); x0, y0:
 // its first pencil.  WIDE: 64-bit cells.  sh[b]: bits given up by scale block
 // b of the unit (its scale 2^(sg - sh[b]), sh[b] <= SH_MAX).  tm[grid]: the
-// unit's exact totals at the common scale 2^sg (valid in thread 0).
-template <int N, int MAS, int G, class CT, bool WIDE>
+// unit's exact totals at the common scale 2^sg (valid in thread 0).  SPILLED:
+// the tile's spilled entries too.
+template <int N, int MAS, int G, class CT, bool WIDE, bool SPILLED>
 __device__ __forceinline__ void tile_unit(const DepGeom& g, const ColEntries& te, int sg, const int (&sh)[Unit<N, G, CT, WIDE>::NSB],
                                           int x0, int y0, int kz_cols, const float2* __restrict__ tw, float2* __restrict__ spec,
                                           unsigned char* smem, const unsigned* list, long long (*s_part)[G],
                                           long long (&tm)[G], bool clear) {
-  using Cell = typename std::conditional<WIDE, unsigned long long, int>::type;
+  using Cell = UnitCell<N, G, CT, WIDE>;
   using U = Unit<N, G, CT, WIDE>;
-  constexpr int R = MAS, UX = U::UX, UY = U::UY, PAIRS = U::PAIRS, NT = U::NT, NSB = U::NSB;
+  constexpr int UY = U::UY, PAIRS = U::PAIRS, NT = U::NT, NSB = U::NSB;
   constexpr int P = N / 2 + 8, NX = G == 2 ? N : N / 2;
   constexpr int SBY = U::SBY;                                  // scale blocks along y
   Cell* acc = reinterpret_cast<Cell*>(smem);                   // [2 PAIRS][N] fixed-point cells
@@ -164,69 +234,17 @@ __device__ __forceinline__ void tile_unit(const DepGeom& g, const ColEntries& te
     for (int k = tid; k < (int)(U::CELLS * sizeof(Cell) / 16); k += NT) a4[k] = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
   }
+  // the entries whose places are kept, then the others (a loop that asks for each entry which it is: 512^3
+  // deposit/z 750 -> 740 us)
 #pragma unroll 1
-  for (int q = 0; q < 2; ++q) {
-  const unsigned en = q ? te.n[1] : te.n[0];
-  for (unsigned i = tid; i < en; i += NT) {
-    const float4 e = q ? te.extra[i] : __ldg(te.entries + (i < U::LIST ? list[i] : column_index(te, i)));
-#pragma unroll
-    for (int grid = 0; grid < G; ++grid) {
-      Axis<R> ax, ay, az;
-      make_axis<MAS, 0, N>(g, e.x, grid, ax);
-      make_axis<MAS, 0, N>(g, e.y, grid, ay);
-      make_axis<MAS, 0, N>(g, e.z, grid, az);
-      int lx[R], ly[R], zz[R];
-      local_nodes<R>(ax, N, x0, UX, lx);
-      local_nodes<R>(ay, N, y0, UY, ly);
-      // z weight times the particle weight at each block's scale (exact: powers of two)
-      float wz[NSB][R];
-#pragma unroll
-      for (int r = 0; r < R; ++r) zz[r] = wrapn(az.first + r, N);
-#pragma unroll
-      for (int b = 0; b < NSB; ++b) {
-        const float wsc = __fmul_rn(e.w, up[b]);
-#pragma unroll
-        for (int r = 0; r < R; ++r) wz[b][r] = __fmul_rn(az.w[r], wsc);
-      }
-#pragma unroll
-      for (int rx = 0; rx < R; ++rx) {
-        if (lx[rx] < 0) continue;
-        // with one block row the block depends on x only: select the z weights once per x node
-        float wzx[R];
-        if constexpr (SBY == 1) {
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            float wzb[NSB];
-#pragma unroll
-            for (int k = 0; k < NSB; ++k) wzb[k] = wz[k][r];
-            wzx[r] = pick_block<NSB>(lx[rx] >> 2, wzb);
-          }
-        }
-#pragma unroll
-        for (int ry = 0; ry < R; ++ry) {
-          if (ly[ry] < 0) continue;
-          const float wxy = __fmul_rn(ax.w[rx], ay.w[ry]);
-          const int row = U::cell_row(lx[rx], ly[ry], grid);
-#pragma unroll
-          for (int rz = 0; rz < R; ++rz) {
-            float wzr;
-            if constexpr (SBY == 1) {
-              wzr = wzx[rz];
-            } else {
-              float wzb[NSB];
-#pragma unroll
-              for (int k = 0; k < NSB; ++k) wzb[k] = wz[k][rz];
-              wzr = pick_block<NSB>((lx[rx] >> 2) * SBY + (ly[ry] >> 2), wzb);
-            }
-            const int v = __float2int_rn(__fmul_rn(wxy, wzr));
-            if constexpr (WIDE) atomicAdd(&acc[row + zz[rz]], (unsigned long long)(long long)v);
-            else atomicAdd(&acc[row + zz[rz]], v);
-          }
-        }
-      }
-    }
+  for (unsigned q = 0; q < 2; ++q) {
+    const unsigned en = q ? te.n[0] : min(te.n[0], (unsigned)U::LIST);
+    for (unsigned i = q * U::LIST + tid; i < en; i += NT)
+      add_entry<N, MAS, G, CT, WIDE>(g, __ldg(te.entries + (q ? column_index(te, i) : list[i])), up, x0, y0, acc);
   }
-  }
+  if constexpr (SPILLED)
+    for_spilled<NT>(te.ctr->cat, te.n[1], [&](unsigned i) { return spilled_column(te, i); },
+                    [&](const float4& e) { add_entry<N, MAS, G, CT, WIDE>(g, e, up, x0, y0, acc); });
   __syncthreads();
 
   // z transform: a thread transforms columns 2cp and 2cp+1 (one scale block), the same column pair in
@@ -281,7 +299,7 @@ __device__ __forceinline__ void tile_unit(const DepGeom& g, const ColEntries& te
 }
 
 // Every unit of a tile; writes the tile's totals.  sh: the shifts of the tile's scale blocks.
-template <int N, int MAS, int G, class CT, bool WIDE>
+template <int N, int MAS, int G, class CT, bool WIDE, bool SPILLED>
 __device__ __forceinline__ void tile_units(const DepGeom& g, const ColEntries& te, int sg, const int (&sh)[CT::NSB],
                                            int x0, int y0, int kz_cols, const float2* __restrict__ tw,
                                            float2* __restrict__ spec, unsigned char* smem, const unsigned* list,
@@ -302,7 +320,7 @@ __device__ __forceinline__ void tile_units(const DepGeom& g, const ColEntries& t
       for (int b = 0; b < U::NSB; ++b) shu[b] = sh[b];
     }
     long long tm[G];
-    tile_unit<N, MAS, G, CT, WIDE>(g, te, sg, shu, x0 + ux, y0 + uy, kz_cols, tw, spec, smem, list,
+    tile_unit<N, MAS, G, CT, WIDE, SPILLED>(g, te, sg, shu, x0 + ux, y0 + uy, kz_cols, tw, spec, smem, list,
                                    s_part, tm, U::NU > 1 && u > 0);
     if (threadIdx.x == 0) {
 #pragma unroll
@@ -321,12 +339,61 @@ __device__ __forceinline__ void tile_units(const DepGeom& g, const ColEntries& t
 template <int N, int MAS, int G, class CT>
 __device__ __noinline__ void tile_units_wide(const DepGeom& g, ColEntries te, int sg, unsigned packed, int x0, int y0,
                                              int kz_cols, const float2* __restrict__ tw, float2* __restrict__ spec,
-                                             unsigned char* smem, const unsigned* list, long long (*s_part)[G],
-                                             long long* tile_mass) {
+                                             long long (*s_part)[G], long long* tile_mass) {
+  using U = Unit<N, G, CT, false>;
+  extern __shared__ __align__(16) int acc_smem[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(acc_smem);
+  const unsigned* list = reinterpret_cast<const unsigned*>(acc_smem + U::CELLS + CT::NSB * N);
   int sh[CT::NSB];
 #pragma unroll
   for (int b = 0; b < CT::NSB; ++b) sh[b] = (int)((packed >> (8 * b)) & 0xffu);
-  tile_units<N, MAS, G, CT, true>(g, te, sg, sh, x0, y0, kz_cols, tw, spec, smem, list, s_part, tile_mass);
+  tile_units<N, MAS, G, CT, true, true>(g, te, sg, sh, x0, y0, kz_cols, tw, spec, smem, list, s_part, tile_mass);
+}
+
+// Adds entry e to the per-block plane counts zc [NSB][N] of the tile at
+// (x0, y0).
+template <int N, int MAS, int G, class CT>
+__device__ __forceinline__ void count_planes(const DepGeom& g, const float4& e, int x0, int y0, int* zc) {
+  constexpr int R = MAS, W = R + G - 1;
+  // the union of the grids' nodes along each axis: first .. last (the second grid's first node
+  // is the first grid's or the next one), as the bucketing counts them.  Every entry of the
+  // bucket reaches the tile, so an axis with one block row needs no test
+  int first[3], last[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    if ((a == 0 && CT::SBX == 1) || (a == 1 && CT::SBY == 1)) {
+      first[a] = last[a] = 0;
+      continue;
+    }
+    Axis<R> a0;
+    make_axis<MAS, 0, N>(g, a == 0 ? e.x : (a == 1 ? e.y : e.z), 0, a0);
+    first[a] = a0.first;
+    last[a] = a0.first + R - 1;
+    if constexpr (G == 2) {
+      Axis<R> a1;
+      make_axis<MAS, 0, N>(g, a == 0 ? e.x : (a == 1 ? e.y : e.z), 1, a1);
+      last[a] = a1.first + R - 1;
+    }
+  }
+  // scale blocks reached along x and y
+  unsigned mx = CT::SBX == 1 ? 1u : 0u, my = CT::SBY == 1 ? 1u : 0u;
+#pragma unroll
+  for (int r = 0; r < W; ++r) {
+    if constexpr (CT::SBX > 1) {
+      const int cx = wrapn(first[0] + r, N) - x0;
+      if (first[0] + r <= last[0] && cx >= 0 && cx < CT::TX) mx |= 1u << (cx >> 2);
+    }
+    if constexpr (CT::SBY > 1) {
+      const int cy = wrapn(first[1] + r, N) - y0;
+      if (first[1] + r <= last[1] && cy >= 0 && cy < CT::TY) my |= 1u << (cy >> 2);
+    }
+  }
+#pragma unroll
+  for (int bx = 0; bx < CT::SBX; ++bx)
+#pragma unroll
+    for (int by = 0; by < CT::SBY; ++by)
+      if (((mx >> bx) & 1u) && ((my >> by) & 1u))
+        for (int zn = first[2]; zn <= last[2]; ++zn) atomicAdd(&zc[(bx * CT::SBY + by) * N + wrapn(zn, N)], 1);
 }
 
 // Per-block plane counts of a tile (zc [NSB][N], zeroed on entry) and the
@@ -334,79 +401,39 @@ __device__ __noinline__ void tile_units_wide(const DepGeom& g, ColEntries te, in
 // (then sh[] holds SH_MAX + 1 for those blocks).  An entry covers block b in
 // plane z when its nodes (any grid) reach b's 4 x-columns, its 4 y-columns
 // and z.
-template <int N, int MAS, int G, class CT>
+template <int N, int MAS, int G, class CT, bool SPILLED>
 __device__ __forceinline__ bool block_scales(const DepGeom& g, const ColEntries& te, int x0, int y0, int* zc,
                                              unsigned* list, int* s_max, int (&sh)[CT::NSB]) {
-  constexpr int R = MAS, NT = Unit<N, G, CT, false>::NT, NSB = CT::NSB, W = R + G - 1;
+  constexpr int NT = Unit<N, G, CT, false>::NT, NSB = CT::NSB;
   constexpr unsigned LIST = Unit<N, G, CT, false>::LIST;
   const int tid = threadIdx.x;
   // this pass is the tile's first touch of its bucket: a thread issues EB entry loads at once
   constexpr int EB = 4;
 #pragma unroll 1
-  for (int q = 0; q < 2; ++q) {
-  const unsigned en = q ? te.n[1] : te.n[0];
-  for (unsigned i0 = tid; i0 < en; i0 += EB * NT) {
-    float4 ev[EB];
+  for (unsigned q = 0; q < 2; ++q) {                   // the entries whose places are kept, then the others
+    const unsigned en = q ? te.n[0] : min(te.n[0], LIST);
+    for (unsigned i0 = q * LIST + tid; i0 < en; i0 += EB * NT) {
+      float4 ev[EB];
 #pragma unroll
-    for (int k = 0; k < EB; ++k) {
-      const unsigned i = i0 + k * NT;
-      ev[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (i < en) {
-        if (q) {
-          ev[k] = te.extra[i];
-        } else {
+      for (int k = 0; k < EB; ++k) {
+        const unsigned i = i0 + k * NT;
+        ev[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < en) {
           const unsigned at = column_index(te, i);
-          if (i < LIST) list[i] = at;                  // read by this thread only, in the deposit
+          if (q == 0) list[i] = at;                    // read by this thread only, in the deposit
           ev[k] = __ldg(te.entries + at);
         }
       }
-    }
 #pragma unroll
-    for (int k = 0; k < EB; ++k) {
-      if (i0 + k * NT >= en) break;
-      const float4 e = ev[k];
-      // the union of the grids' nodes along each axis: first .. last (the second grid's first node
-      // is the first grid's or the next one), as the bucketing counts them.  Every entry of the
-      // bucket reaches the tile, so an axis with one block row needs no test
-      int first[3], last[3];
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        if ((a == 0 && CT::SBX == 1) || (a == 1 && CT::SBY == 1)) {
-          first[a] = last[a] = 0;
-          continue;
-        }
-        Axis<R> a0;
-        make_axis<MAS, 0, N>(g, a == 0 ? e.x : (a == 1 ? e.y : e.z), 0, a0);
-        first[a] = a0.first;
-        last[a] = a0.first + R - 1;
-        if constexpr (G == 2) {
-          Axis<R> a1;
-          make_axis<MAS, 0, N>(g, a == 0 ? e.x : (a == 1 ? e.y : e.z), 1, a1);
-          last[a] = a1.first + R - 1;
-        }
+      for (int k = 0; k < EB; ++k) {
+        if (i0 + k * NT >= en) break;
+        count_planes<N, MAS, G, CT>(g, ev[k], x0, y0, zc);
       }
-      // scale blocks reached along x and y
-      unsigned mx = CT::SBX == 1 ? 1u : 0u, my = CT::SBY == 1 ? 1u : 0u;
-#pragma unroll
-      for (int r = 0; r < W; ++r) {
-        if constexpr (CT::SBX > 1) {
-          const int cx = wrapn(first[0] + r, N) - x0;
-          if (first[0] + r <= last[0] && cx >= 0 && cx < CT::TX) mx |= 1u << (cx >> 2);
-        }
-        if constexpr (CT::SBY > 1) {
-          const int cy = wrapn(first[1] + r, N) - y0;
-          if (first[1] + r <= last[1] && cy >= 0 && cy < CT::TY) my |= 1u << (cy >> 2);
-        }
-      }
-#pragma unroll
-      for (int bx = 0; bx < CT::SBX; ++bx)
-#pragma unroll
-        for (int by = 0; by < CT::SBY; ++by)
-          if (((mx >> bx) & 1u) && ((my >> by) & 1u))
-            for (int zn = first[2]; zn <= last[2]; ++zn) atomicAdd(&zc[(bx * CT::SBY + by) * N + wrapn(zn, N)], 1);
     }
   }
-  }
+  if constexpr (SPILLED)
+    for_spilled<NT>(te.ctr->cat, te.n[1], [&](unsigned i) { return spilled_column(te, i); },
+                    [&](const float4& e) { count_planes<N, MAS, G, CT>(g, e, x0, y0, zc); });
   __syncthreads();
   // a node weight of TSC (<= 0.75^3) or PCS (<= (2/3)^3) is below 1/2: one more bit
   constexpr int WBIT = (MAS == GBP_TSC || MAS == GBP_PCS) ? 1 : 0;
@@ -428,12 +455,12 @@ __device__ __forceinline__ bool block_scales(const DepGeom& g, const ColEntries&
   return heavy;
 }
 
-template <int N, int MAS, int G, class CT>
-__global__ void __launch_bounds__(Unit<N, G, CT, false>::NT, Unit<N, G, CT, false>::MINB)
-deposit_fftz_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ entries, const unsigned* __restrict__ counts,
-                    const __grid_constant__ Spill sp, DepCounters* ctr, int kz_cols,
-                    const float2* __restrict__ tw, float2* __restrict__ spec, long long* __restrict__ tile_mass) {
-  pdl_wait();
+// A tile's plane counts, scales and units; the cells and the plane counts are
+// zero on entry.
+template <int N, int MAS, int G, class CT, bool SPILLED>
+__device__ __forceinline__ void column_tile(const DepGeom& g, const ColEntries& te, int sg, int x0, int y0, int kz_cols,
+                                            const float2* __restrict__ tw, float2* __restrict__ spec,
+                                            long long* __restrict__ tile_mass) {
   using U = Unit<N, G, CT, false>;
   constexpr int NT = U::NT, NSB = CT::NSB;
   extern __shared__ __align__(16) int acc_smem[];
@@ -441,9 +468,38 @@ deposit_fftz_kernel(const __grid_constant__ DepGeom g, const float4* __restrict_
   unsigned* list = reinterpret_cast<unsigned*>(zc + NSB * N);
   __shared__ long long s_part[NT / 32][G];
   __shared__ int s_max[NT / 32];
+  int sh[NSB];
+  const bool heavy = block_scales<N, MAS, G, CT, SPILLED>(g, te, x0, y0, zc, list, s_max, sh);
+  if (heavy) {                                         // uniform over the CTA
+    unsigned packed = 0;
+#pragma unroll
+    for (int b = 0; b < NSB; ++b) packed |= (unsigned)(sh[b] > SH_MAX ? 0 : sh[b]) << (8 * b);
+    tile_units_wide<N, MAS, G, CT>(g, te, sg, packed, x0, y0, kz_cols, tw, spec, s_part, tile_mass);
+  } else {
+    tile_units<N, MAS, G, CT, false, SPILLED>(g, te, sg, sh, x0, y0, kz_cols, tw, spec,
+                                              reinterpret_cast<unsigned char*>(acc_smem), list, s_part, tile_mass);
+  }
+}
+
+// A tile with spilled entries.
+template <int N, int MAS, int G, class CT>
+__device__ __noinline__ void column_spilled_tile(const DepGeom& g, ColEntries te, int sg, int x0, int y0, int kz_cols,
+                                                 const float2* __restrict__ tw, float2* __restrict__ spec,
+                                                 long long* __restrict__ tile_mass) {
+  column_tile<N, MAS, G, CT, true>(g, te, sg, x0, y0, kz_cols, tw, spec, tile_mass);
+}
+
+template <int N, int MAS, int G, class CT>
+__global__ void __launch_bounds__(Unit<N, G, CT, false>::NT, Unit<N, G, CT, false>::MINB)
+deposit_fftz_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ entries, const unsigned* __restrict__ counts,
+                    const __grid_constant__ Spill sp, DepCounters* ctr, int kz_cols,
+                    const float2* __restrict__ tw, float2* __restrict__ spec, long long* __restrict__ tile_mass) {
+  pdl_wait();
+  using U = Unit<N, G, CT, false>;
+  constexpr int NT = U::NT;
+  extern __shared__ __align__(16) int acc_smem[];
   __shared__ ColRuns s_runs;
-  const int tid = threadIdx.x;
-  const int t = blockIdx.x;
+  const int tid = threadIdx.x, t = blockIdx.x;
   const int ty = t % g.nt[1], tx = t / g.nt[1];
   const int x0 = tx * CT::TX, y0 = ty * CT::TY;
   static_assert(U::CELLS * sizeof(int) >= Unit<N, G, CT, true>::CELLS * 8, "the 64-bit cells lie in what is cleared");
@@ -451,19 +507,10 @@ deposit_fftz_kernel(const __grid_constant__ DepGeom g, const float4* __restrict_
   const ColEntries te = column_entries(g, tx, ty, entries, counts, sp, ctr, s_runs);
   if (tid == 0 && te.n[0] + te.n[1] > g.flag_cap) atomicOr(&ctr->outgrown, 1u);
   const int sg = fixed_scale_exp(ctr->maxw_bits, 0);
-  for (int k = tid; k < NSB * N; k += NT) zc[k] = 0;
+  for (int k = tid; k < CT::NSB * N; k += NT) acc_smem[U::CELLS + k] = 0;
   __syncthreads();
-  int sh[NSB];
-  const bool heavy = block_scales<N, MAS, G, CT>(g, te, x0, y0, zc, list, s_max, sh);
-  unsigned char* cells = reinterpret_cast<unsigned char*>(acc_smem);
-  if (heavy) {                                         // uniform over the CTA
-    unsigned packed = 0;
-#pragma unroll
-    for (int b = 0; b < NSB; ++b) packed |= (unsigned)(sh[b] > SH_MAX ? 0 : sh[b]) << (8 * b);
-    tile_units_wide<N, MAS, G, CT>(g, te, sg, packed, x0, y0, kz_cols, tw, spec, cells, list, s_part, tile_mass);
-  } else {
-    tile_units<N, MAS, G, CT, false>(g, te, sg, sh, x0, y0, kz_cols, tw, spec, cells, list, s_part, tile_mass);
-  }
+  if (te.n[1]) column_spilled_tile<N, MAS, G, CT>(g, te, sg, x0, y0, kz_cols, tw, spec, tile_mass);
+  else column_tile<N, MAS, G, CT, false>(g, te, sg, x0, y0, kz_cols, tw, spec, tile_mass);
 }
 
 struct PartLayout {

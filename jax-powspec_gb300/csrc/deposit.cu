@@ -21,8 +21,8 @@
 //
 // Passes 1-3 are one unless a large mesh holds few particles: fill_kernel
 // gives each tile a bucket of fixed capacity and writes every entry at the
-// slot its count atomic returns, or on the tile's spill lists when the bucket
-// is full (deposit_core.cuh, deposit_layout).
+// slot its count atomic returns, or in the spill table when the bucket is
+// full (deposit_core.cuh, deposit_layout).
 //
 // Integer accumulation makes each cell's sum independent of particle order
 // and scheduling, so the mesh is bitwise reproducible; no float atomics are
@@ -34,6 +34,52 @@
 namespace gbp {
 namespace {
 
+// Adds entry e to the cells of the tile at (x0, y0, z0), ex x ey x ez of them.
+template <int MAS, int CM>
+__device__ __forceinline__ void add_entry(const DepGeom& g, const float4& e, int grid, float sc, int x0, int y0, int z0,
+                                          int ex, int ey, int ez, unsigned* lo, unsigned* hi) {
+  constexpr int R = Scheme<MAS, CM>::R;
+  Axis<R> ax, ay, az;
+  make_axis<MAS, CM>(g, e.x, grid, ax);
+  make_axis<MAS, CM>(g, e.y, grid, ay);
+  make_axis<MAS, CM>(g, e.z, grid, az);
+  int lx[R], ly[R], lz[R];
+  local_nodes<R>(ax, g.N, x0, ex, lx);
+  local_nodes<R>(ay, g.N, y0, ey, ly);
+  local_nodes<R>(az, g.N, z0, ez, lz);
+#pragma unroll
+  for (int rx = 0; rx < R; ++rx) {
+    if (lx[rx] < 0) continue;
+#pragma unroll
+    for (int ry = 0; ry < R; ++ry) {
+      if (ly[ry] < 0) continue;
+      // src/mas.py:149 (and :76) weights corner (ix, iyp, izp) with
+      // mdx*mdy*ddz; the compat variants keep that (wxy_bug).  The
+      // product order ((wx*wy)*wz)*w is the reference's.
+      const float wxy = __fmul_rn(ax.w[rx], ay.w[ry]);
+      const float wxy_bug = __fmul_rn(ax.w[rx], ay.w[0]);
+      const int row = (lx[rx] * TILE + ly[ry]) * TILE;
+      int q[R];
+      unsigned old[R];
+#pragma unroll
+      for (int rz = 0; rz < R; ++rz) {         // issue the row's low-word adds together
+        if (lz[rz] < 0) continue;
+        const bool bug = CM != 0 && rx == 0 && ry == 1 && rz == 1;
+        const float c = __fmul_rn(__fmul_rn(bug ? wxy_bug : wxy, az.w[rz]), e.w);
+        q[rz] = __float2int_rn(__fmul_rn(c, sc));
+        old[rz] = atomicAdd(&lo[row + lz[rz]], static_cast<unsigned>(q[rz]));
+      }
+#pragma unroll
+      for (int rz = 0; rz < R; ++rz) {         // then the carries into the high words
+        if (lz[rz] < 0) continue;
+        const unsigned add = static_cast<unsigned>(q[rz]);
+        const int dh = (q[rz] < 0 ? -1 : 0) + (old[rz] + add < old[rz] ? 1 : 0);
+        if (dh) atomicAdd(&hi[row + lz[rz]], static_cast<unsigned>(dh));
+      }
+    }
+  }
+}
+
 // Pass 4: one CTA per tile; the grids go one after the other through the
 // same shared memory (more CTAs per SM), re-reading the bucket from L2.
 //
@@ -42,53 +88,66 @@ namespace {
 // 32-bit atomic on the low word, whose return value tells whether it carried
 // into the high word, which then gets the (rare) second atomic.  The integer
 // sums are exact whatever the order of the adds.
-template <int MAS, int G, int CM>
-__global__ void __launch_bounds__(DEP_THREADS)
-deposit_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ entries, const unsigned* __restrict__ counts,
-               const unsigned* __restrict__ offsets, const __grid_constant__ Spill sp, DepCounters* ctr,
-               const float* __restrict__ mesh_in,
-               float* __restrict__ mesh_out, long long* __restrict__ tile_mass) {
-  pdl_wait();
-  constexpr int R = Scheme<MAS, CM>::R;
-  extern __shared__ __align__(16) unsigned acc32[];
-  __shared__ long long s_part[DEP_THREADS / 32];
-  unsigned* lo = acc32;
-  unsigned* hi = acc32 + TILE3;
-  const int t = blockIdx.x;
-  const int tz = t % g.nt[2], ty = (t / g.nt[2]) % g.nt[1], tx = t / (g.nt[2] * g.nt[1]);
-  const int x0 = tx * g.td[0], y0 = ty * g.td[1], z0 = tz * g.td[2];
-  const int ex = min(g.td[0], g.N - x0), ey = min(g.td[1], g.N - y0), ez = min(g.td[2], g.N - z0);
+template <int CM>
+struct Early {
+  static constexpr bool ON = CM != 0;
+  static constexpr int CELLS4 = TILE3 / 4 / DEP_THREADS;      // float4s of the tile per thread
+  float4 v[ON ? CELLS4 : 1];
+};
 
-  // The drop-ins add to a mesh, one grid: its cells are read, and the accumulators cleared, ahead of the
-  // chain count -> bucket entries, which they do not depend on (512^3, 4 Mi particles: 0.335 -> 0.282 ms,
-  // 1.07 GB, 3.8 TB/s).  With two grids the registers cost more than the latency (0.137 -> 0.157 at 360^3).
-  constexpr bool EARLY = CM != 0;
-  constexpr int CELLS4 = TILE3 / 4 / DEP_THREADS;      // float4s of the tile per thread
-  float4 base[EARLY ? CELLS4 : 1];
-  if (EARLY) {
+// A tile's first cell and extent.
+struct TileBox {
+  int x0, y0, z0, ex, ey, ez;
+};
+
+__device__ __forceinline__ TileBox tile_box(const DepGeom& g, int t) {
+  const int tz = t % g.nt[2], ty = (t / g.nt[2]) % g.nt[1], tx = t / (g.nt[2] * g.nt[1]);
+  TileBox b;
+  b.x0 = tx * g.td[0]; b.y0 = ty * g.td[1]; b.z0 = tz * g.td[2];
+  b.ex = min(g.td[0], g.N - b.x0); b.ey = min(g.td[1], g.N - b.y0); b.ez = min(g.td[2], g.N - b.z0);
+  return b;
+}
+
+// The drop-ins add to a mesh, one grid: its cells are read, and the accumulators cleared, ahead of the
+// chain count -> bucket entries, which they do not depend on (512^3, 4 Mi particles: 0.335 -> 0.282 ms,
+// 1.07 GB, 3.8 TB/s).  With two grids the registers cost more than the latency (0.137 -> 0.157 at 360^3).
+template <int CM>
+__device__ __forceinline__ void read_early(const DepGeom& g, const TileBox& b, const float* __restrict__ mesh_in,
+                                           Early<CM>& base) {
+  if constexpr (Early<CM>::ON) {
     const long long n = g.N;
-    if (g.vec_ok && ez == TILE && (g.N & 3) == 0 && mesh_in) {
+    if (g.vec_ok && b.ez == TILE && (g.N & 3) == 0 && mesh_in) {
 #pragma unroll
-      for (int q = 0; q < CELLS4; ++q) {
+      for (int q = 0; q < Early<CM>::CELLS4; ++q) {
         const int k = threadIdx.x + q * DEP_THREADS;
         const int lz = (k % (TILE / 4)) * 4, ly = (k / (TILE / 4)) % TILE, lx = k / (TILE * TILE / 4);
-        if (lx < ex && ly < ey)
-          base[EARLY ? q : 0] =
-              __ldcs(reinterpret_cast<const float4*>(mesh_in + ((x0 + lx) * n + (y0 + ly)) * n + (z0 + lz)));
+        if (lx < b.ex && ly < b.ey)
+          base.v[q] =
+              __ldcs(reinterpret_cast<const float4*>(mesh_in + ((b.x0 + lx) * n + (b.y0 + ly)) * n + (b.z0 + lz)));
       }
     }
-    uint4* a4 = reinterpret_cast<uint4*>(acc32);
-    for (int k = threadIdx.x; k < 2 * TILE3 / 4; k += DEP_THREADS) a4[k] = make_uint4(0u, 0u, 0u, 0u);
   }
-  const TileEntries te = tile_entries(g, t, entries, counts, offsets, sp, ctr);
-  if (threadIdx.x == 0 && te.n[0] + te.n[1] > g.flag_cap) atomicOr(&ctr->outgrown, 1u);
-  const int s = fixed_scale_exp(ctr->maxw_bits, CM);
+}
+
+template <int MAS, int G, int CM, bool SPILLED>
+__device__ __forceinline__ void deposit_tile(const DepGeom& g, const TileEntries& te, int s, const TileBox& box,
+                                             const Early<CM>& base, const float* __restrict__ mesh_in,
+                                             float* __restrict__ mesh_out, long long* __restrict__ tile_mass) {
+  extern __shared__ __align__(16) unsigned acc32[];
+  __shared__ long long s_part[DEP_THREADS / 32];
+  unsigned *lo = acc32, *hi = acc32 + TILE3;
+  constexpr bool EARLY = Early<CM>::ON;
+  const int t = blockIdx.x;
+  const int x0 = box.x0, y0 = box.y0, z0 = box.z0, ex = box.ex, ey = box.ey, ez = box.ez;
   const float sc = ldexpf(1.0f, s);
   const float inv_sc = ldexpf(1.0f, -s);
   const long long N = g.N;
   const long long M = N * N * N;
   const bool vec4 = g.vec_ok && (ez == TILE) && ((g.N & 3) == 0);
 
+  // both grids' code in line but for PCS, which is long (360^3, 1.5 M: CIC 147 -> 135 us; PCS 483 -> 523)
+  constexpr int GRIDS_INLINE = MAS == GBP_PCS ? 1 : G;
+#pragma unroll GRIDS_INLINE
   for (int grid = 0; grid < G; ++grid) {
     if (!EARLY) {
       uint4* a4 = reinterpret_cast<uint4*>(acc32);
@@ -96,52 +155,12 @@ deposit_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ ent
     }
     __syncthreads();
 #pragma unroll 1
-    for (int q = 0; q < 2; ++q) {
-    const float4* ep = q ? te.p[1] : te.p[0];
-    const unsigned en = q ? te.n[1] : te.n[0];
-    for (unsigned i = threadIdx.x; i < en; i += DEP_THREADS) {
-      const float4 e = ep[i];
-      Axis<R> ax, ay, az;
-      make_axis<MAS, CM>(g, e.x, grid, ax);
-      make_axis<MAS, CM>(g, e.y, grid, ay);
-      make_axis<MAS, CM>(g, e.z, grid, az);
-      int lx[R], ly[R], lz[R];
-      local_nodes<R>(ax, g.N, x0, ex, lx);
-      local_nodes<R>(ay, g.N, y0, ey, ly);
-      local_nodes<R>(az, g.N, z0, ez, lz);
-#pragma unroll
-      for (int rx = 0; rx < R; ++rx) {
-        if (lx[rx] < 0) continue;
-#pragma unroll
-        for (int ry = 0; ry < R; ++ry) {
-          if (ly[ry] < 0) continue;
-          // src/mas.py:149 (and :76) weights corner (ix, iyp, izp) with
-          // mdx*mdy*ddz; the compat variants keep that (wxy_bug).  The
-          // product order ((wx*wy)*wz)*w is the reference's.
-          const float wxy = __fmul_rn(ax.w[rx], ay.w[ry]);
-          const float wxy_bug = __fmul_rn(ax.w[rx], ay.w[0]);
-          const int row = (lx[rx] * TILE + ly[ry]) * TILE;
-          int q[R];
-          unsigned old[R];
-#pragma unroll
-          for (int rz = 0; rz < R; ++rz) {         // issue the row's low-word adds together
-            if (lz[rz] < 0) continue;
-            const bool bug = CM != 0 && rx == 0 && ry == 1 && rz == 1;
-            const float c = __fmul_rn(__fmul_rn(bug ? wxy_bug : wxy, az.w[rz]), e.w);
-            q[rz] = __float2int_rn(__fmul_rn(c, sc));
-            old[rz] = atomicAdd(&lo[row + lz[rz]], static_cast<unsigned>(q[rz]));
-          }
-#pragma unroll
-          for (int rz = 0; rz < R; ++rz) {         // then the carries into the high words
-            if (lz[rz] < 0) continue;
-            const unsigned add = static_cast<unsigned>(q[rz]);
-            const int dh = (q[rz] < 0 ? -1 : 0) + (old[rz] + add < old[rz] ? 1 : 0);
-            if (dh) atomicAdd(&hi[row + lz[rz]], static_cast<unsigned>(dh));
-          }
-        }
-      }
-    }
-    }
+    for (unsigned i = threadIdx.x; i < te.n[0]; i += DEP_THREADS)
+      add_entry<MAS, CM>(g, __ldg(te.entries + i), grid, sc, x0, y0, z0, ex, ey, ez, lo, hi);
+    if constexpr (SPILLED)
+      for_spilled<DEP_THREADS>(
+          te.ctr->cat, te.n[1], [&](unsigned i) { return spilled_id(*te.sp, te.t, i); },
+          [&](const float4& e) { add_entry<MAS, CM>(g, e, grid, sc, x0, y0, z0, ex, ey, ez, lo, hi); });
     __syncthreads();
 
     // Write this grid's tile once; sum it exactly for the mean density.
@@ -169,9 +188,9 @@ deposit_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ ent
       };
       if constexpr (EARLY) {
 #pragma unroll
-        for (int q = 0; q < CELLS4; ++q) cell4(threadIdx.x + q * DEP_THREADS, base[q]);
+        for (int q = 0; q < Early<CM>::CELLS4; ++q) cell4(threadIdx.x + q * DEP_THREADS, base.v[q]);
       } else {
-        for (int k = threadIdx.x; k < TILE3 / 4; k += DEP_THREADS) cell4(k, base[0]);
+        for (int k = threadIdx.x; k < TILE3 / 4; k += DEP_THREADS) cell4(k, base.v[0]);
       }
     } else {
       for (int k = threadIdx.x; k < TILE3; k += DEP_THREADS) {
@@ -194,6 +213,38 @@ deposit_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ ent
       tile_mass[(long long)grid * gridDim.x + t] = tm;
     }
   }
+}
+
+// A tile with spilled entries.
+template <int MAS, int G, int CM>
+__device__ __noinline__ void deposit_spilled_tile(DepGeom g, TileEntries te, int s, Early<CM> base,
+                                                  const float* __restrict__ mesh_in, float* __restrict__ mesh_out,
+                                                  long long* __restrict__ tile_mass) {
+  deposit_tile<MAS, G, CM, true>(g, te, s, tile_box(g, blockIdx.x), base, mesh_in, mesh_out, tile_mass);
+}
+
+template <int MAS, int G, int CM>
+__global__ void __launch_bounds__(DEP_THREADS, MAS == GBP_PCS ? 4 : (MAS == GBP_TSC || CM ? 5 : 6))
+deposit_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ entries, const unsigned* __restrict__ counts,
+               const unsigned* __restrict__ offsets, const __grid_constant__ Spill sp, DepCounters* ctr,
+               const float* __restrict__ mesh_in, float* __restrict__ mesh_out, long long* __restrict__ tile_mass) {
+  pdl_wait();
+  extern __shared__ __align__(16) unsigned acc32[];
+  const int t = blockIdx.x;
+  const TileBox box = tile_box(g, t);
+  Early<CM> base;
+  read_early<CM>(g, box, mesh_in, base);
+  if constexpr (Early<CM>::ON) {
+    uint4* a4 = reinterpret_cast<uint4*>(acc32);
+    for (int k = threadIdx.x; k < 2 * TILE3 / 4; k += DEP_THREADS) a4[k] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  const unsigned maxw = ctr->maxw_bits;         // on its way beside the count
+  const TileEntries te = tile_entries(g, t, entries, counts, offsets, sp, ctr);
+  const int s = fixed_scale_exp(maxw, CM);
+  if (threadIdx.x == 0 && te.n[0] + te.n[1] > g.flag_cap) atomicOr(&ctr->outgrown, 1u);
+  // (base goes into both: loads that one of them does not need would be put behind the branch)
+  if (te.n[1]) deposit_spilled_tile<MAS, G, CM>(g, te, s, base, mesh_in, mesh_out, tile_mass);
+  else deposit_tile<MAS, G, CM, false>(g, te, s, box, base, mesh_in, mesh_out, tile_mass);
 }
 
 // Buckets of a fixed capacity filled in one pass, as on the fused path.

@@ -1,7 +1,9 @@
 // Deposit internals shared by the mesh deposit (deposit.cu) and the deposit
 // fused with the z pass of the FFT (depfft.cu): geometry, B-spline and
-// reference-compatible stencils, tile bucketing (count / scan / scatter),
-// int64 fixed-point helpers, statistics and workspace layout.
+// reference-compatible stencils, tile bucketing in one pass (buckets of a
+// fixed capacity and a table for their surplus; count, scan and scatter for a
+// large mesh with few particles), int64 fixed-point helpers, statistics and
+// workspace layout.
 #pragma once
 
 #include <algorithm>
@@ -254,24 +256,99 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-// Fill path: the entries beyond a bucket's capacity.  heads holds HEADS lists
-// per tile of them (node + 1, 0 ends a list), linked through next.
-constexpr unsigned HEADS = CSTRIDE;
+// Fill path: the entries beyond a bucket's capacity.  An entry's slot is its
+// rank among its bucket's attempts, so entry r of bucket b's surplus has a
+// place of its own, r mod 2^lg in the chunk of key (b, r >> lg): an open hash
+// table of chunks that hold particle numbers.  A tile finds any of its
+// surplus entries by one probe and reads the particle from the catalogue, so
+// a clump costs its own tile a few dependent loads per entry, whatever the
+// number of clumps (linked lists that a few threads walked took 13.9 ms where
+// this takes 4.3 for a 512^3 CIC deposit of 4 Mi particles, three quarters of
+// them in 8 clumps, 7.4 against 2.4 with 20), and the table is 6 bytes per
+// entry that can spill where lists and copies of the entries took 40.
 struct Spill {
-  unsigned* heads;      // [ntiles * HEADS], zeroed
-  unsigned* next;       // [nspill]
-  unsigned* tile;       // [nspill] (column tiles: 4 * tile + class)
-  float4* entry;        // [nspill] (u, w)
-  float4* extra;        // [nextra] copies gathered by the tiles, contiguous per tile
+  unsigned long long* keys;   // [chunks], zeroed; 0: free
+  unsigned* ids;              // [chunks << lg] particle numbers
+  unsigned chunks;
+  int lg;
 };
 
-// Puts an entry on list `head`; `lists` (a power of two) of them start at it.
-__device__ __forceinline__ void spill_entry(const Spill& sp, DepCounters* ctr, unsigned tile, size_t head,
-                                            unsigned lists, const float4& e) {
-  const unsigned s = atomicAdd(&ctr->n_spill, 1u);
-  sp.tile[s] = tile;
-  sp.entry[s] = e;
-  sp.next[s] = atomicExch(&sp.heads[head + (s & (lists - 1))], s + 1u);
+__device__ __forceinline__ unsigned long long spill_key(const Spill& sp, unsigned bucket, unsigned rank) {
+  return ((unsigned long long)(bucket + 1u) << 28) | (rank >> sp.lg);      // lg >= 4
+}
+
+__device__ __forceinline__ unsigned spill_home(const Spill& sp, unsigned long long key) {
+  return (unsigned)(((key * 0x9E3779B97F4A7C15ull >> 32) * sp.chunks) >> 32);
+}
+
+// Entry `rank` of bucket `bucket`'s surplus is particle `id`.  The table has
+// half as many chunks again as a catalogue can need, so a probe ends.
+__device__ __forceinline__ void spill_entry(const Spill& sp, unsigned bucket, unsigned rank, unsigned id) {
+  const unsigned long long key = spill_key(sp, bucket, rank);
+  unsigned c = spill_home(sp, key);
+  for (unsigned tries = 0; tries < sp.chunks; ++tries) {
+    unsigned long long k = *const_cast<volatile unsigned long long*>(sp.keys + c);
+    if (k == 0ull) {
+      k = atomicCAS(sp.keys + c, 0ull, key);
+      if (k == 0ull) k = key;
+    }
+    if (k == key) {
+      sp.ids[((size_t)c << sp.lg) + (rank & ((1u << sp.lg) - 1u))] = id;
+      return;
+    }
+    c = c + 1u == sp.chunks ? 0u : c + 1u;
+  }
+}
+
+// The particle of that entry (0xffffffff should it not be there).
+__device__ __forceinline__ unsigned spilled_id(const Spill& sp, unsigned bucket, unsigned rank) {
+  const unsigned long long key = spill_key(sp, bucket, rank);
+  unsigned c = spill_home(sp, key);
+  for (unsigned tries = 0; sp.keys[c] != key; c = c + 1u == sp.chunks ? 0u : c + 1u)
+    if (++tries > sp.chunks) return 0xffffffffu;
+  return sp.ids[((size_t)c << sp.lg) + (rank & ((1u << sp.lg) - 1u))];
+}
+
+// A particle's entry (u, w), as the fill computed it.
+__device__ __forceinline__ float4 particle_entry(const Catalogue& cat, unsigned i) {
+  if (i == 0xffffffffu) return make_float4(0.f, 0.f, 0.f, 0.f);
+  return make_float4(__fmul_rn(__fsub_rn(cat.x[i], cat.ox), cat.inv_cell),
+                     __fmul_rn(__fsub_rn(cat.y[i], cat.oy), cat.inv_cell),
+                     __fmul_rn(__fsub_rn(cat.z[i], cat.oz), cat.inv_cell), cat.w ? cat.w[i] : 1.0f);
+}
+
+// use(entry) of a tile's n spilled entries, thread by thread of NT.  A thread
+// looks up the numbers of four at once and loads the next one's particle
+// before it uses the last.
+template <int NT, class Id, class Use>
+__device__ __forceinline__ void for_spilled(const Catalogue& cat, unsigned n, Id id_of, Use use) {
+  for (unsigned i0 = threadIdx.x; i0 < n; i0 += 4 * NT) {
+    unsigned id[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) id[k] = i0 + k * NT < n ? id_of(i0 + k * NT) : 0xffffffffu;
+    float4 e = particle_entry(cat, id[0]);
+#pragma unroll 1
+    for (unsigned i = i0; i < n && i < i0 + 4 * NT; i += NT) {
+      const float4 next = particle_entry(cat, id[1]);
+      use(e);
+      e = next;
+      id[1] = id[2];
+      id[2] = id[3];
+      id[3] = 0xffffffffu;
+    }
+  }
+}
+
+// The fill kernels leave the catalogue they read (the parameters' or the
+// job's) beside the counters, for the tiles.
+__device__ __forceinline__ void keep_catalogue(const DepGeom& g, DepCounters* ctr) {
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    ctr->cat = Catalogue{g.x, g.y, g.z, g.w, g.ox, g.oy, g.oz, g.inv_cell};
+}
+
+// Number of particle k of a thread's batch (load_batch).
+__device__ __forceinline__ unsigned batch_id(int k) {
+  return (blockIdx.x * CNT_ITEMS + k) * CNT_THREADS + threadIdx.x;
 }
 
 // Block reductions of the weight statistics in a fixed order (deterministic
@@ -344,21 +421,21 @@ count_kernel(DepGeom gp, unsigned* __restrict__ counts, DepCounters* ctr, float4
 // Passes 1 and 3 at once (fill path: buckets of a fixed capacity g.tcap, tile
 // t's at entry t * tcap).  The count of tile t that a particle's atomic
 // returns is also its slot in t's bucket, so the entry is written right away;
-// a slot beyond the capacity puts the particle on one of the tile's spill
-// lists instead, which the tile's CTA collects (tile_entries), so a clump
-// costs its own tile and no second pass over the catalogue (a scan and a
-// scatter that rebuilt all buckets cost 0.15 of the 0.57 ms of a clustered
-// 4 Mi particle 512^3 CIC deposit, now 0.43, and two idle launches when
-// nothing overflowed).  The statistics are those of count_kernel, over the
+// a slot beyond the capacity goes to the spill table instead, where the
+// tile's CTA looks it up, so a clump costs its own tile and no second pass
+// over the catalogue (a scan and a scatter that rebuilt all buckets cost 0.15
+// of the 0.57 ms of a clustered 4 Mi particle 512^3 CIC deposit, and two idle
+// launches when nothing overflowed).  The statistics are those of count_kernel, over the
 // same particle blocks.
 // Registers for 5 CTAs per SM: its returning atomics want warps in flight
 // (0.151 -> 0.142 ms for 4 Mi particles at 512^3 against 4 CTAs per SM).
 template <int MAS, int G, int CM, bool JOB>
 __global__ void __launch_bounds__(CNT_THREADS, 5)
-fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entries, Spill sp, DepCounters* ctr,
-            float4* block_stats) {
+fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entries,
+            const __grid_constant__ Spill sp, DepCounters* ctr, float4* block_stats) {
   pdl_wait();
   const DepGeom g = catalogue_of<JOB>(gp);
+  keep_catalogue(g, ctr);
   const unsigned tcap = g.tcap;
   float maxw = 0.0f;
   ff sw{0.f, 0.f}, sw2{0.f, 0.f};
@@ -391,12 +468,27 @@ fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entr
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         if (tt[q] >= 0) slot[q] = atomicAdd(&counts[tt[q] * CSTRIDE], 1u);
+      bool over = false;
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         if (tt[q] >= 0) {
           if (slot[q] < tcap) entries[(unsigned)tt[q] * tcap + slot[q]] = e;
-          else spill_entry(sp, ctr, (unsigned)tt[q], (size_t)tt[q] * HEADS, HEADS, e);
+          else over = true;
         }
+      if (over) {
+#pragma unroll 1
+        for (int q = 0; q < 8; ++q) {
+          int t = -1;
+          unsigned s = 0;
+#pragma unroll
+          for (int r = 0; r < 8; ++r)
+            if (r == q) {
+              t = tt[r];
+              s = slot[r];
+            }
+          if (t >= 0 && s >= tcap) spill_entry(sp, (unsigned)t, s - tcap, batch_id(k));
+        }
+      }
     } else {
       for (int a = 0; a < nx; ++a)
         for (int b = 0; b < ny; ++b)
@@ -404,7 +496,7 @@ fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entr
             const int t = (pick3(a, x0, x1, x2) * g.nt[1] + pick3(b, y0, y1, y2)) * g.nt[2] + pick3(c, z0, z1, z2);
             const unsigned slot = atomicAdd(&counts[t * CSTRIDE], 1u);
             if (slot < tcap) entries[(unsigned)t * tcap + slot] = e;
-            else spill_entry(sp, ctr, (unsigned)t, (size_t)t * HEADS, HEADS, e);
+            else spill_entry(sp, (unsigned)t, slot - tcap, batch_id(k));
           }
     }
     maxw = fmaxf(maxw, fabsf(w));
@@ -426,7 +518,6 @@ fill_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entr
 // grids: 0.190 -> 0.063 ms; 256^3, 1 M: 0.047 -> 0.022; 1024^3, 16 Mi PCS:
 // 1.28 -> 0.32), for 2 % more in the kernel that finds the runs.
 constexpr int CLS = CSTRIDE / 4;              // words between a tile's four class counters (a sector each)
-constexpr int CLS_HEADS = HEADS / 4;          // spill lists per tile and class
 
 // v[c] by selects (no local memory).
 __device__ __forceinline__ unsigned pick4(unsigned c, const unsigned (&v)[4]) {
@@ -450,10 +541,11 @@ __device__ __forceinline__ int column_axis(const DepGeom& g, int ax, float u, in
 
 template <int MAS, int G, bool JOB>
 __global__ void __launch_bounds__(CNT_THREADS, 5)
-fill_columns_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entries, Spill sp,
-                    DepCounters* ctr, float4* block_stats) {
+fill_columns_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restrict__ entries,
+                    const __grid_constant__ Spill sp, DepCounters* ctr, float4* block_stats) {
   pdl_wait();
   const DepGeom g = catalogue_of<JOB>(gp);
+  keep_catalogue(g, ctr);
   float maxw = 0.0f;
   ff sw{0.f, 0.f}, sw2{0.f, 0.f};
   unsigned kept = 0, bad = 0;
@@ -480,14 +572,21 @@ fill_columns_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restric
     sw = ff_add_f(sw, w);
     sw2 = ff_add_f(sw2, __fmul_rn(w, w));
   }
+  bool over = false;
 #pragma unroll
   for (int k = 0; k < CNT_ITEMS; ++k) {
     if (tc[k] < 0) continue;
     const unsigned t = (unsigned)tc[k] >> 2, c = (unsigned)tc[k] & 3u;
-    if (slot[k] < pick4(c, g.ccap)) {
-      entries[(size_t)t * g.tcap + pick4(c, g.coff) + slot[k]] = e[k];
-    } else {
-      spill_entry(sp, ctr, (unsigned)tc[k], (size_t)t * HEADS + c * CLS_HEADS, CLS_HEADS, e[k]);
+    if (slot[k] < pick4(c, g.ccap)) entries[(size_t)t * g.tcap + pick4(c, g.coff) + slot[k]] = e[k];
+    else over = true;
+  }
+  if (over) {                                 // a loop: in line twice, it cost the others 2-4 % of the pass
+    static_assert(CNT_ITEMS == 2, "selects of two");
+#pragma unroll 1
+    for (int k = 0; k < CNT_ITEMS; ++k) {
+      const int b = k ? tc[1] : tc[0];
+      const unsigned s = k ? slot[1] : slot[0], cap = pick4((unsigned)b & 3u, g.ccap);
+      if (b >= 0 && s >= cap) spill_entry(sp, (unsigned)b, s - cap, batch_id(k));
     }
   }
   flush_block_stats(maxw, sw, sw2, kept, bad, ctr, block_stats);
@@ -498,13 +597,14 @@ fill_columns_kernel(DepGeom gp, unsigned* __restrict__ counts, float4* __restric
 struct ColRuns {
   unsigned pre[16], delta[16];
   unsigned spilled[9], code[9];               // entries beyond the bucket, 4 * tile + class
-  unsigned total, n_spilled, base, fill;
+  unsigned total, n_spilled;
 };
 
 struct ColEntries {
   const float4* entries;
   const ColRuns* runs;
-  const float4* extra;
+  const Spill* sp;
+  const DepCounters* ctr;
   unsigned n[2];                              // in buckets, spilled
 };
 
@@ -518,44 +618,18 @@ __device__ __forceinline__ unsigned column_index(const ColEntries& te, unsigned 
   return i + r.delta[q];
 }
 
-// Collects a column tile's spilled entries into a slice of sp.extra of its own
-// (every thread of the block calls): run by run, eight lanes walk the lists of
-// the run's class; a run that holds more than 64 entries per list and a
-// sixteenth of all spilled ones (a point mass) has the block look through
-// them all instead.
-__device__ __noinline__ const float4* gather_columns(const Spill& sp, DepCounters* ctr, ColRuns& r) {
-  if (threadIdx.x == 0) {
-    r.base = atomicAdd(&ctr->n_extra, r.n_spilled);
-    r.fill = 0;
-  }
-  __syncthreads();
-  float4* out = sp.extra + r.base;
-  auto put = [&](unsigned s) {
-    const unsigned q = atomicAdd(&r.fill, 1u);
-    if (q < r.n_spilled) out[q] = sp.entry[s];
-  };
-  const unsigned all = ctr->n_spill;
-  for (int k = 0; k < 9; ++k) {
-    const unsigned n = r.spilled[k], code = r.code[k];
-    if (n > 64 * CLS_HEADS && n > all / 16) {
-      for (unsigned j = threadIdx.x; j < all; j += blockDim.x)
-        if (sp.tile[j] == code) put(j);
-    } else if (n && threadIdx.x < CLS_HEADS) {
-      unsigned v = sp.heads[(size_t)(code >> 2) * HEADS + (code & 3u) * CLS_HEADS + threadIdx.x];
-      for (unsigned j = 0; v != 0u && j < n; ++j) {
-        put(v - 1u);
-        v = sp.next[v - 1u];
-      }
-    }
-  }
-  __syncthreads();
-  return out;
+// The particle of spilled entry i of a column tile.
+__device__ __forceinline__ unsigned spilled_column(const ColEntries& te, unsigned i) {
+  const ColRuns& r = *te.runs;
+  int q = 0;
+  while (q < 8 && i >= r.spilled[q]) i -= r.spilled[q++];
+  return spilled_id(*te.sp, r.code[q], i);
 }
 
 // Every thread of the block calls; ends with a barrier.
 __device__ __forceinline__ ColEntries column_entries(const DepGeom& g, int tx, int ty, const float4* entries,
-                                                     const unsigned* counts, const Spill& sp, DepCounters* ctr,
-                                                     ColRuns& r) {
+                                                     const unsigned* counts, const Spill& sp,
+                                                     const DepCounters* ctr, ColRuns& r) {
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     unsigned m = 0, code = 0, c = 0;
@@ -592,62 +666,36 @@ __device__ __forceinline__ ColEntries column_entries(const DepGeom& g, int tx, i
   ColEntries te;
   te.entries = entries;
   te.runs = &r;
+  te.sp = &sp;
+  te.ctr = ctr;
   te.n[0] = r.total;
   te.n[1] = r.n_spilled;
-  te.extra = nullptr;
-  if (te.n[1]) te.extra = gather_columns(sp, ctr, r);
   return te;
 }
 
 // The entries of one tile in two parts: n[0] in its bucket, n[1] beyond its
-// capacity (fill path).  Loops over a tile's entries take the parts in turn:
-// the rare second one costs the first nothing per entry.
+// capacity (fill path).  A tile that has any of the rare second part goes
+// through a copy of its code out of line: a call, or a second loop, in the
+// common one would cost it registers (512^3 CIC, 4 Mi particles: 279 -> 387 us
+// with the call in the middle).
 struct TileEntries {
-  const float4* p[2];
-  unsigned n[2];
+  const float4* entries;
+  const Spill* sp;
+  const DepCounters* ctr;
+  unsigned t, n[2];
 };
 
-// Collects a tile's n spilled entries into a slice of `extra` of its own
-// (every thread of the block calls).  One warp walks the tile's HEADS lists;
-// a tile that holds more than 64 entries per list and a sixteenth of all
-// spilled ones (a point mass) has the block look through them all instead.
-__device__ __noinline__ const float4* gather_spilled(const Spill& sp, DepCounters* ctr, int t, unsigned n) {
-  __shared__ unsigned s_base, s_n;
-  if (threadIdx.x == 0) {
-    s_base = atomicAdd(&ctr->n_extra, n);
-    s_n = 0;
-  }
-  __syncthreads();
-  float4* out = sp.extra + s_base;
-  auto put = [&](unsigned s) {
-    const unsigned q = atomicAdd(&s_n, 1u);
-    if (q < n) out[q] = sp.entry[s];
-  };
-  const unsigned all = ctr->n_spill;
-  if (n > 64 * HEADS && n > all / 16) {
-    for (unsigned k = threadIdx.x; k < all; k += blockDim.x)
-      if (sp.tile[k] == (unsigned)t) put(k);
-  } else if (threadIdx.x < HEADS) {
-    unsigned v = sp.heads[(size_t)t * HEADS + threadIdx.x];
-    for (unsigned k = 0; v != 0u && k < n; ++k) {
-      put(v - 1u);
-      v = sp.next[v - 1u];
-    }
-  }
-  __syncthreads();
-  return out;
-}
-
-// Every thread of the block calls; ends with the list complete.
 __device__ __forceinline__ TileEntries tile_entries(const DepGeom& g, int t, const float4* entries,
                                                     const unsigned* counts, const unsigned* offsets, const Spill& sp,
-                                                    DepCounters* ctr) {
+                                                    const DepCounters* ctr) {
   TileEntries te;
   const unsigned c = counts[(long long)t * CSTRIDE];
+  te.entries = entries + (g.tcap ? (size_t)t * g.tcap : (size_t)offsets[t]);
+  te.sp = &sp;
+  te.ctr = ctr;
+  te.t = (unsigned)t;
   te.n[0] = g.tcap ? min(c, g.tcap) : c;
   te.n[1] = c - te.n[0];
-  te.p[0] = entries + (g.tcap ? (size_t)t * g.tcap : (size_t)offsets[t]);
-  te.p[1] = te.n[1] ? gather_spilled(sp, ctr, t, te.n[1]) : te.p[0];
   return te;
 }
 
@@ -737,17 +785,18 @@ struct DepLayout {
   unsigned flag_cap;    // DepGeom::flag_cap
   unsigned ccap[4], coff[4];   // column tiles: each class's part of the bucket
   size_t nentries;      // entries the bucket buffer holds
-  size_t nspill;        // fill path: entries that may lie beyond their buckets
-  size_t nextra;        // and copies of them that the tiles may gather
+  size_t chunks;        // fill path: chunks of 2^lg entries of the spill table
+  int lg;
   size_t scan_bytes;
   size_t total;
 };
 
 // Bytes at the start of the workspace that one memset clears per call: the
-// counters, the tiles' entry counts and their fill counters or spill list
-// heads (adjacent).
+// counters, the tiles' entry counts and their fill counters or the spill
+// table's keys (adjacent).
 inline size_t zeroed_bytes(const DepLayout& L) {
-  return align256(sizeof(DepCounters)) + 2 * align256((size_t)L.ntiles * CSTRIDE * sizeof(unsigned));
+  const size_t counts = align256((size_t)L.ntiles * CSTRIDE * sizeof(unsigned));
+  return align256(sizeof(DepCounters)) + counts + (L.tcap ? align256(L.chunks * sizeof(unsigned long long)) : counts);
 }
 
 struct StrideLoad {
@@ -760,6 +809,16 @@ inline thrust::transform_iterator<StrideLoad, thrust::counting_iterator<int>> st
 }
 
 void finish_layout(DepLayout& L);
+
+// Spill table of `nlists` buckets whose surplus is at most `most` entries:
+// chunks of about a bucket's mean fill (16 to 128 entries, so that neither
+// part-filled chunks nor keys take much), half as many again as can be in use
+// (every full one, and a part-filled one per bucket).
+void size_spill(DepLayout& L, double most, double nlists) {
+  L.lg = 4;
+  while (L.lg < 7 && most / nlists > (double)(1 << L.lg)) ++L.lg;
+  L.chunks = (size_t)(1.5 * std::min(most, nlists + most / (double)(1 << L.lg))) + 16;
+}
 
 // Mean entries per tile of a uniform catalogue of n particles (a span of
 // `width` nodes reaches the next tile along an axis with probability
@@ -823,14 +882,15 @@ int deposit_layout(int64_t n, int N, int mas, int interlace, int compat, const i
   L.nblocks = (int)((n + (long long)CNT_THREADS * CNT_ITEMS - 1) / ((long long)CNT_THREADS * CNT_ITEMS));
   L.tcap = 0;
   L.nentries = (size_t)n * L.maxrep + 1;
-  L.nspill = L.nextra = 0;
+  L.chunks = 0;
+  L.lg = 4;
   L.flag_cap = 0xffffffffu;
   if (fill && n > 0) {
     const double mean = mean_fill(n, N, width, L), cap = bucket_capacity(mean);
     if (mean >= 32.0) L.flag_cap = (unsigned)std::min(cap, 4294967295.0);
     if ((mean >= 32.0 || cap * (double)L.ntiles <= 16777216.0) && cap * (double)L.ntiles < 4294967295.0) {
       L.tcap = (unsigned)cap;
-      L.nspill = L.nextra = L.nentries;
+      size_spill(L, (double)n * L.maxrep, L.ntiles);
       L.nentries = (size_t)L.tcap * (size_t)L.ntiles + 1;
     }
   }
@@ -840,7 +900,7 @@ int deposit_layout(int64_t n, int N, int mas, int interlace, int compat, const i
 
 // Column tiles of tx x ty pencils (both powers of two >= 4 that divide N/2),
 // always one pass: class c's part of a bucket holds twice its mean fill of a
-// uniform catalogue plus 48 (what overflows it costs a list;
+// uniform catalogue plus 48 (what overflows it goes to the spill table;
 // GBP_STATS_REFILLED is reported at the capacity a bucket of all the tile's
 // entries would have).  Nodes first .. last of all grids span MAS - 1 cells,
 // or half a cell more on average with two grids, so they reach the next tile
@@ -873,8 +933,7 @@ int column_layout(int64_t n, int N, int mas, int interlace, int tx, int ty, DepL
   if (off * (double)L.ntiles >= 4294967295.0) return GBP_ERR_UNSUPPORTED;
   L.tcap = (unsigned)off;
   L.nentries = (size_t)L.tcap * (size_t)L.ntiles + 1;
-  L.nspill = (size_t)n + 1;
-  L.nextra = (size_t)n * L.maxrep + 1;
+  size_spill(L, (double)n, 4.0 * L.ntiles);
   finish_layout(L);
   return GBP_OK;
 }
@@ -885,21 +944,21 @@ void finish_layout(DepLayout& L) {
   if (!L.tcap) cub::DeviceScan::ExclusiveSum(nullptr, L.scan_bytes, strided_counts(nullptr), (unsigned*)nullptr, L.ntiles);
   const size_t nbl = (size_t)(L.nblocks > 0 ? L.nblocks : 1);
   L.total = zeroed_bytes(L) + align256((size_t)L.ntiles * 2 * sizeof(long long)) + align256((size_t)L.ntiles * 4) + align256(nbl * sizeof(float4)) +
-            align256(L.nentries * sizeof(float4)) + align256(L.scan_bytes) + 2 * align256(L.nspill * sizeof(unsigned)) +
-            align256(L.nspill * sizeof(float4)) + align256(L.nextra * sizeof(float4));
+            align256(L.nentries * sizeof(float4)) + align256(L.scan_bytes) +
+            align256((L.chunks << L.lg) * sizeof(unsigned));
 }
 
 // Workspace slices shared by both deposit paths.
 struct DepBuffers {
   DepCounters* ctr;
   unsigned* counts;      // [ntiles * CSTRIDE] entries per tile (count pass)
-  unsigned* fills;       // [ntiles * CSTRIDE] entries written so far (count path's scatter)
+  unsigned* fills;       // [ntiles * CSTRIDE] entries written so far (count path's scatter; else nullptr)
   unsigned* offsets;     // [ntiles] first entry of each tile (exclusive scan of the counts)
   float4* block_stats;
   long long* tile_mass;  // [2][ntiles]
   float4* entries;
   void* scan_tmp;
-  Spill spill;           // fill path (its heads share the bytes of fills)
+  Spill spill;           // fill path
 };
 
 inline DepBuffers carve_deposit(void* workspace, const DepLayout& L) {
@@ -908,17 +967,16 @@ inline DepBuffers carve_deposit(void* workspace, const DepLayout& L) {
   const int nbl = L.nblocks > 0 ? L.nblocks : 1;
   b.ctr = cv.take<DepCounters>(1);
   b.counts = cv.take<unsigned>((size_t)L.ntiles * CSTRIDE);
-  b.fills = cv.take<unsigned>((size_t)L.ntiles * CSTRIDE);
+  b.fills = L.tcap ? nullptr : cv.take<unsigned>((size_t)L.ntiles * CSTRIDE);
+  b.spill.keys = L.tcap ? cv.take<unsigned long long>(L.chunks) : nullptr;
   b.offsets = cv.take<unsigned>(L.ntiles);
   b.block_stats = cv.take<float4>(nbl);
   b.tile_mass = cv.take<long long>((size_t)L.ntiles * 2);
   b.entries = cv.take<float4>(L.nentries);
   b.scan_tmp = cv.take<char>(L.scan_bytes);
-  b.spill.heads = b.fills;
-  b.spill.next = cv.take<unsigned>(L.nspill);
-  b.spill.tile = cv.take<unsigned>(L.nspill);
-  b.spill.entry = cv.take<float4>(L.nspill);
-  b.spill.extra = cv.take<float4>(L.nextra);
+  b.spill.ids = cv.take<unsigned>(L.chunks << L.lg);
+  b.spill.chunks = (unsigned)L.chunks;
+  b.spill.lg = L.lg;
   return b;
 }
 

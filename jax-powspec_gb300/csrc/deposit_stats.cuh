@@ -10,12 +10,16 @@
 
 namespace gbp {
 
+struct Catalogue {
+  const float *x, *y, *z, *w;
+  float ox, oy, oz, inv_cell;
+};
+
 struct DepCounters {           // zeroed by one memset per call; integers: any order gives the same totals
   unsigned int maxw_bits;
-  unsigned int n_spill;        // fill path: entries beyond their bucket's capacity
-  unsigned int n_extra;        // spilled entries gathered by their tiles so far
   unsigned int outgrown;       // some tile has more entries than DepGeom::flag_cap
   unsigned long long kept, bad;
+  Catalogue cat;               // what the fill kernel read
 };
 
 struct StatsFold {
