@@ -908,29 +908,33 @@ int deposit_layout(int64_t n, int N, int mas, int interlace, int compat, const i
 int column_layout(int64_t n, int N, int mas, int interlace, int tx, int ty, DepLayout& L) {
   if (n < 0) return GBP_ERR_INVALID;
   if (mas < GBP_NGP || mas > GBP_PCS) return GBP_ERR_INVALID;
-  const int td[3] = {tx, ty, N};
-  L.maxrep = 4;
+  const int td[3] = {tx, ty, N}, width = mas + (interlace ? 1 : 0);
+  L.maxrep = 1;
   for (int a = 0; a < 3; ++a) {
     L.td[a] = td[a];
     L.ts[a] = __builtin_ctz(td[a]);
     L.nt[a] = N / td[a];
+    if (a < 2) L.maxrep *= max_tiles_axis(N, td[a], width);
   }
   L.ntiles = L.nt[0] * L.nt[1];
   if ((double)n * L.maxrep >= 4294967295.0) return GBP_ERR_UNSUPPORTED;
   L.nblocks = (int)((n + (long long)CNT_THREADS * CNT_ITEMS - 1) / ((long long)CNT_THREADS * CNT_ITEMS));
-  const double all = mean_fill(n, N, mas + (interlace ? 1 : 0), L);
+  const double all = mean_fill(n, N, width, L);
   L.flag_cap = all >= 32.0 ? (unsigned)std::min(bucket_capacity(all), 4294967295.0) : 0xffffffffu;
   const double span = mas - 1 + (interlace ? 0.5 : 0.0), mean = (double)n / (double)L.ntiles;
+  // entries are numbered in 32 bits: less than twice the mean beyond 2.1e9 particles (NGP on one grid, whose
+  // particles touch one tile, takes up to 4.29e9), the surplus in the table
+  const double slack = 4.0 * 52.0 * (double)L.ntiles;
+  const double f = n > 0 ? std::min(2.0, (4294967295.0 - slack) / (double)n) : 2.0;
   double off = 0.0;
   for (int c = 0; c < 4; ++c) {
     const double px = span / tx, py = span / ty;
     const double m = mean * ((c & 2) ? px : 1.0 - px) * ((c & 1) ? py : 1.0 - py);
-    const double cap = 4.0 * std::ceil((2.0 * m + 48.0) / 4.0);
+    const double cap = 4.0 * std::ceil((f * m + 48.0) / 4.0);
     L.coff[c] = (unsigned)off;
     L.ccap[c] = (unsigned)cap;
     off += cap;
   }
-  if (off * (double)L.ntiles >= 4294967295.0) return GBP_ERR_UNSUPPORTED;
   L.tcap = (unsigned)off;
   L.nentries = (size_t)L.tcap * (size_t)L.ntiles + 1;
   size_spill(L, (double)n, 4.0 * L.ntiles);

@@ -95,3 +95,32 @@ def test_spilled_particles_change_no_bit(N, clumps, per, mas, interlace):
             assert list(q.deposit_stats()[0].mass) == list(read_stats(r.stats).mass), tiles
         small.close()
         big.close()
+
+
+def test_fused_workspace_and_limits():
+    """What the fused path takes: the buckets (twice the catalogue), a table for the surplus and little else, for
+    every tile shape; a catalogue is refused only when an entry per tile it can touch has no 32-bit number (one grid
+    of NGP touches one tile, other schemes four)."""
+    from gbpowspec import _lib, _native
+    dev = torch.device("cuda", 0)
+    lib = _lib.load()
+    size = C.c_size_t(0)
+
+    def need(N, n, mas, grids, tiles=None):
+        plan = _native.FFTPlan(N, grids, dev)
+        if tiles:
+            plan.set_tiles(*tiles)
+        bins = _native.bins_for(np.arange(1, N // 2).astype(np.float32), N, dev)
+        st = lib.gbp_particles_power_workspace_size(n, plan.handle, bins.handle, mas, 7, C.byref(size))
+        plan.close()
+        return st, size.value
+    for N, n, mas, grids in ((512, 4 << 20, 3, 2), (256, 1 << 20, 3, 2), (128, 1 << 20, 2, 2), (128, 1 << 20, 2, 1),
+                             (1024, 16 << 20, 4, 2)):
+        for tiles in _native.tile_variants(N):
+            st, b = need(N, n, mas, grids, tiles)
+            assert st == 0 and b <= 72 * n + 4096 * (N // 4) ** 2, (N, tiles, b / n)
+    assert need(512, 4_200_000_000, 1, 1)[0] == 0
+    assert need(512, 2_000_000_000, 1, 1)[0] == 0
+    assert need(512, 1_070_000_000, 2, 1)[0] == 0
+    for mas, grids, n in ((1, 1, 4_294_967_295), (1, 2, 1_080_000_000), (2, 1, 1_080_000_000)):
+        assert need(512, n, mas, grids)[0] == _lib.GBP_ERR_UNSUPPORTED
