@@ -66,8 +66,8 @@ struct ColTile {
 // packed complex columns: column q = (a, ly) with a = the pencil's x (two
 // grids) or x / 2 (one grid), a = q / UY, ly = q % UY.  Columns 2cp and
 // 2cp + 1 always lie in one scale block.  The unit is the tile where its
-// cells fit UNIT_BYTES, else 4x4 pencils of it; with 64-bit cells half of
-// that or less.  At 512^3 a unit of 64 KB (512 threads, 64-thread named
+// cells fit UNIT_BYTES, else 4x4 pencils of it; with 64-bit cells the same on
+// the smallest meshes, else half of that or less.  At 512^3 a unit of 64 KB (512 threads, 64-thread named
 // barriers, two CTAs per SM) beats one of 128 KB in a 1024-thread CTA (0.84
 // against 0.89 ms for 8x4 tiles of two grids, 4 Mi particles TSC); at 1024^3
 // 4x4 pencils in one CTA beat two visits of the bucket by 4x2 (7.7 against
@@ -80,21 +80,29 @@ struct Unit {
   static constexpr size_t PENCIL = (size_t)N * G * sizeof(int);          // bytes of a pencil's 32-bit cells
   static constexpr bool WHOLE = CT::TX * CT::TY * PENCIL <= UNIT_BYTES<N>;
   static constexpr int NARROW_X = WHOLE ? CT::TX : 4, NARROW_Y = WHOLE ? CT::TY : 4;
-  static constexpr int UX = WIDE ? 4 : NARROW_X;
-  static constexpr int UY = WIDE ? (NARROW_X * NARROW_Y == 16 ? 2 : 4) : NARROW_Y;
-  static constexpr int NUY = CT::TY / UY, NU = (CT::TX / UX) * NUY;      // units per tile
-  static constexpr int PAIRS = UX * UY * G / 2;
-  static constexpr int SBY = UY >= 4 ? UY / 4 : 1, NSB = UX / 4 * SBY;   // scale blocks it spans
   // threads of the CTA: a butterfly pair (two columns) of the 32-bit unit's radix-8 stages each
   static constexpr int NFFT = NARROW_X * NARROW_Y * G * N / 32;
   static constexpr int NT = NFFT < 256 ? 256 : NFFT;
   // 64 registers a thread for every size: the kernel waits at the barriers between its phases, and a fourth
   // block of 256 threads hides them (256^3 TSC weighted 253 -> 244 us a call, 24 mocks of 128^3 1543 -> 1446)
   static constexpr int MINB = NT >= 1024 ? 1 : (NT >= 512 ? 2 : 4);   // CTAs per SM the registers are sized for
-  static constexpr size_t CELLS = (size_t)2 * PAIRS * N;
   static constexpr int LIST = 4 * NT;              // entries whose places are kept between the two passes
-  static constexpr size_t SMEM = (CELLS + (size_t)CT::NSB * N + LIST) * sizeof(int);   // cells, plane counts, list
-  static_assert(UX * UY * (WIDE ? 2 : 1) <= NARROW_X * NARROW_Y && NT <= 1024, "64-bit cells fit the same bytes");
+  // ints beside the cells: plane counts, list
+  static constexpr size_t REST = (size_t)CT::NSB * N + LIST;
+  // 64-bit cells of the whole 32-bit unit where they take 16 KB, so that a dense clump's entries are visited once
+  // (64^3 TSC on one grid, 8 clumps of 9,000: 1.42 -> 1.24 ms; 128^3 CIC on one grid, 8 of 98,000: 10.1 -> 6.0);
+  // 32 KB would speed up clumps at 128^3 with two grids too (11.3 -> 8.2 ms) but cost ordinary mocks in lanes 2 %
+  static constexpr size_t NARROW_BYTES = NARROW_X * NARROW_Y * PENCIL;
+  static constexpr bool WIDE_WHOLE = 2 * NARROW_BYTES <= 16 * 1024;
+  static constexpr int UX = WIDE && !WIDE_WHOLE ? 4 : NARROW_X;
+  static constexpr int UY = WIDE && !WIDE_WHOLE ? (NARROW_X * NARROW_Y == 16 ? 2 : 4) : NARROW_Y;
+  static constexpr int NUY = CT::TY / UY, NU = (CT::TX / UX) * NUY;      // units per tile
+  static constexpr int PAIRS = UX * UY * G / 2;
+  static constexpr int SBY = UY >= 4 ? UY / 4 : 1, NSB = UX / 4 * SBY;   // scale blocks it spans
+  static constexpr size_t CELLS = (size_t)2 * PAIRS * N;
+  static constexpr size_t ROOM = NARROW_BYTES / sizeof(int) * (WIDE_WHOLE ? 2 : 1);     // ints the cells may take
+  static constexpr size_t SMEM = (ROOM + REST) * sizeof(int);
+  static_assert(CELLS * (WIDE ? 2 : 1) <= ROOM && NT <= 1024, "the unit's cells fit");
   // First cell of pencil (lx, ly) of a grid.
   __device__ static __forceinline__ int cell_row(int lx, int ly, int grid) {
     if constexpr (G == 2) return ((lx * UY + ly) * 2 + grid) * N;
@@ -321,7 +329,7 @@ __device__ __forceinline__ void tile_units(const DepGeom& g, const ColEntries& t
     }
     long long tm[G];
     tile_unit<N, MAS, G, CT, WIDE, SPILLED>(g, te, sg, shu, x0 + ux, y0 + uy, kz_cols, tw, spec, smem, list,
-                                   s_part, tm, U::NU > 1 && u > 0);
+                                   s_part, tm, (WIDE && U::WIDE_WHOLE) || u > 0);
     if (threadIdx.x == 0) {
 #pragma unroll
       for (int q = 0; q < G; ++q) total[q] += tm[q];
@@ -343,7 +351,7 @@ __device__ __noinline__ void tile_units_wide(const DepGeom& g, ColEntries te, in
   using U = Unit<N, G, CT, false>;
   extern __shared__ __align__(16) int acc_smem[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(acc_smem);
-  const unsigned* list = reinterpret_cast<const unsigned*>(acc_smem + U::CELLS + CT::NSB * N);
+  const unsigned* list = reinterpret_cast<const unsigned*>(acc_smem + U::ROOM + CT::NSB * N);
   int sh[CT::NSB];
 #pragma unroll
   for (int b = 0; b < CT::NSB; ++b) sh[b] = (int)((packed >> (8 * b)) & 0xffu);
@@ -464,7 +472,7 @@ __device__ __forceinline__ void column_tile(const DepGeom& g, const ColEntries& 
   using U = Unit<N, G, CT, false>;
   constexpr int NT = U::NT, NSB = CT::NSB;
   extern __shared__ __align__(16) int acc_smem[];
-  int* zc = acc_smem + U::CELLS;                       // [NSB][N] entries covering each block's planes
+  int* zc = acc_smem + U::ROOM;                       // [NSB][N] entries covering each block's planes
   unsigned* list = reinterpret_cast<unsigned*>(zc + NSB * N);
   __shared__ long long s_part[NT / 32][G];
   __shared__ int s_max[NT / 32];
@@ -502,12 +510,11 @@ deposit_fftz_kernel(const __grid_constant__ DepGeom g, const float4* __restrict_
   const int tid = threadIdx.x, t = blockIdx.x;
   const int ty = t % g.nt[1], tx = t / g.nt[1];
   const int x0 = tx * CT::TX, y0 = ty * CT::TY;
-  static_assert(U::CELLS * sizeof(int) >= Unit<N, G, CT, true>::CELLS * 8, "the 64-bit cells lie in what is cleared");
   for (int k = tid; k < (int)(U::CELLS / 4); k += NT) reinterpret_cast<uint4*>(acc_smem)[k] = make_uint4(0u, 0u, 0u, 0u);
   const ColEntries te = column_entries(g, tx, ty, entries, counts, sp, ctr, s_runs);
   if (tid == 0 && te.n[0] + te.n[1] > g.flag_cap) atomicOr(&ctr->outgrown, 1u);
   const int sg = fixed_scale_exp(ctr->maxw_bits, 0);
-  for (int k = tid; k < CT::NSB * N; k += NT) acc_smem[U::CELLS + k] = 0;
+  for (int k = tid; k < CT::NSB * N; k += NT) acc_smem[U::ROOM + k] = 0;
   __syncthreads();
   if (te.n[1]) column_spilled_tile<N, MAS, G, CT>(g, te, sg, x0, y0, kz_cols, tw, spec, tile_mass);
   else column_tile<N, MAS, G, CT, false>(g, te, sg, x0, y0, kz_cols, tw, spec, tile_mass);

@@ -51,6 +51,16 @@ def test_surplus_is_collected_in_parallel():
     assert many < 2.0 * one + 0.2, (one, many)
 
 
+def test_dense_tiles_of_small_meshes_are_visited_once():
+    """Eight clumps of 98,304 particles at 128^3, one grid: two visits of each dense tile's entries took 10.1 ms,
+    one takes 6.0."""
+    from gbpowspec import PkConfig, PowerSpectrum
+    N, n = 128, 98_304
+    x, y, z = _clumps(N, 262_144, 8, n, 7, float(N))
+    ps = PowerSpectrum(PkConfig(n_mesh=N, box_size=float(N), mas="cic", interlace=False))
+    assert _ms(lambda: ps.run(x, y, z)) < 8.0
+
+
 @pytest.mark.parametrize("mas,interlace", [("ngp", False), ("cic", True), ("tsc", False), ("pcs", False),
                                            ("pcs", True)])
 @pytest.mark.parametrize("N,clumps,per", [(48, 5, 6000), (64, 1, 30_000), (64, 30, 900), (128, 40, 3000)])
