@@ -3,19 +3,21 @@
 The deposit fused with the z pass buckets particles by column tile (tx x ty
 pencils over all of z) and deposits one tile per CTA; the tile is also the
 bucket of the particle sort.  Its best shape depends on the device, the
-mesh, the scheme, interlacing and the particle count: small tiles replicate
-more particles across tile faces (more bucket entries, more sort traffic),
-large ones hold more shared memory per CTA (fewer CTAs per SM).  Every
-shape gives the same P_l bit for bit (fixed-point scales per 4x4 block), so
-the choice is pure speed.
+mesh, the scheme, interlacing and the particle count: small tiles read more
+of their neighbours' entries (those whose stencils cross a face), large ones
+hold more shared memory per CTA (fewer CTAs per SM).  Every shape gives the
+same P_l bit for bit (fixed-point scales per 4x4 block), so the choice is
+pure speed.
 
 ``Tuner.best(N, mas, interlace, n)`` returns the shape to use.  The first
-call for a (device, N, MAS, grids, n-bucket) key times every shape the
+call for a (device, N, MAS, grids, n-bucket, KERNELS) key times every shape the
 library offers (gbp_column_tile_variants) on a seeded lognormal catalogue
 of n particles (CUDA events, median of a few runs after a warm-up), keeps
 the fastest and writes it to a JSON cache (GBP_TUNE_CACHE, default
 ~/.cache/gbpowspec/tiles.json); later calls, in this process or another,
-read it.  n-buckets are powers of two (round(log2 n)).  PowerSpectrum,
+read it.  n-buckets are powers of two (round(log2 n)); KERNELS numbers the
+kernels the timings were made with, so what an older build wrote is measured
+again.  PowerSpectrum,
 BatchRunner and the Server take ``tiles="auto"`` to use it.
 """
 from __future__ import annotations
@@ -26,6 +28,10 @@ import os
 import threading
 
 __all__ = ["Tuner", "default_tuner"]
+
+# Raised when a change of the bucketing, deposit/z or lane code can change which tile is fastest (1: entries
+# replicated per tile; 2: every particle written once, where 512^3 with two grids went from 8x4 to 4x4).
+KERNELS = 2
 
 
 def _default_path() -> str:
@@ -56,7 +62,7 @@ class Tuner:
     @staticmethod
     def key(device: str, N: int, mas: str, interlace: bool, n: int) -> str:
         bucket = int(round(math.log2(max(int(n), 1))))
-        return f"{device}|N{int(N)}|{mas.lower()}|G{2 if interlace else 1}|n2^{bucket}"
+        return f"{device}|N{int(N)}|{mas.lower()}|G{2 if interlace else 1}|n2^{bucket}|k{KERNELS}"
 
     def _load(self) -> dict:
         if self._cache is None:
