@@ -914,7 +914,8 @@ int column_layout(int64_t n, int N, int mas, int interlace, int tx, int ty, DepL
     L.td[a] = td[a];
     L.ts[a] = __builtin_ctz(td[a]);
     L.nt[a] = N / td[a];
-    if (a < 2) L.maxrep *= max_tiles_axis(N, td[a], width);
+    // tiles that `width` consecutive nodes can touch (td divides N): no enumeration in a call's host time
+    if (a < 2) L.maxrep *= std::min(L.nt[a], 1 + (width + td[a] - 2) / td[a]);
   }
   L.ntiles = L.nt[0] * L.nt[1];
   if ((double)n * L.maxrep >= 4294967295.0) return GBP_ERR_UNSUPPORTED;
