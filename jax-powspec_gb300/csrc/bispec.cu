@@ -247,7 +247,7 @@ bispec_x_kernel(PowGeom g, const int* __restrict__ shell_bins, int k2_max, int p
       const float2 w = __ldg(g.tw + xk);
       const float2 d = unpack_mode(s[c * TST + xswz<L::M2>(xk & (NX - 1))],
                                    s[(XB_C + c) * TST + xswz<L::M2>((NX - xk) & (NX - 1))], w.x, w.y);
-      const float f = 0.5f * c2[ax] * c2[ay] * c2[kz];
+      const float f = c2[ax] * c2[ay] * c2[kz];
       const float dr = d.x * f, di = slab ? -d.y * f : d.y * f;
       return make_float2(dr * m.y + di * m.x, dr * m.x - di * m.y);
     };
@@ -384,7 +384,7 @@ __device__ __forceinline__ void bispec_pairs(const PowGeom& g, const Smem& t, co
     bin[j] = bin_of(g, t, k2);
     const int sp = xswz<L::M2>(p & (L::NX - 1)), sm = xswz<L::M2>((L::NX - p) & (L::NX - 1));
     const float2 e = __ldg(g.tw + p);
-    const float c = 0.25f * cyz * t.c2[p];       // unpack_mode is twice the mode
+    const float c = cyz * t.c2[p];               // of d; D and J, unscaled fields, come out twice the mode
     float q[BK_NV] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int h = 0; h < 2; ++h) {                // kx = p, then kx = -p (the same mode when p = 0 or N/2)
@@ -399,8 +399,8 @@ __device__ __forceinline__ void bispec_pairs(const PowGeom& g, const Smem& t, co
       q[2] += J.x;
       q[3] += 1.0f;
     }
-    v[j][0] = w * q[0] * (4.0f * c * c);
-    v[j][1] = w * q[1] * c;
+    v[j][0] = w * q[0] * (c * c);
+    v[j][1] = w * q[1] * (0.5f * c);
     v[j][2] = w * q[2] * 0.5f;
     v[j][3] = w * q[3];
   }

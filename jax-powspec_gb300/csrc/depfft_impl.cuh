@@ -229,12 +229,12 @@ __device__ __forceinline__ void tile_unit(const DepGeom& g, const ColEntries& te
   Cell* acc = reinterpret_cast<Cell*>(smem);                   // [2 PAIRS][N] fixed-point cells
   float4* cs4 = reinterpret_cast<float4*>(smem);               // [PAIRS/2][N] slots of two columns, alias the cells
   const int tid = threadIdx.x;
-  // 2^s and 2^-s of each block: s = sg - sh in [-110, 100], one normal float each
+  // 2^s and the packed transform's scale times 2^-s of each block: s = sg - sh in [-110, 100], one normal float each
   float up[NSB], dn[NSB];
 #pragma unroll
   for (int b = 0; b < NSB; ++b) {
     up[b] = ldexpf(1.0f, sg - sh[b]);
-    dn[b] = ldexpf(1.0f, sh[b] - sg);
+    dn[b] = ldexpf(fft::PACK_SCALE<G>, sh[b] - sg);
   }
 
   if (clear) {

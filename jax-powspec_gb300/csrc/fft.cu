@@ -145,7 +145,8 @@ fftz_packed_kernel(const float* __restrict__ mesh, float2* __restrict__ out, int
   float2* o1 = o0 + (long long)NX * N * P;
   auto gin = [base](int j, int cp) {
     const float* b = base + 2 * cp % PACK_W * XM + 2 * cp / PACK_W * N + j;    // planes 2cp % PACK_W and the next
-    return make_float4(__ldcg(b), __ldcg(b + IM), __ldcg(b + XM), __ldcg(b + IM + XM));
+    constexpr float S = fft::PACK_SCALE<G>;
+    return make_float4(S * __ldcg(b), S * __ldcg(b + IM), S * __ldcg(b + XM), S * __ldcg(b + IM + XM));
   };
   auto sin_ = [](int j, int cp) { return s4[cp * N + zsw(j)]; };
   auto sout = [](int j, int cp, float4 v) { s4[cp * N + zsw(j)] = v; };

@@ -221,6 +221,13 @@ struct PackedRows {
   __device__ static __forceinline__ int kz(int k) { return (k >> 3) * BLOCK + (k & 7); }
 };
 
+// Scale of the fields that the z passes of the packed transform read: with it
+// unpack_mode (xpass.cuh) gives the mode F(k), or (F0 + phi F1) / 2 of two
+// grids, itself, and its square overflows no earlier than |F|^2 does (a power
+// of two: the same bits as a factor on the square).
+template <int G>
+constexpr float PACK_SCALE = G == 2 ? 0.25f : 0.5f;
+
 // Stores Z[k] of two columns of a packed z pass, whose entries lie `step`
 // apart: kz = k goes to slab 0 (o0) when k <= N/2, kz = -(N - k) to slab 1
 // (o1) as entry N - k when N - k <= N/2; only kz < kz_cols are kept.

@@ -211,7 +211,7 @@ grad_x_kernel(PowGeom g, const float4* __restrict__ coef, float2* __restrict__ o
         const float2 eym = make_float2(e.x, ay == H ? ey.y : -ey.y);
         const float2 eyz = fft::cmul(ey, ez), emz = fft::cmul(eym, ez);
         for (int p = lane + 32 * (warp % L::HALVES); p <= H; p += 32 * L::HALVES) {
-          const float A = amp(p) * 0.125f;         // f = 1/2, D = unpack_mode / 4
+          const float A = amp(p) * 0.5f;           // f = 1/2
           const float2 ep = t.eph[p], em = make_float2(ep.x, p == H ? ep.y : -ep.y);
           const float2 zp = a[at(p)], zm = a[at(-p)], wp = b[at(p)], wm = b[at(-p)];
           // H0, H1 = H0 conj(phi) of a mode with Z(k) = u, Z(-k) = v
@@ -235,7 +235,7 @@ grad_x_kernel(PowGeom g, const float4* __restrict__ coef, float2* __restrict__ o
           }
         }
       } else {
-        const float f = plane ? 1.0f : 0.5f;       // D = unpack_mode / 2; the planes twice
+        const float f = plane ? 2.0f : 1.0f;       // the planes twice
         for (int p = lane + 32 * (warp % L::HALVES); p <= N / 4; p += 32 * L::HALVES) {
           const int r = H - p;
           const float Ap = amp(p) * f, Ar = amp(r) * f;

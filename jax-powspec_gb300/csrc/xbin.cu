@@ -146,8 +146,7 @@ __device__ __forceinline__ void xbin_item(const PowGeom& g, const Smem& t, const
     const float2 ez = t.eph[kzc];
     eyz = make_float2(ey.x * ez.x - ey.y * ez.y, ey.x * ez.y + ey.y * ez.x);
   }
-  // |unpack_mode / 2|^2, and |(a + b)/2|^2 of an interlaced pair: the 1/4 or 1/16 rides on the constant
-  const float cyz = t.c2[ay] * t.c2[kzc] * (INTER ? 0.0625f : 0.25f);
+  const float cyz = t.c2[ay] * t.c2[kzc];
   const int kyz2 = ky * ky + kzc * kzc;
   const float fz2 = (float)(kzc * kzc);
   const float2* a_col = s + c * TST;

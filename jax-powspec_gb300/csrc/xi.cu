@@ -140,7 +140,7 @@ xi_x_kernel(PowGeom g, float2* __restrict__ out, int xmax) {
     x_forward<N, false, false>(s, g.s0, y, kb, g.twx, tid);
     const int c = warp / L::HALVES, kz = kb * XB_C + c;
     const int ky = signed_k(y, N), ay = ky < 0 ? -ky : ky;
-    const float cyz = kz <= H ? 0.25f * t.c2[ay] * t.c2[kz] : 0.0f;
+    const float cyz = kz <= H ? t.c2[ay] * t.c2[kz] : 0.0f;
     const float2* a = s + c * TST;
     const float2* b = s + (XB_C + c) * TST;
     for (int p = lane + 32 * (warp % L::HALVES); p <= H; p += 32 * L::HALVES) {

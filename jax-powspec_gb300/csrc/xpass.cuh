@@ -53,7 +53,7 @@ __device__ __forceinline__ int xswz(int x) {
   else return x ^ ((x >> 4) & (M2 - 1));
 }
 
-// (A + B) - i f (A - B), B = conj b, f = (fr, fi): four times |.|^2's root is the mode.
+// (A + B) - i f (A - B), B = conj b, f = (fr, fi): the mode (the fields come scaled, fft::PACK_SCALE).
 __device__ __forceinline__ float2 unpack_mode(float2 a, float2 b, float fr, float fi) {
   const float sx = a.x + b.x, sy = a.y - b.y, dx = a.x - b.x, dy = a.y + b.y;
   return make_float2(sx + (fr * dy + fi * dx), sy + (fi * dy - fr * dx));
