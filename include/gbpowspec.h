@@ -95,9 +95,11 @@ typedef struct gbp_deposit_stats {
   int flags;            /* GBP_STATS_* bits below                           */
 } gbp_deposit_stats;
 
-/* flags bit: a tile's bucket outgrew the fixed capacity the one-pass
- * bucketing gives it (a strongly clustered catalogue), and its surplus went
- * through per-tile lists; the results are the same. */
+/* flags bit: some tile holds more entries than twice the mean of a uniform
+ * catalogue plus 64 (a strongly clustered catalogue; not reported where that
+ * mean is below 32).  A fill level, the same for every way of bucketing: what
+ * a bucket cannot hold goes through a table of surplus entries, with the same
+ * results, and part of a bucket may spill before the flag is raised. */
 #define GBP_STATS_REFILLED 1
 
 int gbp_deposit_workspace_size(int64_t n_particles, int n_mesh, int mas,
@@ -291,7 +293,7 @@ int gbp_fft_power(gbp_fft_plan plan, const float* mesh, void* spectrum,
  * is scratch of the plan's spectrum size.  The particles are bucketed by
  * column tile in one pass, each written once, into buckets of fixed capacity
  * (twice the mean fill of a uniform catalogue of n_particles and a little);
- * what overflows one (a dense clump) goes to lists that the tile collects in
+ * what overflows one (a dense clump) goes to a table where the tile finds it in
  * the same call, same results.  GBP_STATS_REFILLED in stats_out->flags: some
  * tile holds more than twice the mean plus 64 entries.
  * Replaces src/mas.py:88-153 + src/correlations.py:7-56 for the production

@@ -29,14 +29,15 @@
 //   4. adds up the tile's exact integer total at the common scale 2^s_g
 //      (the mean density).
 //
-// With two grids a tile is taken in units of 4x4 (1024^3: 4x2) pencils whose
-// both grids fit in shared memory together; with one grid the unit is the
-// tile.
+// A tile is taken in units whose cells, all grids', fit in shared memory
+// together: the tile itself where they do (UNIT_BYTES), else 4x4 pencils.
 //
 // A block whose densest plane would cost more than SH_MAX bits (a dense
-// clump) makes its whole tile wide: 64-bit cells (4x2 or 4x4 pencils at a
-// time in the same shared memory), the clumped blocks at the common scale,
-// the others at their own.
+// clump) makes its whole tile wide: 64-bit cells (the unit's on the smallest
+// meshes, else half a unit at a time in the same shared memory), the clumped
+// blocks at the common scale, the others at their own.  A tile with entries
+// beyond its bucket's capacity takes a copy of the code out of line that looks
+// them up too.
 //
 // Then the y pass (fft.cu) and the x pass fused with the binning (xbin.cu)
 // finish the transform and the P_l sums.  HBM traffic per grid: the
@@ -217,9 +218,9 @@ __device__ __forceinline__ void add_entry(const DepGeom& g, const float4& e,
 // unit's exact totals at the common scale 2^sg (valid in thread 0).  SPILLED:
 // the tile's spilled entries too.
 template <int N, int MAS, int G, class CT, bool WIDE, bool SPILLED>
-__device__ __forceinline__ void tile_unit(const DepGeom& g, const ColEntries& te, int sg, const int (&sh)[Unit<N, G, CT, WIDE>::NSB],
-                                          int x0, int y0, int kz_cols, const float2* __restrict__ tw, float2* __restrict__ spec,
-                                          unsigned char* smem, const unsigned* list, long long (*s_part)[G],
+__device__ __forceinline__ void tile_unit(const DepGeom& g, const ColEntries& te, int sg,
+                                          const int (&sh)[Unit<N, G, CT, WIDE>::NSB], int x0, int y0, int kz_cols,
+                                          const float2* __restrict__ tw, float2* __restrict__ spec, unsigned char* smem, const unsigned* list, long long (*s_part)[G],
                                           long long (&tm)[G], bool clear) {
   using Cell = UnitCell<N, G, CT, WIDE>;
   using U = Unit<N, G, CT, WIDE>;
@@ -229,7 +230,7 @@ __device__ __forceinline__ void tile_unit(const DepGeom& g, const ColEntries& te
   Cell* acc = reinterpret_cast<Cell*>(smem);                   // [2 PAIRS][N] fixed-point cells
   float4* cs4 = reinterpret_cast<float4*>(smem);               // [PAIRS/2][N] slots of two columns, alias the cells
   const int tid = threadIdx.x;
-  // 2^s and the packed transform's scale times 2^-s of each block: s = sg - sh in [-110, 100], one normal float each
+  // 2^s of each block, and 2^-s times the packed transform's scale: s = sg - sh in [-110, 100], normal floats
   float up[NSB], dn[NSB];
 #pragma unroll
   for (int b = 0; b < NSB; ++b) {
@@ -329,7 +330,7 @@ __device__ __forceinline__ void tile_units(const DepGeom& g, const ColEntries& t
     }
     long long tm[G];
     tile_unit<N, MAS, G, CT, WIDE, SPILLED>(g, te, sg, shu, x0 + ux, y0 + uy, kz_cols, tw, spec, smem, list,
-                                   s_part, tm, (WIDE && U::WIDE_WHOLE) || u > 0);
+                                                  s_part, tm, (WIDE && U::WIDE_WHOLE) || u > 0);
     if (threadIdx.x == 0) {
 #pragma unroll
       for (int q = 0; q < G; ++q) total[q] += tm[q];
@@ -499,8 +500,8 @@ __device__ __noinline__ void column_spilled_tile(const DepGeom& g, ColEntries te
 
 template <int N, int MAS, int G, class CT>
 __global__ void __launch_bounds__(Unit<N, G, CT, false>::NT, Unit<N, G, CT, false>::MINB)
-deposit_fftz_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ entries, const unsigned* __restrict__ counts,
-                    const __grid_constant__ Spill sp, DepCounters* ctr, int kz_cols,
+deposit_fftz_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ entries,
+                    const unsigned* __restrict__ counts, const __grid_constant__ Spill sp, DepCounters* ctr, int kz_cols,
                     const float2* __restrict__ tw, float2* __restrict__ spec, long long* __restrict__ tile_mass) {
   pdl_wait();
   using U = Unit<N, G, CT, false>;
@@ -510,7 +511,8 @@ deposit_fftz_kernel(const __grid_constant__ DepGeom g, const float4* __restrict_
   const int tid = threadIdx.x, t = blockIdx.x;
   const int ty = t % g.nt[1], tx = t / g.nt[1];
   const int x0 = tx * CT::TX, y0 = ty * CT::TY;
-  for (int k = tid; k < (int)(U::CELLS / 4); k += NT) reinterpret_cast<uint4*>(acc_smem)[k] = make_uint4(0u, 0u, 0u, 0u);
+  for (int k = tid; k < (int)(U::CELLS / 4); k += NT)
+    reinterpret_cast<uint4*>(acc_smem)[k] = make_uint4(0u, 0u, 0u, 0u);
   const ColEntries te = column_entries(g, tx, ty, entries, counts, sp, ctr, s_runs);
   if (tid == 0 && te.n[0] + te.n[1] > g.flag_cap) atomicOr(&ctr->outgrown, 1u);
   const int sg = fixed_scale_exp(ctr->maxw_bits, 0);
@@ -600,7 +602,8 @@ int particles_power_n(DepGeom g, int64_t n_launch, gbp_fft_plan plan, gbp_bins B
   } else if (tx == 8 && ty == 4) {
     if constexpr (N <= 512) r = dispatch_mas<N, ColTile<N, 8, 4>>(mas, G, g, L.dep, b, B->kz_cols, plan->tw, spec, st);
   } else if (tx == 8 && ty == 8) {
-    if constexpr (N == 128 || N == 256) r = dispatch_mas<N, ColTile<N, 8, 8>>(mas, G, g, L.dep, b, B->kz_cols, plan->tw, spec, st);
+    if constexpr (N == 128 || N == 256)
+      r = dispatch_mas<N, ColTile<N, 8, 8>>(mas, G, g, L.dep, b, B->kz_cols, plan->tw, spec, st);
   }
   if (r) return r;
   // up to 256^3 the statistics are a block of the last fold (as fast as a kernel of its own less the launch,

@@ -946,9 +946,11 @@ int column_layout(int64_t n, int N, int mas, int interlace, int tx, int ty, DepL
 // The rest of a layout, from its tiles, blocks and buckets.
 void finish_layout(DepLayout& L) {
   L.scan_bytes = 0;
-  if (!L.tcap) cub::DeviceScan::ExclusiveSum(nullptr, L.scan_bytes, strided_counts(nullptr), (unsigned*)nullptr, L.ntiles);
+  if (!L.tcap)
+    cub::DeviceScan::ExclusiveSum(nullptr, L.scan_bytes, strided_counts(nullptr), (unsigned*)nullptr, L.ntiles);
   const size_t nbl = (size_t)(L.nblocks > 0 ? L.nblocks : 1);
-  L.total = zeroed_bytes(L) + align256((size_t)L.ntiles * 2 * sizeof(long long)) + align256((size_t)L.ntiles * 4) + align256(nbl * sizeof(float4)) +
+  L.total = zeroed_bytes(L) + align256((size_t)L.ntiles * 2 * sizeof(long long)) + align256((size_t)L.ntiles * 4) +
+            align256(nbl * sizeof(float4)) +
             align256(L.nentries * sizeof(float4)) + align256(L.scan_bytes) +
             align256((L.chunks << L.lg) * sizeof(unsigned));
 }
@@ -993,15 +995,15 @@ int bucket_particles(const DepGeom& g, const DepLayout& L, const DepBuffers& b, 
   if (L.tcap) {
     if (L.nblocks > 0) {
       GBP_TRACE("deposit_fill", st);
-      GBP_CUDA_TRY(launch_pdl(job ? fill_kernel<MAS, G, CM, CM == 0> : fill_kernel<MAS, G, CM, false>, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts,
-                              b.entries, b.spill, b.ctr, b.block_stats));
+      GBP_CUDA_TRY(launch_pdl(job ? fill_kernel<MAS, G, CM, CM == 0> : fill_kernel<MAS, G, CM, false>,
+                              dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts, b.entries, b.spill, b.ctr, b.block_stats));
     }
     return GBP_OK;
   }
   if (L.nblocks > 0) {
     GBP_TRACE("deposit_count", st);
-    GBP_CUDA_TRY(launch_pdl(job ? count_kernel<MAS, G, CM, CM == 0> : count_kernel<MAS, G, CM, false>, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts, b.ctr,
-                            b.block_stats));
+    GBP_CUDA_TRY(launch_pdl(job ? count_kernel<MAS, G, CM, CM == 0> : count_kernel<MAS, G, CM, false>,
+                            dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts, b.ctr, b.block_stats));
   }
   {
     GBP_TRACE("deposit_scan", st);
@@ -1011,8 +1013,8 @@ int bucket_particles(const DepGeom& g, const DepLayout& L, const DepBuffers& b, 
   }
   if (L.nblocks > 0) {
     GBP_TRACE("deposit_scatter", st);
-    GBP_CUDA_TRY(launch_pdl(job ? scatter_kernel<MAS, G, CM, CM == 0> : scatter_kernel<MAS, G, CM, false>, dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.offsets,
-                            b.fills, b.entries));
+    GBP_CUDA_TRY(launch_pdl(job ? scatter_kernel<MAS, G, CM, CM == 0> : scatter_kernel<MAS, G, CM, false>,
+                            dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.offsets, b.fills, b.entries));
   }
   return GBP_OK;
 }

@@ -91,9 +91,9 @@ template <int N, int R, int CP, int NT, bool MID_SYNC, bool END_SYNC, bool IFAST
 __device__ __forceinline__ void stage2(In in, Out out, const float2* __restrict__ tw, int p, int tid) {
   constexpr int NB = CP * (N / R);
   constexpr int PER = GS > 0 ? 8 / R : (NB + NT - 1) / NT;
-  static_assert(GS == 0 || (IFAST && GS == GROUP<N> && CP * (N / 8) % GS == 0 && CP * (N / 8) <= NT),
+  static_assert(GS == 0 || (IFAST && GS == GROUP<N> && CP * (N / 8) % (GS > 0 ? GS : 1) == 0 && CP * (N / 8) <= NT),
                 "whole groups, one first-stage butterfly per thread");
-  static_assert(GS <= 32 || NT / GS <= MAX_GROUPS, "more groups than named barriers");
+  static_assert(GS <= 32 || NT / (GS > 0 ? GS : 1) <= MAX_GROUPS, "more groups than named barriers");
   // number of butterfly q of the thread, column pair by column pair
   constexpr int STEP = GS > 0 ? GS : NT;
   const int b0 = GS > 0 && PER > 1 ? tid + tid / STEP * STEP * (PER - 1) : tid;

@@ -28,8 +28,9 @@
 // W and their derivatives dW/du of its stencil nodes (per grid), times the
 // gradient mesh there: dLoss/dw_i = sum grad W, dLoss/du_a = w_i sum grad
 // dW/du_a, and dLoss/dx_a = inv_cell dLoss/du_a.  The explicit dependence of
-// the normalisation and of the shot noise on the weights is added on the
-// host side (gbpowspec/grad.py); it is nb-sized arithmetic.
+// the normalisation and of the shot noise on the weights is two numbers per
+// call (grad_coef_kernel, or gbpowspec/grad.py on the cuFFT path), which the
+// gather adds to dLoss/dw_i.
 #include <cufft.h>
 #include <math.h>
 

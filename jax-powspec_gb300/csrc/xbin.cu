@@ -18,8 +18,8 @@
 //                      phi = exp(i pi (kx + ky + kz) / N)  (times 1/2)
 //          one grid:   E + w O, the same with w = exp(-2 pi i kx / N) and
 //                      Z taken at kx mod N/2,
-//      that is ((A + B) - i f (A - B)) / 2 with f = phi or w.  The modes x
-//      and N - x of a column (kx and -kx) share |k|, mu, the window and the
+//      that is ((A + B) - i f (A - B)) / 2 with f = phi or w (the fields come
+//      times 1/4 or 1/2, so the mode needs no factor).  The modes x and N - x of a column (kx and -kx) share |k|, mu, the window and the
 //      bin, and the four values they need, so they are summed first and
 //      looked up once; a warp walks one column over half of the |kx| range
 //      (or all of it; x = N/2 alone is added after the last pair), so bins

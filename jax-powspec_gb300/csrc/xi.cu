@@ -122,8 +122,9 @@ xi_reduce_kernel(const float2* __restrict__ part_ff, int C, int nb, int nbe, dou
 }
 
 // Items (y, kb) of the packed transform: x pass, power of the 8 columns at
-// (ky, kz), transform of the N (real, even) powers along x, x planes 0 .. xmax
-// stored to out [xmax + 1][N][P].
+// (ky, kz), transform of the N powers (real; the columns at (ky, kz) and
+// (-ky, -kz) mirror each other) along x, x planes 0 .. xmax stored to out
+// [xmax + 1][N][P].
 template <int N>
 __global__ void __launch_bounds__(XLayout<N, false>::NT, 1024 / XLayout<N, false>::NT)
 xi_x_kernel(PowGeom g, float2* __restrict__ out, int xmax) {

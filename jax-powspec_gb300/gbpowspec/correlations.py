@@ -57,8 +57,8 @@ def _upload(a: np.ndarray, dev: torch.device) -> torch.Tensor:
     """A small host table on the device, through a pinned copy that torch's host allocator keeps until the transfer,
     enqueued on the current stream, is done (pageable memory may be read by the GPU after the call returns where it
     can reach host pages).  Waiting for the transfer, as a blocking copy does, left the GPU idle for 0.1-0.3 ms a call
-    (256^3: xi_vec 0.33 -> 0.24 ms, bispec 1.11 -> 0.81; the pinned copies cost 20-30 us each of that back).  Under stream capture the blocking copy refuses, as a
-    graph would keep the table's address."""
+    (256^3: xi_vec 0.33 -> 0.24 ms, bispec 1.11 -> 0.81; the pinned copies cost 20-30 us each of that back).  Under
+    stream capture the blocking copy refuses, as a graph would keep the table's address."""
     t = torch.from_numpy(a)
     if torch.cuda.is_current_stream_capturing():
         return t.to(dev)
