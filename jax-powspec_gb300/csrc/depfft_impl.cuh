@@ -220,8 +220,9 @@ __device__ __forceinline__ void add_entry(const DepGeom& g, const float4& e,
 template <int N, int MAS, int G, class CT, bool WIDE, bool SPILLED>
 __device__ __forceinline__ void tile_unit(const DepGeom& g, const ColEntries& te, int sg,
                                           const int (&sh)[Unit<N, G, CT, WIDE>::NSB], int x0, int y0, int kz_cols,
-                                          const float2* __restrict__ tw, float2* __restrict__ spec, unsigned char* smem, const unsigned* list, long long (*s_part)[G],
-                                          long long (&tm)[G], bool clear) {
+                                          const float2* __restrict__ tw, float2* __restrict__ spec, unsigned char* smem,
+                                          const unsigned* list, long long (*s_part)[G], long long (&tm)[G],
+                                          bool clear) {
   using Cell = UnitCell<N, G, CT, WIDE>;
   using U = Unit<N, G, CT, WIDE>;
   constexpr int UY = U::UY, PAIRS = U::PAIRS, NT = U::NT, NSB = U::NSB;
@@ -501,8 +502,9 @@ __device__ __noinline__ void column_spilled_tile(const DepGeom& g, ColEntries te
 template <int N, int MAS, int G, class CT>
 __global__ void __launch_bounds__(Unit<N, G, CT, false>::NT, Unit<N, G, CT, false>::MINB)
 deposit_fftz_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ entries,
-                    const unsigned* __restrict__ counts, const __grid_constant__ Spill sp, DepCounters* ctr, int kz_cols,
-                    const float2* __restrict__ tw, float2* __restrict__ spec, long long* __restrict__ tile_mass) {
+                    const unsigned* __restrict__ counts, const __grid_constant__ Spill sp, DepCounters* ctr,
+                    int kz_cols, const float2* __restrict__ tw, float2* __restrict__ spec,
+                    long long* __restrict__ tile_mass) {
   pdl_wait();
   using U = Unit<N, G, CT, false>;
   constexpr int NT = U::NT;

@@ -226,8 +226,9 @@ __device__ __noinline__ void deposit_spilled_tile(DepGeom g, TileEntries te, int
 template <int MAS, int G, int CM>
 __global__ void __launch_bounds__(DEP_THREADS, MAS == GBP_PCS ? 4 : (MAS == GBP_TSC || CM ? 5 : 6))
 deposit_kernel(const __grid_constant__ DepGeom g, const float4* __restrict__ entries,
-               const unsigned* __restrict__ counts, const unsigned* __restrict__ offsets, const __grid_constant__ Spill sp, DepCounters* ctr,
-               const float* __restrict__ mesh_in, float* __restrict__ mesh_out, long long* __restrict__ tile_mass) {
+               const unsigned* __restrict__ counts, const unsigned* __restrict__ offsets,
+               const __grid_constant__ Spill sp, DepCounters* ctr, const float* __restrict__ mesh_in,
+               float* __restrict__ mesh_out, long long* __restrict__ tile_mass) {
   pdl_wait();
   extern __shared__ __align__(16) unsigned acc32[];
   const int t = blockIdx.x;

@@ -996,7 +996,8 @@ int bucket_particles(const DepGeom& g, const DepLayout& L, const DepBuffers& b, 
     if (L.nblocks > 0) {
       GBP_TRACE("deposit_fill", st);
       GBP_CUDA_TRY(launch_pdl(job ? fill_kernel<MAS, G, CM, CM == 0> : fill_kernel<MAS, G, CM, false>,
-                              dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts, b.entries, b.spill, b.ctr, b.block_stats));
+                              dim3(L.nblocks), dim3(CNT_THREADS), 0, st, g, b.counts, b.entries, b.spill, b.ctr,
+                              b.block_stats));
     }
     return GBP_OK;
   }

@@ -139,7 +139,7 @@ fftz_packed_kernel(const float* __restrict__ mesh, float2* __restrict__ out, int
   using R = fft::PackedRows<N>;
   constexpr int ROWS = PAIRS / PACK_W;
   const int x = blockIdx.x / (N / ROWS) * PACK_W, y = blockIdx.x % (N / ROWS) * ROWS;
-  constexpr long long XM = G == 2 ? (long long)N * N : 2LL * N * N;            // mesh: from one packed plane to the next
+  constexpr long long XM = G == 2 ? (long long)N * N : 2LL * N * N;   // mesh: from one packed plane to the next
   const float* base = mesh + x * XM + (long long)y * N;
   float2* o0 = out + R::at(x, y);
   float2* o1 = o0 + (long long)NX * N * P;
@@ -281,8 +281,8 @@ int launch_cols(float2* data, long long plane_stride, long long row_stride, int 
   const size_t smem = (size_t)SL * fft::ColBlock<N, SL>::SLAB * sizeof(float2);
   auto kc = fft_cols_kernel<N, PRUNE, W, SL>;
   GBP_CUDA_TRY(cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  GBP_CUDA_TRY(launch_pdl(kc, dim3((unsigned)(nplanes / SL * nkb)), dim3(N / 2 * SL), smem, st, data, plane_stride, row_stride,
-                          nplanes, nkb, k2_max, tw));
+  GBP_CUDA_TRY(launch_pdl(kc, dim3((unsigned)(nplanes / SL * nkb)), dim3(N / 2 * SL), smem, st, data, plane_stride,
+                          row_stride, nplanes, nkb, k2_max, tw));
   return GBP_OK;
 }
 
@@ -355,8 +355,8 @@ int run_y_inverse(int G, float2* spec, int kz_cols, int k2_max, const float2* tw
   auto k = fft_cols_inv_kernel<N, SL>;
   GBP_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   GBP_TRACE("fft_y_inverse", st);
-  GBP_CUDA_TRY(launch_pdl(k, dim3((unsigned)(G * N / SL * (kz_cols / 8))), dim3(N / 2 * SL), smem, st, spec, G * N, kz_cols / 8,
-                          k2_max, tw));
+  GBP_CUDA_TRY(launch_pdl(k, dim3((unsigned)(G * N / SL * (kz_cols / 8))), dim3(N / 2 * SL), smem, st, spec,
+                          G * N, kz_cols / 8, k2_max, tw));
   return GBP_OK;
 }
 
@@ -442,7 +442,8 @@ int own_fft_r2c(int N, int G, const float* mesh, float2* spec, const float2* tw,
 int own_fft_z_packed(int N, int G, const float* mesh, float2* spec, int kz_cols, const float2* tw,
                      cudaStream_t st) {
 #define GBP_Z(NN) \
-  case NN: return G == 2 ? run_z_packed<NN, 2>(mesh, spec, kz_cols, tw, st) : run_z_packed<NN, 1>(mesh, spec, kz_cols, tw, st)
+  case NN:       \
+    return G == 2 ? run_z_packed<NN, 2>(mesh, spec, kz_cols, tw, st) : run_z_packed<NN, 1>(mesh, spec, kz_cols, tw, st)
   switch (N) {
     GBP_Z(64);
     GBP_Z(128);
@@ -489,7 +490,8 @@ int own_fft_y_inverse(int N, int G, float2* spec, int kz_cols, int k2_max, const
 
 int own_fft_z_unpack(int N, int G, const float2* spec, float* mesh, int kz_cols, const float2* tw, cudaStream_t st) {
 #define GBP_Z(NN) \
-  case NN: return G == 2 ? run_z_unpack<NN, 2>(spec, mesh, kz_cols, tw, st) : run_z_unpack<NN, 1>(spec, mesh, kz_cols, tw, st)
+  case NN:       \
+    return G == 2 ? run_z_unpack<NN, 2>(spec, mesh, kz_cols, tw, st) : run_z_unpack<NN, 1>(spec, mesh, kz_cols, tw, st)
   switch (N) {
     GBP_Z(64);
     GBP_Z(128);

@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(XLayout<N, INTER>::NT, N >= 1024 && INTER ? 1 
 grad_x_kernel(PowGeom g, const float4* __restrict__ coef, float2* __restrict__ out) {
   pdl_wait();
   using L = XLayout<N, INTER>;
-  constexpr int P = N / 2 + 8, TST = L::TST, NX = L::NX, NT = L::NT, H = N / 2, M2 = L::M2;
+  constexpr int TST = L::TST, NX = L::NX, NT = L::NT, H = N / 2, M2 = L::M2;
   extern __shared__ __align__(16) unsigned char smem[];
   float2* s = reinterpret_cast<float2*>(smem);
   const Smem t = load_tables<1, INTER>(g, smem + L::data_bytes());

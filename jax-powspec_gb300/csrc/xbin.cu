@@ -19,9 +19,10 @@
 //          one grid:   E + w O, the same with w = exp(-2 pi i kx / N) and
 //                      Z taken at kx mod N/2,
 //      that is ((A + B) - i f (A - B)) / 2 with f = phi or w (the fields come
-//      times 1/4 or 1/2, so the mode needs no factor).  The modes x and N - x of a column (kx and -kx) share |k|, mu, the window and the
-//      bin, and the four values they need, so they are summed first and
-//      looked up once; a warp walks one column over half of the |kx| range
+//      times 1/4 or 1/2, so the mode needs no factor).  The modes x and N - x
+//      of a column (kx and -kx) share |k|, mu, the window and the bin, and the
+//      four values they need, so they are summed first and looked up once; a
+//      warp walks one column over half of the |kx| range
 //      (or all of it; x = N/2 alone is added after the last pair), so bins
 //      are monotone along the walk.  A lane owns consecutive pairs; runs of
 //      equal bin are summed in-lane, joined across lanes by one warp
@@ -362,5 +363,6 @@ extern "C" int gbp_fft_power(gbp_fft_plan plan, const float* mesh, void* spectru
   if (r) return r;
   r = own_fft_y_packed(B->N, plan->grids, spec, B->kz_cols, B->last_closed, plan->tw, st);
   if (r) return r;
-  return xbin_power(plan, spec, B, mas_order, ells, mass, sums_out, nmodes_out, ksum_out, workspace, ws_bytes, st, StatsFold{});
+  return xbin_power(plan, spec, B, mas_order, ells, mass, sums_out, nmodes_out, ksum_out, workspace, ws_bytes, st,
+                    StatsFold{});
 }
